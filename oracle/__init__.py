@@ -24,9 +24,10 @@ def build_port() -> str:
 
 def build_ref(refdir: str | None = None) -> str | None:
     """Compile the reference from its own sources into _ref/ (x86 container only). The checkout is
-    named by the argument or the CHEMTENSOR_REFERENCE_DIR environment variable; None if absent."""
+    named by the argument or the CHEMTENSOR_REFERENCE_DIR environment variable; None if it or its
+    sources are absent."""
     refdir = refdir or os.environ.get("CHEMTENSOR_REFERENCE_DIR")
-    if not refdir or not os.path.isdir(refdir):
+    if not refdir or not os.path.isdir(os.path.join(refdir, "src")):
         return None
     subprocess.run(["make", "-s", "-C", HERE, "ref", f"REFDIR={refdir}"], check=True)
     return REF
