@@ -437,12 +437,12 @@ static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int
 		// cores to pay for their operand packing (FP64 is then both faster and exact). Its key comes
 		// from the output blocks and contributions, which the FP64 lowering has too: a product that
 		// stays on FP64 is lowered once, one on the tensor cores twice
-		DotLowering l = lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm);
+		DotLowering l = lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm, 64, true);
 		const int bn = tuned_tile_width(c, s, axs, t, axt, nmult, precision, out_perm, l);
 		if (bn == 0) return upload_dot_plan(c, std::move(l), GEMM_FP64, 64);
 		return upload_dot_plan(c, lower_dot(s, axs, t, axt, nmult, precision, c.num_sms(), out_perm, bn), precision, bn);
 	}
-	DotLowering l = lower_dot(s, axs, t, axt, nmult, z ? (int)GEMM_FP64 : precision, c.num_sms(), out_perm);
+	DotLowering l = lower_dot(s, axs, t, axt, nmult, z ? (int)GEMM_FP64 : precision, c.num_sms(), out_perm, 64, !z);
 	return upload_dot_plan(c, std::move(l), precision, 64);
 }
 
@@ -470,11 +470,38 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 	const size_t o_tiles = pk.add(l.tiles);
 	const size_t o_splits = pk.add(l.splits);
 	const size_t o_tcons = pk.add(l.tcons), o_apacks = pk.add(l.apacks), o_bpacks = pk.add(l.bpacks);
-	const size_t o_zt = pk.add(zt);
+	const size_t o_zt = pk.add(zt), o_st = pk.add(l.stiles);
+	const size_t o_so = pk.add(l.souts);
+	size_t o_side[2][4] = {};
+	for (int q = 0; q < 2 && !l.stiles.empty(); q++)
+	{
+		o_side[q][0] = pk.add(l.spack[q].runs);
+		o_side[q][1] = pk.add(l.spack[q].groups);
+		o_side[q][2] = pk.add(l.spack[q].items);
+		o_side[q][3] = pk.add(l.spack[q].chunks);
+	}
 	// at least 16 bytes, from the packer's own storage (a product without output blocks packs nothing)
 	if (pk.bytes.size() < 16) pk.bytes.resize(16);
 	p.desc = c.upload(pk.bytes.data(), pk.bytes.size());
 	p.nztiles = (int)zt.size();
+	p.nstiles = (int)l.stiles.size();
+	p.stiles = at<SliceTile>(p.desc, o_st);
+	p.souts = at<SliceOut>(p.desc, o_so);
+	p.orient = l.orient;
+	for (int q = 0; q < 2; q++)
+	{
+		DotPlan::Side& d = p.side[q];
+		d.runs = at<SliceRun>(p.desc, o_side[q][0]);
+		d.groups = at<SliceGroup>(p.desc, o_side[q][1]);
+		d.items = at<SliceItem>(p.desc, o_side[q][2]);
+		d.chunks = at<SliceChunk>(p.desc, o_side[q][3]);
+		d.nitems = (int)l.spack[q].items.size();
+		d.ngroups = (int)l.spack[q].groups.size();
+		d.nchunks = (int)l.spack[q].chunks.size();
+		d.nblocks = l.spack[q].blocks;
+		d.bytes = l.spack[q].bytes;
+	}
+	p.c_blocks = l.out->nblocks;
 	p.ztiles = at<ZTile>(p.desc, o_zt);
 	p.tcons = at<TcContrib>(p.desc, o_tcons);
 	p.apacks = at<TcPack>(p.desc, o_apacks);
@@ -516,14 +543,60 @@ void DotPlan::run(Ctx& c, const double* A, const double* B, double* C) const
 		c.gemm_flops += flops;
 		return;
 	}
-	double* w = work ? (double*)work->ptr : nullptr;
-	int* cnt = counters ? (int*)counters->ptr : nullptr;
-	if (ntiles[0] > 0)
+	if (ntiles[0] > 0 || nstiles > 0)
 	{
 		KScope ks(c, K_GEMM, 1, flops, 0);
-		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops);
+		launch_f64(c, A, B, C);
 	}
 	c.gemm_flops += flops;
+}
+
+void DotPlan::launch_f64(Ctx& c, const double* A, const double* B, double* C) const
+{
+	double* w = work ? (double*)work->ptr : nullptr;
+	int* cnt = counters ? (int*)counters->ptr : nullptr;
+	if (nstiles > 0)
+	{
+		DBuf e(&c, (size_t)(side[0].nblocks + side[1].nblocks) * sizeof(int));
+		int *ea = (int*)e.ptr, *eb = ea + side[0].nblocks;
+		CTG_CUDA(cudaMemsetAsync(e.ptr, 0, e.bytes, c.stream()));
+		DBuf pa(&c, (size_t)slice_bytes(0)), pb(&c, (size_t)slice_bytes(1));
+		block_exps(c, 0, A, ea);
+		block_exps(c, 1, B, eb);
+		slice_pack(c, 0, A, ea, pa.ptr);
+		slice_pack(c, 1, B, eb, pb.ptr);
+		run_slices(c, A, B, pa.ptr, pb.ptr, C, nullptr);
+	}
+	else if (ntiles[0] > 0)
+		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops);
+}
+
+// the groups' exponents in front of the digits, which start on a 256-byte boundary
+static size_t slice_head(const DotPlan::Side& d) { return ((size_t)d.ngroups * sizeof(int) + 255) & ~(size_t)255; }
+
+i64 DotPlan::slice_bytes(int s) const { return (i64)slice_head(side[s]) + std::max<i64>(side[s].bytes, 16); }
+
+void DotPlan::block_exps(Ctx& c, int s, const double* x, int* exps, int* clear, int nclear) const
+{
+	launch_block_exps(side[s].nchunks, side[s].chunks, x, exps, clear, nclear, c.stream());
+}
+
+void DotPlan::slice_pack(Ctx& c, int s, const double* x, const int* exps, void* pack) const
+{
+	const Side& d = side[s];
+	// orient 0: B lies along the MMA rows
+	launch_slice_pack(d.nitems, d.items, d.groups, d.runs, (orient == 0) == (s == 1), x, exps, (char*)pack + slice_head(d),
+	                  (int*)pack, c.stream());
+}
+
+void DotPlan::run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C, int* exp_c) const
+{
+	const int x = orient ? 0 : 1;
+	const void* pack[2] = {apack, bpack};
+	launch_gemm_slices(nstiles, stiles, outs, souts, cons, splits, counters ? (int*)counters->ptr : nullptr, orient, A, B,
+	                   (const char*)pack[x] + slice_head(side[x]), (const char*)pack[1 - x] + slice_head(side[1 - x]),
+	                   (const int*)pack[x], (const int*)pack[1 - x], C, exp_c, work ? (double*)work->ptr : nullptr, c.tc_error(),
+	                   c.num_sms(), c.stream());
 }
 
 void DotPlan::run_z(Ctx& c, const double* A, const double* B, double* C, bool conj_a, bool conj_b) const
@@ -651,7 +724,7 @@ std::string tune_key(const DotLowering& l, int precision)
 double time_tc_variant(Ctx& c, DotLowering&& l, int precision, int bn, const Meta& s, const Meta& t)
 {
 	DotPlan p = upload_dot_plan(c, std::move(l), bn == 0 ? (int)GEMM_FP64 : precision, bn == 0 ? 64 : bn);
-	if (p.ntiles[0] == 0) return 0.0;
+	if (p.ntiles[0] == 0 && p.nstiles == 0) return 0.0;
 	if (bn == 0)
 	{
 		DBuf A(&c, (size_t)std::max<i64>(s.nnz, 1) * sizeof(double));
@@ -665,9 +738,7 @@ double time_tc_variant(Ctx& c, DotLowering&& l, int precision, int bn, const Met
 		for (int rep = 0; rep < 3; rep++)
 		{
 			CTG_CUDA(cudaEventRecord(e[0], c.stream()));
-			launch_gemm_f64(p.ntiles[0], p.tiles[0], p.outs, p.cons, p.splits, p.counters ? (int*)p.counters->ptr : nullptr,
-			                (const double*)A.ptr, (const double*)B.ptr, (double*)C.ptr,
-			                p.work ? (double*)p.work->ptr : nullptr, c.stream());
+			p.launch_f64(c, (const double*)A.ptr, (const double*)B.ptr, (double*)C.ptr);
 			CTG_CUDA(cudaEventRecord(e[1], c.stream()));
 			CTG_CUDA(cudaEventSynchronize(e[1]));
 			float ms = 0;
@@ -735,7 +806,7 @@ static int tuned_tile_width(Ctx& c, const Meta& s, int axs, const Meta& t, int a
 	const int forced = g_forced_tc_bn.load();
 	if (forced) return forced;
 	if (env_forced) return env_forced;
-	if (l64.tiles.empty()) return 64;
+	if (l64.tiles.empty() && l64.stiles.empty()) return 64;
 	const std::string key = tune_key(l64, precision);
 	TuneTable& tt = tune_table();
 	{
@@ -759,7 +830,7 @@ static int tuned_tile_width(Ctx& c, const Meta& s, int axs, const Meta& t, int a
 			e.bn = widths[i];
 		}
 	}
-	e.ms[3] = time_tc_variant(c, lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm), precision, 0, s, t);
+	e.ms[3] = time_tc_variant(c, lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm, 64, true), precision, 0, s, t);
 	if (e.ms[3] < best) e.bn = 0;
 	std::lock_guard<std::mutex> g(tt.mu);
 	if (const TuneEntry* prev = tt.find(key)) return prev->bn;    // another thread tuned it meanwhile

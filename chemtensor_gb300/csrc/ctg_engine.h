@@ -169,6 +169,19 @@ struct DotPlan {
 	int nsplits = 0;
 	DBufPtr work;                        // their partial sums
 	DBufPtr counters;                    // their completion counters (one int per split tile)
+	// FP64 on the tensor cores by digit slices (then ntiles is 0); side 0 is operand A, 1 is B
+	int nstiles = 0, orient = 0;
+	const SliceTile* stiles = nullptr;
+	const SliceOut* souts = nullptr;
+	struct Side {
+		const SliceRun* runs = nullptr;
+		const SliceGroup* groups = nullptr;
+		const SliceItem* items = nullptr;
+		const SliceChunk* chunks = nullptr;
+		int nitems = 0, ngroups = 0, nchunks = 0, nblocks = 0;
+		i64 bytes = 0;
+	} side[2];
+	int c_blocks = 0;                    // blocks of the result
 	i64 a_entries = 0, b_entries = 0;    // entries of the two operand tensors
 	// tensor-core path: packed operand records (see launch_tc_pack) and per-contribution records
 	const TcContrib* tcons = nullptr;
@@ -184,6 +197,15 @@ struct DotPlan {
 	int nztiles = 0;
 	const ZTile* ztiles = nullptr;
 	void run(Ctx& c, const double* A, const double* B, double* C) const;
+	// the FP64 product's launches alone (no counters)
+	void launch_f64(Ctx& c, const double* A, const double* B, double* C) const;
+	// a product by digit slices in parts, so that an operand used by many runs is packed once, and the
+	// exponents of a result's blocks for the next product come from this one. A packed operand is one
+	// buffer: the groups' exponents, then the digits (slice_bytes)
+	i64 slice_bytes(int s) const;
+	void block_exps(Ctx& c, int s, const double* x, int* exps, int* clear = nullptr, int nclear = 0) const;
+	void slice_pack(Ctx& c, int s, const double* x, const int* exps, void* pack) const;
+	void run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C, int* exp_c) const;
 	// complex128 entries, operands optionally read conjugated
 	void run_z(Ctx& c, const double* A, const double* B, double* C, bool conj_a, bool conj_b) const;
 	// tensor-core path in parts, so that an operand used by many runs is packed once; src_f32: the

@@ -1,0 +1,818 @@
+// ctg_gemm_slices.cu - FP64 block GEMM on the tensor cores by exact digit slices (ctg_slices.h).
+//
+// GB300 retires about two FP64 FMAs per clock and SM, its tensor cores about four thousand FP16 ones:
+// the 36 digit products that stand for one FP64 product cost a fiftieth of the FMA. The sums over
+// the digits are exact, so a result carries one rounding and the cut at 2^-62 of its operands' blocks'
+// largest entries, less than the rounding of an FMA chain.
+//
+//   k_block_exps   the largest exponent of every block of an operand (the scale of its digits)
+//   k_slice_pack   cuts an operand into FP16 digits: per group of rows (the blocks with the same free
+//                  indices) the terms of all its blocks one after the other, 16 terms at a time, in the
+//                  canonical K-major core-matrix layout, so that a stage of the GEMM is two bulk copies.
+//                  An entry is converted once here, and once per tile that reads it in the GEMM: with ten
+//                  warps of the GEMM converting, its MMAs waited for them three quarters of the time
+//   k_gemm_slices  persistent, one CTA per SM, output tiles of 128 x 64 (SliceTile): warp 0 copies the
+//                  digits of 16 terms per stage (up to 32 + 16 KiB), warp 1 issues the MMAs, warps 4-19 add
+//                  the orders up and write.
+// The 64 columns of a tile are two halves of 32 with an accumulator each in tensor memory: columns 32 o ..
+// 32 o + 31 of it hold order o. Digit s of the 128 rows meets the digits 0 .. 7 - s of the 32 columns,
+// which lie one after the other as rows of one B operand, in one MMA of N = 32 (8 - s) that writes
+// the orders s .. 7: eight MMAs per half and 16 terms stand for 36 products, and the A digits are read
+// once each. The tile is 64 wide because a stage then moves 48 KiB for 1240 cycles of MMAs (39 bytes a
+// cycle and SM out of L2; 66 with 32 columns), and tensor memory holds no more. Every 128 terms the
+// epilogue takes the sums over: half 0 while the MMAs of half 1 run, and conversely.
+// Measured, three products of a local-Hamiltonian application at D = 1024 (4.1e9 FMAs): 7.65 ms on the
+// FP64 pipe, 0.62 ms here and 0.24 ms for the digits (1.06 ms with the conversion inside the GEMM). The
+// first two products are bound by the epilogue (integer instructions on 2e7 results, tensor pipe 28 and
+// 37 % busy), the third, with ten times the terms, by the copies out of L2 (46 %).
+// A tile with an operand block that is not finite or tiny, or whose results may leave the normal range,
+// takes its entries from FP64 sums over the operands. Every wait is bounded and ends when another warp
+// has failed.
+#include <algorithm>
+#include <mutex>
+
+#include "ctg_kernels.h"
+#include "ctg_launch.cuh"
+#include "ctg_slices.h"
+#include "ctg_tcgen05.cuh"
+
+namespace ctg {
+
+namespace {
+
+constexpr int SL_M = SLICE_TILE_ROWS, SL_HALF = SLICE_HALF;
+constexpr int SL_EPI = 16, SL_EPI_WARP0 = 4;    // epilogue warps: a tensor-memory quarter by 8 columns of each half
+constexpr int SL_THREADS = 32 * (SL_EPI_WARP0 + SL_EPI);
+constexpr int SL_LBO = 128;                     // bytes between the two core matrices of 16 terms
+constexpr int SL_A_SBO = SLICE_ROW8_BYTES, SL_B_SBO = 256;       // between groups of 8 rows
+constexpr int SL_A_DIGIT = 256;                 // between the digits of a row
+constexpr int SL_A_BYTES = SL_M / 8 * SLICE_ROW8_BYTES;          // 32 KiB
+constexpr int SL_B_BYTES = 2 * SLICE_COL32_BYTES;                // 16 KiB
+constexpr int SL_STAGE = SL_A_BYTES + SL_B_BYTES;
+constexpr int SL_STAGES = 4;
+constexpr int SL_ACC = SLICES * SL_HALF;        // accumulator columns of a half
+constexpr int SL_FLUSH = SLICE_K / SLICE_STAGE_K;                // stages between flushes
+constexpr int SL_LD = 5;                        // staging row of the epilogue (4 columns)
+constexpr int SL_EPI_BYTES = SL_EPI * 32 * SL_LD * 8;
+constexpr int SL_TILES = 32;                    // tiles described at a time (twice)
+// one tile, as the other warps need it
+struct SliceInfo {
+	i64 xs, ys;                          // digits of its first stage (bytes)
+	i64 co, sr0, sr1, sc0;               // output layout (GemmOut)
+	int r1, c1;
+	int tile;                            // -1: no more tiles
+	int xstep, ystep, xbytes, ybytes;    // digits (bytes) between stages, and of one
+	int nch, halves;
+	int m0, n0, m, n;
+	int split, sp, block, e, f;          // e, f: largest biased exponents of its operand blocks
+};
+constexpr int SL_BARS = 2 * SL_STAGES + 4 + 4 + 1;
+constexpr int SL_SMEM = SL_STAGES * SL_STAGE + SL_EPI_BYTES + 2 * SL_TILES * (int)sizeof(SliceInfo) + SL_BARS * 8 + 32;
+constexpr int SL_WAIT = 1 << 21;                // polls before a wait is declared failed
+constexpr uint32_t SL_POLL_NS = 1000;           // longest a poll suspends its warp
+static_assert(SL_SMEM <= 227 * 1024, "shared memory per CTA");
+static_assert(2 * SL_ACC <= 512, "tensor memory");
+static_assert((SL_EPI_WARP0 & 3) == 0, "a warp reads the tensor-memory quarter warp % 4");
+
+// instruction descriptor: FP32 D, FP16 (format 0) K-major A and B, M = 128, N columns
+__device__ __forceinline__ uint32_t slice_idesc(int n)
+{
+	return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(SL_M >> 4) << 24);
+}
+
+__device__ __forceinline__ bool elect_one()
+{
+	uint32_t p;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(p));
+	return p != 0;
+}
+
+__device__ __forceinline__ void slice_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate)
+{
+	asm volatile(
+		"{\n\t.reg .pred p;\n\t"
+		"setp.ne.b32 p, %4, 0;\n\t"
+		"tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+		:
+		: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate));
+}
+
+// bounded wait for the given phase parity; false after SL_WAIT polls, or when *abort is set
+__device__ __forceinline__ bool slice_wait(uint64_t* bar, uint32_t parity, const volatile int* abort)
+{
+	const uint32_t mbar = smem_u32(bar);
+	for (int it = 0; it < SL_WAIT; it++)
+	{
+		uint32_t done;
+		asm volatile(
+			"{\n\t.reg .pred p;\n\t"
+			"mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+			"selp.b32 %0, 1, 0, p;\n\t}"
+			: "=r"(done)
+			: "r"(mbar), "r"(parity), "r"(SL_POLL_NS)
+			: "memory");
+		if (done) return true;
+		if (abort && *abort) return false;
+	}
+	return false;
+}
+
+// acc + x w for w = 2^24, 2^16, 2^8 or 1: one multiply-add instead of the shift and the two adds that a
+// constant factor would become
+__device__ __forceinline__ int64_t add_order(int64_t acc, int x, int w)
+{
+	int64_t r;
+	asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(x), "r"(w), "l"(acc));
+	return r;
+}
+
+// biased exponent of a number; 1 for denormal numbers, 0 for zero
+__device__ __forceinline__ int exponent_code(double x)
+{
+	const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+	return hi >= 0x00100000u ? (int)(hi >> 20) : (hi | (uint32_t)__double2loint(x)) ? 1 : 0;
+}
+
+// ------------------------------------------------------------------------------------
+// exponents and digits of an operand
+// ------------------------------------------------------------------------------------
+
+// largest exponent code of every operand block, SLICE_CHUNK entries per CTA
+__global__ void __launch_bounds__(256)
+k_block_exps(const SliceChunk* __restrict__ chunks, const double* __restrict__ x, int* __restrict__ exps, int* __restrict__ clear,
+             int nclear)
+{
+	pdl_wait();
+	pdl_trigger();
+	const SliceChunk ch = chunks[blockIdx.x];
+	int e = 0;
+	for (int i = threadIdx.x; i < ch.n; i += 256) e = max(e, exponent_code(x[ch.off + i]));
+	e = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
+	if ((threadIdx.x & 31) == 0 && e > 0) atomicMax(exps + ch.block, e);
+	for (int i = blockIdx.x * 256 + threadIdx.x; i < nclear; i += gridDim.x * 256) clear[i] = 0;
+}
+
+// bytes 0 and 1 (or 2 and 3) of w, biased digits u = d + 128 of two numbers, as FP16 pairs with the
+// numbers' signs: 0x6400 + u is the FP16 pattern of 1024 + u, and sgn (1024 + u) - sgn 1152 = sgn d
+__device__ __forceinline__ uint32_t digits_f16x2(uint32_t w, bool upper, uint32_t sgn, uint32_t off)
+{
+	const uint32_t p = __byte_perm(w, 0x64646464u, upper ? 0x4342 : 0x4140);
+	uint32_t r;
+	asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(p), "r"(sgn), "r"(off));
+	return r;
+}
+
+// One warp per item: 32 rows of a group by SLICE_ITEM stages of its terms, 8 terms at a time (each lane a
+// row: its 8 entries become 16 bytes of each of the 8 digits). The entries of the next 8 terms are on
+// their way while these are cut.
+constexpr int PACK_WARPS = 4;
+__global__ void __launch_bounds__(PACK_WARPS * 32, 8)
+k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups,
+             const SliceRun* __restrict__ runs, int rows8, const double* __restrict__ x, const int* __restrict__ exps,
+             unsigned char* __restrict__ dst, int* __restrict__ gexps)
+{
+	pdl_wait();
+	pdl_trigger();
+	const int item = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	if (item >= nitems) return;
+	const SliceItem im = items[item];
+	const SliceGroup g = groups[im.group];
+	int E = 0;
+	for (int c = lane; c < g.nrun; c += 32) E = max(E, exps[runs[g.run0 + c].block]);
+	E = (int)__reduce_max_sync(0xffffffffu, (unsigned)E);
+	if (im.row0 == 0 && im.u0 == 0 && lane == 0) gexps[im.group] = E;
+	// blocks with smaller exponents are summed in FP64, or hold zeros only
+	E = max(E, SLICE_EXP_MIN);
+	const int row = im.row0 + lane;
+	const bool valid = row < g.rows;
+	// destination of the lane's row in stage 0, first 8 terms, digit 0; bytes between digits and stages
+	unsigned char* out = dst + g.base + (lane & 7) * 16;
+	const int groups8 = (g.rows + 7) / 8, groups32 = (g.rows + 31) / 32;
+	const int digit = rows8 ? SL_A_DIGIT : SLICE_COL32_BYTES / SLICES;
+	const i64 stage = rows8 ? (i64)groups8 * SLICE_ROW8_BYTES : (i64)groups32 * SLICE_COL32_BYTES;
+	out += rows8 ? (i64)(row >> 3) * SLICE_ROW8_BYTES : (i64)(row >> 5) * SLICE_COL32_BYTES + (lane >> 3) * SL_B_SBO;
+	const bool store = rows8 ? (row >> 3) < groups8 : true;
+	// place in the terms: block c of the group, term kk of it
+	int c = im.run - 1, kk = 0, kend = 0, sk = 0;
+	const double* p = nullptr;
+	auto next = [&]() {
+		kk = 0;
+		if (++c < g.nrun)
+		{
+			const SliceRun r = runs[g.run0 + c];
+			kend = r.k;
+			sk = r.sk;
+			p = x + r.off + (i64)(valid ? row : 0) * r.sr;
+		}
+	};
+	next();
+	kk = im.kk;
+	auto read8 = [&](double v[8]) {
+		if (c < g.nrun && kend - kk >= 8)
+		{
+			const double* s = p + (i64)kk * sk;
+#pragma unroll
+			for (int t = 0; t < 8; t++) v[t] = valid ? s[(i64)t * sk] : 0.0;
+			kk += 8;
+			if (kk == kend) next();
+			return;
+		}
+#pragma unroll
+		for (int t = 0; t < 8; t++)
+		{
+			v[t] = 0.0;
+			if (c < g.nrun)
+			{
+				if (valid) v[t] = p[(i64)kk * sk];
+				if (++kk == kend) next();
+			}
+		}
+	};
+	const int stages = (g.ktot + SLICE_STAGE_K - 1) / SLICE_STAGE_K;
+	const int n8 = 2 * min(SLICE_ITEM, stages - im.u0);
+	out += (i64)im.u0 * stage;
+	double v[8];
+	read8(v);
+	for (int u = 0; u < n8; u++)
+	{
+		uint32_t dig[8][2], sgn[4], off[4];
+#pragma unroll
+		for (int q = 0; q < 4; q++)
+		{
+			const uint32_t ha = (uint32_t)__double2hiint(v[2 * q]), hb = (uint32_t)__double2hiint(v[2 * q + 1]);
+			const uint64_t da = slice_digits(ha, (uint32_t)__double2loint(v[2 * q]), E);
+			const uint64_t db = slice_digits(hb, (uint32_t)__double2loint(v[2 * q + 1]), E);
+			dig[2 * q][0] = (uint32_t)(da >> 32);
+			dig[2 * q][1] = (uint32_t)da;
+			dig[2 * q + 1][0] = (uint32_t)(db >> 32);
+			dig[2 * q + 1][1] = (uint32_t)db;
+			// +-1 and -+1152 in FP16, by the numbers' signs
+			const uint32_t s2 = __byte_perm(ha, hb, 0x7030) & 0x80008000u;
+			sgn[q] = s2 | 0x3c003c00u;
+			off[q] = s2 ^ 0xe480e480u;
+		}
+		if (u + 1 < n8) read8(v);
+		unsigned char* d = out + (i64)(u >> 1) * stage + (u & 1) * SL_LBO;
+#pragma unroll
+		for (int h = 0; h < 4; h++)
+		{
+			// digits 2 h and 2 h + 1: bytes 3 and 2 (h even) or 1 and 0 of word h / 2
+			uint32_t w0[4], w1[4];
+#pragma unroll
+			for (int q = 0; q < 4; q++)
+			{
+				const uint32_t b = __byte_perm(dig[2 * q][h >> 1], dig[2 * q + 1][h >> 1], (h & 1) ? 0x4051 : 0x6273);
+				w0[q] = digits_f16x2(b, false, sgn[q], off[q]);
+				w1[q] = digits_f16x2(b, true, sgn[q], off[q]);
+			}
+			if (store)
+			{
+				*(uint4*)(d + 2 * h * digit) = make_uint4(w0[0], w0[1], w0[2], w0[3]);
+				*(uint4*)(d + (2 * h + 1) * digit) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+			}
+		}
+	}
+}
+
+// ------------------------------------------------------------------------------------
+// the products
+// ------------------------------------------------------------------------------------
+
+// whether the results of two groups with these exponents are summed in FP64
+__device__ __forceinline__ bool sum_again(int e, int f)
+{
+	return e == 0x7ff || f == 0x7ff || e < SLICE_EXP_MIN || f < SLICE_EXP_MIN || !slice_in_range(slice_top(e, f));
+}
+
+// n entries of an output block from (i, j) on, along its columns (along = 1) or rows, by FP64 sums
+__device__ __noinline__ void slice_entries_f64(const GemmOut& o, const GemmContrib* cons, const double* A, const double* B, int i,
+                                               int j, int along, int n, double* C, int* exp_c)
+{
+	for (; n > 0; n--, along ? j++ : i++)
+	{
+		double s = 0.0;
+		for (int c = o.c0; c < o.c0 + o.nc; c++)
+		{
+			const GemmContrib g = cons[c];
+			const double* a = A + g.a_off + (i64)i * g.sAm;
+			const double* b = B + g.b_off + (i64)j * g.sBn;
+			for (int kk = 0; kk < g.k; kk++) s = fma(a[(i64)kk * g.sAk], b[(i64)kk * g.sBk], s);
+		}
+		C[gemm_out_index(o, i, j)] = s;
+		if (exp_c && exponent_code(s)) atomicMax(exp_c + o.block, exponent_code(s));
+	}
+}
+
+__global__ void __launch_bounds__(SL_THREADS, 1)
+k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
+              const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const unsigned char* xpack,
+              const unsigned char* ypack, const int* xexps, const int* yexps, double* C, int* exp_c, double* work, int* error)
+{
+	extern __shared__ __align__(1024) unsigned char smem[];
+	double* stage_out = (double*)(smem + SL_STAGES * SL_STAGE);
+	SliceInfo* infos = (SliceInfo*)((unsigned char*)stage_out + SL_EPI_BYTES);
+	uint64_t* full = (uint64_t*)(infos + 2 * SL_TILES);                       // copies landed
+	uint64_t* empty = full + SL_STAGES;                                       // MMAs of a stage done
+	uint64_t* acc_full = empty + SL_STAGES;                                   // accumulators ready
+	uint64_t* acc_empty = acc_full + 2;                                       // accumulators read
+	uint64_t* info_full = acc_empty + 2;                                      // tiles described
+	uint64_t* info_empty = info_full + 2;                                     // their descriptions read
+	uint64_t* split_bar = info_empty + 2;                                     // epilogue: steps of a split tile
+	uint32_t* tmem_slot = (uint32_t*)(split_bar + 1);
+	volatile int* abort = (volatile int*)(tmem_slot + 1);
+	volatile int* last_share = abort + 1;
+	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+	if (warp == 1)
+	{
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512)
+		             : "memory");
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+	}
+	if (tid == 0)
+	{
+		for (int st = 0; st < SL_STAGES; st++)
+		{
+			mbar_init(smem_u32(full + st), 1);
+			mbar_init(smem_u32(empty + st), 1);
+		}
+		for (int b = 0; b < 2; b++)
+		{
+			mbar_init(smem_u32(acc_full + b), 1);
+			mbar_init(smem_u32(acc_empty + b), SL_EPI);
+			mbar_init(smem_u32(info_full + b), 1);
+			mbar_init(smem_u32(info_empty + b), SL_EPI + 2);
+		}
+		mbar_init(smem_u32(split_bar), SL_EPI);
+		*abort = 0;
+	}
+	asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	tc_fence_before();
+	__syncthreads();
+	tc_fence_after();
+	const uint32_t tmem = *tmem_slot;
+	// everything up to here overlaps the tail of the previous kernel in the stream
+	pdl_wait();
+
+	// the description of the CTA's tile number it (every lane of a warp, in order): null at the end
+	auto tile_info = [&](int it, bool& ok) -> const SliceInfo* {
+		const int batch = (it / SL_TILES) & 1;
+		if (it % SL_TILES == 0) ok = __all_sync(0xffffffffu, slice_wait(info_full + batch, (uint32_t)((it / (2 * SL_TILES)) & 1), abort));
+		const SliceInfo* f = infos + batch * SL_TILES + it % SL_TILES;
+		return ok && f->tile >= 0 ? f : nullptr;
+	};
+	// after the last use of it
+	auto tile_done = [&](int it) {
+		if (it % SL_TILES != SL_TILES - 1) return;
+		__syncwarp();
+		if (lane == 0) mbar_arrive(smem_u32(info_empty + ((it / SL_TILES) & 1)));
+	};
+
+	if (warp == 0)
+	{
+		// copies: the stages of every tile in order
+		int g = 0;
+		bool ok = true;
+		for (int it = 0; ok; it++)
+		{
+			const SliceInfo* f = tile_info(it, ok);
+			if (!f) break;
+			const uint32_t xb = f->xbytes, yb = f->ybytes;
+			const int xstep = f->xstep, ystep = f->ystep, nch = f->nch;
+			const unsigned char *xs = xpack + f->xs, *ys = ypack + f->ys;
+			for (int u = 0; u < nch; u++, g++, xs += xstep, ys += ystep)
+			{
+				const int st = g % SL_STAGES;
+				if (g >= SL_STAGES) ok = slice_wait(empty + st, (uint32_t)(((g / SL_STAGES) - 1) & 1), abort);
+				ok = __all_sync(0xffffffffu, ok);
+				if (!ok) break;
+				if (lane == 0)
+				{
+					const uint32_t sa = smem_u32(smem + st * SL_STAGE), bar = smem_u32(full + st);
+					mbar_expect_tx(bar, xb + yb);
+					bulk_copy(sa, xs, xb, bar);
+					bulk_copy(sa + SL_A_BYTES, ys, yb, bar);
+				}
+				__syncwarp();
+			}
+			tile_done(it);
+		}
+		if (!ok && lane == 0)
+		{
+			*abort = 1;
+			atomicExch(error, 1);
+		}
+		// the copies of the last stages must land before shared memory is released
+		for (int u = max(g - SL_STAGES, 0); u < g; u++) slice_wait(full + u % SL_STAGES, (uint32_t)((u / SL_STAGES) & 1), nullptr);
+	}
+	else if (warp == 1)
+	{
+		// the whole warp walks the stages (its state stays in uniform registers), one lane issues
+		int g = 0, f = 0;                  // stages, flushes of a half
+		bool ok = true;
+		const bool one = elect_one();
+		const uint32_t s0 = smem_u32(smem);
+		for (int it = 0; ok; it++)
+		{
+			const SliceInfo* info = tile_info(it, ok);
+			if (!info) break;
+			const int nch = info->nch, halves = info->halves;
+			for (int u = 0; u < nch && ok; u++, g++)
+			{
+				const int st = g % SL_STAGES;
+				const bool first = u % SL_FLUSH == 0, last = u % SL_FLUSH == SL_FLUSH - 1 || u == nch - 1;
+				ok = slice_wait(full + st, (uint32_t)((g / SL_STAGES) & 1), abort);
+				if (!ok) break;
+				for (int h = 0; h < halves; h++)
+				{
+					const int fh = f + h, b = fh & 1;
+					if (first && fh >= 2)
+					{
+						ok = slice_wait(acc_empty + b, (uint32_t)(((fh >> 1) - 1) & 1), abort);
+						if (!ok) break;
+					}
+					tc_fence_after();
+					if (one)
+					{
+						const uint64_t da = make_desc(s0 + st * SL_STAGE, SL_LBO, SL_A_SBO);
+						const uint64_t db = make_desc(s0 + st * SL_STAGE + SL_A_BYTES + h * SLICE_COL32_BYTES, SL_LBO, SL_B_SBO);
+						const uint32_t acc = tmem + (uint32_t)(b * SL_ACC);
+#pragma unroll
+						for (int s = 0; s < SLICES; s++)
+							slice_mma(acc + (uint32_t)(s * SL_HALF), da + (uint64_t)(s * (SL_A_DIGIT >> 4)), db,
+							          slice_idesc(SL_HALF * (SLICES - s)), s > 0 || !first);
+						if (last) mma_commit(smem_u32(acc_full + b));
+						if (h == halves - 1) mma_commit(smem_u32(empty + st));
+					}
+					__syncwarp();
+				}
+				if (last) f += halves;
+			}
+			tile_done(it);
+		}
+		if (!ok && lane == 0)
+		{
+			*abort = 1;
+			atomicExch(error, 1);
+		}
+		// no MMA may still run when tensor memory is freed
+		if (g > 0) slice_wait(empty + (g - 1) % SL_STAGES, (uint32_t)(((g - 1) / SL_STAGES) & 1), nullptr);
+		pdl_trigger();
+	}
+	else if (warp == 2)
+	{
+		// descriptions, 32 tiles at a time, one per lane: no other warp waits for global memory but for its
+		// data. Tiles come in order of falling work; each pass over the CTAs reverses the order of the
+		// one before
+		const int grid = gridDim.x, me = blockIdx.x, npass = (ntiles + grid - 1) / grid;
+		bool ok = true;
+		for (int p0 = 0; ok; p0 += SL_TILES)
+		{
+			const int batch = (p0 / SL_TILES) & 1;
+			if (p0 >= 2 * SL_TILES)
+				ok = __all_sync(0xffffffffu, slice_wait(info_empty + batch, (uint32_t)((p0 / (2 * SL_TILES) - 1) & 1), abort));
+			if (!ok) break;
+			const int pass = p0 + lane, ti = pass * grid + ((pass & 1) ? grid - 1 - me : me);
+			SliceInfo f = {};
+			f.tile = -1;
+			if (pass < npass && ti < ntiles)
+			{
+				const SliceTile t = tiles[ti];
+				const GemmOut o = outs[t.out];
+				f.tile = ti;
+				f.nch = t.u1 - t.u0;
+				f.halves = t.halves;
+				f.m0 = t.m0;
+				f.n0 = t.n0;
+				f.m = o.m;
+				f.n = o.n;
+				f.co = o.c_off;
+				f.sr0 = o.sr0;
+				f.sr1 = o.sr1;
+				f.sc0 = o.sc0;
+				f.r1 = o.r1;
+				f.c1 = o.c1;
+				f.split = t.split;
+				f.sp = t.sp;
+				f.block = o.block;
+				if (f.nch > 0)
+				{
+					const SliceOut s = souts[t.out];
+					const int x8 = (orient ? t.m0 : t.n0) >> 3, y32 = (orient ? t.n0 : t.m0) >> 5;
+					f.xstep = s.x8 * SLICE_ROW8_BYTES;
+					f.ystep = s.y32 * SLICE_COL32_BYTES;
+					f.xbytes = min(SL_M / 8, s.x8 - x8) * SLICE_ROW8_BYTES;
+					f.ybytes = min(2, s.y32 - y32) * SLICE_COL32_BYTES;
+					f.xs = s.xbase + (i64)t.u0 * f.xstep + (i64)x8 * SLICE_ROW8_BYTES;
+					f.ys = s.ybase + (i64)t.u0 * f.ystep + (i64)y32 * SLICE_COL32_BYTES;
+					f.e = xexps[s.xgroup];
+					f.f = yexps[s.ygroup];
+				}
+			}
+			infos[batch * SL_TILES + lane] = f;
+			__syncwarp();
+			if (lane == 0) mbar_arrive(smem_u32(info_full + batch));
+			if (p0 + SL_TILES > npass) break;      // the batch had a lane without a tile: the end is marked
+		}
+		if (!ok && lane == 0)
+		{
+			*abort = 1;
+			atomicExch(error, 1);
+		}
+	}
+	else if (warp >= SL_EPI_WARP0)
+	{
+		const int q = warp & 3, part = (warp - SL_EPI_WARP0) >> 2;
+		const int gr = q * 32 + lane;                          // MMA row
+		double* sw = stage_out + (warp - SL_EPI_WARP0) * 32 * SL_LD;
+		int f = 0, nsp = 0;
+		int wt[4] = {1 << 24, 1 << 16, 1 << 8, 1};
+		asm("" : "+r"(wt[0]), "+r"(wt[1]), "+r"(wt[2]), "+r"(wt[3]));
+		// the sums of the halves between the flushes of a tile with several
+		int64_t kept[32];
+		bool ok = true;
+		for (int it = 0; ok; it++)
+		{
+			const SliceInfo* info = tile_info(it, ok);
+			if (!info) break;
+			const SliceInfo& tile = *info;
+			const int nch = tile.nch, halves = tile.halves;
+			// MMA rows of this warp inside the output block
+			const int rows = min(32, (orient ? tile.m - tile.m0 : tile.n - tile.n0) - q * 32);
+			const int nfl = max((nch + SL_FLUSH - 1) / SL_FLUSH, 1);
+			// a last flush of 32 terms at most (32 x 7 x 2^14 < 2^22) leaves the integers in the low bits of
+			// sum + 1.5 2^23: minus the offsets that their patterns will add, 0x4b400000 times the weights
+			// (the sums of the orders 0 .. 2 stay below 2^22 for 128 terms, and always go that way: the integer
+			// conversion runs at an eighth of the rate)
+			const bool few_last = nch > 0 && (nch - 1) % SL_FLUSH < 2;
+			const int64_t start_hi = -0x4b400000ll * ((int64_t)nfl * 0x01010100ll + (few_last ? 1 : 0));
+			const int64_t start_lo = few_last ? -0x4b400000ll * 0x01010101ll : 0;
+			for (int fl = 0; fl < nfl && ok; fl++)
+			{
+#pragma unroll 1
+				for (int h = 0; h < halves; h++)
+				{
+					// MMA columns of this warp; one without columns waits and arrives like the others, so that no
+					// warp gets more than a phase of a barrier ahead or behind
+					const int gc = h * SL_HALF + part * 8;
+					const int cols = min(8, (orient ? tile.n - tile.n0 : tile.m - tile.m0) - gc);
+					const bool active = rows > 0 && cols > 0;
+					int64_t hi[8], lo[8];
+					if (fl == 0)
+					{
+#pragma unroll
+						for (int c = 0; c < 8; c++)
+						{
+							hi[c] = start_hi;
+							lo[c] = start_lo;
+						}
+					}
+					else
+					{
+#pragma unroll
+						for (int c = 0; c < 8; c++)
+						{
+							hi[c] = kept[h * 16 + c];
+							lo[c] = kept[h * 16 + 8 + c];
+						}
+					}
+					if (nch > 0)
+					{
+						const int b = f & 1;
+						ok = __all_sync(0xffffffffu, slice_wait(acc_full + b, (uint32_t)((f >> 1) & 1), abort));
+						f++;
+						if (!ok) break;
+						if (active)
+						{
+							tc_fence_after();
+							const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * SL_ACC + part * 8);
+							const bool few = few_last && fl == nfl - 1;
+#pragma unroll
+							for (int op = 0; op < SLICES; op += 2)
+							{
+								uint32_t v[16];
+								asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+								             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+								             : "r"(ta + (uint32_t)(op * SL_HALF)));
+								asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+								             : "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+								             : "r"(ta + (uint32_t)((op + 1) * SL_HALF)));
+								asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+								for (int c = 0; c < 16; c++)
+								{
+									const float x = __uint_as_float(v[c]);
+									v[c] = few || op + c / 8 <= 2 ? __float_as_uint(x + 12582912.0f) : (uint32_t)__float2int_rn(x);
+								}
+								// orders op and op + 1 have the weights 2^24, 2^16 (op % 4 == 0) or 2^8, 1 in their half
+								const int w0 = (op & 2) ? wt[2] : wt[0], w1 = (op & 2) ? wt[3] : wt[1];
+#pragma unroll
+								for (int c = 0; c < 8; c++)
+								{
+									int64_t& acc = op < 4 ? hi[c] : lo[c];
+									acc = add_order(add_order(acc, (int)v[c], w0), (int)v[8 + c], w1);
+								}
+							}
+							tc_fence_before();
+						}
+						__syncwarp();
+						if (lane == 0) mbar_arrive(smem_u32(acc_empty + b));
+					}
+					if (fl < nfl - 1)
+					{
+#pragma unroll
+						for (int c = 0; c < 8; c++)
+						{
+							kept[h * 16 + c] = hi[c];
+							kept[h * 16 + 8 + c] = lo[c];
+						}
+						continue;
+					}
+					if (!active) continue;
+					if (tile.split >= 0)
+					{
+						// a share of a split tile: its sums as they are
+						const GemmSplit sp = splits[tile.split];
+						int64_t* w = (int64_t*)(work + sp.part + (i64)tile.sp * sp.stride);
+						if (lane < rows)
+						{
+#pragma unroll
+							for (int c = 0; c < 8; c++)
+								if (c < cols) *(longlong2*)(w + 2 * (orient ? gr * sp.ld + gc + c : (gc + c) * sp.ld + gr)) = make_longlong2(hi[c], lo[c]);
+						}
+						continue;
+					}
+					// results in place of the sums; `again`: they are summed in FP64 below
+					const int top = slice_top(tile.e, tile.f);
+					const bool zero = tile.e == 0 || tile.f == 0, again = !zero && sum_again(tile.e, tile.f);
+					int emax = 0;
+					if (zero)
+					{
+#pragma unroll
+						for (int c = 0; c < 8; c++) hi[c] = 0;
+					}
+					else
+					{
+#pragma unroll
+						for (int c = 0; c < 8; c++) hi[c] = (int64_t)slice_value(hi[c], lo[c], top);
+					}
+					// columns past the block's end have zero digits
+#pragma unroll
+					for (int c = 0; c < 8; c++) emax = max(emax, (int)((uint32_t)((uint64_t)hi[c] >> 32) & 0x7fffffffu));
+					emax = again || lane >= rows ? 0 : emax >> 20;
+					if (exp_c)
+					{
+						emax = (int)__reduce_max_sync(0xffffffffu, (unsigned)emax);
+						if (lane == 0 && emax > 0) atomicMax(exp_c + tile.block, emax);
+					}
+					if (orient == 0)
+					{
+						// lanes are neighbouring columns of the output block: coalesced
+						if (lane < rows)
+						{
+							const int j = tile.n0 + gr, jq = j / tile.c1, r1 = tile.r1;
+							const i64 sr1 = tile.sr1, wrap = tile.sr0 - (i64)(r1 - 1) * sr1;
+							const int i = tile.m0 + gc, ih = i / r1;
+							int il = i - ih * r1;
+							double* ci = C + tile.co + (i64)jq * tile.sc0 + (j - jq * tile.c1) + (i64)ih * tile.sr0 + (i64)il * sr1;
+#pragma unroll
+							for (int c = 0; c < 8; c++)
+							{
+								if (c < cols) *ci = __longlong_as_double(hi[c]);
+								// the next row: a step inside the run of low row indices, or past its end
+								const bool end = ++il == r1;
+								ci += end ? wrap : sr1;
+								if (end) il = 0;
+							}
+						}
+					}
+					else
+					{
+						// lanes are rows of the output block: turned in shared memory, so that 4 lanes write 4
+						// neighbouring columns of a row
+						const int i = min(tile.m0 + gr, tile.m - 1), iq = i / tile.r1;
+						const i64 ro = tile.co + (i64)iq * tile.sr0 + (i64)(i - iq * tile.r1) * tile.sr1;
+						const int c = lane & 3;
+#pragma unroll
+						for (int c0 = 0; c0 < 8; c0 += 4)
+						{
+							if (cols <= c0) break;
+#pragma unroll
+							for (int t = 0; t < 4; t++) sw[lane * SL_LD + t] = __longlong_as_double(hi[c0 + t]);
+							__syncwarp();
+							const int j = tile.n0 + gc + min(c0 + c, cols - 1), jq = j / tile.c1;
+							const i64 co = (i64)jq * tile.sc0 + (j - jq * tile.c1);
+#pragma unroll
+							for (int t = 0; t < 4; t++)
+							{
+								const int rr = t * 8 + (lane >> 2);
+								const i64 rof = __shfl_sync(0xffffffffu, ro, rr);
+								if (rr < rows && c0 + c < cols) C[rof + co] = sw[rr * SL_LD + c];
+							}
+							__syncwarp();
+						}
+					}
+					__syncwarp();
+					if (again && lane < rows) slice_entries_f64(outs[tiles[tile.tile].out], cons, A, B, orient ? tile.m0 + gr : tile.m0 + gc, orient ? tile.n0 + gc : tile.n0 + gr, orient, cols, C, exp_c);
+				}
+			}
+			if (!ok) break;
+			if (tile.split >= 0)
+			{
+				// the CTA that completes a split tile last adds the shares (integers of one scale) and rounds
+				const GemmSplit sp = splits[tile.split];
+				auto step = [&]() {
+					__syncwarp();
+					if (lane == 0) mbar_arrive(smem_u32(split_bar));
+					ok = __all_sync(0xffffffffu, slice_wait(split_bar, (uint32_t)(nsp & 1), abort));
+					nsp++;
+				};
+				__threadfence();
+				step();
+				if (!ok) break;
+				if (warp == SL_EPI_WARP0 && lane == 0) *last_share = atomicAdd(counters + tile.split, 1) == sp.nsplit - 1;
+				step();
+				if (!ok) break;
+				if (*last_share)
+				{
+					__threadfence();
+					int emax = 0;
+					for (int e = tid - 32 * SL_EPI_WARP0; e < sp.rows * sp.cols; e += 32 * SL_EPI)
+					{
+						const int i = e / sp.cols, j = e - i * sp.cols;
+						const longlong2* pw = (const longlong2*)(work + sp.part) + (i64)i * sp.ld + j;
+						int64_t hi = 0, lo = 0;
+						for (int p = 0; p < sp.nsplit; p++)
+						{
+							const longlong2 v = __ldcg(pw + (i64)p * (sp.stride / 2));
+							hi += v.x;
+							lo += v.y;
+						}
+						const bool zero = tile.e == 0 || tile.f == 0;
+						const double sum = zero ? 0.0 : __longlong_as_double((long long)slice_value(hi, lo, slice_top(tile.e, tile.f)));
+						C[gemm_out_index(outs[sp.out], sp.m0 + i, sp.n0 + j)] = sum;
+						if (!zero && sum_again(tile.e, tile.f))
+							slice_entries_f64(outs[sp.out], cons, A, B, sp.m0 + i, sp.n0 + j, 0, 1, C, exp_c);
+						else emax = max(emax, exponent_code(sum));
+					}
+					if (exp_c && emax > 0) atomicMax(exp_c + tile.block, emax);
+					if (tid == 32 * SL_EPI_WARP0) counters[tile.split] = 0;
+				}
+				// nobody overwrites *last_share before every warp has read it
+				step();
+				if (!ok) break;
+			}
+			tile_done(it);
+		}
+		if (!ok && lane == 0)
+		{
+			*abort = 1;
+			atomicExch(error, 1);
+		}
+	}
+	tc_fence_before();
+	__syncthreads();
+	if (warp == 1)
+	{
+		tc_fence_after();
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+	}
+}
+
+}  // namespace
+
+void launch_block_exps(int nchunks, const SliceChunk* chunks, const double* x, int* exps, int* clear, int nclear, cudaStream_t st)
+{
+	if (nchunks <= 0)
+	{
+		if (nclear > 0) CTG_CUDA(cudaMemsetAsync(clear, 0, (size_t)nclear * sizeof(int), st));
+		return;
+	}
+	launch_pdl(launch_config(dim3(nchunks), dim3(256), 0, st), k_block_exps, chunks, x, exps, clear, nclear);
+}
+
+void launch_slice_pack(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, bool rows8,
+                       const double* x, const int* exps, void* dst, int* gexps, cudaStream_t st)
+{
+	if (nitems <= 0) return;
+	launch_pdl(launch_config(dim3((nitems + PACK_WARPS - 1) / PACK_WARPS), dim3(PACK_WARPS * 32), 0, st), k_slice_pack, nitems, items,
+	           groups, runs, rows8 ? 1 : 0, x, exps, (unsigned char*)dst, gexps);
+}
+
+void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
+                        const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const void* xpack,
+                        const void* ypack, const int* xexps, const int* yexps, double* C, int* exp_c, double* work, int* error,
+                        int num_sms, cudaStream_t st)
+{
+	if (ntiles <= 0) return;
+	static std::once_flag attr_once;
+	std::call_once(attr_once, [] {
+		CTG_CUDA(cudaFuncSetAttribute(k_gemm_slices, cudaFuncAttributeMaxDynamicSharedMemorySize, SL_SMEM));
+	});
+	// persistent: one CTA per SM (its shared memory admits one)
+	const cudaLaunchConfig_t cfg = launch_config(dim3(std::min(ntiles, num_sms)), dim3(SL_THREADS), SL_SMEM, st);
+	launch_pdl(cfg, k_gemm_slices, ntiles, tiles, outs, souts, cons, splits, counters, orient, A, B, (const unsigned char*)xpack,
+	           (const unsigned char*)ypack, xexps, yexps, C, exp_c, work, error);
+}
+
+}  // namespace ctg

@@ -36,6 +36,7 @@
 #include <mutex>
 
 #include "ctg_kernels.h"
+#include "ctg_tcgen05.cuh"
 
 namespace ctg {
 
@@ -101,22 +102,6 @@ struct Cfg {
 	static_assert(TMEM_COLS <= 512, "tensor memory");
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p)
-{
-	return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// shared-memory matrix descriptor (no swizzle, K-major)
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr)
-{
-	uint64_t d = 0;
-	d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-	d |= (uint64_t)((TC_LBO >> 4) & 0x3FFF) << 16;
-	d |= (uint64_t)((TC_SBO >> 4) & 0x3FFF) << 32;
-	d |= (uint64_t)1 << 46;                // descriptor version for this architecture
-	return d;                              // base offset 0, swizzle none
-}
-
 // instruction descriptor: FP32 D, K-major A and B, M = 128, N = BN; A / B format BF16 (1, kind::f16)
 // or TF32 (2, kind::tf32)
 template <int FMT, int BN>
@@ -150,57 +135,6 @@ __device__ __forceinline__ void mma(uint32_t tmem_d, uint64_t adesc, uint64_t bd
 			:
 			: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"((uint32_t)accumulate));
 }
-
-__device__ __forceinline__ void mma_commit(uint32_t mbar)
-{
-	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t mbar, int count)
-{
-	asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(count) : "memory");
-}
-
-// bounded wait for the given phase parity; returns false after `limit` polls, or when *abort is set
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, long long limit, const volatile int* abort = nullptr)
-{
-	for (long long it = 0; it < limit; it++)
-	{
-		if (abort && *abort) return false;
-		uint32_t done = 0;
-		asm volatile(
-			"{\n\t.reg .pred p;\n\t"
-			"mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-			"selp.b32 %0, 1, 0, p;\n\t}"
-			: "=r"(done)
-			: "r"(mbar), "r"(parity)
-			: "memory");
-		if (done) return true;
-		if (it > 64) __nanosleep(64);
-	}
-	return false;
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t mbar, uint32_t bytes)
-{
-	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t mbar)
-{
-	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
-}
-
-// global -> shared bulk copy completing on an mbarrier (16-byte aligned addresses, size a multiple of 16)
-__device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t mbar)
-{
-	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-	             "l"(src), "r"(bytes), "r"(mbar)
-	             : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t canon_offset(int row, int kbyte)
 {
@@ -431,8 +365,8 @@ k_gemm_tc(int ntiles, const GemmTile* __restrict__ tiles, const GemmOut* __restr
 						{
 							int pa, pb;
 							F::prod(pr, pa, pb);
-							const uint64_t da = make_desc(sa + (uint32_t)(pa * A_PART_BYTES) + koff);
-							const uint64_t db = make_desc(sb + (uint32_t)(pb * BN * TC_KB) + koff);
+							const uint64_t da = make_desc(sa + (uint32_t)(pa * A_PART_BYTES) + koff, TC_LBO, TC_SBO);
+							const uint64_t db = make_desc(sb + (uint32_t)(pb * BN * TC_KB) + koff, TC_LBO, TC_SBO);
 							mma<FMT>(dacc, da, db, idesc, u > 0 || k > 0 || pr > 0);
 						}
 					}

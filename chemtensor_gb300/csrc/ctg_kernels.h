@@ -24,6 +24,7 @@ struct GemmOut {
 	// of column axes rearranged, the last column run innermost), so that no transpose pass is needed.
 	int r1, c1;
 	i64 sr0, sr1, sc0;
+	int block, pad;    // the block's number in the result's (transposed) structure
 };
 
 __host__ __device__ inline i64 gemm_out_index(const GemmOut& o, int i, int j)
@@ -76,6 +77,59 @@ int tile_cols(int cls);
 void launch_gemm_f64(int ntiles, const GemmTile* tiles, const GemmOut* outs, const GemmContrib* cons,
                      const GemmSplit* splits, int* counters, const double* A, const double* B, double* C, double* work,
                      cudaStream_t st, double flops = 0.0);
+
+// The same sums on the tensor cores by exact digit slices (ctg_gemm_slices.cu): FP64 operands and
+// results, each result rounded once. One operand of the product (x) lies along the 128 rows of the MMA
+// tiles, the other (y) along their 64 columns (two halves of 32): orient 0: x = B (the tile's 128 are
+// columns of the output block, its 64 rows of it), orient 1: x = A. The rows of an operand with the same
+// free indices form a group; the terms of its blocks follow each other, in the order of the output
+// blocks' contributions, which is the same for the two groups of an output block.
+constexpr int SLICE_TILE_ROWS = 128, SLICE_TILE_COLS = 64, SLICE_HALF = 32;
+constexpr int SLICE_STAGE_K = 16;                                   // terms of a stage
+constexpr int SLICE_ROW8_BYTES = 2048, SLICE_COL32_BYTES = 8192;    // digits of 8 rows of x, of 32 of y, per stage
+struct SliceTile {
+	int out;
+	int m0, n0;        // tile origin inside the output block
+	int u0, u1;        // stages (u0 = u1: no terms, the tile is zero)
+	int halves;        // 1 or 2
+	int split, sp;     // share of a split tile (GemmSplit, counters; two integers per entry in the work space)
+};
+struct SliceOut {      // an output block's groups: packed digits (bytes), rows / 8 of x, rows / 32 of y, numbers
+	i64 xbase, ybase;
+	int x8, y32;
+	int xgroup, ygroup;
+};
+struct SliceRun {      // one block of a group: first entry, terms, strides of rows and terms, its number
+	i64 off;
+	int k, sr, sk, block;
+};
+struct SliceGroup {
+	i64 base;          // packed digits (bytes)
+	int run0, nrun;
+	int rows, ktot;
+};
+constexpr int SLICE_ITEM = 4;                                       // stages of an item at most
+struct SliceItem {     // 32 rows of a group, stages from u0 on: they begin in block run of the group, at its term kk
+	int group, row0, u0;
+	int run, kk;
+};
+// largest biased exponent of every block of an operand into exps (zero before the launch): 0 a block of
+// zeros, 1 denormal numbers at most, 0x7ff a number that is not finite. Also sets clear[0 .. nclear) to zero.
+constexpr int SLICE_CHUNK = 4096;
+struct SliceChunk {
+	i64 off;
+	int n, block;
+};
+void launch_block_exps(int nchunks, const SliceChunk* chunks, const double* x, int* exps, int* clear, int nclear, cudaStream_t st);
+// digits of an operand (rows8: as x, else as y) from its blocks' exponents; gexps receives the groups'
+void launch_slice_pack(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, bool rows8,
+                       const double* x, const int* exps, void* dst, int* gexps, cudaStream_t st);
+// tiles are listed by falling work; exp_c (optional, zero before the launch) receives the largest biased
+// exponents of the result's blocks; *error becomes 1 if a bounded wait ran out
+void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
+                        const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const void* xpack,
+                        const void* ypack, const int* xexps, const int* yexps, double* C, int* exp_c, double* work, int* error,
+                        int num_sms, cudaStream_t st);
 
 // Same work lists on the tcgen05 tensor cores with FP32 accumulation, output tiles of
 // tc_tile_rows() x BN (BN = 64, 128 or 256, chosen per product). Operand formats (TcFormat):

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstdlib>
 #include <unordered_map>
 
 namespace ctg {
@@ -12,6 +13,8 @@ namespace ctg {
 thread_local double g_plan_stage[12];
 
 namespace {
+
+constexpr int SLICE_SPLIT = 8;             // fewest stages of a share of a split tile on the digit slices
 
 double host_seconds()
 {
@@ -107,6 +110,162 @@ CopyLowering rows_lowering(std::shared_ptr<Meta> out, std::vector<RowDesc>&& d, 
 	return p;
 }
 
+// tiles of an output block on the digit slices, with the 128 MMA rows along its columns (orient 0) or rows (1)
+i64 slice_ntiles(const GemmOut& o, int orient, int cols)
+{
+	auto up = [](int a, int b) { return (i64)((a + b - 1) / b); };
+	return orient ? up(o.m, SLICE_TILE_ROWS) * up(o.n, cols) : up(o.n, SLICE_TILE_ROWS) * up(o.m, cols);
+}
+
+// SM clocks of a tile of `halves` halves and k terms on the digit slices: the MMAs, and the epilogue that
+// they wait for
+double slice_clocks(double halves, i64 k)
+{
+	return halves * (1500.0 + 640.0 * (double)((k + SLICE_STAGE_K - 1) / SLICE_STAGE_K));
+}
+
+// the operand along the MMA rows: the choice with the fewer half tiles (weighted by their terms)
+int slice_orient(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum, double clocks[2])
+{
+	clocks[0] = clocks[1] = 0;
+	for (size_t b = 0; b < outs.size(); b++)
+		for (int o = 0; o < 2; o++) clocks[o] += slice_clocks((double)slice_ntiles(outs[b], o, SLICE_HALF), ksum[b]);
+	return clocks[1] < clocks[0] ? 1 : 0;
+}
+
+// SM clocks of the three launches that a product by digit slices has besides the GEMM (exponents, digits)
+constexpr double SLICE_OVERHEAD = 50000;
+
+// Digit slices or the FP64 pipe, by the SM clocks that each takes: the FP64 tiles at 2.1 FMAs a clock
+// (padding included), against the MMAs, the conversion of the operands' entries and the launches. Both
+// sides measured: a D = 1024 local-Hamiltonian product of 1.1e9 FMAs 2.0 ms against 0.2 ms, the
+// products of a Hubbard chain at D = 256 (3e6 .. 9e6 FMAs in 300 .. 1500 output blocks) 15 .. 60 us
+// against 40 .. 55 us.
+bool use_slices(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum, const std::vector<GemmTile>* tiles, i64 entries,
+                int num_sms)
+{
+	static const int forced = [] {
+		const char* e = getenv("CTGPU_SLICE_GEMM");
+		return e ? atoi(e) : -1;
+	}();
+	if (forced == 0) return false;
+	if (forced == 1) return true;
+	double clocks[2], f64 = 0;
+	const int o = slice_orient(outs, ksum, clocks);
+	for (int k = 0; k < NUM_TILE_CLASSES; k++)
+		for (const GemmTile& t : tiles[k])
+			f64 += (double)TILE_ROWS[k] * TILE_COLS[k] * (double)ksum[(size_t)t.out] / 2.1;
+	return (clocks[o] + 2.0 * (double)entries) / num_sms + SLICE_OVERHEAD < f64 / num_sms;
+}
+
+// how an operand is packed: the groups (runs of `keys` with one free index) that some output block uses
+struct SliceKey {
+	i64 f;
+	int block;
+};
+void slice_pack(const Meta& m, const std::vector<SliceKey>& keys, const std::vector<char>& used, bool leading,
+                const std::vector<i64>& lead, const std::vector<i64>& trail, bool rows8, SlicePack& p, std::vector<int>& group_at)
+{
+	p.blocks = m.nblocks;
+	for (int b = 0; b < m.nblocks; b++)
+		for (i64 e = 0, n = m.block_size(b); e < n; e += SLICE_CHUNK)
+			p.chunks.push_back(SliceChunk{m.boff[b] + e, (int)std::min<i64>(SLICE_CHUNK, n - e), b});
+	group_at.assign(keys.size(), -1);
+	for (size_t x = 0; x < keys.size();)
+	{
+		size_t y = x;
+		while (y < keys.size() && keys[y].f == keys[x].f) y++;
+		if (used[x])
+		{
+			SliceGroup g = {};
+			g.base = p.bytes;
+			g.run0 = (int)p.runs.size();
+			g.nrun = (int)(y - x);
+			for (size_t q = x; q < y; q++)
+			{
+				const int b = keys[q].block;
+				const i64 l = lead[(size_t)b], t = trail[(size_t)b];
+				SliceRun r = {};
+				r.off = m.boff[b];
+				r.k = (int)(leading ? l : t);
+				r.sr = (int)(leading ? 1 : t);
+				r.sk = (int)(leading ? t : 1);
+				r.block = b;
+				p.runs.push_back(r);
+				g.ktot += r.k;
+				g.rows = (int)(leading ? t : l);
+				CTG_CHECK(r.off + (i64)(g.rows - 1) * r.sr + (i64)(r.k - 1) * r.sk < m.nnz, "dot: operand out of range");
+			}
+			const i64 stages = (g.ktot + SLICE_STAGE_K - 1) / SLICE_STAGE_K;
+			p.bytes += stages * (rows8 ? (i64)((g.rows + 7) / 8) * SLICE_ROW8_BYTES : (i64)((g.rows + 31) / 32) * SLICE_COL32_BYTES);
+			group_at[x] = (int)p.groups.size();
+			int run = 0, kk = 0;                  // first term of the item's stages
+			for (int u0 = 0; u0 < stages; u0 += SLICE_ITEM)
+			{
+				for (int r0 = 0; r0 < g.rows; r0 += 32) p.items.push_back(SliceItem{(int)p.groups.size(), r0, u0, run, kk});
+				for (kk += SLICE_ITEM * SLICE_STAGE_K; run < g.nrun && kk >= p.runs[(size_t)(g.run0 + run)].k; run++)
+					kk -= p.runs[(size_t)(g.run0 + run)].k;
+			}
+			p.groups.push_back(g);
+		}
+		x = y;
+	}
+}
+
+// tiles, cut into shares of at least SLICE_SPLIT stages where one holds more than a fair share of the work
+void slice_tiles(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum, int num_sms, DotLowering& p)
+{
+	double total = 0;
+	for (size_t b = 0; b < outs.size(); b++)
+		total += slice_clocks((double)slice_ntiles(outs[b], p.orient, SLICE_HALF), ksum[b]);
+	const double target = std::max(total / num_sms, slice_clocks(1, SLICE_SPLIT * SLICE_STAGE_K));
+	i64 wsz = 0;
+	for (size_t b = 0; b < outs.size(); b++)
+	{
+		const GemmOut& o = outs[b];
+		const int tr = p.orient ? SLICE_TILE_ROWS : SLICE_TILE_COLS, tc = p.orient ? SLICE_TILE_COLS : SLICE_TILE_ROWS;
+		const i64 stages = (ksum[b] + SLICE_STAGE_K - 1) / SLICE_STAGE_K;
+		for (int m0 = 0; m0 < o.m; m0 += tr)
+			for (int n0 = 0; n0 < o.n; n0 += tc)
+			{
+				SliceTile t = {};
+				t.out = (int)b;
+				t.m0 = m0;
+				t.n0 = n0;
+				t.halves = (p.orient ? o.n - n0 : o.m - m0) > SLICE_HALF ? 2 : 1;
+				t.split = -1;
+				const i64 S = std::max<i64>(1, std::min<i64>(stages / SLICE_SPLIT, (i64)std::ceil(slice_clocks(t.halves, ksum[b]) / target)));
+				if (S > 1)
+				{
+					GemmSplit g = {};
+					g.out = (int)b;
+					g.m0 = m0;
+					g.n0 = n0;
+					g.rows = std::min(tr, o.m - m0);
+					g.cols = std::min(tc, o.n - n0);
+					g.nsplit = (int)S;
+					g.ld = tc;
+					g.stride = 2 * tr * tc;        // two 64-bit integers per entry
+					g.part = wsz;
+					wsz += S * g.stride;
+					t.split = (int)p.splits.size();
+					p.splits.push_back(g);
+				}
+				for (i64 q = 0; q < S; q++)
+				{
+					t.sp = (int)q;
+					t.u0 = (int)(q * stages / S);
+					t.u1 = (int)((q + 1) * stages / S);
+					p.stiles.push_back(t);
+				}
+			}
+	}
+	std::stable_sort(p.stiles.begin(), p.stiles.end(), [](const SliceTile& x, const SliceTile& y) {
+		return (x.u1 - x.u0) * x.halves > (y.u1 - y.u0) * y.halves;
+	});
+	p.work_doubles = wsz;
+}
+
 }  // namespace
 
 
@@ -115,7 +274,7 @@ CopyLowering rows_lowering(std::shared_ptr<Meta> out, std::vector<RowDesc>&& d, 
 // ------------------------------------------------------------------------------------
 
 DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision, int num_sms,
-                      const int* out_perm, int tc_bn)
+                      const int* out_perm, int tc_bn, bool slices)
 {
 	CTG_CHECK(!is_tc_precision(precision) || tc_bn == 64 || tc_bn == 128 || tc_bn == 256,
 	          "dot: tensor-core tile width must be 64, 128 or 256");
@@ -197,6 +356,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 	geometry(t, nldt, t_lead, t_trail);
 	constexpr int KCH = 16;                      // k chunk of the FP64 kernels
 	std::vector<i64> nchunk((size_t)r.nblocks, 0), ksum((size_t)r.nblocks, 0);
+	std::vector<std::pair<size_t, size_t>> run_at((size_t)r.nblocks);   // first keys of its operands' runs
 	// The output blocks are cut into ranges lowered side by side on the host threads (each range
 	// into its own lists, joined in range order afterwards, so the plan does not depend on the
 	// number of threads); small products stay on the calling thread.
@@ -232,6 +392,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			o.sr1 = o.n;
 			o.c1 = o.n;
 			o.sc0 = 0;
+			o.block = b;
 			o.c0 = (int)R.cons.size();             // range-local until the join
 			i64 fs = 0, ft = 0;
 			for (int i = 0; i < nfs; i++) fs = fs * r.nb[i] + ir[i];
@@ -250,6 +411,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			size_t t1 = t0;
 			while (t1 < kt.size() && kt[t1].f == ft) t1++;
 			CTG_CHECK(s1 - s0 == t1 - t0, "dot: operand block runs differ");
+			run_at[(size_t)b] = {s0, t0};
 			const double mn2 = 2.0 * (double)o.m * (double)o.n;
 			i64 nch = 0;
 			for (size_t x = s0, y = t0; x < s1; x++, y++)
@@ -437,6 +599,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			}
 			GemmOut& o = outs[(size_t)b];
 			o.c_off = outp->boff[bp];
+			o.block = bp;
 			o.r1 = (int)size[1];
 			o.sr0 = stride[0];
 			o.sr1 = stride[1];
@@ -446,6 +609,41 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			CTG_CHECK(o.c_off + (i64)o.m * o.n <= outp->nnz, "dot: transposed output block out of range");
 		}
 		p.out = outp;
+	}
+	if (slices && precision == GEMM_FP64 && use_slices(outs, ksum, tiles, s.nnz + t.nnz, num_sms))
+	{
+		g_plan_stage[1] += host_seconds() - ts0;
+		double clocks[2];
+		p.orient = slice_orient(outs, ksum, clocks);
+		// groups: the operands' runs that an output block with contributions uses
+		std::vector<SliceKey> ka(ks.size()), kb(kt.size());
+		for (size_t i = 0; i < ks.size(); i++) ka[i] = SliceKey{ks[i].f, ks[i].b};
+		for (size_t i = 0; i < kt.size(); i++) kb[i] = SliceKey{kt[i].f, kt[i].b};
+		std::vector<char> ua(ks.size(), 0), ub(kt.size(), 0);
+		for (size_t b = 0; b < outs.size(); b++)
+			if (outs[b].nc > 0) ua[run_at[b].first] = ub[run_at[b].second] = 1;
+		std::vector<int> ga, gb;
+		slice_pack(s, ka, ua, axs == AX_LEADING, s_lead, s_trail, p.orient == 1, p.spack[0], ga);
+		slice_pack(t, kb, ub, axt == AX_LEADING, t_lead, t_trail, p.orient == 0, p.spack[1], gb);
+		p.souts.resize(outs.size());
+		for (size_t b = 0; b < outs.size(); b++)
+		{
+			if (outs[b].nc == 0) continue;
+			const int x = p.orient ? 0 : 1;
+			const int gi[2] = {ga[run_at[b].first], gb[run_at[b].second]};
+			const SliceGroup &gx = p.spack[x].groups[(size_t)gi[x]], &gy = p.spack[1 - x].groups[(size_t)gi[1 - x]];
+			CTG_CHECK(gx.ktot == ksum[b] && gy.ktot == ksum[b] && gx.rows == (x ? outs[b].n : outs[b].m) &&
+			              gy.rows == (x ? outs[b].m : outs[b].n),
+			          "dot: groups of an output block");
+			p.souts[b] = SliceOut{gx.base, gy.base, (gx.rows + 7) / 8, (gy.rows + 31) / 32, gi[x], gi[1 - x]};
+		}
+		slice_tiles(outs, ksum, num_sms, p);
+		p.outs = std::move(outs);
+		p.cons = std::move(cons);
+		p.flops = flops;
+		p.a_entries = s.nnz;
+		p.b_entries = t.nnz;
+		return p;
 	}
 	// Split-K: on GB300 one SM retires about two FP64 FMAs per clock, so a block GEMM with fewer
 	// tiles than SMs leaves most of the FP64 pipes idle. Tiles whose work exceeds a fair share of

@@ -13,12 +13,28 @@
 
 namespace ctg {
 
+// one operand of a product by digit slices
+struct SlicePack {
+	std::vector<SliceRun> runs;
+	std::vector<SliceGroup> groups;
+	std::vector<SliceItem> items;
+	std::vector<SliceChunk> chunks;      // pieces of its blocks, for their exponents
+	i64 bytes = 0;                       // of the packed digits
+	int blocks = 0;
+};
+
 // block_sparse_tensor_dot (block_sparse_tensor.c:1826-2001) as GEMM work lists
 struct DotLowering {
 	std::shared_ptr<Meta> out;
 	std::vector<GemmOut> outs;           // one per output block
 	std::vector<GemmContrib> cons;       // operand block pairs, grouped by output block
 	std::vector<GemmTile> tiles;         // every CTA's tile, all tile classes in one list
+	// FP64 on the tensor cores by digit slices (then `tiles` is empty): tiles, the output blocks' groups,
+	// which operand lies along the MMA rows (SliceTile), and how the operands (A, B) are packed
+	std::vector<SliceTile> stiles;
+	std::vector<SliceOut> souts;
+	int orient = 0;
+	SlicePack spack[2];
 	std::vector<GemmSplit> splits;       // tiles whose sum is split over several CTAs
 	i64 work_doubles = 0;                // partial-sum scratch of the split tiles
 	// tensor-core path: packed operand records and their per-contribution indices
@@ -31,8 +47,10 @@ struct DotLowering {
 // out_perm (optional, r.ndim entries): write the result in the layout of its transpose by out_perm,
 // which must arrange two runs of row axes and two runs of column axes (each run kept in order) with
 // the last column run innermost. tc_bn: column width of the tensor-core tiles (64, 128 or 256).
+// slices (FP64 only): the product may run on the tensor cores by digit slices where the rule in
+// use_slices says that this is faster.
 DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision, int num_sms,
-                      const int* out_perm = nullptr, int tc_bn = 64);
+                      const int* out_perm = nullptr, int tc_bn = 64, bool slices = false);
 
 // data movement: kind 0 block permutation (PermDesc), 1 row map (RowDesc + maps), 2 axis scaling
 // (ScaleDesc + maps)

@@ -31,3 +31,11 @@ def test_block_enumeration_matches_brute_force(tmp_path):
 @pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
 def test_cluster_jacobi_schedule_covers_every_pair_once(tmp_path):
     _build_and_run(tmp_path, "check_schedule", [os.path.join(ROOT, "tests", "host", "check_schedule.cpp")], [])
+
+
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_digit_slices_and_their_tiles(tmp_path):
+    _build_and_run(tmp_path, "check_slices",
+                   [os.path.join(ROOT, "tests", "host", "check_slices.cpp")] +
+                   [os.path.join(CSRC, f) for f in ("ctg_plan.cpp", "ctg_meta.cpp", "ctg_pool.cpp")],
+                   [f"-L{CUDA}/lib64", "-lcudart", "-lpthread"])
