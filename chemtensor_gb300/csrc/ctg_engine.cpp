@@ -1095,7 +1095,7 @@ DTensor view_trace_unit(const DTensor& t)
 // SVD and RQ of block-sparse matrices
 // ------------------------------------------------------------------------------------
 
-int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, double discard_weight)
+int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, double discard_weight, bool steady)
 {
 	const Meta& am = a.m();
 	pend = SvdPending();
@@ -1284,14 +1284,14 @@ int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, do
 		if (groups.size() == 1)
 			launch_svd_group(groups[0].l, groups[0].first, groups[0].count, (const SvdDesc*)desc->ptr, a.data(),
 			                 res.u.data(), (double*)res.s->ptr, res.vh.data(), (double*)scratch.ptr, (int*)status.ptr,
-			                 (double*)tail.ptr, c.stream(), tsp, discard2);
+			                 (double*)tail.ptr, c.stream(), tsp, discard2, steady);
 		else
 		{
 			c.fork(ng);
 			for (size_t g = 0; g < groups.size(); g++)
 				launch_svd_group(groups[g].l, groups[g].first, groups[g].count, (const SvdDesc*)desc->ptr, a.data(),
 				                 res.u.data(), (double*)res.s->ptr, res.vh.data(), (double*)scratch.ptr,
-				                 (int*)status.ptr, (double*)tail.ptr, c.aux((int)g), tsp, discard2);
+				                 (int*)status.ptr, (double*)tail.ptr, c.aux((int)g), tsp, discard2, steady);
 			c.join(ng);
 		}
 	}

@@ -259,9 +259,12 @@ SvdLaunch svd_launch_for(int m, int n, int want, int max_cluster);
 // cluster exchanges to phase_ts[8 block + 4 ..].
 // discard2: the caller discards every singular value whose square is below it (0: none); the
 // refinement of the mixed path then leaves the mutual rotations of those columns out.
+// steady: the basis within (nearly) equal singular values, which is free, has to stay what the fixed
+// five FP32 sweeps from rank 32 on make it: for callers whose later arithmetic rounds coarsely, such
+// as products of split BF16 entries, where another basis shows at 1e-6 of a molecule's energies.
 void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* descs, const double* a, double* u,
                       double* s, double* vh, double* scratch, int* status, double* flops, cudaStream_t st,
-                      unsigned long long* phase_ts = nullptr, double discard2 = 0.0);
+                      unsigned long long* phase_ts = nullptr, double discard2 = 0.0, bool steady = false);
 
 // Householder RQ of a row-major m x n block: A = R Q with Q (k x n) orthonormal rows, R (m x k), k = min(m, n).
 // Scratch holds n*m + n*k + k doubles per block.

@@ -44,10 +44,23 @@ constexpr int SVD_THREADS = 256;
 constexpr int NWARPS = SVD_THREADS / 32;
 constexpr int SVD_STEP_PAIRS = 32;            // most column pairs of one inner step (group size <= 32)
 constexpr int SVD_SMEM_LIMIT = 220 * 1024;    // dynamic shared memory per CTA (227 KB less static use)
-constexpr int SVD_F32_SWEEPS = 5;             // default: most FP32 preconditioning sweeps
+constexpr int SVD_F32_SWEEPS = 5;             // default: FP32 preconditioning sweeps before the angles are asked
+constexpr int SVD_F32_MORE = 3;               // most further FP32 sweeps while pairs still turn by a wide angle
 constexpr int SVD_F32_SWEEPS_MAX = 8;         // capacity of the FP32 sweep flags
+// Default: cosine and tangent of the angle above which a rotation asks for a further FP32 sweep. An
+// FP32 sweep of a block of 100 to 190 columns costs ~75 us, a pass of the FP64 finish that starts too
+// far away ~0.7 ms; the angles shrink quadratically, so after a sweep without an angle above 1e-2 the
+// next would leave ~1e-4, which the finish takes in its own first pass. Ground-state searches, ms
+// (two states each; blocks of up to 190 | up to 90 columns): five sweeps 320, 315 | 74.7, 74.6; six
+// always 285, 285 | 76.9, 76.1; while above 1e-4 297, 290 | 78.6, 76.6; above 1e-2 288, 286 | 74.1,
+// 75.0; above 5e-2 299, 299 | 73.6, 74.4; above 0.2 314, 315 | 72.3, 74.6. Starting to ask after
+// four sweeps instead of five: within 2 % either way.
+constexpr float SVD_F32_WIDE = 0.01f;
 constexpr float SVD_F32_COS = 0.0f;           // default: FP32 sweeps rotate every pair above N eps_32
-constexpr int SVD_F32_MIN_RANK = 32;          // default: smallest rank preconditioned in FP32
+// Default: smallest rank preconditioned in FP32. A spin chain at bond dimension 32 (ranks up to 32):
+// 104.9 ms from rank 32 on, 101.2 from 20, 99.1 from 16, 99.0 from 12 and 98.9 from 8 on.
+constexpr int SVD_F32_MIN_RANK = 16;
+constexpr int SVD_F32_MIN_STEADY = 32;        // the same where the caller wants the basis steady
 constexpr int SVD_F32_CLUSTER = 8;            // default: CTAs of the FP32 sweeps
 constexpr int SVD_OUT_RC = 32;                // reflectors staged per round of the output phase
 
@@ -491,8 +504,10 @@ __device__ __forceinline__ float warp_sumf(float v)
 // pairs: inner product (every lane gets the sum), classical Jacobi rotation (tan theta the
 // smaller root of t^2 + 2 zeta t - 1 = 0, computed by every lane), rotation of the two records.
 // One CTA barrier per step.
+// local_rot[0]: a pair was rotated; local_rot[1]: a pair whose cosine and tangent of the angle both
+// lay above `wide`, one of its squared norms above tail2.
 __device__ void jacobi_step32(const Tour32& t, int buf, int mode, int step, int cA, int cB, int npad, float tol2,
-                              int* local_rot)
+                              int* local_rot, float wide, float tail2)
 {
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int np = mode == 0 ? npad : t.bs;
@@ -561,7 +576,8 @@ __device__ void jacobi_step32(const Tour32& t, int buf, int mode, int step, int 
 			{
 				*pa = fmaf(-tn, g, al);
 				*pb = fmaf(tn, g, be);
-				*local_rot = 1;
+				local_rot[0] = 1;
+				if (fabsf(tn) > wide && g * g > wide * wide * al * be && fmaxf(al, be) > tail2) local_rot[1] = 1;
 			}
 		}
 	}
@@ -877,9 +893,13 @@ __device__ int qr_pivoted_cluster(cg::cluster_group& cluster, double* smem, cons
 // cluster (a tour over 2 cf groups; the others only keep the cluster barriers in step): their
 // cost is latency and barriers, not arithmetic, and fewer, larger groups need fewer rounds. On
 // return, V (r x r, orthogonal to FP32 accuracy, column g at xs.V + g r) is in global memory.
+// At most nsw sweeps, and up to SVD_F32_MORE further ones while the last of them still rotated a pair
+// by a wide angle (SVD_F32_WIDE; not counted where both columns lie in the tail that the caller
+// discards). Every CTA reads the same flags after the same barrier, so all take the same decision.
 __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, double* smem, const SvdScratch& xs, int M,
-                                 int cf, int rank, int nsw, float cos_min, long long* cyc)
+                                 int cf, int rank, int nsw, float cos_min, float wide, float tail2, long long* cyc)
 {
+	const int last = min(nsw + SVD_F32_MORE, SVD_F32_SWEEPS_MAX);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const long long c0 = cyc ? clock64() : 0;
 	const int N = t.N, r = t.r;
@@ -914,8 +934,8 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 		}
 		__syncthreads();
 		const float tol2 = fmaxf((float)N * FLT_EPSILON * (float)N * FLT_EPSILON, cos_min * cos_min);
-		int buf = 0, done32 = nsw;
-		for (int sweep = 0; sweep < nsw; sweep++)
+		int buf = 0, done32 = 0;
+		for (int sweep = 0; sweep < last; sweep++)
 		{
 			round_groups(0, rank, f.nm, A, B);
 			for (int slot = 0; slot < 2; slot++)
@@ -942,7 +962,7 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 					if (lane == 0) f.nrm(buf, slot)[c] = acc;
 				}
 			}
-			if (tid == 0) *local_rot = 0;
+			if (tid == 0) local_rot[0] = local_rot[1] = 0;
 			__syncthreads();
 			for (int rho = 0; rho < f.nm; rho++)
 			{
@@ -951,13 +971,13 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 				if (rho == 0)
 				{
 					const int npad = f.bs + (f.bs & 1);
-					for (int st = 0; st < npad - 1; st++) jacobi_step32(f, buf, 0, st, cA, cB, npad, tol2, local_rot);
+					for (int st = 0; st < npad - 1; st++) jacobi_step32(f, buf, 0, st, cA, cB, npad, tol2, local_rot, wide, tail2);
 				}
-				for (int st = 0; st < f.bs; st++) jacobi_step32(f, buf, 1, st, cA, cB, 0, tol2, local_rot);
+				for (int st = 0; st < f.bs; st++) jacobi_step32(f, buf, 1, st, cA, cB, 0, tol2, local_rot, wide, tail2);
 				if (cf > 1)
 				{
 					const long long cx = cyc ? clock64() : 0;
-					if (tid == 0 && rho == f.nm - 1 && *local_rot) atomicOr(xs.flags32 + sweep, 1);
+					if (tid == 0 && rho == f.nm - 1 && local_rot[0]) atomicOr(xs.flags32 + sweep, local_rot[1] ? 3 : 1);
 					const int rho1 = (rho + 1) % f.nm;
 					for (int slot = 0; slot < 2; slot++)
 					{
@@ -976,18 +996,15 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 					if (cyc) cyc[10] += clock64() - cx;
 				}
 			}
-			bool conv;
-			if (cf > 1) conv = __ldcg(xs.flags32 + sweep) == 0;
+			int rot;
+			if (cf > 1) rot = __ldcg(xs.flags32 + sweep);
 			else
 			{
-				conv = *local_rot == 0;
+				rot = local_rot[0] | 2 * local_rot[1];
 				__syncthreads();
 			}
-			if (conv)
-			{
-				done32 = sweep + 1;
-				break;
-			}
+			done32 = sweep + 1;
+			if (rot == 0 || (done32 >= nsw && !(rot & 2))) break;
 		}
 		if (cyc) cyc[2] += done32;
 		// V (FP32) to global memory, column g at V + g r
@@ -1006,10 +1023,11 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 	else if (cf > 1)
 	{
 		// the barriers of the working CTAs' rounds, and their convergence decision
-		for (int sweep = 0; sweep < nsw; sweep++)
+		for (int sweep = 0; sweep < last; sweep++)
 		{
 			for (int rho = 0; rho < f.nm; rho++) cluster.sync();
-			if (__ldcg(xs.flags32 + sweep) == 0) break;
+			const int rot = __ldcg(xs.flags32 + sweep);
+			if (rot == 0 || (sweep + 1 >= nsw && !(rot & 2))) break;
 		}
 	}
 	cluster.sync();
@@ -1763,7 +1781,7 @@ __global__ void __launch_bounds__(SVD_THREADS, 1)
 k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restrict__ a, double* __restrict__ u,
            double* __restrict__ s, double* __restrict__ vh, double* __restrict__ scratch, int* __restrict__ status,
            double* __restrict__ flops, int cl, int smem_bytes, unsigned long long* __restrict__ phase_ts, int f32_min,
-           int f32_cl, int refine, double tail2, int f32_sweeps, float f32_cos)
+           int f32_cl, int refine, double tail2, int f32_sweeps, float f32_cos, float f32_wide)
 {
 	extern __shared__ __align__(16) double smem[];
 	cg::cluster_group cluster = cg::this_cluster();
@@ -1858,8 +1876,8 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	int rf_iters = 0;
 	if (mixed)
 	{
-		precondition_f32(cluster, t, smem, xs, M, cf, rank, f32_sweeps, f32_cos, cyc);
 		const double us = __ldcg(xs.misc + 2);
+		precondition_f32(cluster, t, smem, xs, M, cf, rank, f32_sweeps, f32_cos, f32_wide, (float)(tail2 / (us * us)), cyc);
 		refined = finish_mixed(cluster, t, smem, xs, M, cl, rank, refine != 0, (float)(tail2 / (us * us)), jflops, cyc,
 		                       rf_iters);
 	}
@@ -2460,7 +2478,7 @@ static int svd_f32_cluster()
 	return v;
 }
 
-// most FP32 preconditioning sweeps (CTGPU_SVD_F32_SWEEPS overrides, 1 to SVD_F32_SWEEPS_MAX)
+// FP32 preconditioning sweeps before the angles are asked (CTGPU_SVD_F32_SWEEPS overrides, 1 to SVD_F32_SWEEPS_MAX)
 static int svd_f32_sweeps()
 {
 	static const int v = [] {
@@ -2478,6 +2496,17 @@ static float svd_f32_cos()
 	static const float v = [] {
 		const char* e = getenv("CTGPU_SVD_F32_COS");
 		return e ? (float)atof(e) : SVD_F32_COS;
+	}();
+	return v;
+}
+
+// cosine and tangent above which a rotation of an FP32 sweep asks for a further one
+// (CTGPU_SVD_F32_WIDE overrides; default SVD_F32_WIDE)
+static float svd_f32_wide()
+{
+	static const float v = [] {
+		const char* e = getenv("CTGPU_SVD_F32_WIDE");
+		return e ? (float)atof(e) : SVD_F32_WIDE;
 	}();
 	return v;
 }
@@ -2571,7 +2600,7 @@ SvdLaunch svd_launch_for(int m, int n, int want, int max_cluster)
 
 void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* descs, const double* a, double* u,
                       double* s, double* vh, double* scratch, int* status, double* flops, cudaStream_t st,
-                      unsigned long long* phase_ts, double discard2)
+                      unsigned long long* phase_ts, double discard2, bool steady)
 {
 	if (count <= 0) return;
 	cudaLaunchConfig_t cfg = {};
@@ -2591,6 +2620,8 @@ void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* d
 		CTG_CUDA(cudaLaunchKernelEx(&cfg, k_svd_global, descs, first, a, u, s, vh, scratch, status, 0.0, flops, g.cluster));
 		return;
 	}
+	// the steady form's threshold lies above the default one, so the launch's shared memory holds it too
+	const int f32_min = steady && svd_f32_min() > 0 ? std::max(svd_f32_min(), SVD_F32_MIN_STEADY) : svd_f32_min();
 	static std::once_flag attr_once[64];
 	int dev = 0;
 	CTG_CUDA(cudaGetDevice(&dev));
@@ -2600,8 +2631,8 @@ void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* d
 			CTG_CUDA(cudaFuncSetAttribute(k_svd_tour, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
 		});
 	CTG_CUDA(cudaLaunchKernelEx(&cfg, k_svd_tour, descs, first, a, u, s, vh, scratch, status, flops, g.cluster, g.smem,
-	                             phase_ts, svd_f32_min(), svd_f32_cluster(), svd_refine(), discard2, svd_f32_sweeps(),
-	                             svd_f32_cos()));
+	                             phase_ts, f32_min, svd_f32_cluster(), svd_refine(), discard2, svd_f32_sweeps(),
+	                             svd_f32_cos(), steady ? FLT_MAX : svd_f32_wide()));
 }
 
 }  // namespace ctg
