@@ -429,7 +429,7 @@ static int tuned_tile_width(Ctx& c, const Meta& s, int axs, const Meta& t, int a
 static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision,
                               const int* out_perm)
 {
-	// complex128: the FP64 work lists (outputs, contributions) with tiles of the complex GEMM
+	// complex128: the FP64 lists and tiles, over complex entries
 	const bool z = precision == GEMM_Z64;
 	if (is_tc_precision(precision))
 	{
@@ -448,17 +448,6 @@ static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int
 
 static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 {
-	const bool z = precision == GEMM_Z64;
-	std::vector<ZTile> zt;
-	if (z)
-	{
-		for (size_t b = 0; b < l.outs.size(); b++)
-			for (int m0 = 0; m0 < l.outs[b].m; m0 += 32)
-				for (int n0 = 0; n0 < l.outs[b].n; n0 += 32) zt.push_back(ZTile{(int)b, m0, n0, 0});
-		l.tiles.clear();
-		l.splits.clear();
-		l.work_doubles = 0;
-	}
 	DotPlan p;
 	p.out = l.out;
 	p.precision = precision;
@@ -470,7 +459,7 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 	const size_t o_tiles = pk.add(l.tiles);
 	const size_t o_splits = pk.add(l.splits);
 	const size_t o_tcons = pk.add(l.tcons), o_apacks = pk.add(l.apacks), o_bpacks = pk.add(l.bpacks);
-	const size_t o_zt = pk.add(zt), o_st = pk.add(l.stiles);
+	const size_t o_st = pk.add(l.stiles);
 	const size_t o_so = pk.add(l.souts);
 	size_t o_side[2][4] = {};
 	for (int q = 0; q < 2 && !l.stiles.empty(); q++)
@@ -483,7 +472,6 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 	// at least 16 bytes, from the packer's own storage (a product without output blocks packs nothing)
 	if (pk.bytes.size() < 16) pk.bytes.resize(16);
 	p.desc = c.upload(pk.bytes.data(), pk.bytes.size());
-	p.nztiles = (int)zt.size();
 	p.nstiles = (int)l.stiles.size();
 	p.stiles = at<SliceTile>(p.desc, o_st);
 	p.souts = at<SliceOut>(p.desc, o_so);
@@ -502,7 +490,6 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 		d.bytes = l.spack[q].bytes;
 	}
 	p.c_blocks = l.out->nblocks;
-	p.ztiles = at<ZTile>(p.desc, o_zt);
 	p.tcons = at<TcContrib>(p.desc, o_tcons);
 	p.apacks = at<TcPack>(p.desc, o_apacks);
 	p.bpacks = at<TcPack>(p.desc, o_bpacks);
@@ -512,7 +499,8 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 	p.cons = at<GemmContrib>(p.desc, o_cons);
 	p.splits = at<GemmSplit>(p.desc, o_splits);
 	p.nsplits = (int)l.splits.size();
-	if (l.work_doubles > 0) p.work = std::make_shared<DBuf>(&c, (size_t)l.work_doubles * sizeof(double));
+	const size_t entry = precision == GEMM_Z64 ? 2 * sizeof(double) : sizeof(double);
+	if (l.work_doubles > 0) p.work = std::make_shared<DBuf>(&c, (size_t)l.work_doubles * entry);
 	if (!l.splits.empty())
 	{
 		// completion counters of the split tiles: zero now, and reset by the kernel after each use
@@ -603,7 +591,8 @@ void DotPlan::run_z(Ctx& c, const double* A, const double* B, double* C, bool co
 {
 	CTG_CHECK(precision == GEMM_Z64, "complex GEMM on a real plan");
 	KScope ks(c, K_GEMM, 1, 4.0 * flops, 0);
-	launch_gemm_z(nztiles, ztiles, outs, cons, A, B, C, conj_a ? 1 : 0, conj_b ? 1 : 0, c.stream());
+	launch_gemm_z(ntiles[0], tiles[0], outs, cons, splits, counters ? (int*)counters->ptr : nullptr, A, B, C,
+	              work ? (double*)work->ptr : nullptr, conj_a, conj_b, c.stream(), 4.0 * flops);
 	c.gemm_flops += 4.0 * flops;
 }
 
@@ -991,8 +980,6 @@ DTensor op_dot(Ctx& c, const DTensor& s, int axs, const DTensor& t, int axt, int
 		CTG_CHECK(s.cplx && t.cplx, "dot: real and complex operands");
 		DotPlan p = make_dot_plan(c, s.m(), axs, t.m(), axt, nmult, GEMM_Z64);
 		DTensor r = c.empty(p.out, true);
-		if (p.out->nnz > 0)
-			CTG_CUDA(cudaMemsetAsync(r.data(), 0, (size_t)p.out->nnz * 2 * sizeof(double), c.stream()));
 		p.run_z(c, s.data(), t.data(), r.data(), s.conj, t.conj);
 		return r;
 	}

@@ -193,9 +193,6 @@ struct DotPlan {
 	double flops = 0;
 	double flops_cls[NUM_TILE_CLASSES] = {};
 	int precision = GEMM_FP64;
-	// complex128 (precision GEMM_Z64): tiles of the complex GEMM
-	int nztiles = 0;
-	const ZTile* ztiles = nullptr;
 	void run(Ctx& c, const double* A, const double* B, double* C) const;
 	// the FP64 product's launches alone (no counters)
 	void launch_f64(Ctx& c, const double* A, const double* B, double* C) const;

@@ -9,34 +9,55 @@ namespace ctg {
 // ------------------------------------------------------------------------------------
 
 constexpr int GEMM_THREADS = 256;     // 16 x 16 thread grid for every tile class
-constexpr int GEMM_SMEM_DOUBLES = 16 * (128 + 1 + 8 + 1);
+constexpr int GEMM_SMEM_ENTRIES = 16 * (128 + 1 + 8 + 1);
 constexpr int GEMM_DIRECT_K = 4;      // contributions up to this k skip the shared-memory staging
 
-template <int BM, int BN, int BK, int TM, int TN>
-__device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOut* __restrict__ outs,
-                                              const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits,
-                                              int* __restrict__ counters, const double* __restrict__ A,
-                                              const double* __restrict__ B, double* __restrict__ C,
-                                              double* __restrict__ work, double* sm)
+// entry arithmetic of the tiles: T = double, or double2 for complex128. `flip` has the sign bit set
+// where the operand is conjugated.
+__device__ __forceinline__ double gemm_entry(double x, unsigned) { return x; }
+__device__ __forceinline__ double2 gemm_entry(double2 x, unsigned flip)
+{
+	return make_double2(x.x, __hiloint2double(__double2hiint(x.y) ^ (int)flip, __double2loint(x.y)));
+}
+__device__ __forceinline__ void gemm_mac(double& c, double a, double b) { c = fma(a, b, c); }
+__device__ __forceinline__ void gemm_mac(double2& c, double2 a, double2 b)
+{
+	c.x = fma(a.x, b.x, c.x);
+	c.y = fma(a.x, b.y, c.y);
+	c.x = fma(-a.y, b.y, c.x);
+	c.y = fma(a.y, b.x, c.y);
+}
+__device__ __forceinline__ void gemm_add(double& c, double x) { c += x; }
+__device__ __forceinline__ void gemm_add(double2& c, double2 x)
+{
+	c.x += x.x;
+	c.y += x.y;
+}
+
+template <class T, int BM, int BN, int BK, int TM, int TN>
+__device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* __restrict__ outs,
+                                          const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits,
+                                          int* __restrict__ counters, const T* __restrict__ A, const T* __restrict__ B,
+                                          T* __restrict__ C, T* __restrict__ work, T* sm, unsigned fa, unsigned fb)
 {
 	constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
-	static_assert(NT == GEMM_THREADS && BK * (BM + 1 + BN + 1) <= GEMM_SMEM_DOUBLES, "tile class layout");
-	double (*As)[BM + 1] = reinterpret_cast<double (*)[BM + 1]>(sm);
-	double (*Bs)[BN + 1] = reinterpret_cast<double (*)[BN + 1]>(sm + BK * (BM + 1));
+	static_assert(NT == GEMM_THREADS && BK * (BM + 1 + BN + 1) <= GEMM_SMEM_ENTRIES, "tile class layout");
+	T (*As)[BM + 1] = reinterpret_cast<T (*)[BM + 1]>(sm);
+	T (*Bs)[BN + 1] = reinterpret_cast<T (*)[BN + 1]>(sm + BK * (BM + 1));
 	const GemmOut o = outs[tile.out];
 	const int tid = threadIdx.x;
 	const int tx = tid % NTX, ty = tid / NTX;
-	double acc[TM][TN];
+	T acc[TM][TN];
 #pragma unroll
 	for (int i = 0; i < TM; i++)
 #pragma unroll
-		for (int j = 0; j < TN; j++) acc[i][j] = 0.0;
+		for (int j = 0; j < TN; j++) acc[i][j] = T();
 
 	for (int c = tile.c0; c <= tile.c1; c++)
 	{
 		const GemmContrib g = cons[c];
-		const double* a = A + g.a_off;
-		const double* b = B + g.b_off;
+		const T* a = A + g.a_off;
+		const T* b = B + g.b_off;
 		const int kb = (c == tile.c0 ? tile.k0 : 0), ke = (c == tile.c1 ? tile.k1 : g.k);
 		if (ke - kb <= GEMM_DIRECT_K)
 		{
@@ -46,23 +67,23 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 #pragma unroll 1
 			for (int kk = kb; kk < ke; kk++)
 			{
-				double av[TM], bv[TN];
+				T av[TM], bv[TN];
 #pragma unroll
 				for (int i = 0; i < TM; i++)
 				{
 					const int gi = tile.m0 + ty + i * NTY;
-					av[i] = gi < o.m ? a[(i64)gi * g.sAm + (i64)kk * g.sAk] : 0.0;
+					av[i] = gi < o.m ? gemm_entry(a[(i64)gi * g.sAm + (i64)kk * g.sAk], fa) : T();
 				}
 #pragma unroll
 				for (int j = 0; j < TN; j++)
 				{
 					const int gj = tile.n0 + tx + j * NTX;
-					bv[j] = gj < o.n ? b[(i64)kk * g.sBk + (i64)gj * g.sBn] : 0.0;
+					bv[j] = gj < o.n ? gemm_entry(b[(i64)kk * g.sBk + (i64)gj * g.sBn], fb) : T();
 				}
 #pragma unroll
 				for (int i = 0; i < TM; i++)
 #pragma unroll
-					for (int j = 0; j < TN; j++) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+					for (int j = 0; j < TN; j++) gemm_mac(acc[i][j], av[i], bv[j]);
 			}
 			continue;
 		}
@@ -75,7 +96,7 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 				{
 					const int kk = e % BK, i = e / BK;
 					const int gi = tile.m0 + i, gk = k0 + kk;
-					As[kk][i] = (gi < o.m && gk < ke) ? a[(i64)gi * g.sAm + gk] : 0.0;
+					As[kk][i] = (gi < o.m && gk < ke) ? gemm_entry(a[(i64)gi * g.sAm + gk], fa) : T();
 				}
 			}
 			else
@@ -84,7 +105,7 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 				{
 					const int i = e % BM, kk = e / BM;
 					const int gi = tile.m0 + i, gk = k0 + kk;
-					As[kk][i] = (gi < o.m && gk < ke) ? a[(i64)gi * g.sAm + (i64)gk * g.sAk] : 0.0;
+					As[kk][i] = (gi < o.m && gk < ke) ? gemm_entry(a[(i64)gi * g.sAm + (i64)gk * g.sAk], fa) : T();
 				}
 			}
 			// B tile: BK x BN
@@ -94,7 +115,7 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 				{
 					const int j = e % BN, kk = e / BN;
 					const int gj = tile.n0 + j, gk = k0 + kk;
-					Bs[kk][j] = (gj < o.n && gk < ke) ? b[(i64)gk * g.sBk + gj] : 0.0;
+					Bs[kk][j] = (gj < o.n && gk < ke) ? gemm_entry(b[(i64)gk * g.sBk + gj], fb) : T();
 				}
 			}
 			else
@@ -103,14 +124,14 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 				{
 					const int kk = e % BK, j = e / BK;
 					const int gj = tile.n0 + j, gk = k0 + kk;
-					Bs[kk][j] = (gj < o.n && gk < ke) ? b[(i64)gk * g.sBk + (i64)gj * g.sBn] : 0.0;
+					Bs[kk][j] = (gj < o.n && gk < ke) ? gemm_entry(b[(i64)gk * g.sBk + (i64)gj * g.sBn], fb) : T();
 				}
 			}
 			__syncthreads();
 			const int kmax = min(BK, ke - k0);
 			for (int kk = 0; kk < kmax; kk++)
 			{
-				double av[TM], bv[TN];
+				T av[TM], bv[TN];
 #pragma unroll
 				for (int i = 0; i < TM; i++) av[i] = As[kk][ty + i * NTY];
 #pragma unroll
@@ -118,7 +139,7 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 #pragma unroll
 				for (int i = 0; i < TM; i++)
 #pragma unroll
-					for (int j = 0; j < TN; j++) acc[i][j] = fma(av[i], bv[j], acc[i][j]);
+					for (int j = 0; j < TN; j++) gemm_mac(acc[i][j], av[i], bv[j]);
 			}
 			__syncthreads();
 		}
@@ -128,7 +149,7 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 		// partial sum of a split tile (full BM x BN, leading dimension BN); the CTA that completes
 		// the split last adds the partial sums in share order (deterministic) and writes C
 		const GemmSplit sp = splits[tile.split];
-		double* w = work + sp.part + (i64)tile.sp * sp.stride;
+		T* w = work + sp.part + (i64)tile.sp * sp.stride;
 #pragma unroll
 		for (int i = 0; i < TM; i++)
 #pragma unroll
@@ -143,9 +164,9 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 		for (int e = tid; e < sp.rows * sp.cols; e += NT)
 		{
 			const int i = e / sp.cols, j = e - i * sp.cols;
-			const double* pw = work + sp.part + (i64)i * sp.ld + j;
-			double sum = 0.0;
-			for (int q = 0; q < sp.nsplit; q++) sum += __ldcg(pw + (i64)q * sp.stride);
+			const T* pw = work + sp.part + (i64)i * sp.ld + j;
+			T sum = T();
+			for (int q = 0; q < sp.nsplit; q++) gemm_add(sum, __ldcg(pw + (i64)q * sp.stride));
 			C[gemm_out_index(o, sp.m0 + i, sp.n0 + j)] = sum;
 		}
 		if (tid == 0) counters[tile.split] = 0;
@@ -165,6 +186,28 @@ __device__ __forceinline__ void gemm_tile_f64(const GemmTile& tile, const GemmOu
 	}
 }
 
+template <class T>
+__device__ __forceinline__ void gemm_any_tile(const GemmTile& tile, const GemmOut* __restrict__ outs,
+                                              const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits,
+                                              int* __restrict__ counters, const T* __restrict__ A, const T* __restrict__ B,
+                                              T* __restrict__ C, T* __restrict__ work, T* sm, unsigned fa, unsigned fb)
+{
+	switch (tile.cls)
+	{
+	case TILE_L: gemm_tile<T, 64, 64, 16, 4, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_M: gemm_tile<T, 32, 32, 16, 2, 2>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_W: gemm_tile<T, 16, 64, 16, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_T: gemm_tile<T, 64, 16, 16, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_R8: gemm_tile<T, 8, 32, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_R4: gemm_tile<T, 4, 64, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_C8: gemm_tile<T, 32, 8, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_C4: gemm_tile<T, 64, 4, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_W8: gemm_tile<T, 8, 128, 16, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_T8: gemm_tile<T, 128, 8, 16, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	default:     gemm_tile<T, 16, 16, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	}
+}
+
 __global__ void __launch_bounds__(GEMM_THREADS, 3)
 k_gemm_f64(const GemmTile* __restrict__ tiles, const GemmOut* __restrict__ outs, const GemmContrib* __restrict__ cons,
            const GemmSplit* __restrict__ splits, int* __restrict__ counters, const double* __restrict__ A,
@@ -172,22 +215,25 @@ k_gemm_f64(const GemmTile* __restrict__ tiles, const GemmOut* __restrict__ outs,
 {
 	pdl_wait();
 	pdl_trigger();
-	__shared__ double sm[GEMM_SMEM_DOUBLES];
-	const GemmTile tile = tiles[blockIdx.x];
-	switch (tile.cls)
-	{
-	case TILE_L: gemm_tile_f64<64, 64, 16, 4, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_M: gemm_tile_f64<32, 32, 16, 2, 2>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_W: gemm_tile_f64<16, 64, 16, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_T: gemm_tile_f64<64, 16, 16, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_R8: gemm_tile_f64<8, 32, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_R4: gemm_tile_f64<4, 64, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_C8: gemm_tile_f64<32, 8, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_C4: gemm_tile_f64<64, 4, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_W8: gemm_tile_f64<8, 128, 16, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	case TILE_T8: gemm_tile_f64<128, 8, 16, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	default:     gemm_tile_f64<16, 16, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm); break;
-	}
+	__shared__ double sm[GEMM_SMEM_ENTRIES];
+	gemm_any_tile(tiles[blockIdx.x], outs, cons, splits, counters, A, B, C, work, sm, 0u, 0u);
+}
+
+// complex128: the tiles, split shares and lists of the real product, four FMAs per pair of entries.
+// Bound by the FP64 pipe on large blocks and by latency on small ones (tens of blocks of 1 to 60 rows).
+// A tile of its own, 32 x 32 with all contributions on one CTA, left most SMs idle and spent six FP64
+// instructions per pair: 164 us per product of a Hubbard chain at bond dimension 64 (628 products,
+// 103 ms), 20 us with the work lists' narrow tiles and split shares (12.7 ms). Two blocks per SM: the
+// 4 x 4 complex accumulators and operands of TILE_L need 128 registers.
+__global__ void __launch_bounds__(GEMM_THREADS, 2)
+k_gemm_z(const GemmTile* __restrict__ tiles, const GemmOut* __restrict__ outs, const GemmContrib* __restrict__ cons,
+         const GemmSplit* __restrict__ splits, int* __restrict__ counters, const double2* __restrict__ A,
+         const double2* __restrict__ B, double2* __restrict__ C, double2* __restrict__ work, unsigned flip_a, unsigned flip_b)
+{
+	pdl_wait();
+	pdl_trigger();
+	__shared__ double2 sm[GEMM_SMEM_ENTRIES];
+	gemm_any_tile(tiles[blockIdx.x], outs, cons, splits, counters, A, B, C, work, sm, flip_a, flip_b);
 }
 
 int tile_rows(int cls)
@@ -211,6 +257,19 @@ void launch_gemm_f64(int ntiles, const GemmTile* tiles, const GemmOut* outs, con
 	const cudaLaunchConfig_t cfg = launch_config(dim3(ntiles), dim3(GEMM_THREADS), 0, st);
 	if (flops < 2e8) launch_pdl(cfg, k_gemm_f64, tiles, outs, cons, splits, counters, A, B, C, work);
 	else CTG_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_f64, tiles, outs, cons, splits, counters, A, B, C, work));
+}
+
+void launch_gemm_z(int ntiles, const GemmTile* tiles, const GemmOut* outs, const GemmContrib* cons,
+                   const GemmSplit* splits, int* counters, const double* A, const double* B, double* C, double* work,
+                   bool conj_a, bool conj_b, cudaStream_t st, double flops)
+{
+	if (ntiles <= 0) return;
+	const cudaLaunchConfig_t cfg = launch_config(dim3(ntiles), dim3(GEMM_THREADS), 0, st);
+	const double2 *a = (const double2*)A, *b = (const double2*)B;
+	double2 *o = (double2*)C, *w = (double2*)work;
+	const unsigned fa = conj_a ? 0x80000000u : 0u, fb = conj_b ? 0x80000000u : 0u;
+	if (flops < 2e8) launch_pdl(cfg, k_gemm_z, tiles, outs, cons, splits, counters, a, b, o, w, fa, fb);
+	else CTG_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_z, tiles, outs, cons, splits, counters, a, b, o, w, fa, fb));
 }
 
 // ------------------------------------------------------------------------------------

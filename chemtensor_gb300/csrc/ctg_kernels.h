@@ -277,14 +277,11 @@ void launch_rq_householder(int nblocks, const RqDesc* descs, const double* a, do
                            cudaStream_t st);
 
 // ---- complex128 (interleaved real / imaginary parts, element offsets and strides) -------
-// Tiles of the complex block GEMM: 32 x 32 of output block `out`, all of its contributions.
-struct ZTile {
-	int out, m0, n0, pad;
-};
-// C = sum op(A) op(B) over the same GemmOut / GemmContrib lists as the FP64 GEMM; conj_a / conj_b
-// conjugate the operand's entries as they are read.
-void launch_gemm_z(int ntiles, const ZTile* tiles, const GemmOut* outs, const GemmContrib* cons, const double* A,
-                   const double* B, double* C, int conj_a, int conj_b, cudaStream_t st);
+// C = sum op(A) op(B) over the FP64 GEMM's lists (work: complex entries); conj_a / conj_b conjugate the
+// operand's entries as they are read (the conjugated bra of the environment updates, chain_ops.c:116-245).
+void launch_gemm_z(int ntiles, const GemmTile* tiles, const GemmOut* outs, const GemmContrib* cons,
+                   const GemmSplit* splits, int* counters, const double* A, const double* B, double* C, double* work,
+                   bool conj_a, bool conj_b, cudaStream_t st, double flops);
 // complex SVD of each block (SvdDesc offsets in complex elements, s_off in doubles, w_off in
 // complex elements of scratch); status[b] = 1 if block b did not converge
 i64 svd_z_scratch(int m, int n);
