@@ -1162,8 +1162,9 @@ int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, do
 		pend.zstatus = std::make_shared<DBuf>(&c, zd.size() * sizeof(int));
 		pend.zblocks = (int)zd.size();
 		KScope ks(c, K_SVD, 1);
-		launch_svd_z((int)zd.size(), (const SvdDesc*)desc->ptr, a.data(), res.u.data(), (double*)res.s->ptr,
-		             res.vh.data(), (double*)scratch.ptr, (int*)pend.zstatus->ptr, c.stream());
+		launch_svd_z((int)zd.size(), (const SvdDesc*)desc->ptr, zd.data(), a.data(), res.u.data(), (double*)res.s->ptr,
+		             res.vh.data(), (double*)scratch.ptr, (int*)pend.zstatus->ptr, discard2, svd_max_cluster(c.device()),
+		             c.stream());
 		return 0;
 	}
 	std::vector<SvdDesc> descs;

@@ -283,10 +283,11 @@ void launch_gemm_z(int ntiles, const GemmTile* tiles, const GemmOut* outs, const
                    const GemmSplit* splits, int* counters, const double* A, const double* B, double* C, double* work,
                    bool conj_a, bool conj_b, cudaStream_t st, double flops);
 // complex SVD of each block (SvdDesc offsets in complex elements, s_off in doubles, w_off in
-// complex elements of scratch); status[b] = 1 if block b did not converge
+// complex elements of scratch); status[b] = 1 if block b did not converge. host: the descriptors in
+// host memory; discard2 as for launch_svd_group; max_cluster: largest cluster the device schedules.
 i64 svd_z_scratch(int m, int n);
-void launch_svd_z(int nblocks, const SvdDesc* descs, const double* a, double* u, double* s, double* vh, double* work,
-                  int* status, cudaStream_t st);
+void launch_svd_z(int nblocks, const SvdDesc* descs, const SvdDesc* host, const double* a, double* u, double* s, double* vh,
+                  double* work, int* status, double discard2, int max_cluster, cudaStream_t st);
 // complex QR / RQ of each block (RqDesc offsets in complex elements; scratch of
 // m n + max(m, n) min(m, n) + min(m, n) complex elements per block)
 void launch_qr_z(int nblocks, const RqDesc* descs, const double* a, double* r, double* q, double* scratch, cudaStream_t st);
