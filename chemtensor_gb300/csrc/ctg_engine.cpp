@@ -556,7 +556,7 @@ void DotPlan::launch_f64(Ctx& c, const double* A, const double* B, double* C) co
 		run_slices(c, A, B, pa.ptr, pb.ptr, C, nullptr);
 	}
 	else if (ntiles[0] > 0)
-		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops);
+		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops, flops_cls[TILE_L] > 0);
 }
 
 // the groups' exponents in front of the digits, which start on a 256-byte boundary

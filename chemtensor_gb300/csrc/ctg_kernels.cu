@@ -9,8 +9,118 @@ namespace ctg {
 // ------------------------------------------------------------------------------------
 
 constexpr int GEMM_THREADS = 256;     // 16 x 16 thread grid for every tile class
-constexpr int GEMM_SMEM_ENTRIES = 16 * (128 + 1 + 8 + 1);
-constexpr int GEMM_DIRECT_K = 4;      // contributions up to this k skip the shared-memory staging
+constexpr int GEMM_BK = 16;           // terms per stage
+constexpr int GEMM_TERMS = 64;        // terms whose operand positions are tabulated at a time
+constexpr int GEMM_RING = 2 * GEMM_BK * (128 + 1 + 8 + 1);      // entries of the ring of stages, real product
+constexpr int GEMM_RING_Z = GEMM_BK * (128 + 1 + 8 + 1);        // complex entries
+
+// The sum of a tile runs over its contributions and each one's inner index. GEMM_TERMS consecutive terms of
+// that one list are tabulated: where the term's column of A and row of B lie.
+struct GemmTerms {
+	i64 a[GEMM_TERMS], b[GEMM_TERMS];
+	int sa[GEMM_TERMS], sb[GEMM_TERMS];
+	int start[GEMM_TERMS];            // first term of the contributions, scratch of the tabulation
+	GemmContrib con[GEMM_TERMS];
+	int half;                         // terms of the first 32 contributions
+	int count, next_c, next_k;        // terms tabulated; where the list goes on
+	int a_by_k, b_by_k;               // consecutive terms are consecutive entries
+};
+
+// The next (at most GEMM_TERMS) terms from contribution c, inner index k on. All threads call it; the first
+// 64 take a contribution each, add up the terms before theirs and look up their own term's contribution.
+__device__ __forceinline__ void gemm_terms(GemmTerms& w, const GemmTile& tile, const GemmContrib* __restrict__ cons, int c, int k)
+{
+	const int tid = threadIdx.x, lane = tid & 31;
+	if (c == tile.c1)
+	{
+		// the last (mostly the only) contribution: its terms follow one another, nothing to add up or look up
+		const GemmContrib g = cons[c];
+		if (tid < GEMM_TERMS)
+		{
+			w.a[tid] = g.a_off + (i64)(k + tid) * g.sAk;
+			w.b[tid] = g.b_off + (i64)(k + tid) * g.sBk;
+			w.sa[tid] = g.sAm;
+			w.sb[tid] = g.sBn;
+		}
+		if (tid == 0)
+		{
+			const bool whole = tile.k1 - k <= GEMM_TERMS;
+			w.count = whole ? tile.k1 - k : GEMM_TERMS;
+			w.next_c = whole ? c + 1 : c;
+			w.next_k = k + GEMM_TERMS;
+			w.a_by_k = g.sAk == 1 && g.sAm != 1;
+			w.b_by_k = g.sBk == 1 && g.sBn != 1;
+		}
+		__syncthreads();
+		return;
+	}
+	int n = 0, incl = 0;
+	if (tid < GEMM_TERMS)
+	{
+		if (c + tid <= tile.c1)
+		{
+			const GemmContrib g = cons[c + tid];
+			w.con[tid] = g;
+			n = (c + tid == tile.c1 ? tile.k1 : g.k) - (tid == 0 ? k : 0);
+		}
+		incl = n;
+#pragma unroll
+		for (int o = 1; o < 32; o <<= 1)
+		{
+			const int v = __shfl_up_sync(0xffffffffu, incl, o);
+			if (lane >= o) incl += v;
+		}
+		if (tid == 31) w.half = incl;
+	}
+	__syncthreads();
+	if (tid < GEMM_TERMS)
+	{
+		if (tid >= 32) incl += w.half;
+		const int first = incl - n;
+		w.start[tid] = first;
+		// the contribution with the table's last term, or the last one of all
+		if (n > 0 && first < GEMM_TERMS && (incl >= GEMM_TERMS || c + tid == tile.c1))
+		{
+			const bool whole = incl <= GEMM_TERMS;
+			w.count = whole ? incl : GEMM_TERMS;
+			w.next_c = whole ? c + tid + 1 : c + tid;
+			w.next_k = whole ? 0 : GEMM_TERMS - first + (tid == 0 ? k : 0);
+		}
+		if (tid == 0)
+		{
+			if (c > tile.c1) w.count = 0;
+			w.a_by_k = n > 0 && w.con[0].sAk == 1 && w.con[0].sAm != 1;
+			w.b_by_k = n > 0 && w.con[0].sBk == 1 && w.con[0].sBn != 1;
+		}
+	}
+	__syncthreads();
+	if (tid < w.count)
+	{
+		int j = 0;
+#pragma unroll
+		for (int step = GEMM_TERMS / 2; step > 0; step >>= 1)
+			if (w.start[j + step] <= tid) j += step;
+		const GemmContrib g = w.con[j];
+		const int kk = tid - w.start[j] + (j == 0 ? k : 0);
+		w.a[tid] = g.a_off + (i64)kk * g.sAk;
+		w.b[tid] = g.b_off + (i64)kk * g.sBk;
+		w.sa[tid] = g.sAm;
+		w.sb[tid] = g.sBn;
+	}
+	__syncthreads();
+}
+
+__device__ __forceinline__ void gemm_copy(double* dst, const double* src)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void gemm_copy(double2* dst, const double2* src)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void gemm_copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void gemm_copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 // entry arithmetic of the tiles: T = double, or double2 for complex128. `flip` has the sign bit set
 // where the operand is conjugated.
@@ -34,16 +144,16 @@ __device__ __forceinline__ void gemm_add(double2& c, double2 x)
 	c.y += x.y;
 }
 
-template <class T, int BM, int BN, int BK, int TM, int TN>
+template <class T, int RING, int BM, int BN, int TM, int TN>
 __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* __restrict__ outs,
                                           const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits,
                                           int* __restrict__ counters, const T* __restrict__ A, const T* __restrict__ B,
-                                          T* __restrict__ C, T* __restrict__ work, T* sm, unsigned fa, unsigned fb)
+                                          T* __restrict__ C, T* __restrict__ work, T* sm, GemmTerms& w, unsigned fa, unsigned fb)
 {
-	constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
-	static_assert(NT == GEMM_THREADS && BK * (BM + 1 + BN + 1) <= GEMM_SMEM_ENTRIES, "tile class layout");
-	T (*As)[BM + 1] = reinterpret_cast<T (*)[BM + 1]>(sm);
-	T (*Bs)[BN + 1] = reinterpret_cast<T (*)[BN + 1]>(sm + BK * (BM + 1));
+	constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY, BK = GEMM_BK;
+	constexpr int STAGE = BK * (BM + 1 + BN + 1);
+	constexpr int NST = RING / STAGE < GEMM_TERMS / BK ? RING / STAGE : GEMM_TERMS / BK;      // stages in flight
+	static_assert(NT == GEMM_THREADS && NST >= 1, "tile class layout");
 	const GemmOut o = outs[tile.out];
 	const int tid = threadIdx.x;
 	const int tx = tid % NTX, ty = tid / NTX;
@@ -53,107 +163,85 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 #pragma unroll
 		for (int j = 0; j < TN; j++) acc[i][j] = T();
 
-	for (int c = tile.c0; c <= tile.c1; c++)
-	{
-		const GemmContrib g = cons[c];
-		const T* a = A + g.a_off;
-		const T* b = B + g.b_off;
-		const int kb = (c == tile.c0 ? tile.k0 : 0), ke = (c == tile.c1 ? tile.k1 : g.k);
-		if (ke - kb <= GEMM_DIRECT_K)
+	// rows and columns beyond the block and terms beyond the table stay unset: what they give is not stored
+	auto load = [&](int st) {
+		T* as = sm + (st % NST) * STAGE;
+		T* bs = as + BK * (BM + 1);
+		const int k0 = st * BK;
+#pragma unroll
+		for (int e = tid; e < BM * BK; e += NT)
 		{
-			// short contraction (most contributions of a block-sparse DMRG contraction have k <= 2):
-			// operands straight from global memory through L1, no staging and no barrier. Same
-			// accumulation order as the staged path.
-#pragma unroll 1
-			for (int kk = kb; kk < ke; kk++)
-			{
-				T av[TM], bv[TN];
-#pragma unroll
-				for (int i = 0; i < TM; i++)
-				{
-					const int gi = tile.m0 + ty + i * NTY;
-					av[i] = gi < o.m ? gemm_entry(a[(i64)gi * g.sAm + (i64)kk * g.sAk], fa) : T();
-				}
-#pragma unroll
-				for (int j = 0; j < TN; j++)
-				{
-					const int gj = tile.n0 + tx + j * NTX;
-					bv[j] = gj < o.n ? gemm_entry(b[(i64)kk * g.sBk + (i64)gj * g.sBn], fb) : T();
-				}
-#pragma unroll
-				for (int i = 0; i < TM; i++)
-#pragma unroll
-					for (int j = 0; j < TN; j++) gemm_mac(acc[i][j], av[i], bv[j]);
-			}
-			continue;
+			const int kk = w.a_by_k ? e % BK : e / BM, i = w.a_by_k ? e / BK : e % BM;
+			if (k0 + kk < w.count && tile.m0 + i < o.m)
+				gemm_copy(as + kk * (BM + 1) + i, A + w.a[k0 + kk] + (i64)(tile.m0 + i) * w.sa[k0 + kk]);
 		}
-		for (int k0 = kb; k0 < ke; k0 += BK)
+#pragma unroll
+		for (int e = tid; e < BN * BK; e += NT)
 		{
-			// A tile: BM x BK; the thread-to-element map follows the unit-stride index
-			if (g.sAk == 1)
-			{
-				for (int e = tid; e < BM * BK; e += NT)
-				{
-					const int kk = e % BK, i = e / BK;
-					const int gi = tile.m0 + i, gk = k0 + kk;
-					As[kk][i] = (gi < o.m && gk < ke) ? gemm_entry(a[(i64)gi * g.sAm + gk], fa) : T();
-				}
-			}
-			else
-			{
-				for (int e = tid; e < BM * BK; e += NT)
-				{
-					const int i = e % BM, kk = e / BM;
-					const int gi = tile.m0 + i, gk = k0 + kk;
-					As[kk][i] = (gi < o.m && gk < ke) ? gemm_entry(a[(i64)gi * g.sAm + (i64)gk * g.sAk], fa) : T();
-				}
-			}
-			// B tile: BK x BN
-			if (g.sBn == 1)
-			{
-				for (int e = tid; e < BK * BN; e += NT)
-				{
-					const int j = e % BN, kk = e / BN;
-					const int gj = tile.n0 + j, gk = k0 + kk;
-					Bs[kk][j] = (gj < o.n && gk < ke) ? gemm_entry(b[(i64)gk * g.sBk + gj], fb) : T();
-				}
-			}
-			else
-			{
-				for (int e = tid; e < BK * BN; e += NT)
-				{
-					const int kk = e % BK, j = e / BK;
-					const int gj = tile.n0 + j, gk = k0 + kk;
-					Bs[kk][j] = (gj < o.n && gk < ke) ? gemm_entry(b[(i64)gk * g.sBk + (i64)gj * g.sBn], fb) : T();
-				}
-			}
+			const int kk = w.b_by_k ? e % BK : e / BN, j = w.b_by_k ? e / BK : e % BN;
+			if (k0 + kk < w.count && tile.n0 + j < o.n)
+				gemm_copy(bs + kk * (BN + 1) + j, B + w.b[k0 + kk] + (i64)(tile.n0 + j) * w.sb[k0 + kk]);
+		}
+	};
+	bool first = true;
+	for (int c = tile.c0, k = tile.k0; first || c <= tile.c1;)
+	{
+		gemm_terms(w, tile, cons, c, k);
+		// the lists belong to the plan: the operands are the first access that has to wait for the kernel before
+		if (first)
+		{
+			pdl_wait();
+			pdl_trigger();
+			first = false;
+		}
+		const int count = w.count, nst = (count + BK - 1) / BK;
+		if (count == 0) break;
+#pragma unroll
+		for (int st = 0; st < NST; st++)
+		{
+			if (st < nst) load(st);
+			gemm_copy_commit();
+		}
+		for (int st = 0; st < nst; st++)
+		{
+			gemm_copy_wait<NST - 1>();
 			__syncthreads();
-			const int kmax = min(BK, ke - k0);
+			const T* as = sm + (st % NST) * STAGE;
+			const T* bs = as + BK * (BM + 1);
+			const int kmax = min(BK, count - st * BK);
 			for (int kk = 0; kk < kmax; kk++)
 			{
 				T av[TM], bv[TN];
 #pragma unroll
-				for (int i = 0; i < TM; i++) av[i] = As[kk][ty + i * NTY];
+				for (int i = 0; i < TM; i++) av[i] = gemm_entry(as[kk * (BM + 1) + ty + i * NTY], fa);
 #pragma unroll
-				for (int j = 0; j < TN; j++) bv[j] = Bs[kk][tx + j * NTX];
+				for (int j = 0; j < TN; j++) bv[j] = gemm_entry(bs[kk * (BN + 1) + tx + j * NTX], fb);
 #pragma unroll
 				for (int i = 0; i < TM; i++)
 #pragma unroll
 					for (int j = 0; j < TN; j++) gemm_mac(acc[i][j], av[i], bv[j]);
 			}
-			__syncthreads();
+			if (st + NST < nst)
+			{
+				__syncthreads();
+				load(st + NST);
+			}
+			gemm_copy_commit();
 		}
+		c = w.next_c;
+		k = w.next_k;
+		__syncthreads();                  // the table and the ring are free again
 	}
 	if (tile.split >= 0)
 	{
 		// partial sum of a split tile (full BM x BN, leading dimension BN); the CTA that completes
 		// the split last adds the partial sums in share order (deterministic) and writes C
 		const GemmSplit sp = splits[tile.split];
-		T* w = work + sp.part + (i64)tile.sp * sp.stride;
+		T* part = work + sp.part + (i64)tile.sp * sp.stride;
 #pragma unroll
 		for (int i = 0; i < TM; i++)
 #pragma unroll
-			for (int j = 0; j < TN; j++) w[(ty + i * NTY) * BN + tx + j * NTX] = acc[i][j];
+			for (int j = 0; j < TN; j++) part[(ty + i * NTY) * BN + tx + j * NTX] = acc[i][j];
 		__threadfence();
 		__syncthreads();
 		__shared__ int last;
@@ -166,6 +254,7 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 			const int i = e / sp.cols, j = e - i * sp.cols;
 			const T* pw = work + sp.part + (i64)i * sp.ld + j;
 			T sum = T();
+#pragma unroll 4
 			for (int q = 0; q < sp.nsplit; q++) gemm_add(sum, __ldcg(pw + (i64)q * sp.stride));
 			C[gemm_out_index(o, sp.m0 + i, sp.n0 + j)] = sum;
 		}
@@ -186,37 +275,56 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 	}
 }
 
-template <class T>
+template <class T, int RING, bool LARGE>
 __device__ __forceinline__ void gemm_any_tile(const GemmTile& tile, const GemmOut* __restrict__ outs,
                                               const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits,
                                               int* __restrict__ counters, const T* __restrict__ A, const T* __restrict__ B,
-                                              T* __restrict__ C, T* __restrict__ work, T* sm, unsigned fa, unsigned fb)
+                                              T* __restrict__ C, T* __restrict__ work, unsigned fa, unsigned fb)
 {
+	__shared__ T sm[RING];
+	__shared__ GemmTerms w;
+	if (LARGE && tile.cls == TILE_L)
+	{
+		gemm_tile<T, RING, 64, 64, 4, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb);
+		return;
+	}
 	switch (tile.cls)
 	{
-	case TILE_L: gemm_tile<T, 64, 64, 16, 4, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_M: gemm_tile<T, 32, 32, 16, 2, 2>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_W: gemm_tile<T, 16, 64, 16, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_T: gemm_tile<T, 64, 16, 16, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_R8: gemm_tile<T, 8, 32, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_R4: gemm_tile<T, 4, 64, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_C8: gemm_tile<T, 32, 8, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_C4: gemm_tile<T, 64, 4, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_W8: gemm_tile<T, 8, 128, 16, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	case TILE_T8: gemm_tile<T, 128, 8, 16, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
-	default:     gemm_tile<T, 16, 16, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, fa, fb); break;
+	case TILE_M: gemm_tile<T, RING, 32, 32, 2, 2>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_W: gemm_tile<T, RING, 16, 64, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_T: gemm_tile<T, RING, 64, 16, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_R8: gemm_tile<T, RING, 8, 32, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_R4: gemm_tile<T, RING, 4, 64, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_C8: gemm_tile<T, RING, 32, 8, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_C4: gemm_tile<T, RING, 64, 4, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_W8: gemm_tile<T, RING, 8, 128, 1, 4>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	case TILE_T8: gemm_tile<T, RING, 128, 8, 4, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
+	default: gemm_tile<T, RING, 16, 16, 1, 1>(tile, outs, cons, splits, counters, A, B, C, work, sm, w, fa, fb); break;
 	}
 }
 
-__global__ void __launch_bounds__(GEMM_THREADS, 3)
+// Bound by the FP64 pipe where the blocks are large, by latency where they are small: a tile's chain is tile,
+// contributions, operands, FMAs, result, and only the last two use the pipe. So
+//   - the lists are read before the wait on the kernel before (they belong to the plan);
+//   - up to 64 terms are one flat list over all contributions, staged by asynchronous copies with up to four
+//     stages in flight: short contributions (k of 1 to 20) share stages and latency. Staging each
+//     contribution by itself, every load exposed, took as long per contribution as now per tile;
+//   - tiles come longest first and split shares are small (see lower_dot): the SMs' FP64 times of one product
+//     had differed by 29 to 81 percent of its duration.
+// Clock stamps in a product of 891 tiles of one to thirteen terms: 2100 cycles to the table, 1050 to the
+// operands, 3500 of FMAs (five blocks on the SM), 700 to the result. Four blocks per SM for LARGE = false:
+// 94.0 ms of a spin-chain search and 69.8 of a Hubbard one (D = 100) against 95.4 and 71.4 with five, 94.8
+// and 72.8 with six and a ring of half the size.
+// Before and after, all of it: Hubbard L = 32, D = 256 search 286 -> 269 ms, D = 100 74.0 -> 69.8, spin chain
+// L = 20, D = 32 98.5 -> 94.0, one-site Hubbard D = 256 69.3 -> 68.1.
+// LARGE: the product has TILE_L tiles.
+template <bool LARGE>
+__global__ void __launch_bounds__(GEMM_THREADS, LARGE ? 3 : 4)
 k_gemm_f64(const GemmTile* __restrict__ tiles, const GemmOut* __restrict__ outs, const GemmContrib* __restrict__ cons,
            const GemmSplit* __restrict__ splits, int* __restrict__ counters, const double* __restrict__ A,
            const double* __restrict__ B, double* __restrict__ C, double* __restrict__ work)
 {
-	pdl_wait();
-	pdl_trigger();
-	__shared__ double sm[GEMM_SMEM_ENTRIES];
-	gemm_any_tile(tiles[blockIdx.x], outs, cons, splits, counters, A, B, C, work, sm, 0u, 0u);
+	gemm_any_tile<double, GEMM_RING, LARGE>(tiles[blockIdx.x], outs, cons, splits, counters, A, B, C, work, 0u, 0u);
 }
 
 // complex128: the tiles, split shares and lists of the real product, four FMAs per pair of entries.
@@ -230,10 +338,7 @@ k_gemm_z(const GemmTile* __restrict__ tiles, const GemmOut* __restrict__ outs, c
          const GemmSplit* __restrict__ splits, int* __restrict__ counters, const double2* __restrict__ A,
          const double2* __restrict__ B, double2* __restrict__ C, double2* __restrict__ work, unsigned flip_a, unsigned flip_b)
 {
-	pdl_wait();
-	pdl_trigger();
-	__shared__ double2 sm[GEMM_SMEM_ENTRIES];
-	gemm_any_tile(tiles[blockIdx.x], outs, cons, splits, counters, A, B, C, work, sm, flip_a, flip_b);
+	gemm_any_tile<double2, GEMM_RING_Z, true>(tiles[blockIdx.x], outs, cons, splits, counters, A, B, C, work, flip_a, flip_b);
 }
 
 int tile_rows(int cls)
@@ -248,15 +353,16 @@ int tile_cols(int cls)
 
 void launch_gemm_f64(int ntiles, const GemmTile* tiles, const GemmOut* outs, const GemmContrib* cons,
                      const GemmSplit* splits, int* counters, const double* A, const double* B, double* C, double* work,
-                     cudaStream_t st, double flops)
+                     cudaStream_t st, double flops, bool large)
 {
 	if (ntiles <= 0) return;
 	// programmatic dependent launch for the short products of a sweep (tens of microseconds); a
 	// product of milliseconds gains nothing from it and lost 2 % with it (the next kernel's blocks
 	// scheduled beside its last waves)
 	const cudaLaunchConfig_t cfg = launch_config(dim3(ntiles), dim3(GEMM_THREADS), 0, st);
-	if (flops < 2e8) launch_pdl(cfg, k_gemm_f64, tiles, outs, cons, splits, counters, A, B, C, work);
-	else CTG_CUDA(cudaLaunchKernelEx(&cfg, k_gemm_f64, tiles, outs, cons, splits, counters, A, B, C, work));
+	const auto kernel = large ? k_gemm_f64<true> : k_gemm_f64<false>;
+	if (flops < 2e8) launch_pdl(cfg, kernel, tiles, outs, cons, splits, counters, A, B, C, work);
+	else CTG_CUDA(cudaLaunchKernelEx(&cfg, kernel, tiles, outs, cons, splits, counters, A, B, C, work));
 }
 
 void launch_gemm_z(int ntiles, const GemmTile* tiles, const GemmOut* outs, const GemmContrib* cons,

@@ -73,10 +73,11 @@ int tile_rows(int cls);
 int tile_cols(int cls);
 
 // every tile of every class in one launch (256 threads per CTA, the tile's class picks its shape);
-// split tiles use `counters` (one per GemmSplit, zero before the launch and again after it)
+// split tiles use `counters` (one per GemmSplit, zero before the launch and again after it). large: the
+// list has TILE_L tiles.
 void launch_gemm_f64(int ntiles, const GemmTile* tiles, const GemmOut* outs, const GemmContrib* cons,
                      const GemmSplit* splits, int* counters, const double* A, const double* B, double* C, double* work,
-                     cudaStream_t st, double flops = 0.0);
+                     cudaStream_t st, double flops = 0.0, bool large = true);
 
 // The same sums on the tensor cores by exact digit slices (ctg_gemm_slices.cu): FP64 operands and
 // results, each result rounded once. One operand of the product (x) lies along the 128 rows of the MMA

@@ -355,7 +355,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 	geometry(s, nlds, s_lead, s_trail);
 	geometry(t, nldt, t_lead, t_trail);
 	constexpr int KCH = 16;                      // k chunk of the FP64 kernels
-	std::vector<i64> nchunk((size_t)r.nblocks, 0), ksum((size_t)r.nblocks, 0);
+	std::vector<i64> ksum((size_t)r.nblocks, 0);
 	std::vector<std::pair<size_t, size_t>> run_at((size_t)r.nblocks);   // first keys of its operands' runs
 	// The output blocks are cut into ranges lowered side by side on the host threads (each range
 	// into its own lists, joined in range order afterwards, so the plan does not depend on the
@@ -413,7 +413,6 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			CTG_CHECK(s1 - s0 == t1 - t0, "dot: operand block runs differ");
 			run_at[(size_t)b] = {s0, t0};
 			const double mn2 = 2.0 * (double)o.m * (double)o.n;
-			i64 nch = 0;
 			for (size_t x = s0, y = t0; x < s1; x++, y++)
 			{
 				CTG_CHECK(ks[x].c == kt[y].c, "dot: missing partner block");
@@ -439,9 +438,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 				if (is_tc_precision(precision)) R.con_blocks.emplace_back(bs, bt);
 				R.flops += mn2 * (double)k;
 				ksum[(size_t)b] += k;
-				nch += (k + KCH - 1) / KCH;
 			}
-			nchunk[(size_t)b] = nch;
 			o.nc = (int)R.cons.size() - o.c0;
 			CTG_CHECK(o.m >= 1 && o.n >= 1 && o.c_off + (i64)o.m * o.n <= r.nnz, "dot: output block out of range");
 		}
@@ -647,7 +644,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 	}
 	// Split-K: on GB300 one SM retires about two FP64 FMAs per clock, so a block GEMM with fewer
 	// tiles than SMs leaves most of the FP64 pipes idle. Tiles whose work exceeds a fair share of
-	// the whole product are cut into shares of consecutive 16-wide k chunks, one CTA each; their
+	// the whole product are cut into shares of consecutive chunks of 16 terms, one CTA each; their
 	// partial sums are added in a fixed order (deterministic) by the CTA that completes the split last.
 	g_plan_stage[1] += host_seconds() - ts0;
 	ts0 = host_seconds();
@@ -658,8 +655,11 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 		double total = 0;
 		for (int k = 0; k < NUM_TILE_CLASSES; k++)
 			for (const GemmTile& t : tiles[k])
-				total += (double)TILE_ROWS[k] * TILE_COLS[k] * (double)(nchunk[(size_t)t.out] * KCH);
-		const double target = std::max(total / (2.0 * num_sms), 16384.0);
+				total += (double)TILE_ROWS[k] * TILE_COLS[k] * (double)ksum[(size_t)t.out];
+		// shares of an eighth of an SM's part, at least 16 terms of a 16 x 16 tile (2048 clocks of the FP64
+		// pipe). With half of a part and 64 terms: Hubbard L = 32, D = 256 272.1 ms (269.6 with these), D = 100
+		// 71.9 (69.8), spin chain D = 32 94.9 (94.0), one-site Hubbard D = 256 69.2 (68.1).
+		const double target = std::max(total / (8.0 * num_sms), 4096.0);
 		std::vector<std::pair<int, int>> pos;
 		for (int k = 0; k < NUM_TILE_CLASSES; k++)
 		{
@@ -668,25 +668,33 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			for (const GemmTile& t : tiles[k])
 			{
 				const GemmOut& o = outs[(size_t)t.out];
-				const i64 n = nchunk[(size_t)t.out];
-				const double w = (double)tr * tc * (double)(n * KCH);
+				const i64 n = (ksum[(size_t)t.out] + KCH - 1) / KCH;
+				const double w = (double)tr * tc * (double)ksum[(size_t)t.out];
 				const int S = (int)std::min<double>((double)n, std::ceil(w / target));
 				if (S <= 1)
 				{
 					kept.push_back(t);
 					continue;
 				}
+				// first term of every chunk, and the end
 				pos.clear();
-				for (int cc = o.c0; cc < o.c0 + o.nc; cc++)
-					for (int kk = 0; kk < cons[(size_t)cc].k; kk += KCH) pos.emplace_back(cc, kk);
+				i64 at = 0;
+				for (int cc = o.c0; cc < o.c0 + o.nc; at += cons[(size_t)cc++].k)
+					while ((i64)pos.size() * KCH < at + cons[(size_t)cc].k) pos.emplace_back(cc, (int)((i64)pos.size() * KCH - at));
+				pos.emplace_back(o.c0 + o.nc - 1, cons[(size_t)(o.c0 + o.nc - 1)].k);
 				for (int sp = 0; sp < S; sp++)
 				{
 					const i64 a = sp * n / S, e = (sp + 1) * n / S;
 					GemmTile u = t;
 					u.c0 = pos[(size_t)a].first;
 					u.k0 = pos[(size_t)a].second;
-					u.c1 = pos[(size_t)e - 1].first;
-					u.k1 = std::min(pos[(size_t)e - 1].second + KCH, cons[(size_t)u.c1].k);
+					u.c1 = pos[(size_t)e].first;
+					u.k1 = pos[(size_t)e].second;
+					if (u.k1 == 0)                       // the chunk starts a contribution: up to the end of the one before
+					{
+						u.c1--;
+						u.k1 = cons[(size_t)u.c1].k;
+					}
 					u.split = (int)splits.size();
 					u.sp = sp;
 					kept.push_back(u);
@@ -760,6 +768,35 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 	for (int k = 0; k < NUM_TILE_CLASSES; k++) ntiles += tiles[k].size();
 	p.tiles.reserve(ntiles);
 	for (int k = 0; k < NUM_TILE_CLASSES; k++) p.tiles.insert(p.tiles.end(), tiles[k].begin(), tiles[k].end());
+	if (!is_tc_precision(precision))
+	{
+		// Longest first, by steps of an eighth of a binary order of magnitude: the blocks that start together
+		// are spread evenly over the SMs, and the short ones fill up behind them. In the order of the
+		// classes: Hubbard L = 32, D = 256 286.8 ms, longest first 272.5.
+		auto weight = [&](const GemmTile& t) {
+			i64 terms = ksum[(size_t)t.out];
+			if (t.split >= 0)
+			{
+				terms = (i64)t.k1 - t.k0;
+				for (int c = t.c0; c < t.c1; c++) terms += cons[(size_t)c].k;
+			}
+			const unsigned long long v = (unsigned long long)(terms * TILE_ROWS[t.cls] * TILE_COLS[t.cls]) * 8 + 8;
+			const int e = 63 - __builtin_clzll(v);
+			return e * 8 + (int)((v >> (e - 3)) & 7);
+		};
+		constexpr int STEPS = 64 * 8;
+		std::vector<unsigned short> w(p.tiles.size());
+		int at[STEPS + 1] = {};
+		for (size_t q = 0; q < w.size(); q++)
+		{
+			w[q] = (unsigned short)(STEPS - 1 - weight(p.tiles[q]));
+			at[w[q] + 1]++;
+		}
+		for (int q = 1; q <= STEPS; q++) at[q] += at[q - 1];
+		std::vector<GemmTile> sorted(p.tiles.size());
+		for (size_t q = 0; q < w.size(); q++) sorted[(size_t)at[w[q]]++] = p.tiles[q];
+		p.tiles.swap(sorted);
+	}
 	if (is_tc_precision(precision) && !p.tiles.empty())
 	{
 		// the persistent tensor-core kernel takes tiles in list order, one per CTA at a time: tiles
