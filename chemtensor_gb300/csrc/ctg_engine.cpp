@@ -1466,11 +1466,8 @@ int op_rq(Ctx& c, const DTensor& a, DTensor& r, DTensor& q)
 	DBufPtr desc = c.upload(descs.data(), descs.size() * sizeof(RqDesc));
 	DBuf scratch(&c, (size_t)std::max<i64>(woff, 1) * a.width() * sizeof(double));
 	KScope ks(c, K_RQ, 1);
-	if (a.cplx)
-		launch_qr_z((int)descs.size(), (const RqDesc*)desc->ptr, a.data(), r.data(), q.data(), (double*)scratch.ptr, c.stream());
-	else
-		launch_rq_householder((int)descs.size(), (const RqDesc*)desc->ptr, a.data(), r.data(), q.data(), (double*)scratch.ptr,
-		                      c.stream());
+	launch_qr((int)descs.size(), (const RqDesc*)desc->ptr, descs.data(), a.data(), r.data(), q.data(), (double*)scratch.ptr, a.cplx,
+	          c.stream());
 	return 0;
 }
 
@@ -1540,11 +1537,8 @@ int op_qr(Ctx& c, const DTensor& a, DTensor& q, DTensor& r)
 	DBufPtr desc = c.upload(descs.data(), descs.size() * sizeof(RqDesc));
 	DBuf scratch(&c, (size_t)std::max<i64>(woff, 1) * a.width() * sizeof(double));
 	KScope ks(c, K_RQ, 1);
-	if (a.cplx)
-		launch_qr_z((int)descs.size(), (const RqDesc*)desc->ptr, a.data(), r.data(), q.data(), (double*)scratch.ptr, c.stream());
-	else
-		launch_rq_householder((int)descs.size(), (const RqDesc*)desc->ptr, a.data(), r.data(), q.data(), (double*)scratch.ptr,
-		                      c.stream());
+	launch_qr((int)descs.size(), (const RqDesc*)desc->ptr, descs.data(), a.data(), r.data(), q.data(), (double*)scratch.ptr, a.cplx,
+	          c.stream());
 	return 0;
 }
 

@@ -267,15 +267,15 @@ void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* d
                       double* s, double* vh, double* scratch, int* status, double* flops, cudaStream_t st,
                       unsigned long long* phase_ts = nullptr, double discard2 = 0.0, bool steady = false);
 
-// Householder RQ of a row-major m x n block: A = R Q with Q (k x n) orthonormal rows, R (m x k), k = min(m, n).
-// Scratch holds n*m + n*k + k doubles per block.
+// Householder QR or RQ of a row-major m x n block: A = Q R or A = R Q, k = min(m, n). Offsets in entries.
 struct RqDesc {
-	i64 a_off, r_off, q_off, w_off;   // w_off: scratch of m n + max(m, n) min(m, n) + min(m, n) doubles
+	i64 a_off, r_off, q_off, w_off;   // w_off: scratch of m n + max(m, n) min(m, n) + min(m, n) entries
 	int m, n;
 	int qr;                           // 1: A = Q R (dgeqrf convention), 0: A = R Q (dgerqf convention)
 };
-void launch_rq_householder(int nblocks, const RqDesc* descs, const double* a, double* r, double* q, double* scratch,
-                           cudaStream_t st);
+// host: the descriptors in host memory
+void launch_qr(int nblocks, const RqDesc* descs, const RqDesc* host, const double* a, double* r, double* q, double* scratch,
+               bool cplx, cudaStream_t st);
 
 // ---- complex128 (interleaved real / imaginary parts, element offsets and strides) -------
 // C = sum op(A) op(B) over the FP64 GEMM's lists (work: complex entries); conj_a / conj_b conjugate the
@@ -289,9 +289,6 @@ void launch_gemm_z(int ntiles, const GemmTile* tiles, const GemmOut* outs, const
 i64 svd_z_scratch(int m, int n);
 void launch_svd_z(int nblocks, const SvdDesc* descs, const SvdDesc* host, const double* a, double* u, double* s, double* vh,
                   double* work, int* status, double discard2, int max_cluster, cudaStream_t st);
-// complex QR / RQ of each block (RqDesc offsets in complex elements; scratch of
-// m n + max(m, n) min(m, n) + min(m, n) complex elements per block)
-void launch_qr_z(int nblocks, const RqDesc* descs, const double* a, double* r, double* q, double* scratch, cudaStream_t st);
 
 // ---- Lanczos (krylov.c:24-89) ------------------------------------------------------
 // Device-resident scalars of one Lanczos run.

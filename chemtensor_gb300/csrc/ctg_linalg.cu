@@ -1,6 +1,5 @@
-// ctg_linalg.cu - FP64 dense linear algebra on the device: per-block SVD
-// (one-sided Jacobi), per-block RQ (Householder) and the Lanczos vector
-// operations with deterministic warp-shuffle reductions.
+// ctg_linalg.cu - the Lanczos vector operations in FP64 on the device, with deterministic warp-shuffle
+// reductions.
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -22,154 +21,6 @@ __device__ __forceinline__ double warp_sum(double v)
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
 	return v;
-}
-
-// ------------------------------------------------------------------------------------
-// block QR / RQ by Householder reflections, one CTA per block.
-// QR (desc.qr = 1) follows LAPACK dgeqrf + dorgqr in dense_tensor_qr_fill (dense_tensor.c:2253-2651):
-// A = Q R, R upper triangular with diagonal entries -sign(alpha) * |x| of the reflectors.
-// RQ (desc.qr = 0) follows dgerqf + dorgrq in dense_tensor_rq_fill (dense_tensor.c:2680-2880):
-// dgerqf eliminates the rows of A from the last one upwards, each towards its trailing column; that
-// is the QR above applied to W = J A^T J (J reverses an index), with A = (J R_W^T J) (J Q_W^T J).
-// Both run the same column-Householder loop on a column-major work matrix W (p x s).
-// ------------------------------------------------------------------------------------
-
-constexpr int RQ_THREADS = 256;
-
-__device__ double block_sum(double v, double* red)
-{
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	v = warp_sum(v);
-	__syncthreads();
-	if (lane == 0) red[warp] = v;
-	__syncthreads();
-	double t = 0;
-	for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
-	return t;
-}
-
-__global__ void __launch_bounds__(RQ_THREADS)
-k_rq_householder(const RqDesc* __restrict__ descs, const double* __restrict__ a, double* __restrict__ r,
-                 double* __restrict__ q, double* __restrict__ scratch)
-{
-	__shared__ double red[RQ_THREADS / 32];
-	__shared__ double sh_beta, sh_tau, sh_scale;
-	const RqDesc d = descs[blockIdx.x];
-	const int m = d.m, n = d.n;
-	const bool qr = d.qr != 0;
-	const int k = min(m, n);
-	const int p = qr ? m : n, s = qr ? n : m;   // W is p x s, column-major
-	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = RQ_THREADS / 32;
-	double* B = scratch + d.w_off;             // W, p x s
-	double* Q = B + (i64)p * s;                // Q_W, p x k
-	double* tau = Q + (i64)p * k;              // k
-	const double* ab = a + d.a_off;
-	for (i64 e = tid; e < (i64)p * s; e += RQ_THREADS)
-	{
-		const i64 i = e % p, j = e / p;
-		B[e] = qr ? ab[i * n + j] : ab[(m - 1 - j) * n + (n - 1 - i)];
-	}
-	__syncthreads();
-	for (int c = 0; c < k; c++)
-	{
-		double* bc = B + (i64)c * p;
-		double part = 0;
-		for (int i = c + 1 + tid; i < p; i += RQ_THREADS) part = fma(bc[i], bc[i], part);
-		const double xnorm2 = block_sum(part, red);
-		if (tid == 0)
-		{
-			const double alpha = bc[c];
-			if (xnorm2 == 0.0)
-			{
-				sh_tau = 0.0;
-				sh_beta = alpha;
-				sh_scale = 0.0;
-			}
-			else
-			{
-				const double beta = -copysign(sqrt(alpha * alpha + xnorm2), alpha);
-				sh_tau = (beta - alpha) / beta;
-				sh_beta = beta;
-				sh_scale = 1.0 / (alpha - beta);
-			}
-		}
-		__syncthreads();
-		const double tc = sh_tau;
-		for (int i = c + 1 + tid; i < p; i += RQ_THREADS) bc[i] *= sh_scale;
-		__syncthreads();
-		if (tid == 0) { bc[c] = sh_beta; tau[c] = tc; }
-		__syncthreads();
-		// apply H = I - tau v v^T (v = (1, bc[c+1:])) to the remaining columns
-		if (tc != 0.0)
-		{
-			for (int c2 = c + 1 + warp; c2 < s; c2 += nwarps)
-			{
-				double* b2 = B + (i64)c2 * p;
-				double acc = 0;
-				for (int i = c + lane; i < p; i += 32) acc = fma(i == c ? 1.0 : bc[i], b2[i], acc);
-				acc = warp_sum(acc) * tc;
-				for (int i = c + lane; i < p; i += 32) b2[i] -= acc * (i == c ? 1.0 : bc[i]);
-			}
-		}
-		__syncthreads();
-	}
-	// Q_W = H_0 ... H_{k-1} E (p x k), accumulated backwards, column-major
-	for (i64 e = tid; e < (i64)p * k; e += RQ_THREADS) Q[e] = (e / p == e % p) ? 1.0 : 0.0;
-	__syncthreads();
-	for (int c = k - 1; c >= 0; c--)
-	{
-		const double tc = tau[c];
-		const double* bc = B + (i64)c * p;
-		if (tc != 0.0)
-		{
-			for (int j = warp; j < k; j += nwarps)
-			{
-				double* qj = Q + (i64)j * p;
-				double acc = 0;
-				for (int i = c + lane; i < p; i += 32) acc = fma(i == c ? 1.0 : bc[i], qj[i], acc);
-				acc = warp_sum(acc) * tc;
-				for (int i = c + lane; i < p; i += 32) qj[i] -= acc * (i == c ? 1.0 : bc[i]);
-			}
-		}
-		__syncthreads();
-	}
-	if (qr)
-	{
-		// R (k x n) = upper part of W; Q (m x k) = Q_W
-		for (i64 e = tid; e < (i64)k * n; e += RQ_THREADS)
-		{
-			const i64 i = e / n, j = e % n;
-			r[d.r_off + e] = (i <= j) ? B[i + (i64)p * j] : 0.0;
-		}
-		for (i64 e = tid; e < (i64)m * k; e += RQ_THREADS)
-		{
-			const i64 i = e / k, j = e % k;
-			q[d.q_off + e] = Q[i + (i64)p * j];
-		}
-	}
-	else
-	{
-		// R (m x k): R[i][j] = R_W[k-1-j][m-1-i]; Q (k x n): Q[j][i] = Q_W[n-1-i][k-1-j]
-		for (i64 e = tid; e < (i64)m * k; e += RQ_THREADS)
-		{
-			const i64 i = e / k, j = e % k;
-			const i64 a0 = k - 1 - j, b0 = m - 1 - i;
-			r[d.r_off + e] = (a0 <= b0) ? B[a0 + (i64)p * b0] : 0.0;
-		}
-		for (i64 e = tid; e < (i64)k * n; e += RQ_THREADS)
-		{
-			const i64 j = e / n, i = e % n;
-			q[d.q_off + e] = Q[(n - 1 - i) + (i64)p * (k - 1 - j)];
-		}
-	}
-}
-
-void launch_rq_householder(int nblocks, const RqDesc* descs, const double* a, double* r, double* q, double* scratch,
-                           cudaStream_t st)
-{
-	if (nblocks <= 0) return;
-	k_rq_householder<<<nblocks, RQ_THREADS, 0, st>>>(descs, a, r, q, scratch);
-	CTG_CUDA(cudaGetLastError());
 }
 
 // ------------------------------------------------------------------------------------
