@@ -343,8 +343,7 @@ DTensor head_tensor(Ctx& c, const DTensor& a0, double value)
 
 // mps_split_tensor_svd (src/state/mps.c:1119-1159) -> split_block_sparse_matrix_svd (bond_ops.c:15-138)
 int split_mps_svd(Ctx& c, const DTensor& a, i64 d, const std::vector<q32>& qsite, double tol, i64 max_vdim, bool distr_left,
-                  DTensor& a0, DTensor& a1, double* entropy, std::vector<double>* kept = nullptr, long* near_ties = nullptr,
-                  bool steady = false)
+                  DTensor& a0, DTensor& a1, double* entropy, std::vector<double>* kept = nullptr, long* near_ties = nullptr)
 {
 	const i64 dd[2] = {d, d};
 	const int od[2] = {TENSOR_AXIS_OUT, TENSOR_AXIS_OUT};
@@ -356,7 +355,7 @@ int split_mps_svd(Ctx& c, const DTensor& a, i64 d, const std::vector<q32>& qsite
 	SvdPending pend;
 	// relative truncation: the discarded squares sum to at most tol ||a||_F^2; a is the normalised
 	// Lanczos solution, so tol / 2 is a safe lower bound of that budget
-	int ret = op_svd_launch(c, am, sv, pend, tol > 0 ? 0.5 * tol : 0.0, steady);
+	int ret = op_svd_launch(c, am, sv, pend, tol > 0 ? 0.5 * tol : 0.0);
 	if (ret < 0) return ret;
 	// the one host synchronisation of a bond step: the truncation needs the singular values
 	double* sigma = c.pinned_doubles((size_t)sv.ns);
@@ -690,6 +689,12 @@ double time_local_hamiltonian(Ctx& c, const DTensor& a, const DTensor& w, const 
 // dmrg_twosite
 // ------------------------------------------------------------------------------------
 
+struct SteadyScope {
+	Ctx& c;
+	SteadyScope(Ctx& ctx, bool on) : c(ctx) { c.steady = on; }
+	~SteadyScope() { c.steady = false; }
+};
+
 int dmrg_twosite_gpu(const struct mpo* H, int num_sweeps, int maxiter, double tol_split, i64 max_vdim, struct mps* psi,
                      double* en_sweeps, double* entropy, const DmrgOptions& opt, DmrgStats* stats)
 {
@@ -715,6 +720,9 @@ int dmrg_twosite_gpu(const struct mpo* H, int num_sweeps, int maxiter, double to
 		const double want = std::min(0.25 * (double)free_b, std::max(256.0 * 1048576.0, 400.0 * two_site));
 		c.reserve((size_t)want);
 	}
+	const bool reduced = is_tc_precision(opt.precision) && psi->a[0].dtype == CT_DOUBLE_REAL &&
+	                     num_sweeps > std::max(opt.final_fp64_sweeps, 0);
+	const SteadyScope steady(c, reduced);
 	c.gemm_flops = 0;
 	c.kernel_launches = 0;
 	c.profile = false;
@@ -797,7 +805,7 @@ int dmrg_twosite_gpu(const struct mpo* H, int num_sweeps, int maxiter, double to
 		double ent = 0;
 		// synchronises once (for the singular values); the Lanczos scalars have arrived by then
 		r = split_mps_svd(c, aopt, psi->d, qsite, tol_split, max_vdim, !left_to_right, A[i], A[i + 1], &ent,
-		                  &st->bond_sigma[(size_t)i], &st->near_ties, is_tc_precision(prec));
+		                  &st->bond_sigma[(size_t)i], &st->near_ties);
 		if (g_inject_tridiag_failure > 0)
 		{
 			// host-side fault injection (tests of the error path): this eigensolve reports failure

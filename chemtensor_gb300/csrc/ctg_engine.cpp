@@ -437,12 +437,12 @@ static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int
 		// cores to pay for their operand packing (FP64 is then both faster and exact). Its key comes
 		// from the output blocks and contributions, which the FP64 lowering has too: a product that
 		// stays on FP64 is lowered once, one on the tensor cores twice
-		DotLowering l = lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm, 64, true);
+		DotLowering l = lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm, 64, true, c.steady);
 		const int bn = tuned_tile_width(c, s, axs, t, axt, nmult, precision, out_perm, l);
 		if (bn == 0) return upload_dot_plan(c, std::move(l), GEMM_FP64, 64);
 		return upload_dot_plan(c, lower_dot(s, axs, t, axt, nmult, precision, c.num_sms(), out_perm, bn), precision, bn);
 	}
-	DotLowering l = lower_dot(s, axs, t, axt, nmult, z ? (int)GEMM_FP64 : precision, c.num_sms(), out_perm, 64, !z);
+	DotLowering l = lower_dot(s, axs, t, axt, nmult, z ? (int)GEMM_FP64 : precision, c.num_sms(), out_perm, 64, !z, c.steady);
 	return upload_dot_plan(c, std::move(l), precision, 64);
 }
 
@@ -900,11 +900,13 @@ static void dump_plan_request(int kind, const std::vector<i64>& params, const Me
 	fflush(f);
 }
 
+constexpr i64 PLAN_STEADY = 1 << 16;      // beside the precision in a plan's key
+
 DotPlan make_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision,
                       const int* out_perm)
 {
 	PlanTimer plan_timer(c);
-	std::vector<i64> params = {axs, axt, nmult, precision};
+	std::vector<i64> params = {axs, axt, nmult, precision + (c.steady ? PLAN_STEADY : 0)};
 	if (out_perm)
 		for (int i = 0; i < s.ndim + t.ndim - 2 * nmult; i++) params.push_back(out_perm[i]);
 	const uint64_t key = plan_key(0, params, s, &t);
@@ -1082,7 +1084,7 @@ DTensor view_trace_unit(const DTensor& t)
 // SVD and RQ of block-sparse matrices
 // ------------------------------------------------------------------------------------
 
-int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, double discard_weight, bool steady)
+int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, double discard_weight)
 {
 	const Meta& am = a.m();
 	pend = SvdPending();
@@ -1272,14 +1274,14 @@ int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, do
 		if (groups.size() == 1)
 			launch_svd_group(groups[0].l, groups[0].first, groups[0].count, (const SvdDesc*)desc->ptr, a.data(),
 			                 res.u.data(), (double*)res.s->ptr, res.vh.data(), (double*)scratch.ptr, (int*)status.ptr,
-			                 (double*)tail.ptr, c.stream(), tsp, discard2, steady);
+			                 (double*)tail.ptr, c.stream(), tsp, discard2, c.steady);
 		else
 		{
 			c.fork(ng);
 			for (size_t g = 0; g < groups.size(); g++)
 				launch_svd_group(groups[g].l, groups[g].first, groups[g].count, (const SvdDesc*)desc->ptr, a.data(),
 				                 res.u.data(), (double*)res.s->ptr, res.vh.data(), (double*)scratch.ptr,
-				                 (int*)status.ptr, (double*)tail.ptr, c.aux((int)g), tsp, discard2, steady);
+				                 (int*)status.ptr, (double*)tail.ptr, c.aux((int)g), tsp, discard2, c.steady);
 			c.join(ng);
 		}
 	}
@@ -1467,7 +1469,7 @@ int op_rq(Ctx& c, const DTensor& a, DTensor& r, DTensor& q)
 	DBuf scratch(&c, (size_t)std::max<i64>(woff, 1) * a.width() * sizeof(double));
 	KScope ks(c, K_RQ, 1);
 	launch_qr((int)descs.size(), (const RqDesc*)desc->ptr, descs.data(), a.data(), r.data(), q.data(), (double*)scratch.ptr, a.cplx,
-	          c.stream());
+	          c.steady, c.stream());
 	return 0;
 }
 
@@ -1538,7 +1540,7 @@ int op_qr(Ctx& c, const DTensor& a, DTensor& q, DTensor& r)
 	DBuf scratch(&c, (size_t)std::max<i64>(woff, 1) * a.width() * sizeof(double));
 	KScope ks(c, K_RQ, 1);
 	launch_qr((int)descs.size(), (const RqDesc*)desc->ptr, descs.data(), a.data(), r.data(), q.data(), (double*)scratch.ptr, a.cplx,
-	          c.stream());
+	          c.steady, c.stream());
 	return 0;
 }
 

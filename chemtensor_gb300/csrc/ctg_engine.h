@@ -112,6 +112,12 @@ public:
 	// n doubles of pinned host memory (contents valid until the next call); only call while no
 	// asynchronous copy into it is pending
 	double* pinned_doubles(size_t n);
+	// Set while this thread runs a search with reduced-precision sweeps. The noise of split-BF16 products is
+	// 1e-5 of a first sweep's energies, and a single changed rounding in their FP64 operands (or another basis
+	// within equal singular values) gives other noise. So such searches keep the arithmetic that they have always
+	// had where a faster one would round differently: the block SVD's starting basis (launch_svd_group), the
+	// shares of split FP64 sums (lower_dot), the real QR / RQ (launch_qr).
+	bool steady = false;
 	// optional per-kernel-class timing with CUDA events on this stream (resolved at sync points)
 	bool profile = false;
 	KProf prof[K_NUM_CLASSES];
@@ -290,9 +296,8 @@ struct SvdPending {
 // to at most this (the relative truncation of the two-site split times a lower bound of ||a||_F^2;
 // 0: the full SVD is needed). Every value whose square is below discard_weight / (2 k), k the total
 // number of singular values, is then certainly discarded, and the block SVD may leave the mutual
-// rotations of such columns out. steady: see launch_svd_group.
-int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, double discard_weight = 0.0,
-                  bool steady = false);
+// rotations of such columns out.
+int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, double discard_weight = 0.0);
 // 0, or -1 if a block did not converge (diagnostics on stderr)
 int op_svd_finish(Ctx& c, const SvdPending& pend);
 // launch, synchronise, finish. Returns 0 or -1.

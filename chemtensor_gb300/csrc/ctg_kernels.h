@@ -260,9 +260,7 @@ SvdLaunch svd_launch_for(int m, int n, int want, int max_cluster);
 // cluster exchanges to phase_ts[8 block + 4 ..].
 // discard2: the caller discards every singular value whose square is below it (0: none); the
 // refinement of the mixed path then leaves the mutual rotations of those columns out.
-// steady: the basis within (nearly) equal singular values, which is free, has to stay what the fixed
-// five FP32 sweeps from rank 32 on make it: for callers whose later arithmetic rounds coarsely, such
-// as products of split BF16 entries, where another basis shows at 1e-6 of a molecule's energies.
+// steady (see Ctx::steady): five FP32 sweeps from rank 32 on, whatever the angles.
 void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* descs, const double* a, double* u,
                       double* s, double* vh, double* scratch, int* status, double* flops, cudaStream_t st,
                       unsigned long long* phase_ts = nullptr, double discard2 = 0.0, bool steady = false);
@@ -273,9 +271,9 @@ struct RqDesc {
 	int m, n;
 	int qr;                           // 1: A = Q R (dgeqrf convention), 0: A = R Q (dgerqf convention)
 };
-// host: the descriptors in host memory
+// host: the descriptors in host memory; steady: see Ctx::steady
 void launch_qr(int nblocks, const RqDesc* descs, const RqDesc* host, const double* a, double* r, double* q, double* scratch,
-               bool cplx, cudaStream_t st);
+               bool cplx, bool steady, cudaStream_t st);
 
 // ---- complex128 (interleaved real / imaginary parts, element offsets and strides) -------
 // C = sum op(A) op(B) over the FP64 GEMM's lists (work: complex entries); conj_a / conj_b conjugate the

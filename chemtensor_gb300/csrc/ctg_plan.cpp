@@ -274,7 +274,7 @@ void slice_tiles(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum,
 // ------------------------------------------------------------------------------------
 
 DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision, int num_sms,
-                      const int* out_perm, int tc_bn, bool slices)
+                      const int* out_perm, int tc_bn, bool slices, bool steady)
 {
 	CTG_CHECK(!is_tc_precision(precision) || tc_bn == 64 || tc_bn == 128 || tc_bn == 256,
 	          "dot: tensor-core tile width must be 64, 128 or 256");
@@ -652,14 +652,21 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 	i64 wsz = 0;
 	if (!is_tc_precision(precision))
 	{
+		// steady: every contribution's chunks by themselves, larger shares (see lower_dot's declaration)
+		std::vector<i64> nchunk((size_t)r.nblocks, 0);
+		for (size_t b = 0; b < outs.size(); b++)
+		{
+			if (!steady) nchunk[b] = (ksum[b] + KCH - 1) / KCH;
+			for (int cc = outs[b].c0; steady && cc < outs[b].c0 + outs[b].nc; cc++) nchunk[b] += (cons[(size_t)cc].k + KCH - 1) / KCH;
+		}
+		auto terms = [&](int out) { return (double)(steady ? nchunk[(size_t)out] * KCH : ksum[(size_t)out]); };
 		double total = 0;
 		for (int k = 0; k < NUM_TILE_CLASSES; k++)
-			for (const GemmTile& t : tiles[k])
-				total += (double)TILE_ROWS[k] * TILE_COLS[k] * (double)ksum[(size_t)t.out];
+			for (const GemmTile& t : tiles[k]) total += (double)TILE_ROWS[k] * TILE_COLS[k] * terms(t.out);
 		// shares of an eighth of an SM's part, at least 16 terms of a 16 x 16 tile (2048 clocks of the FP64
 		// pipe). With half of a part and 64 terms: Hubbard L = 32, D = 256 272.1 ms (269.6 with these), D = 100
 		// 71.9 (69.8), spin chain D = 32 94.9 (94.0), one-site Hubbard D = 256 69.2 (68.1).
-		const double target = std::max(total / (8.0 * num_sms), 4096.0);
+		const double target = steady ? std::max(total / (2.0 * num_sms), 16384.0) : std::max(total / (8.0 * num_sms), 4096.0);
 		std::vector<std::pair<int, int>> pos;
 		for (int k = 0; k < NUM_TILE_CLASSES; k++)
 		{
@@ -668,8 +675,8 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			for (const GemmTile& t : tiles[k])
 			{
 				const GemmOut& o = outs[(size_t)t.out];
-				const i64 n = (ksum[(size_t)t.out] + KCH - 1) / KCH;
-				const double w = (double)tr * tc * (double)ksum[(size_t)t.out];
+				const i64 n = nchunk[(size_t)t.out];
+				const double w = (double)tr * tc * terms(t.out);
 				const int S = (int)std::min<double>((double)n, std::ceil(w / target));
 				if (S <= 1)
 				{
@@ -680,7 +687,10 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 				pos.clear();
 				i64 at = 0;
 				for (int cc = o.c0; cc < o.c0 + o.nc; at += cons[(size_t)cc++].k)
-					while ((i64)pos.size() * KCH < at + cons[(size_t)cc].k) pos.emplace_back(cc, (int)((i64)pos.size() * KCH - at));
+				{
+					for (int kk = 0; steady && kk < cons[(size_t)cc].k; kk += KCH) pos.emplace_back(cc, kk);
+					while (!steady && (i64)pos.size() * KCH < at + cons[(size_t)cc].k) pos.emplace_back(cc, (int)((i64)pos.size() * KCH - at));
+				}
 				pos.emplace_back(o.c0 + o.nc - 1, cons[(size_t)(o.c0 + o.nc - 1)].k);
 				for (int sp = 0; sp < S; sp++)
 				{

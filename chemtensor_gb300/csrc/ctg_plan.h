@@ -49,8 +49,11 @@ struct DotLowering {
 // the last column run innermost. tc_bn: column width of the tensor-core tiles (64, 128 or 256).
 // slices (FP64 only): the product may run on the tensor cores by digit slices where the rule in
 // use_slices says that this is faster.
+// steady (FP64): the sums of split tiles keep the order of shares that this library has always given them,
+// for callers whose later arithmetic rounds coarsely (see Ctx::steady); it costs 1 to 3 percent.
 DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision, int num_sms,
-                      const int* out_perm = nullptr, int tc_bn = 64, bool slices = false);
+                      const int* out_perm = nullptr, int tc_bn = 64, bool slices = false,
+                      bool steady = false);
 
 // data movement: kind 0 block permutation (PermDesc), 1 row map (RowDesc + maps), 2 axis scaling
 // (ScaleDesc + maps)

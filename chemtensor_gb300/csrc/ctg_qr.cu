@@ -304,6 +304,138 @@ k_qr_householder(const RqDesc* __restrict__ descs, const T* __restrict__ a, T* _
 			q[d.q_off + e] = conj_of(B[(n - 1 - e % n) + (i64)p * (k - 1 - e / n)]);
 }
 
+// The real QR / RQ whose rounding reduced-precision searches keep (Ctx::steady): matrix in the scratch, scaled
+// reflectors, IEEE square roots and divisions, a warp per column. 131 us where the kernel above takes 83.
+constexpr int RQ_THREADS = 256;
+
+__device__ double block_sum(double v, double* red)
+{
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	v = warp_sum(v);
+	__syncthreads();
+	if (lane == 0) red[warp] = v;
+	__syncthreads();
+	double t = 0;
+	for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += red[w];
+	return t;
+}
+
+__global__ void __launch_bounds__(RQ_THREADS)
+k_qr_steady(const RqDesc* __restrict__ descs, const double* __restrict__ a, double* __restrict__ r,
+                 double* __restrict__ q, double* __restrict__ scratch)
+{
+	__shared__ double red[RQ_THREADS / 32];
+	__shared__ double sh_beta, sh_tau, sh_scale;
+	const RqDesc d = descs[blockIdx.x];
+	const int m = d.m, n = d.n;
+	const bool qr = d.qr != 0;
+	const int k = min(m, n);
+	const int p = qr ? m : n, s = qr ? n : m;   // W is p x s, column-major
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = RQ_THREADS / 32;
+	double* B = scratch + d.w_off;             // W, p x s
+	double* Q = B + (i64)p * s;                // Q_W, p x k
+	double* tau = Q + (i64)p * k;              // k
+	const double* ab = a + d.a_off;
+	for (i64 e = tid; e < (i64)p * s; e += RQ_THREADS)
+	{
+		const i64 i = e % p, j = e / p;
+		B[e] = qr ? ab[i * n + j] : ab[(m - 1 - j) * n + (n - 1 - i)];
+	}
+	__syncthreads();
+	for (int c = 0; c < k; c++)
+	{
+		double* bc = B + (i64)c * p;
+		double part = 0;
+		for (int i = c + 1 + tid; i < p; i += RQ_THREADS) part = fma(bc[i], bc[i], part);
+		const double xnorm2 = block_sum(part, red);
+		if (tid == 0)
+		{
+			const double alpha = bc[c];
+			if (xnorm2 == 0.0)
+			{
+				sh_tau = 0.0;
+				sh_beta = alpha;
+				sh_scale = 0.0;
+			}
+			else
+			{
+				const double beta = -copysign(sqrt(alpha * alpha + xnorm2), alpha);
+				sh_tau = (beta - alpha) / beta;
+				sh_beta = beta;
+				sh_scale = 1.0 / (alpha - beta);
+			}
+		}
+		__syncthreads();
+		const double tc = sh_tau;
+		for (int i = c + 1 + tid; i < p; i += RQ_THREADS) bc[i] *= sh_scale;
+		__syncthreads();
+		if (tid == 0) { bc[c] = sh_beta; tau[c] = tc; }
+		__syncthreads();
+		// apply H = I - tau v v^T (v = (1, bc[c+1:])) to the remaining columns
+		if (tc != 0.0)
+		{
+			for (int c2 = c + 1 + warp; c2 < s; c2 += nwarps)
+			{
+				double* b2 = B + (i64)c2 * p;
+				double acc = 0;
+				for (int i = c + lane; i < p; i += 32) acc = fma(i == c ? 1.0 : bc[i], b2[i], acc);
+				acc = warp_sum(acc) * tc;
+				for (int i = c + lane; i < p; i += 32) b2[i] -= acc * (i == c ? 1.0 : bc[i]);
+			}
+		}
+		__syncthreads();
+	}
+	// Q_W = H_0 ... H_{k-1} E (p x k), accumulated backwards, column-major
+	for (i64 e = tid; e < (i64)p * k; e += RQ_THREADS) Q[e] = (e / p == e % p) ? 1.0 : 0.0;
+	__syncthreads();
+	for (int c = k - 1; c >= 0; c--)
+	{
+		const double tc = tau[c];
+		const double* bc = B + (i64)c * p;
+		if (tc != 0.0)
+		{
+			for (int j = warp; j < k; j += nwarps)
+			{
+				double* qj = Q + (i64)j * p;
+				double acc = 0;
+				for (int i = c + lane; i < p; i += 32) acc = fma(i == c ? 1.0 : bc[i], qj[i], acc);
+				acc = warp_sum(acc) * tc;
+				for (int i = c + lane; i < p; i += 32) qj[i] -= acc * (i == c ? 1.0 : bc[i]);
+			}
+		}
+		__syncthreads();
+	}
+	if (qr)
+	{
+		// R (k x n) = upper part of W; Q (m x k) = Q_W
+		for (i64 e = tid; e < (i64)k * n; e += RQ_THREADS)
+		{
+			const i64 i = e / n, j = e % n;
+			r[d.r_off + e] = (i <= j) ? B[i + (i64)p * j] : 0.0;
+		}
+		for (i64 e = tid; e < (i64)m * k; e += RQ_THREADS)
+		{
+			const i64 i = e / k, j = e % k;
+			q[d.q_off + e] = Q[i + (i64)p * j];
+		}
+	}
+	else
+	{
+		// R (m x k): R[i][j] = R_W[k-1-j][m-1-i]; Q (k x n): Q[j][i] = Q_W[n-1-i][k-1-j]
+		for (i64 e = tid; e < (i64)m * k; e += RQ_THREADS)
+		{
+			const i64 i = e / k, j = e % k;
+			const i64 a0 = k - 1 - j, b0 = m - 1 - i;
+			r[d.r_off + e] = (a0 <= b0) ? B[a0 + (i64)p * b0] : 0.0;
+		}
+		for (i64 e = tid; e < (i64)k * n; e += RQ_THREADS)
+		{
+			const i64 j = e / n, i = e % n;
+			q[d.q_off + e] = Q[(n - 1 - i) + (i64)p * (k - 1 - j)];
+		}
+	}
+}
+
 template <class T>
 void launch_qr_blocks(int nblocks, const RqDesc* descs, const RqDesc* host, const double* a, double* r, double* q,
                       double* scratch, cudaStream_t st)
@@ -324,9 +456,14 @@ void launch_qr_blocks(int nblocks, const RqDesc* descs, const RqDesc* host, cons
 }  // namespace
 
 void launch_qr(int nblocks, const RqDesc* descs, const RqDesc* host, const double* a, double* r, double* q, double* scratch,
-               bool cplx, cudaStream_t st)
+               bool cplx, bool steady, cudaStream_t st)
 {
-	if (cplx) launch_qr_blocks<double2>(nblocks, descs, host, a, r, q, scratch, st);
+	if (steady && !cplx && nblocks > 0)
+	{
+		k_qr_steady<<<nblocks, RQ_THREADS, 0, st>>>(descs, a, r, q, scratch);
+		CTG_CUDA(cudaGetLastError());
+	}
+	else if (cplx) launch_qr_blocks<double2>(nblocks, descs, host, a, r, q, scratch, st);
 	else launch_qr_blocks<double>(nblocks, descs, host, a, r, q, scratch, st);
 }
 

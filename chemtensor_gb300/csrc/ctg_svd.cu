@@ -60,7 +60,7 @@ constexpr float SVD_F32_COS = 0.0f;           // default: FP32 sweeps rotate eve
 // Default: smallest rank preconditioned in FP32. A spin chain at bond dimension 32 (ranks up to 32):
 // 104.9 ms from rank 32 on, 101.2 from 20, 99.1 from 16, 99.0 from 12 and 98.9 from 8 on.
 constexpr int SVD_F32_MIN_RANK = 16;
-constexpr int SVD_F32_MIN_STEADY = 32;        // the same where the caller wants the basis steady
+constexpr int SVD_F32_MIN_FULL = 32;          // the same where the caller keeps all factors or a steady basis
 constexpr int SVD_F32_CLUSTER = 8;            // default: CTAs of the FP32 sweeps
 constexpr int SVD_OUT_RC = 32;                // reflectors staged per round of the output phase
 
@@ -2620,8 +2620,10 @@ void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* d
 		CTG_CUDA(cudaLaunchKernelEx(&cfg, k_svd_global, descs, first, a, u, s, vh, scratch, status, 0.0, flops, g.cluster));
 		return;
 	}
-	// the steady form's threshold lies above the default one, so the launch's shared memory holds it too
-	const int f32_min = steady && svd_f32_min() > 0 ? std::max(svd_f32_min(), SVD_F32_MIN_STEADY) : svd_f32_min();
+	// The signs of the factors' columns are the sweeps' choice. Callers of the full SVD see them, so ranks below
+	// SVD_F32_MIN_FULL keep the FP64 sweeps' signs there; a truncating caller (the two-site split) does not.
+	const bool full = steady || discard2 == 0.0;
+	const int f32_min = full && svd_f32_min() > 0 ? std::max(svd_f32_min(), SVD_F32_MIN_FULL) : svd_f32_min();
 	static std::once_flag attr_once[64];
 	int dev = 0;
 	CTG_CUDA(cudaGetDevice(&dev));
