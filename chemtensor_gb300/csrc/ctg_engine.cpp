@@ -1250,6 +1250,7 @@ int op_svd_launch(Ctx& c, const DTensor& a, SvdResult& res, SvdPending& pend, do
 		{
 			groups.back().count++;
 			groups.back().l.smem = std::max(groups.back().l.smem, cfg[b].smem);
+			groups.back().l.threads = std::max(groups.back().l.threads, cfg[b].threads);
 		}
 		else groups.push_back(Group{cfg[b], b, 1});
 	}

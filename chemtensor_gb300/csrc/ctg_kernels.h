@@ -246,6 +246,7 @@ i64 svd_scratch_doubles(int m, int n);
 // Jacobi columns live in global memory (blocks too large for the shared-memory path).
 struct SvdLaunch {
 	int cluster = 1;
+	int threads = 256;
 	int smem = 0;
 	int global = 0;
 };
@@ -260,7 +261,7 @@ SvdLaunch svd_launch_for(int m, int n, int want, int max_cluster);
 // cluster exchanges to phase_ts[8 block + 4 ..].
 // discard2: the caller discards every singular value whose square is below it (0: none); the
 // refinement of the mixed path then leaves the mutual rotations of those columns out.
-// steady (see Ctx::steady): five FP32 sweeps from rank 32 on, whatever the angles.
+// steady (see Ctx::steady): five FP32 sweeps from rank 32 on and 256 threads, whatever the angles and the size.
 void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* descs, const double* a, double* u,
                       double* s, double* vh, double* scratch, int* status, double* flops, cudaStream_t st,
                       unsigned long long* phase_ts = nullptr, double discard2 = 0.0, bool steady = false);

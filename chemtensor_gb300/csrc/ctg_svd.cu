@@ -40,8 +40,16 @@ namespace ctg {
 
 namespace {
 
+// Threads per CTA. The FP32 sweeps give a warp per column pair: a block of more than 128 columns has more
+// than eight pairs per step on their sub-cluster of eight CTAs, and with eight warps two rounds of them.
+// 256 | 384 | 512 threads: 200 x 150 3.65 | 2.73 | 2.81 ms, Hubbard search at D = 256 (blocks of up to 190
+// columns) 269.6 | 253.2 | 266.1; at D = 100 (up to 90) 69.4 | 71.1 | 73.9, spin chain at D = 32 94.4 | 97.3 | 99.6.
 constexpr int SVD_THREADS = 256;
-constexpr int NWARPS = SVD_THREADS / 32;
+constexpr int SVD_THREADS_MAX = 384;
+constexpr int SVD_WIDE_COLUMNS = 128;         // blocks of more columns: SVD_THREADS_MAX
+constexpr int SVD_WARPS_MAX = SVD_THREADS_MAX / 32;
+__device__ __forceinline__ int svd_threads() { return (int)blockDim.x; }
+__device__ __forceinline__ int svd_warps() { return (int)(blockDim.x >> 5); }
 constexpr int SVD_STEP_PAIRS = 32;            // most column pairs of one inner step (group size <= 32)
 constexpr int SVD_SMEM_LIMIT = 220 * 1024;    // dynamic shared memory per CTA (227 KB less static use)
 constexpr int SVD_F32_SWEEPS = 5;             // default: FP32 preconditioning sweeps before the angles are asked
@@ -63,6 +71,7 @@ constexpr int SVD_F32_MIN_RANK = 16;
 constexpr int SVD_F32_MIN_FULL = 32;          // the same where the caller keeps all factors or a steady basis
 constexpr int SVD_F32_CLUSTER = 8;            // default: CTAs of the FP32 sweeps
 constexpr int SVD_OUT_RC = 32;                // reflectors staged per round of the output phase
+constexpr int SVD_OUT_WARPS = 8;              // warps with a column in the output phase (twelve: 7.5 for 6.8 ms per sweep)
 
 // shared memory (doubles) of the Jacobi tour: two buffers of two column groups (records of 2 N),
 // their norms and the per-step pair data
@@ -113,7 +122,7 @@ __device__ double block_sum(double v, double* red)
 	if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
 	__syncthreads();
 	double t = 0;
-	for (int w = 0; w < NWARPS; w++) t += red[w];
+	for (int w = 0; w < svd_warps(); w++) t += red[w];
 	return t;
 }
 
@@ -126,12 +135,12 @@ __device__ double block_sum(double v, double* red)
 __device__ int qr_pivoted_cta(double* W, int M, int N, double* nrm, double* ref, double* tau, int* perm,
                               double rank_thresh2)
 {
-	__shared__ double red[NWARPS];
+	__shared__ double red[SVD_WARPS_MAX];
 	__shared__ double sh_beta, sh_tau, sh_scale;
 	__shared__ int sh_piv, sh_stop;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const double tol3z = sqrt(DBL_EPSILON);
-	for (int j = warp; j < N; j += NWARPS)
+	for (int j = warp; j < N; j += svd_warps())
 	{
 		const double* wj = W + (i64)j * M;
 		double acc = 0;
@@ -169,7 +178,7 @@ __device__ int qr_pivoted_cta(double* W, int M, int N, double* nrm, double* ref,
 		{
 			double* wk = W + (i64)k * M;
 			double* wp = W + (i64)p * M;
-			for (int i = tid; i < M; i += SVD_THREADS)
+			for (int i = tid; i < M; i += svd_threads())
 			{
 				const double t = wk[i];
 				wk[i] = wp[i];
@@ -191,7 +200,7 @@ __device__ int qr_pivoted_cta(double* W, int M, int N, double* nrm, double* ref,
 		__syncthreads();
 		double* wk = W + (i64)k * M;
 		double part = 0;
-		for (int i = k + 1 + tid; i < M; i += SVD_THREADS) part = fma(wk[i], wk[i], part);
+		for (int i = k + 1 + tid; i < M; i += svd_threads()) part = fma(wk[i], wk[i], part);
 		const double xnorm2 = block_sum(part, red);
 		if (tid == 0)
 		{
@@ -212,11 +221,11 @@ __device__ int qr_pivoted_cta(double* W, int M, int N, double* nrm, double* ref,
 		}
 		__syncthreads();
 		const double tk = sh_tau;
-		for (int i = k + 1 + tid; i < M; i += SVD_THREADS) wk[i] *= sh_scale;
+		for (int i = k + 1 + tid; i < M; i += svd_threads()) wk[i] *= sh_scale;
 		__syncthreads();
 		if (tid == 0) { wk[k] = sh_beta; tau[k] = tk; }
 		__syncthreads();
-		for (int j = k + 1 + warp; j < N; j += NWARPS)
+		for (int j = k + 1 + warp; j < N; j += svd_warps())
 		{
 			double* wj = W + (i64)j * M;
 			if (tk != 0.0)
@@ -423,7 +432,7 @@ __device__ void jacobi_step(const Tour& t, int buf, int mode, int step, int cA, 
 	const long long c0 = cyc ? clock64() : 0;
 	const int np = mode == 0 ? npad : t.bs;
 	const int len = t.N + t.r;
-	for (int k = warp; k < np; k += NWARPS)
+	for (int k = warp; k < np; k += svd_warps())
 	{
 		int sp, cp, sq, cq;
 		if (!step_pair(t, mode, step, k, cA, cB, npad, sp, cp, sq, cq)) continue;
@@ -512,7 +521,7 @@ __device__ void jacobi_step32(const Tour32& t, int buf, int mode, int step, int 
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int np = mode == 0 ? npad : t.bs;
 	const int len = t.N + t.r;
-	for (int k = warp; k < np; k += NWARPS)
+	for (int k = warp; k < np; k += svd_warps())
 	{
 		int sp, cp, sq, cq;
 		if (!step_pair_idx(mode, step, k, t.bs, cA, cB, npad, sp, cp, sq, cq)) continue;
@@ -663,13 +672,13 @@ __device__ int qr_pivoted_cluster(cg::cluster_group& cluster, double* smem, cons
 	double* hbeta = htau + 32;                           // [2][16] candidate beta per CTA
 	int* hidx = (int*)(hbeta + 32);                      // [2][16] candidate column per CTA
 	int* qdone = hidx + 32;                              // [nloc_max] step that took the column, or -1
-	__shared__ double red[NWARPS];
+	__shared__ double red[SVD_WARPS_MAX];
 	__shared__ double sh_tau, sh_beta, sh_best;
 	__shared__ int sh_jl;
 
 	// load the own columns (B oriented tall) and their squared sums
 	double psum = 0;
-	for (i64 e = tid; e < (i64)nloc * M; e += SVD_THREADS)
+	for (i64 e = tid; e < (i64)nloc * M; e += svd_threads())
 	{
 		const int jl = (int)(e / M), row = (int)(e % M);
 		const int col = rank + cl * jl;
@@ -686,9 +695,9 @@ __device__ int qr_pivoted_cluster(cg::cluster_group& cluster, double* smem, cons
 	int ex = 0;
 	if (total > 0) frexp(sqrt(total), &ex);
 	const double sc = ldexp(1.0, -ex);
-	for (i64 e = tid; e < (i64)nloc * M; e += SVD_THREADS) qcol[e] *= sc;
+	for (i64 e = tid; e < (i64)nloc * M; e += svd_threads()) qcol[e] *= sc;
 	__syncthreads();
-	for (int jl = warp; jl < nloc; jl += NWARPS)
+	for (int jl = warp; jl < nloc; jl += svd_warps())
 	{
 		const double* w = qcol + (i64)jl * M;
 		double acc = 0;
@@ -807,7 +816,7 @@ __device__ int qr_pivoted_cluster(cg::cluster_group& cluster, double* smem, cons
 		if (owner != rank)                                   // uniform in the CTA
 		{
 			const double* src = cluster.map_shared_rank(cbuf, (unsigned)owner);
-			for (int i = k + tid; i < M; i += SVD_THREADS) vloc[i] = src[i];
+			for (int i = k + tid; i < M; i += svd_threads()) vloc[i] = src[i];
 			vbuf = vloc;
 			__syncthreads();
 		}
@@ -816,7 +825,7 @@ __device__ int qr_pivoted_cluster(cg::cluster_group& cluster, double* smem, cons
 		if (pjl >= 0)
 		{
 			double* w = qcol + (i64)pjl * M;
-			for (int i = k + 1 + tid; i < M; i += SVD_THREADS) w[i] = cbuf[i];
+			for (int i = k + 1 + tid; i < M; i += svd_threads()) w[i] = cbuf[i];
 			if (tid == 0)
 			{
 				w[k] = hbeta[par * 16 + owner];
@@ -831,7 +840,7 @@ __device__ int qr_pivoted_cluster(cg::cluster_group& cluster, double* smem, cons
 			q0 = q1;
 		}
 		// d. apply the reflector to the own remaining columns, downdate their norms
-		for (int jl = warp; jl < nloc; jl += NWARPS)
+		for (int jl = warp; jl < nloc; jl += svd_warps())
 		{
 			if (jl == pjl || qdone[jl] >= 0) continue;
 			double* w = qcol + (i64)jl * M;
@@ -864,9 +873,9 @@ __device__ int qr_pivoted_cluster(cg::cluster_group& cluster, double* smem, cons
 	}
 	// columns to global memory in pivot order, the remaining ones after them in source order
 	int* gdone = (int*)xs.T;                             // scratch until the Jacobi writes T
-	for (int jl = tid; jl < nloc; jl += SVD_THREADS) gdone[rank + cl * jl] = qdone[jl];
+	for (int jl = tid; jl < nloc; jl += svd_threads()) gdone[rank + cl * jl] = qdone[jl];
 	cluster.sync();
-	for (int jl = warp; jl < nloc; jl += NWARPS)
+	for (int jl = warp; jl < nloc; jl += svd_warps())
 	{
 		const int j = rank + cl * jl;
 		int pos = qdone[jl];
@@ -922,7 +931,7 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 		{
 			const int x = slot ? B : A;
 			float* dst = f.col(0, slot, 0);
-			for (i64 e = tid; e < (i64)f.cnt(x) * f.ld; e += SVD_THREADS)
+			for (i64 e = tid; e < (i64)f.cnt(x) * f.ld; e += svd_threads())
 			{
 				const int c = (int)(e / f.ld), i = (int)(e % f.ld);
 				const int g = x * f.bs + c;
@@ -941,7 +950,7 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 			for (int slot = 0; slot < 2; slot++)
 			{
 				const int nc = f.cnt(slot ? B : A);
-				for (int c = warp; c < nc; c += NWARPS)
+				for (int c = warp; c < nc; c += svd_warps())
 				{
 					const float* col = f.col(buf, slot, c);
 					float acc = 0.0f;
@@ -986,10 +995,10 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 						group_owner(x, rho1, f.nm, pi2, slot2);
 						const float4* src = (const float4*)f.col(buf, slot, 0);
 						float4* dst = (float4*)cluster.map_shared_rank(f.col(buf ^ 1, slot2, 0), (unsigned)pi2);
-						for (i64 e = tid; e < (i64)nc * f.ld / 4; e += SVD_THREADS) dst[e] = src[e];
+						for (i64 e = tid; e < (i64)nc * f.ld / 4; e += svd_threads()) dst[e] = src[e];
 						const float* nsrc = f.nrm(buf, slot);
 						float* ndst = cluster.map_shared_rank(f.nrm(buf ^ 1, slot2), (unsigned)pi2);
-						for (int e = tid; e < nc; e += SVD_THREADS) ndst[e] = nsrc[e];
+						for (int e = tid; e < nc; e += svd_threads()) ndst[e] = nsrc[e];
 					}
 					cluster.sync();
 					buf ^= 1;
@@ -1013,7 +1022,7 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 		{
 			const int x = slot ? B : A, nc = f.cnt(x);
 			const float* src = f.col(buf, slot, 0);
-			for (i64 e = tid; e < (i64)nc * r; e += SVD_THREADS)
+			for (i64 e = tid; e < (i64)nc * r; e += svd_threads())
 			{
 				const int c = (int)(e / r), i = (int)(e % r);
 				xs.V[(i64)(x * f.bs + c) * r + i] = (double)src[(i64)c * f.ld + N + i];
@@ -1141,7 +1150,7 @@ struct Refine {
 	int* memb;        // members of the cluster being rotated (RF_CLUSTER_MAX)
 	double* cstage;   // that cluster's columns [T; V] (RF_CLUSTER_MAX records of N + r, stride ldc)
 	int* misc;        // [0] non-singleton clusters, [1] failure, [2] edges, [3] labels changed, [4] rotated
-	float* red;       // [NWARPS] block reduction
+	float* red;       // [SVD_WARPS_MAX] block reduction
 	// own columns
 	int A, B, own0, nown;
 };
@@ -1157,7 +1166,7 @@ __host__ __device__ inline i64 refine_doubles(int N, int cl)
 	                  + 4 * 4 * (i64)N                        // key, cid, cnt, qidx
 	                  + 8 * (i64)RF_EDGES_PER_COL * N         // edges
 	                  + 4 * (i64)RF_CLUSTER_MAX               // memb
-	                  + 4 * 8 + 4 * NWARPS                    // misc, red
+	                  + 4 * 8 + 4 * SVD_WARPS_MAX                    // misc, red
 	                  + (i64)N + 16;                          // tail
 	return tour_jac_doubles(N, cl) + (bytes + 7) / 8 + 2;
 }
@@ -1177,14 +1186,14 @@ __device__ void rf_write_own(const Tour& t, const Refine& rf, bool with_t)
 {
 	const int tid = threadIdx.x, N = t.N, r = t.r;
 	if (with_t)
-		for (int e = tid; e < rf.nown * N; e += SVD_THREADS)
+		for (int e = tid; e < rf.nown * N; e += svd_threads())
 		{
 			const int jj = e / N, k = e % N, g = rf_col(t, rf, jj);
 			const double x = rf_rec(t, rf, jj)[k];
 			rf.Tr[(i64)k * r + g] = x;
 			rf.Th[(i64)g * N + k] = split_hilo(x);
 		}
-	for (int e = tid; e < rf.nown * r; e += SVD_THREADS)
+	for (int e = tid; e < rf.nown * r; e += svd_threads())
 	{
 		const int jj = e / r, k = e % r, g = rf_col(t, rf, jj);
 		const double x = rf_rec(t, rf, jj)[N + k];
@@ -1204,7 +1213,7 @@ __device__ double rf_gram(const Tour& t, const Refine& rf, const double* Ar, int
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = t.r;
 	const int nchunk = (r + 31) / 32;
 	double fl = 0;
-	for (int task = warp; task < rf.nown * nchunk; task += NWARPS)
+	for (int task = warp; task < rf.nown * nchunk; task += svd_warps())
 	{
 		const int jj = task % rf.nown, c = task / rf.nown;
 		const int g = rf_col(t, rf, jj);
@@ -1255,7 +1264,7 @@ __device__ void rf_update(const Tour& t, const Refine& rf, bool with_t)
 	const int row0 = with_t ? 0 : N;
 	const int nrows = N + r - row0;
 	const int nb = (rf.nown + JB - 1) / JB;
-	for (int task = tid; task < nrows * nb; task += SVD_THREADS)
+	for (int task = tid; task < nrows * nb; task += svd_threads())
 	{
 		const int kr = row0 + task % nrows, b = task / nrows;
 		const float2* h = kr < N ? rf.Th + kr : rf.Vh + (kr - N);
@@ -1326,7 +1335,7 @@ __device__ double rf_cluster_jacobi(const Tour& t, const Refine& rf, int cl, int
 		}
 		__syncthreads();
 		const int c = rf.misc[5];
-		for (int e = tid; e < c * len; e += SVD_THREADS)
+		for (int e = tid; e < c * len; e += svd_threads())
 		{
 			const int m = e / len, k = e % len, col = rf.memb[m];
 			rf.cstage[(i64)m * ldc + k] = k < N ? __ldcg(rf.Tr + (i64)k * r + col) : __ldcg(rf.Vr + (i64)(k - N) * r + col);
@@ -1383,7 +1392,7 @@ __device__ double rf_cluster_jacobi(const Tour& t, const Refine& rf, int cl, int
 			__syncthreads();
 			if (!any) break;
 		}
-		for (int e = tid; e < c * len; e += SVD_THREADS)
+		for (int e = tid; e < c * len; e += svd_threads())
 		{
 			const int m = e / len, k = e % len, col = rf.memb[m];
 			const double v = rf.cstage[(i64)m * ldc + k];
@@ -1448,13 +1457,13 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		rf.misc = (int*)p;
 		p += 4 * 8;
 		rf.red = (float*)p;
-		p += 4 * NWARPS;
+		p += 4 * SVD_WARPS_MAX;
 		rf.tail = (unsigned char*)p;
 	}
 	double fl = 0;
 
 	// ---- 1. Newton-Schulz on V: own columns from the FP32 phase's output ----
-	for (int e = tid; e < rf.nown * N; e += SVD_THREADS)
+	for (int e = tid; e < rf.nown * N; e += svd_threads())
 	{
 		const int jj = e / N, k = e % N;
 		rf_rec(t, rf, jj)[N + k] = k < r ? __ldcg(xs.V + (i64)rf_col(t, rf, jj) * r + k) : 0.0;
@@ -1467,7 +1476,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		cluster.sync();
 		fl += rf_gram(t, rf, rf.Vr, r, N, true, rf.G);
 		cluster.sync();
-		for (int e = tid; e < rf.nown * r; e += SVD_THREADS)
+		for (int e = tid; e < rf.nown * r; e += svd_threads())
 		{
 			const int jj = e / r, i = e % r;
 			rf.F[jj * r + i] = -0.5f * dbl_to_f32(__ldcg(rf.G + (i64)rf_col(t, rf, jj) * r + i));
@@ -1485,7 +1494,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 	const long long ct = cyc ? clock64() : 0;
 	{
 		const int ngrp = (N + 31) / 32;
-		for (int task = warp; task < ngrp * rf.nown; task += NWARPS)
+		for (int task = warp; task < ngrp * rf.nown; task += svd_warps())
 		{
 			const int gi = ngrp - 1 - task / rf.nown, jj = task % rf.nown;
 			const int i = 32 * gi + lane;
@@ -1539,14 +1548,14 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		lap(6);
 		// diagonal; the discarded tail: the smallest columns whose squared norms sum to at most tail2
 		// (every CTA computes the same sets and values from the same global G)
-		for (int i = tid; i < r; i += SVD_THREADS)
+		for (int i = tid; i < r; i += svd_threads())
 		{
 			const double d = __ldcg(rf.G + (i64)i * r + i);
 			rf.D[i] = d;
 			rf.key[i] = dbl_to_f32(d);
 		}
 		__syncthreads();
-		for (int i = tid; i < r; i += SVD_THREADS)
+		for (int i = tid; i < r; i += svd_threads())
 		{
 			// squared norms up to and including column i in increasing order (ties by index)
 			const float ki = rf.key[i];
@@ -1564,7 +1573,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		// tail) whose first-order angle |G_ig / (D_g - D_i)| would exceed delta, to global memory
 		{
 			float c2 = 0.0f;
-			for (int e = tid; e < rf.nown * r; e += SVD_THREADS)
+			for (int e = tid; e < rf.nown * r; e += svd_threads())
 			{
 				const int jj = e / r, i = e % r, g = rf_col(t, rf, jj);
 				if (i >= g || (rf.tail[i] && rf.tail[g])) continue;
@@ -1588,7 +1597,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		}
 		// clusters: connected components of the edges, labelled by their smallest column
 		if (tid == 0) rf.misc[1] = 0;
-		for (int i = tid; i < r; i += SVD_THREADS)
+		for (int i = tid; i < r; i += svd_threads())
 		{
 			rf.cid[i] = i;
 			rf.cnt[i] = 0;
@@ -1599,7 +1608,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 			fail = 1;
 			break;                                                  // uniform: one global count
 		}
-		for (int e = tid; e < nedge_all; e += SVD_THREADS) rf.edges[e] = __ldcg(rf.gedges + e);
+		for (int e = tid; e < nedge_all; e += svd_threads()) rf.edges[e] = __ldcg(rf.gedges + e);
 		__syncthreads();
 		const int nedge = nedge_all;
 		// minimum-label propagation with pointer jumping (labels are column indices of the same
@@ -1612,7 +1621,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		{
 			if (tid == 0) rf.misc[3] = 0;
 			__syncthreads();
-			for (int e = tid; e < nedge; e += SVD_THREADS)
+			for (int e = tid; e < nedge; e += svd_threads())
 			{
 				const int2 ed = rf.edges[e];
 				const int a = rf.cid[ed.x], b = rf.cid[ed.y];
@@ -1626,7 +1635,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 				}
 			}
 			__syncthreads();
-			for (int i = tid; i < r; i += SVD_THREADS)
+			for (int i = tid; i < r; i += svd_threads())
 			{
 				const int c = rf.cid[i], cc = rf.cid[c];
 				if (cc < c)
@@ -1644,7 +1653,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 			fail = 2;
 			break;
 		}
-		for (int i = tid; i < r; i += SVD_THREADS) atomicAdd(rf.cnt + rf.cid[i], 1);
+		for (int i = tid; i < r; i += svd_threads()) atomicAdd(rf.cnt + rf.cid[i], 1);
 		__syncthreads();
 		if (warp == 0)
 		{
@@ -1680,7 +1689,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 			break;
 		}
 		// first-order generator, own columns (zero inside a cluster and between tail columns)
-		for (int e = tid; e < rf.nown * r; e += SVD_THREADS)
+		for (int e = tid; e < rf.nown * r; e += svd_threads())
 		{
 			const int jj = e / r, i = e % r, g = rf_col(t, rf, jj);
 			float x = 0.0f;
@@ -1708,7 +1717,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		{
 			constexpr int XB = 8;
 			const int nb = (rf.nown + XB - 1) / XB;
-			for (int e = tid; e < nb * r; e += SVD_THREADS)
+			for (int e = tid; e < nb * r; e += svd_threads())
 			{
 				const int b = e / r, i = e % r, j0 = b * XB, nj = min(XB, rf.nown - j0);
 				float acc[XB];
@@ -1758,7 +1767,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 			cluster.sync();
 			fl += rf_cluster_jacobi(t, rf, cl, rank, tol2);
 			cluster.sync();
-			for (int e = tid; e < rf.nown * (N + r); e += SVD_THREADS)
+			for (int e = tid; e < rf.nown * (N + r); e += svd_threads())
 			{
 				const int jj = e / (N + r), k = e % (N + r), g = rf_col(t, rf, jj);
 				rf_rec(t, rf, jj)[k] = k < N ? __ldcg(rf.Tr + (i64)k * r + g) : __ldcg(rf.Vr + (i64)(k - N) * r + g);
@@ -1777,7 +1786,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 	return converged;
 }
 
-__global__ void __launch_bounds__(SVD_THREADS, 1)
+__global__ void __launch_bounds__(SVD_THREADS_MAX, 1)
 k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restrict__ a, double* __restrict__ u,
            double* __restrict__ s, double* __restrict__ vh, double* __restrict__ scratch, int* __restrict__ status,
            double* __restrict__ flops, int cl, int smem_bytes, unsigned long long* __restrict__ phase_ts, int f32_min,
@@ -1795,9 +1804,9 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	const SvdScratch xs = scratch_layout(scratch + d.w_off, M, N);
 	const double* ab = a + d.a_off;
 
-	for (int e = rank * SVD_THREADS + tid; e < SVD_MAX_SWEEPS; e += cl * SVD_THREADS) xs.flags[e] = 0;
-	for (int e = rank * SVD_THREADS + tid; e < SVD_F32_SWEEPS_MAX; e += cl * SVD_THREADS) xs.flags32[e] = 0;
-	for (int e = rank * SVD_THREADS + tid; e < SVD_MAX_SWEEPS; e += cl * SVD_THREADS) xs.cmax[e] = 0;
+	for (int e = rank * svd_threads() + tid; e < SVD_MAX_SWEEPS; e += cl * svd_threads()) xs.flags[e] = 0;
+	for (int e = rank * svd_threads() + tid; e < SVD_F32_SWEEPS_MAX; e += cl * svd_threads()) xs.flags32[e] = 0;
+	for (int e = rank * svd_threads() + tid; e < SVD_MAX_SWEEPS; e += cl * svd_threads()) xs.cmax[e] = 0;
 	const bool stamp = phase_ts && rank == 0 && tid == 0;
 	if (stamp) phase_ts[SVD_PHASE_SLOTS * blk] = globaltimer();
 
@@ -1807,15 +1816,15 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	if (cl > 1) qr_pivoted_cluster(cluster, smem, ab, tall, n, M, N, cl, xs, phase_ts && tid == 0 && rank == 1 ? qcyc : nullptr);
 	else
 	{
-		__shared__ double red[NWARPS];
+		__shared__ double red[SVD_WARPS_MAX];
 		double part = 0;
-		for (i64 e = tid; e < (i64)M * N; e += SVD_THREADS)
+		for (i64 e = tid; e < (i64)M * N; e += svd_threads())
 		{
 			const i64 col = e / M, row = e % M;
 			const double x = tall ? ab[row * n + col] : ab[col * n + row];
 			part = fma(x, x, part);
 		}
-		for (int j = tid; j < N; j += SVD_THREADS) xs.perm[j] = j;
+		for (int j = tid; j < N; j += svd_threads()) xs.perm[j] = j;
 		const double total = block_sum(part, red);
 		// exact power-of-two scaling: keeps products of squared column norms far from underflow
 		int ex = 0;
@@ -1824,7 +1833,7 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 		// the factorisation runs in shared memory when the block fits, then W goes to global memory
 		const bool in_smem = (i64)M * N * 8 <= (i64)smem_bytes;
 		double* Wq = in_smem ? smem : xs.W;
-		for (i64 e = tid; e < (i64)M * N; e += SVD_THREADS)
+		for (i64 e = tid; e < (i64)M * N; e += svd_threads())
 		{
 			const i64 col = e / M, row = e % M;
 			Wq[e] = sc * (tall ? ab[row * n + col] : ab[col * n + row]);
@@ -1832,7 +1841,7 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 		__syncthreads();
 		const int rr = qr_pivoted_cta(Wq, M, N, xs.nrm, xs.sig, xs.tau, xs.perm, DBL_EPSILON * DBL_EPSILON * total * sc * sc);
 		if (in_smem)
-			for (i64 e = tid; e < (i64)M * N; e += SVD_THREADS) xs.W[e] = Wq[e];
+			for (i64 e = tid; e < (i64)M * N; e += svd_threads()) xs.W[e] = Wq[e];
 		if (tid == 0)
 		{
 			xs.misc[0] = (double)rr;
@@ -1889,7 +1898,7 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 		{
 			const int x = slot ? B : A;
 			double* dst = t.col(0, slot, 0);
-			for (i64 e = tid; e < (i64)t.cnt(x) * t.ld; e += SVD_THREADS)
+			for (i64 e = tid; e < (i64)t.cnt(x) * t.ld; e += svd_threads())
 			{
 				const int c = (int)(e / t.ld), i = (int)(e % t.ld);
 				const int g = x * t.bs + c;
@@ -1912,7 +1921,7 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 		for (int slot = 0; slot < 2; slot++)
 		{
 			const int nc = t.cnt(slot ? B : A);
-			for (int c = warp; c < nc; c += NWARPS)
+			for (int c = warp; c < nc; c += svd_warps())
 			{
 				const double* col = t.col(buf, slot, c);
 				double acc = 0;
@@ -1955,10 +1964,10 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 					group_owner(x, rho1, t.nm, pi2, slot2);
 					const double2* src = (const double2*)t.col(buf, slot, 0);
 					double2* dst = (double2*)cluster.map_shared_rank(t.col(buf ^ 1, slot2, 0), (unsigned)pi2);
-					for (i64 e = tid; e < (i64)nc * t.ld / 2; e += SVD_THREADS) dst[e] = src[e];
+					for (i64 e = tid; e < (i64)nc * t.ld / 2; e += svd_threads()) dst[e] = src[e];
 					const double* nsrc = t.nrm(buf, slot);
 					double* ndst = cluster.map_shared_rank(t.nrm(buf ^ 1, slot2), (unsigned)pi2);
-					for (int e = tid; e < nc; e += SVD_THREADS) ndst[e] = nsrc[e];
+					for (int e = tid; e < nc; e += svd_threads()) ndst[e] = nsrc[e];
 				}
 				cluster.sync();
 				buf ^= 1;
@@ -1983,14 +1992,14 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	{
 		const int x = slot ? B : A, nc = t.cnt(x);
 		const double* src = t.col(buf, slot, 0);
-		for (i64 e = tid; e < (i64)nc * t.ld; e += SVD_THREADS)
+		for (i64 e = tid; e < (i64)nc * t.ld; e += svd_threads())
 		{
 			const int c = (int)(e / t.ld), i = (int)(e % t.ld);
 			const int g = x * t.bs + c;
 			if (i < N) xs.T[(i64)g * N + i] = src[e];
 			else if (i - N < r) xs.V[(i64)g * r + (i - N)] = src[e];
 		}
-		for (int c = warp; c < nc; c += NWARPS)
+		for (int c = warp; c < nc; c += svd_warps())
 		{
 			const double* col = t.col(buf, slot, c);
 			double acc = 0;
@@ -2025,29 +2034,29 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	// one warp per column of V; the reflectors are staged in shared memory SVD_OUT_RC at a time (in
 	// the order they are applied, last first), so the serial chain of each column reads shared
 	// memory instead of L2
-	double* ub = smem + (i64)warp * M;
+	double* ub = smem + (i64)warp * M;                    // the first SVD_OUT_WARPS warps only
 	// as many reflectors per round as the shared memory holds (at least 4, at most SVD_OUT_RC)
-	const i64 room = ((i64)smem_bytes / 8 - (i64)NWARPS * M - SVD_OUT_RC) / M;
+	const i64 room = ((i64)smem_bytes / 8 - (i64)SVD_OUT_WARPS * M - SVD_OUT_RC) / M;
 	const int rc = room < 1 ? 1 : (room > SVD_OUT_RC ? SVD_OUT_RC : (int)room);
-	double* ws = smem + (i64)NWARPS * M;                  // staged reflectors, unit leading entry
+	double* ws = smem + (i64)SVD_OUT_WARPS * M;                // staged reflectors, unit leading entry
 	double* ts = ws + (i64)rc * M;                        // their scalars
-	const int nround = (r + cl * NWARPS - 1) / (cl * NWARPS);
+	const int nround = (r + cl * SVD_OUT_WARPS - 1) / (cl * SVD_OUT_WARPS);
 	for (int round = 0; round < nround; round++)
 	{
-		const int c = rank * NWARPS + warp + round * cl * NWARPS;
-		const bool has = c < r;
+		const int c = rank * SVD_OUT_WARPS + warp + round * cl * SVD_OUT_WARPS;
+		const bool has = warp < SVD_OUT_WARPS && c < r;
 		if (has)
 			for (int i = lane; i < M; i += 32) ub[i] = i < r ? __ldcg(xs.V + (i64)c * r + i) : 0.0;
 		for (int k1 = r - 1; k1 >= 0; k1 -= rc)
 		{
 			const int k0 = k1 - rc + 1 > 0 ? k1 - rc + 1 : 0;
 			__syncthreads();
-			for (i64 e = tid; e < (i64)(k1 - k0 + 1) * M; e += SVD_THREADS)
+			for (i64 e = tid; e < (i64)(k1 - k0 + 1) * M; e += svd_threads())
 			{
 				const int k = k0 + (int)(e / M), i = (int)(e % M);
 				ws[e] = i > k ? __ldcg(xs.W + (i64)k * M + i) : (i == k ? 1.0 : 0.0);
 			}
-			for (int e = tid; e <= k1 - k0; e += SVD_THREADS) ts[e] = __ldcg(xs.tau + k0 + e);
+			for (int e = tid; e <= k1 - k0; e += svd_threads()) ts[e] = __ldcg(xs.tau + k0 + e);
 			__syncthreads();
 			if (!has) continue;
 			for (int k = k1; k >= k0; k--)
@@ -2108,8 +2117,8 @@ k_svd_global(const SvdDesc* __restrict__ descs, int first, const double* __restr
 	const bool tall = m >= n;
 	const int M = tall ? m : n, N = tall ? n : m;
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-	const int gtid = rank * SVD_THREADS + tid, gstride = cl * SVD_THREADS;
-	const int gwarp = rank * NWARPS + warp, gwarps = cl * NWARPS;
+	const int gtid = rank * svd_threads() + tid, gstride = cl * svd_threads();
+	const int gwarp = rank * svd_warps() + warp, gwarps = cl * svd_warps();
 
 	double* W = scratch + d.w_off;                        // M x N: B, then R and the Householder vectors
 	double* Q = W + (i64)M * N;                           // M x N: explicit Q (first r columns)
@@ -2132,16 +2141,16 @@ k_svd_global(const SvdDesc* __restrict__ descs, int first, const double* __restr
 	// ---- 1. pivoted QR on the cluster's first CTA ----
 	if (rank == 0)
 	{
-		__shared__ double red[NWARPS];
+		__shared__ double red[SVD_WARPS_MAX];
 		double part = 0;
-		for (i64 e = tid; e < (i64)M * N; e += SVD_THREADS)
+		for (i64 e = tid; e < (i64)M * N; e += svd_threads())
 		{
 			const i64 col = e / M, row = e % M;
 			const double x = tall ? ab[row * n + col] : ab[col * n + row];
 			W[e] = x;
 			part = fma(x, x, part);
 		}
-		for (int j = tid; j < N; j += SVD_THREADS) perm[j] = j;
+		for (int j = tid; j < N; j += svd_threads()) perm[j] = j;
 		const double total = block_sum(part, red);
 		__syncthreads();
 		const int r = qr_pivoted_cta(W, M, N, nrm, sig, tau, perm, DBL_EPSILON * DBL_EPSILON * total);
@@ -2525,7 +2534,7 @@ static int svd_refine()
 static i64 tour_smem_bytes(int M, int N, int cl)
 {
 	const i64 jac = tour_jac_doubles(N, cl);
-	const i64 out = (i64)(NWARPS + 4) * M + SVD_OUT_RC;     // column buffers, at least 4 staged reflectors
+	const i64 out = (i64)(SVD_OUT_WARPS + 4) * M + SVD_OUT_RC;     // column buffers, at least 4 staged reflectors
 	i64 need = jac > out ? jac : out;
 	// FP32 preconditioning and the refinement, where the rank may reach the threshold and their
 	// arrays fit
@@ -2586,6 +2595,7 @@ SvdLaunch svd_launch_for(int m, int n, int want, int max_cluster)
 		if (bsmax <= SVD_STEP_PAIRS && bytes <= SVD_SMEM_LIMIT)
 		{
 			l.cluster = cl;
+			l.threads = N > SVD_WIDE_COLUMNS ? SVD_THREADS_MAX : SVD_THREADS;
 			l.smem = (int)bytes;
 			l.global = 0;
 			return l;
@@ -2605,7 +2615,7 @@ void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* d
 	if (count <= 0) return;
 	cudaLaunchConfig_t cfg = {};
 	cfg.gridDim = dim3((unsigned)(count * g.cluster));
-	cfg.blockDim = dim3(SVD_THREADS);
+	cfg.blockDim = dim3((unsigned)(steady ? SVD_THREADS : g.threads));
 	cfg.dynamicSmemBytes = (size_t)g.smem;
 	cfg.stream = st;
 	cudaLaunchAttribute attr[1];
