@@ -6,6 +6,7 @@
 // HBM for the whole call; the host only handles block structure (integers)
 // and, once per bond, the singular values that decide the truncation.
 #include "ctg_dmrg.h"
+#include "ctg_pool.h"
 
 #include <algorithm>
 #include <chrono>
@@ -69,31 +70,65 @@ Meta meta_from_struct(const struct block_sparse_tensor* t)
 	return m;
 }
 
+// copy(block, first entry inside it, count) over all entries, on the host threads where there are many: a
+// tensor's blocks are scattered heap allocations. A local-Hamiltonian application over 33 MB of operands and result: 3.9 ms with one thread, 2.1
+// with four, 1.9 with eight; 4.9 with one thread and a buffer of its own in between (fresh pages, a second copy).
+// Below half a megabyte waking the threads costs more than it saves
+template <class F>
+static void over_entries(const Meta& m, int width, const F& copy)
+{
+	const i64 bytes = m.nnz * width * (i64)sizeof(double);
+	const int parts = bytes < (i64)1 << 19 ? 1 : (int)std::min<i64>(host_threads(), bytes >> 17);
+	parallel_for(parts, [&](int q) {
+		const i64 lo = m.nnz * q / parts, hi = m.nnz * (q + 1) / parts;
+		int b = (int)(std::upper_bound(m.boff.begin(), m.boff.end(), lo) - m.boff.begin()) - 1;
+		for (b = std::max(b, 0); b < m.nblocks && m.boff[b] < hi; b++)
+		{
+			const i64 x = std::max(lo, m.boff[b]), y = std::min(hi, m.boff[b] + m.block_size(b));
+			if (y > x) copy(b, x - m.boff[b], y - x);
+		}
+	});
+}
+
 DTensor tensor_from_struct(Ctx& c, const struct block_sparse_tensor* t)
 {
 	Meta m = meta_from_struct(t);
 	const int w = t->dtype == CT_DOUBLE_COMPLEX ? 2 : 1;
-	std::vector<double> host((size_t)std::max<i64>(m.nnz, 1) * w);
+	const size_t bytes = (size_t)std::max<i64>(m.nnz, 1) * w * sizeof(double);
+	std::vector<const double*> data((size_t)m.nblocks);
 	for (int b = 0; b < m.nblocks; b++)
 	{
 		const struct dense_tensor* bl = t->blocks[m.linear(m.index(b))];
 		CTG_CHECK(bl != nullptr, "missing dense block in the input tensor");
 		CTG_CHECK(bl->dtype == t->dtype, "dense block of another numeric type");
 		for (int i = 0; i < m.ndim; i++) CTG_CHECK(bl->dim[i] == m.dims(b)[i], "dense block shape mismatch");
-		memcpy(host.data() + m.boff[b] * w, bl->data, (size_t)m.block_size(b) * w * sizeof(double));
+		data[(size_t)b] = (const double*)bl->data;
 	}
+	// straight into the pinned staging area; a tensor larger than that goes through a buffer of its own
+	std::vector<double> own;
+	char* stage = c.stage(bytes);
+	if (!stage) own.resize(bytes / sizeof(double));
+	double* host = stage ? (double*)stage : own.data();
+	if (m.nnz == 0) host[0] = 0.0;
+	over_entries(m, w, [&](int b, i64 first, i64 n) {
+		memcpy(host + (m.boff[b] + first) * w, data[(size_t)b] + first * w, (size_t)(n * w) * sizeof(double));
+	});
 	DTensor d;
 	d.meta = std::make_shared<const Meta>(std::move(m));
 	d.cplx = w == 2;
-	d.buf = c.upload(host.data(), host.size() * sizeof(double));
+	d.buf = stage ? c.upload_staged(stage, bytes) : c.upload(host, bytes);
 	return d;
 }
 
 void tensor_to_struct(Ctx& c, const DTensor& t, struct block_sparse_tensor* out)
 {
-	std::vector<double> host((size_t)std::max<i64>(t.m().nnz, 1) * t.width());
-	copy_to_host(c, t, host.data());
-	write_struct_host(t.m(), host.data(), out, t.cplx);
+	const size_t n = (size_t)std::max<i64>(t.m().nnz, 1) * t.width();
+	std::vector<double> own;
+	char* stage = c.stage(n * sizeof(double));         // read again before anything else is staged
+	if (!stage) own.resize(n);
+	double* host = stage ? (double*)stage : own.data();
+	copy_to_host(c, t, host);
+	write_struct_host(t.m(), host, out, t.cplx);
 }
 
 void write_struct_host(const Meta& m, const double* host, struct block_sparse_tensor* out, bool cplx)
@@ -116,15 +151,20 @@ void write_struct_host(const Meta& m, const double* host, struct block_sparse_te
 	for (int i = 0; i < m.ndim; i++) total *= m.nb[i];
 	out->blocks = (struct dense_tensor**)ct_alloc((size_t)total * sizeof(struct dense_tensor*));
 	memset(out->blocks, 0, (size_t)total * sizeof(struct dense_tensor*));
+	std::vector<double*> data((size_t)m.nblocks);
 	for (int b = 0; b < m.nblocks; b++)
 	{
 		struct dense_tensor* d = (struct dense_tensor*)ct_alloc(sizeof(struct dense_tensor));
 		d->dtype = out->dtype;
 		d->ndim = m.ndim;
 		d->dim = ct_copy(m.dims(b), (size_t)m.ndim);
-		d->data = ct_copy(host + m.boff[b] * w, (size_t)m.block_size(b) * w);
+		d->data = ct_alloc((size_t)(m.block_size(b) * w) * sizeof(double));
+		data[(size_t)b] = (double*)d->data;
 		out->blocks[m.linear(m.index(b))] = d;
 	}
+	over_entries(m, w, [&](int b, i64 first, i64 n) {
+		memcpy(data[(size_t)b] + first * w, host + (m.boff[b] + first) * w, (size_t)(n * w) * sizeof(double));
+	});
 }
 
 void free_struct(struct block_sparse_tensor* t)
@@ -971,7 +1011,7 @@ void mps_vdot_gpu(const struct mps* chi, const struct mps* psi, int device, doub
 	{
 		// mps_contraction_step_right (src/state/mps.c:279-306)
 		DTensor a = tensor_from_struct(c, &psi->a[i]);
-		DTensor b = tensor_from_struct(c, &chi->a[i]);
+		DTensor b = chi->a == psi->a ? a : tensor_from_struct(c, &chi->a[i]);
 		DTensor s1 = op_dot(c, a, AX_TRAILING, r, AX_LEADING, 1);
 		DTensor bc = view_reversed(c, b);
 		bc.conj = b.cplx;                 // <chi| is complex conjugated
@@ -1014,7 +1054,7 @@ void mpo_inner_product_gpu(const struct mps* chi, const struct mpo* op, const st
 	for (int i = L - 1; i >= 0; i--)
 	{
 		DTensor a = tensor_from_struct(c, &psi->a[i]);
-		DTensor b = tensor_from_struct(c, &chi->a[i]);
+		DTensor b = chi->a == psi->a ? a : tensor_from_struct(c, &chi->a[i]);
 		DTensor w = tensor_from_struct(c, &op->a[i]);
 		r = contraction_step_right_ab(c, a, b, w, r);
 	}

@@ -330,6 +330,22 @@ KScope::~KScope()
 	c.kernel_launches += launches;
 }
 
+char* Ctx::stage(size_t bytes)
+{
+	if (bytes > staging_cap_) return nullptr;
+	if (staging_used_ + bytes > staging_cap_) sync();
+	char* p = staging_ + staging_used_;
+	staging_used_ += (bytes + 255) & ~(size_t)255;
+	return p;
+}
+
+DBufPtr Ctx::upload_staged(const char* stage, size_t bytes)
+{
+	auto b = std::make_shared<DBuf>(this, bytes);
+	CTG_CUDA(cudaMemcpyAsync(b->ptr, stage, bytes, cudaMemcpyHostToDevice, st_));
+	return b;
+}
+
 DBufPtr Ctx::upload(const void* host, size_t bytes)
 {
 	CTG_CHECK(host != nullptr || bytes == 0, "upload from a null host pointer");

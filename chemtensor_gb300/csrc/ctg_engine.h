@@ -78,6 +78,10 @@ public:
 	void reserve(size_t bytes);
 	// copy host bytes to a new device buffer (through pinned staging, asynchronous)
 	DBufPtr upload(const void* host, size_t bytes);
+	// room for `bytes` in the pinned staging area, to be filled by the caller for upload_staged or written by a
+	// copy from the device; its contents last until the next sync(). Null if the whole area is smaller.
+	char* stage(size_t bytes);
+	DBufPtr upload_staged(const char* stage, size_t bytes);
 	// block until the stream is idle; recycles the staging arena
 	void sync();
 	DTensor empty(const Meta& m, bool cplx = false);
