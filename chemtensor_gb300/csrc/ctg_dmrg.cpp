@@ -71,9 +71,10 @@ Meta meta_from_struct(const struct block_sparse_tensor* t)
 }
 
 // copy(block, first entry inside it, count) over all entries, on the host threads where there are many: a
-// tensor's blocks are scattered heap allocations. A local-Hamiltonian application over 33 MB of operands and result: 3.9 ms with one thread, 2.1
-// with four, 1.9 with eight; 4.9 with one thread and a buffer of its own in between (fresh pages, a second copy).
-// Below half a megabyte waking the threads costs more than it saves
+// tensor's blocks are scattered heap allocations. A local-Hamiltonian application over 33 MB of operands
+// and result: 3.9 ms with one thread, 2.1 with four, 1.9 with eight; 4.9 with one thread and a buffer of
+// its own in between (fresh pages, a second copy). Half a megabyte is a copy of 50 to 100 us, a few times
+// what waking the threads takes.
 template <class F>
 static void over_entries(const Meta& m, int width, const F& copy)
 {
@@ -663,7 +664,7 @@ int minimize_local_energy(Ctx& c, const DTensor& w, const DTensor& l, const DTen
 	}
 	{
 		KScope ks(c, K_LANCZOS, 1, 3.0 * dn, 24.0 * dn);
-		launch_lz_start(a_start.data(), Vp, n, pp, d_sc, s);
+		launch_lz_start(a_start.data(), Vp, n, pp, d_sc, c.steady, s);
 	}
 	a_opt = c.empty(a_start.meta, a_start.cplx);
 	for (int j = 0; j < maxiter; j++)
@@ -676,13 +677,13 @@ int minimize_local_energy(Ctx& c, const DTensor& w, const DTensor& l, const DTen
 		{
 			KScope ks(c, K_LANCZOS, 1, 9.0 * dn, 72.0 * dn);
 			launch_lz_step(wp, Vp + (i64)j * n, j > 0 ? Vp + (i64)(j - 1) * n : Vp, Vp + (i64)(j + 1) * n, n, nent, j, 0, pp,
-			               d_sc, s);
+			               d_sc, c.steady, s);
 		}
 		else
 		{
 			// alpha of the last step, the tridiagonal eigensolve and the Ritz vector in one launch
 			KScope ks(c, K_LANCZOS, 1, 2.0 * (maxiter + 1) * dn, 8.0 * (maxiter + 3) * dn);
-			launch_lz_finish(wp, Vp, n, maxiter, pp, d_sc, a_opt.data(), s);
+			launch_lz_finish(wp, Vp, n, maxiter, pp, d_sc, a_opt.data(), c.steady, s);
 		}
 		g_host_detail[2] += now_s() - hz;
 	}

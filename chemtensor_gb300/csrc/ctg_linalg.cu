@@ -30,6 +30,7 @@ __device__ __forceinline__ double warp_sum(double v)
 // ------------------------------------------------------------------------------------
 
 constexpr int RED_THREADS = 512;
+constexpr i64 LZ_SMALL_N = 65536;        // vectors of up to this many doubles: 256 threads per block
 
 __device__ void block_partial(double v, double* partial)
 {
@@ -64,7 +65,18 @@ __device__ double final_sum(const double* partial)
 // for vectors of up to LZ_CLUSTER_MAX_N entries: those live in L2 between launches, and a cluster
 // barrier costs a fraction of a grid barrier over 152 blocks. Both partition the entries and order
 // the sums in a fixed way, so that a given n gives the same bits in every run.
+//
+// The steady cluster form (Ctx::steady) keeps the rounding that this library has always had: IEEE square root
+// and division in every thread (a hundred FP64 instructions, each 64 cycles of an SM sub-partition, times four
+// warps), warps' sums added one after the other, three FP64 instructions per entry to orthogonalise. The
+// other one adds by butterflies, derives norm and reciprocal in one warp by ctg_fp64.cuh, needs two
+// FMAs per entry, and starts 256 threads per block for shorter vectors: a butterfly costs five FP64
+// instructions per warp, whatever it adds. A step on the vectors of a spin chain at D = 32 (1e3 doubles)
+// 12.2 -> 9.2 us, of a Hubbard chain at D = 256 (up to 3e5) 22.7 -> 20.1 us; the searches 94.5 -> 91.7 and
+// 254 -> 251 ms, the smallest one (L = 9, D = 16) 9.05 -> 8.55 ms. 256 threads up to 131072 doubles: Hubbard
+// 253.7 ms; 128 threads up to 131072: 257.1.
 struct GridReduce {
+	static constexpr bool steady = true;
 	cg::grid_group g;
 	double* partial;                     // [slot][RED_BLOCKS] in global memory
 	__device__ explicit GridReduce(double* p) : g(cg::this_grid()), partial(p) {}
@@ -76,38 +88,91 @@ struct GridReduce {
 		g.sync();
 		return final_sum(partial + slot * RED_BLOCKS);
 	}
+	__device__ double norm(double v, int slot, double& inv)
+	{
+		const double b = sqrt(sum(v, slot));
+		inv = 1.0 / b;
+		return b;
+	}
 	__device__ void sync() { g.sync(); }
 	__device__ void finish() {}
 };
 
+template <bool STEADY>
 struct ClusterReduce {
+	static constexpr bool steady = STEADY;
 	cg::cluster_group c;
 	double* part;                        // [3] this block's partial sum per slot (shared memory)
 	double* red;                         // [RED_THREADS / 32] per-warp sums (shared memory)
-	double* bc;                          // [3] the cluster's sum per slot (shared memory)
+	double* bc;                          // [3] the cluster's sum per slot (shared memory); [2] also the norm's reciprocal
 	__device__ ClusterReduce(double* p, double* r, double* b) : c(cg::this_cluster()), part(p), red(r), bc(b) {}
 	__device__ int blocks() const { return (int)c.num_blocks(); }
 	__device__ int block() const { return (int)c.block_rank(); }
-	__device__ double sum(double v, int slot)
+	// the sum in the first warp (every lane)
+	__device__ double first_warp_sum(double v, int slot)
 	{
 		v = warp_sum(v);
 		if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
 		__syncthreads();
-		if (threadIdx.x == 0)
+		if constexpr (STEADY)
 		{
-			double t = 0;
-			for (int w = 0; w < RED_THREADS / 32; w++) t += red[w];
-			part[slot] = t;
+			if (threadIdx.x == 0)
+			{
+				double t = 0;
+				for (int w = 0; w < RED_THREADS / 32; w++) t += red[w];
+				part[slot] = t;
+			}
+		}
+		else if (threadIdx.x < 32)
+		{
+			const int nw = (int)blockDim.x >> 5;
+			double t = (int)threadIdx.x < nw ? red[threadIdx.x] : 0.0;
+			for (int o = nw >> 1; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+			if (threadIdx.x == 0) part[slot] = t;
 		}
 		c.sync();
+		if (threadIdx.x >= 32) return 0.0;
+		// the blocks' partial sums in rank order, added by the fixed butterfly of one warp
+		double t = (int)threadIdx.x < blocks() ? *c.map_shared_rank(part + slot, threadIdx.x) : 0.0;
+		if constexpr (STEADY) return warp_sum(t);
+#pragma unroll
+		for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+		return __shfl_sync(0xffffffffu, t, 0);
+	}
+	__device__ double sum(double v, int slot)
+	{
+		v = first_warp_sum(v, slot);
+		if (threadIdx.x == 0) bc[slot] = v;
+		__syncthreads();
+		return bc[slot];
+	}
+	// the square root of the sum and its reciprocal
+	__device__ double norm(double v, int slot, double& inv)
+	{
+		if constexpr (STEADY)
+		{
+			const double b = sqrt(sum(v, slot));
+			inv = 1.0 / b;
+			return b;
+		}
+		v = first_warp_sum(v, slot);
 		if (threadIdx.x < 32)
 		{
-			// the blocks' partial sums in rank order, added by the fixed butterfly of one warp
-			double t = (int)threadIdx.x < blocks() ? *c.map_shared_rank(part + slot, threadIdx.x) : 0.0;
-			t = warp_sum(t);
-			if (threadIdx.x == 0) bc[slot] = t;
+			double b, r;
+			if (v > 1e-290 && v < 1e290) sqrt_rsqrt64(v, b, r);
+			else
+			{
+				b = sqrt(v);
+				r = 1.0 / b;
+			}
+			if (threadIdx.x == 0)
+			{
+				bc[slot] = b;
+				bc[2] = r;
+			}
 		}
 		__syncthreads();
+		inv = bc[2];
 		return bc[slot];
 	}
 	__device__ void sync() { c.sync(); }
@@ -124,8 +189,8 @@ __device__ void lz_step(R& red, double* __restrict__ w, const double* __restrict
                         double* __restrict__ vj1, i64 n, i64 nthr, int j, int last, LanczosScalars* sc)
 {
 	if (sc->stopped) return;               // read before the first barrier: the same in every block
-	const i64 stride = (i64)red.blocks() * RED_THREADS;
-	const i64 first = (i64)red.block() * RED_THREADS + threadIdx.x;
+	const i64 stride = (i64)red.blocks() * blockDim.x;
+	const i64 first = (i64)red.block() * blockDim.x + threadIdx.x;
 	double v = 0;
 	for (i64 i = first; i < n; i += stride) v = fma(w[i], vj[i], v);
 	const double al = red.sum(v, 0);
@@ -140,11 +205,14 @@ __device__ void lz_step(R& red, double* __restrict__ w, const double* __restrict
 	for (i64 i = first; i < n; i += stride)
 	{
 		// w = w' - alpha_j v_j - beta_{j-1} v_{j-1}, evaluated as in krylov.c:44-53
-		const double x = (j > 0) ? w[i] - (al * vj[i] + be * vjm1[i]) : w[i] - al * vj[i];
+		double x;
+		if constexpr (R::steady) x = (j > 0) ? w[i] - (al * vj[i] + be * vjm1[i]) : w[i] - al * vj[i];
+		else x = fma(-al, vj[i], (j > 0) ? fma(-be, vjm1[i], w[i]) : w[i]);
 		w[i] = x;
 		v = fma(x, x, v);
 	}
-	const double b = sqrt(red.sum(v, 1));
+	double inv;
+	const double b = red.norm(v, 1, inv);
 	const bool stop = b < 100.0 * (double)nthr * DBL_EPSILON;
 	if (red.block() == 0 && threadIdx.x == 0)
 	{
@@ -157,7 +225,6 @@ __device__ void lz_step(R& red, double* __restrict__ w, const double* __restrict
 	}
 	if (!stop)
 	{
-		const double inv = 1.0 / b;
 		for (i64 i = first; i < n; i += stride) vj1[i] = inv * w[i];
 	}
 	red.finish();
@@ -171,6 +238,7 @@ k_lz_step(double* __restrict__ w, const double* __restrict__ vj, const double* _
 	lz_step(red, w, vj, vjm1, vj1, n, nthr, j, last, sc);
 }
 
+template <bool STEADY>
 __global__ void __launch_bounds__(RED_THREADS, 1)
 k_lzc_step(double* __restrict__ w, const double* __restrict__ vj, const double* __restrict__ vjm1,
            double* __restrict__ vj1, i64 n, i64 nthr, int j, int last, LanczosScalars* sc)
@@ -178,7 +246,7 @@ k_lzc_step(double* __restrict__ w, const double* __restrict__ vj, const double* 
 	pdl_wait();
 	pdl_trigger();
 	__shared__ double part[3], wred[RED_THREADS / 32], bc[3];
-	ClusterReduce red(part, wred, bc);
+	ClusterReduce<STEADY> red(part, wred, bc);
 	lz_step(red, w, vj, vjm1, vj1, n, nthr, j, last, sc);
 }
 
@@ -186,11 +254,12 @@ k_lzc_step(double* __restrict__ w, const double* __restrict__ vj, const double* 
 template <class R>
 __device__ void lz_start(R& red, const double* __restrict__ v0, double* __restrict__ v, i64 n, LanczosScalars* sc)
 {
-	const i64 stride = (i64)red.blocks() * RED_THREADS;
-	const i64 first = (i64)red.block() * RED_THREADS + threadIdx.x;
+	const i64 stride = (i64)red.blocks() * blockDim.x;
+	const i64 first = (i64)red.block() * blockDim.x + threadIdx.x;
 	double x = 0;
 	for (i64 i = first; i < n; i += stride) x = fma(v0[i], v0[i], x);
-	const double nrm = sqrt(red.sum(x, 0));
+	double inv;
+	const double nrm = red.norm(x, 0, inv);
 	// a start vector of norm zero (or not finite) admits no Lanczos iteration: fewer iterations than
 	// the one eigenvalue asked for, status -1 (krylov.c:218-223); the later kernels see `stopped`
 	const bool bad = !(nrm > 0.0) || !isfinite(nrm);
@@ -203,7 +272,6 @@ __device__ void lz_start(R& red, const double* __restrict__ v0, double* __restri
 	}
 	if (!bad)
 	{
-		const double inv = 1.0 / nrm;
 		for (i64 i = first; i < n; i += stride) v[i] = inv * v0[i];
 	}
 	red.finish();
@@ -216,19 +284,21 @@ k_lz_start(const double* __restrict__ v0, double* __restrict__ v, i64 n, double*
 	lz_start(red, v0, v, n, sc);
 }
 
+template <bool STEADY>
 __global__ void __launch_bounds__(RED_THREADS, 1)
 k_lzc_start(const double* __restrict__ v0, double* __restrict__ v, i64 n, LanczosScalars* sc)
 {
 	pdl_wait();
 	pdl_trigger();
 	__shared__ double part[3], wred[RED_THREADS / 32], bc[3];
-	ClusterReduce red(part, wred, bc);
+	ClusterReduce<STEADY> red(part, wred, bc);
 	lz_start(red, v0, v, n, sc);
 }
 
 __global__ void __launch_bounds__(RED_THREADS, 1)
 k_lz_finish(const double* __restrict__ w, const double* __restrict__ V, i64 n, int maxiter, double* __restrict__ partial,
             LanczosScalars* sc, double* __restrict__ out);
+template <bool STEADY>
 __global__ void __launch_bounds__(RED_THREADS, 1)
 k_lzc_finish(const double* __restrict__ w, const double* __restrict__ V, i64 n, int maxiter, LanczosScalars* sc,
              double* __restrict__ out);
@@ -249,13 +319,12 @@ static void check_coop(const void* fn)
 
 // blocks of the cluster form on this device: 16 (a non-portable cluster size) where every
 // cluster-form kernel can be scheduled with it, else 8; per device, decided once
-static int lz_cluster(const void* fn)
+static int lz_cluster(const void* fn, int which)
 {
 	static std::mutex mu;
-	static int cache[64][3] = {};
+	static int cache[64][6] = {};
 	int dev = 0;
 	CTG_CUDA(cudaGetDevice(&dev));
-	const int which = fn == (const void*)k_lzc_step ? 0 : fn == (const void*)k_lzc_start ? 1 : 2;
 	std::lock_guard<std::mutex> g(mu);
 	int& c = cache[dev & 63][which];
 	if (c) return c;
@@ -292,14 +361,15 @@ static i64 lz_cluster_max_n()
 	return v;
 }
 
+// which: the kernel's number, 0 to 5; the steady form always has RED_THREADS threads
 template <class... Args>
-static void launch_cluster_form(void (*fn)(Args...), cudaStream_t st, Args... args)
+static void launch_cluster_form(int which, void (*fn)(Args...), i64 n, bool steady, cudaStream_t st, Args... args)
 {
-	const int cl = lz_cluster((const void*)fn);
+	const int cl = lz_cluster((const void*)fn, which);
 	cudaLaunchConfig_t cfg = {};
 	cudaLaunchAttribute at[1];
 	cfg.gridDim = dim3(cl);
-	cfg.blockDim = dim3(RED_THREADS);
+	cfg.blockDim = dim3(steady || n > LZ_SMALL_N ? RED_THREADS : 256);
 	cfg.stream = st;
 	at[0].id = cudaLaunchAttributeClusterDimension;
 	at[0].val.clusterDim.x = cl;
@@ -311,11 +381,12 @@ static void launch_cluster_form(void (*fn)(Args...), cudaStream_t st, Args... ar
 }
 
 void launch_lz_step(double* w, const double* vj, const double* vjm1, double* vj1, i64 n, i64 nthr, int j, int last,
-                    double* partial, LanczosScalars* sc, cudaStream_t st)
+                    double* partial, LanczosScalars* sc, bool steady, cudaStream_t st)
 {
 	if (n <= lz_cluster_max_n())
 	{
-		launch_cluster_form(k_lzc_step, st, w, vj, vjm1, vj1, n, nthr, j, last, sc);
+		launch_cluster_form(steady ? 3 : 0, steady ? k_lzc_step<true> : k_lzc_step<false>, n, steady, st, w, vj, vjm1, vj1, n, nthr, j,
+		                    last, sc);
 		return;
 	}
 	check_coop((const void*)k_lz_step);
@@ -323,11 +394,11 @@ void launch_lz_step(double* w, const double* vj, const double* vjm1, double* vj1
 	CTG_CUDA(cudaLaunchCooperativeKernel((const void*)k_lz_step, dim3(RED_BLOCKS), dim3(RED_THREADS), args, 0, st));
 }
 
-void launch_lz_start(const double* v0, double* v, i64 n, double* partial, LanczosScalars* sc, cudaStream_t st)
+void launch_lz_start(const double* v0, double* v, i64 n, double* partial, LanczosScalars* sc, bool steady, cudaStream_t st)
 {
 	if (n <= lz_cluster_max_n())
 	{
-		launch_cluster_form(k_lzc_start, st, v0, v, n, sc);
+		launch_cluster_form(steady ? 4 : 1, steady ? k_lzc_start<true> : k_lzc_start<false>, n, steady, st, v0, v, n, sc);
 		return;
 	}
 	check_coop((const void*)k_lz_start);
@@ -778,8 +849,8 @@ __device__ void lz_finish(R& red, const double* __restrict__ w, const double* __
 	__shared__ double lam;
 	__shared__ int st;
 	const bool stopped = sc->stopped != 0;          // read before the barrier: the same in every block
-	const i64 stride = (i64)red.blocks() * RED_THREADS;
-	const i64 first = (i64)red.block() * RED_THREADS + threadIdx.x;
+	const i64 stride = (i64)red.blocks() * blockDim.x;
+	const i64 first = (i64)red.block() * blockDim.x + threadIdx.x;
 	const int j = maxiter - 1;
 	double alast = 0.0;
 	if (!stopped)
@@ -841,6 +912,7 @@ k_lz_finish(const double* __restrict__ w, const double* __restrict__ V, i64 n, i
 	lz_finish(red, w, V, n, maxiter, sc, out);
 }
 
+template <bool STEADY>
 __global__ void __launch_bounds__(RED_THREADS, 1)
 k_lzc_finish(const double* __restrict__ w, const double* __restrict__ V, i64 n, int maxiter, LanczosScalars* sc,
              double* __restrict__ out)
@@ -848,16 +920,16 @@ k_lzc_finish(const double* __restrict__ w, const double* __restrict__ V, i64 n, 
 	pdl_wait();
 	pdl_trigger();
 	__shared__ double part[3], wred[RED_THREADS / 32], bc[3];
-	ClusterReduce red(part, wred, bc);
+	ClusterReduce<STEADY> red(part, wred, bc);
 	lz_finish(red, w, V, n, maxiter, sc, out);
 }
 
 void launch_lz_finish(const double* w, const double* V, i64 n, int maxiter, double* partial, LanczosScalars* sc,
-                      double* out, cudaStream_t st)
+                      double* out, bool steady, cudaStream_t st)
 {
 	if (n <= lz_cluster_max_n())
 	{
-		launch_cluster_form(k_lzc_finish, st, w, V, n, maxiter, sc, out);
+		launch_cluster_form(steady ? 5 : 2, steady ? k_lzc_finish<true> : k_lzc_finish<false>, n, steady, st, w, V, n, maxiter, sc, out);
 		return;
 	}
 	check_coop((const void*)k_lz_finish);
