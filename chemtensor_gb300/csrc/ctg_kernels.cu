@@ -382,32 +382,71 @@ void launch_gemm_z(int ntiles, const GemmTile* tiles, const GemmOut* outs, const
 // block permutation (dense_tensor_transpose, dense_tensor.c:799-932)
 // ------------------------------------------------------------------------------------
 
+// Permutations and row maps move one to three megabytes of small blocks: bound by latency (chunk, descriptor,
+// source, result) and by the integer divisions of the index arithmetic. The descriptor, which belongs to
+// the plan, goes to shared memory before the wait on the kernel before, and a thread takes COPY_BATCH
+// entries at a time, their divisions and loads side by side. Hubbard chain at D = 256, per launch: permutations
+// 11.6 -> 6.9 us, row maps 6.4 -> 4.5; the two-site search 251 -> 248.5 ms, the one-site search 59.5 -> 57.7, energy and
+// norm 4.45 -> 4.2. Chunks of 1024 instead of 4096 entries: 5.8 and 3.7 us, the searches within their noise.
+constexpr int COPY_BATCH = 4;
+
+// the block's descriptor to shared memory, by all threads
+template <class D>
+__device__ __forceinline__ void copy_desc(D* to, const D* __restrict__ from)
+{
+	static_assert(sizeof(D) % sizeof(int) == 0, "descriptors are whole words");
+	for (int i = threadIdx.x; i < (int)(sizeof(D) / sizeof(int)); i += blockDim.x) ((int*)to)[i] = ((const int*)from)[i];
+	__syncthreads();
+}
+
 // T = double, or double2 for complex128 entries (same descriptors, element units)
 template <class T>
 __global__ void __launch_bounds__(256)
 k_permute(const Chunk* __restrict__ chunks, const PermDesc* __restrict__ descs, const T* __restrict__ src,
           T* __restrict__ dst)
 {
+	__shared__ PermDesc d;
+	const Chunk ch = chunks[blockIdx.x];
+	copy_desc(&d, descs + ch.desc);
 	pdl_wait();
 	pdl_trigger();
-	const Chunk ch = chunks[blockIdx.x];
-	const PermDesc d = descs[ch.desc];
 	const i64 end = min(d.n, ch.start + (i64)COPY_CHUNK);
 	if (d.n < ((i64)1 << 31))
 	{
 		// 32-bit index arithmetic (64-bit integer division is several times slower)
-		for (int e = (int)ch.start + threadIdx.x; e < (int)end; e += blockDim.x)
+		const int nd = d.ndim;
+		const T* s = src + d.src_off;
+		T* t = dst + d.dst_off;
+		for (int e0 = (int)ch.start + threadIdx.x; e0 < (int)end; e0 += COPY_BATCH * blockDim.x)
 		{
-			unsigned r = (unsigned)e;
-			i64 so = 0;
-			for (int i = d.ndim - 1; i >= 0; i--)
+			unsigned r[COPY_BATCH];
+			i64 so[COPY_BATCH];
+			T v[COPY_BATCH];
+#pragma unroll
+			for (int u = 0; u < COPY_BATCH; u++)
+			{
+				r[u] = (unsigned)e0 + u * blockDim.x;
+				so[u] = 0;
+			}
+			for (int i = nd - 1; i > 0; i--)
 			{
 				const unsigned di = (unsigned)d.dims[i];
-				const unsigned q = r / di;
-				so += (i64)(r - q * di) * d.sstr[i];
-				r = q;
+				const i64 st = d.sstr[i];
+#pragma unroll
+				for (int u = 0; u < COPY_BATCH; u++)
+				{
+					const unsigned q = r[u] / di;
+					so[u] += (i64)(r[u] - q * di) * st;
+					r[u] = q;
+				}
 			}
-			dst[d.dst_off + e] = src[d.src_off + so];
+			const i64 st0 = d.sstr[0];
+#pragma unroll
+			for (int u = 0; u < COPY_BATCH; u++)
+				if (e0 + u * (int)blockDim.x < (int)end) v[u] = s[so[u] + (i64)r[u] * st0];
+#pragma unroll
+			for (int u = 0; u < COPY_BATCH; u++)
+				if (e0 + u * (int)blockDim.x < (int)end) t[e0 + u * blockDim.x] = v[u];
 		}
 		return;
 	}
@@ -443,10 +482,11 @@ __global__ void __launch_bounds__(256)
 k_rowmap(const Chunk* __restrict__ chunks, const RowDesc* __restrict__ descs, const i64* __restrict__ maps,
          const T* __restrict__ src, T* __restrict__ dst)
 {
+	__shared__ RowDesc d;
+	const Chunk ch = chunks[blockIdx.x];
+	copy_desc(&d, descs + ch.desc);
 	pdl_wait();
 	pdl_trigger();
-	const Chunk ch = chunks[blockIdx.x];
-	const RowDesc d = descs[ch.desc];
 	const i64 n = d.nlead * d.nrow * d.ntrail;
 	const i64 end = min(n, ch.start + (i64)COPY_CHUNK);
 	const i64* map = maps + d.map_off;
@@ -454,17 +494,33 @@ k_rowmap(const Chunk* __restrict__ chunks, const RowDesc* __restrict__ descs, co
 	{
 		// 32-bit index arithmetic (64-bit integer division is several times slower)
 		const unsigned nt = (unsigned)d.ntrail, nr = (unsigned)d.nrow;
-		for (unsigned e = (unsigned)ch.start + threadIdx.x; e < (unsigned)end; e += blockDim.x)
+		const bool scatter = d.scatter != 0;
+		const i64 srows = d.src_rows, drows = d.dst_rows;
+		const T* s = src + d.src_off;
+		T* o = dst + d.dst_off;
+		for (unsigned e0 = (unsigned)ch.start + threadIdx.x; e0 < (unsigned)end; e0 += COPY_BATCH * blockDim.x)
 		{
-			const unsigned lj = e / nt;
-			const unsigned t = e - lj * nt;
-			const unsigned lead = lj / nr;
-			const unsigned j = lj - lead * nr;
-			const i64 mj = map[j];
-			const i64 srow = d.scatter ? (i64)j : mj;
-			const i64 drow = d.scatter ? mj : (i64)j;
-			dst[d.dst_off + ((i64)lead * d.dst_rows + drow) * d.ntrail + t] =
-				src[d.src_off + ((i64)lead * d.src_rows + srow) * d.ntrail + t];
+			unsigned t[COPY_BATCH], lead[COPY_BATCH], j[COPY_BATCH];
+			i64 mj[COPY_BATCH];
+			T v[COPY_BATCH];
+#pragma unroll
+			for (int u = 0; u < COPY_BATCH; u++)
+			{
+				const unsigned e = e0 + u * blockDim.x;
+				const unsigned lj = e / nt;
+				t[u] = e - lj * nt;
+				lead[u] = lj / nr;
+				j[u] = lj - lead[u] * nr;
+				if (e < (unsigned)end) mj[u] = map[j[u]];
+			}
+#pragma unroll
+			for (int u = 0; u < COPY_BATCH; u++)
+				if (e0 + u * blockDim.x < (unsigned)end)
+					v[u] = s[((i64)lead[u] * srows + (scatter ? (i64)j[u] : mj[u])) * nt + t[u]];
+#pragma unroll
+			for (int u = 0; u < COPY_BATCH; u++)
+				if (e0 + u * blockDim.x < (unsigned)end)
+					o[((i64)lead[u] * drows + (scatter ? mj[u] : (i64)j[u])) * nt + t[u]] = v[u];
 		}
 		return;
 	}
