@@ -2,7 +2,7 @@
 //
 // A kernel launched with the programmatic-stream-serialisation attribute may be scheduled while
 // the kernel before it in the stream is still finishing; it waits at griddepcontrol.wait, before
-// its first global-memory access, until that kernel has completed and its writes are visible. A
+// its first access to memory that kernels write, until that kernel has completed and its writes are visible. A
 // kernel that calls pdl_trigger() lets the next one be scheduled once all of its own blocks have
 // started. The launch setup of consecutive kernels then overlaps their execution instead of
 // following it (a sweep runs a few thousand launches). CTGPU_PDL=0 launches without the attribute.
@@ -16,7 +16,9 @@
 
 namespace ctg {
 
-// first statement of every kernel launched by launch_pdl
+// in every kernel launched by launch_pdl, before the first access to memory that an earlier kernel may have
+// written or may still read. Lists that belong to a plan may be read before it: they were uploaded by a copy
+// in the same stream, for which a kernel launch waits in full, and no kernel writes them.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
