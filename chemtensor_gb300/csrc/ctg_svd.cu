@@ -69,7 +69,13 @@ constexpr float SVD_F32_COS = 0.0f;           // default: FP32 sweeps rotate eve
 // 104.9 ms from rank 32 on, 101.2 from 20, 99.1 from 16, 99.0 from 12 and 98.9 from 8 on.
 constexpr int SVD_F32_MIN_RANK = 16;
 constexpr int SVD_F32_MIN_FULL = 32;          // the same where the caller keeps all factors or a steady basis
-constexpr int SVD_F32_CLUSTER = 8;            // default: CTAs of the FP32 sweeps
+constexpr int SVD_F32_CLUSTER = 8;            // default: most CTAs of the FP32 sweeps
+// A smaller rank takes half the CTAs while their groups then hold no more columns than this: as many pairs per
+// step as a CTA has warps, and half the rounds, each with an exchange over the cluster (1500 clocks, as
+// much as two steps). The order of the pairs, and with it the signs of the columns, is another, so callers
+// that keep all factors keep all CTAs. Spin chain at D = 32 (ranks up to 32) 91.5 -> 89.1 ms, Hubbard chain at
+// D = 100 (up to 90) 70.0 -> 68.5, at D = 256 the same; twelve columns: 92.2, 71.8 and 257.
+constexpr int SVD_F32_PAIRS = 8;
 constexpr int SVD_OUT_RC = 32;                // reflectors staged per round of the output phase
 constexpr int SVD_OUT_WARPS = 8;              // warps with a column in the output phase (twelve: 7.5 for 6.8 ms per sweep)
 
@@ -1790,7 +1796,7 @@ __global__ void __launch_bounds__(SVD_THREADS_MAX, 1)
 k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restrict__ a, double* __restrict__ u,
            double* __restrict__ s, double* __restrict__ vh, double* __restrict__ scratch, int* __restrict__ status,
            double* __restrict__ flops, int cl, int smem_bytes, unsigned long long* __restrict__ phase_ts, int f32_min,
-           int f32_cl, int refine, double tail2, int f32_sweeps, float f32_cos, float f32_wide)
+           int f32_cl, int refine, double tail2, int f32_sweeps, float f32_cos, float f32_wide, int full)
 {
 	extern __shared__ __align__(16) double smem[];
 	cg::cluster_group cluster = cg::this_cluster();
@@ -1878,6 +1884,8 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	long long* cyc = count ? cyc_acc : nullptr;
 	// FP32 sub-cluster: the requested size, or larger until its column groups fit
 	int cf = f32_cl < cl ? f32_cl : cl;
+	if (!full)
+		while (cf > 1 && r <= SVD_F32_PAIRS * cf) cf /= 2;
 	while (cf < cl && f32_tour_bytes(N, r, cf) > (i64)smem_bytes) cf *= 2;
 	const bool mixed = f32_min > 0 && r >= f32_min && 8 * refine_doubles(N, cl) <= (i64)smem_bytes &&
 	                   f32_tour_bytes(N, r, cf) <= (i64)smem_bytes;
@@ -2644,7 +2652,7 @@ void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* d
 		});
 	CTG_CUDA(cudaLaunchKernelEx(&cfg, k_svd_tour, descs, first, a, u, s, vh, scratch, status, flops, g.cluster, g.smem,
 	                             phase_ts, f32_min, svd_f32_cluster(), svd_refine(), discard2, svd_f32_sweeps(),
-	                             svd_f32_cos(), steady ? FLT_MAX : svd_f32_wide()));
+	                             svd_f32_cos(), steady ? FLT_MAX : svd_f32_wide(), full ? 1 : 0));
 }
 
 }  // namespace ctg
