@@ -524,6 +524,7 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 		CTG_CUDA(cudaMemsetAsync(p.counters->ptr, 0, l.splits.size() * sizeof(int), c.stream()));
 	}
 	p.ntiles[0] = (int)l.tiles.size();
+	for (const GemmTile& t : l.tiles) p.large |= t.cls == TILE_L;
 	p.tiles[0] = at<GemmTile>(p.desc, o_tiles);
 	p.flops = l.flops;
 	for (int k = 0; k < NUM_TILE_CLASSES; k++) p.flops_cls[k] = l.flops_cls[k];
@@ -572,7 +573,7 @@ void DotPlan::launch_f64(Ctx& c, const double* A, const double* B, double* C) co
 		run_slices(c, A, B, pa.ptr, pb.ptr, C, nullptr);
 	}
 	else if (ntiles[0] > 0)
-		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops, flops_cls[TILE_L] > 0);
+		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops, large);
 }
 
 // the groups' exponents in front of the digits, which start on a 256-byte boundary

@@ -202,6 +202,7 @@ struct DotPlan {
 	int tc_bn = 64;                      // tile columns, from the tile autotuner
 	double flops = 0;
 	double flops_cls[NUM_TILE_CLASSES] = {};
+	bool large = false;                  // some FP64 tile is a TILE_L (also one without terms)
 	int precision = GEMM_FP64;
 	void run(Ctx& c, const double* A, const double* B, double* C) const;
 	// the FP64 product's launches alone (no counters)

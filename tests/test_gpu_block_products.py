@@ -52,3 +52,39 @@ def test_block_product(gpu, m, n, kind, lead):
     assert np.all(np.abs(got - np.tensordot(A, B, axes)) <= bound)
     for x in (out, ca, cb):
         cs.free_bst(x)
+
+
+_EMPTY_LARGE = """
+import ctypes as C
+import numpy as np
+from chemtensor_gb300 import ctstructs as cs, native
+from helpers import c_bst
+lib = native.lib()
+rng = np.random.default_rng(3)
+k = 60000
+q = lambda *n: np.concatenate([np.full(c, i) for i, c in enumerate(n)]).astype(np.int32)
+a = cs.BlockSparse((140, k), (1, -1), [q(40, 100), np.zeros(k, np.int32)])
+b = cs.BlockSparse((k, 140), (1, -1), [np.zeros(k, np.int32), q(40, 100)])
+for t in (a, b):
+    for idx in t.allowed:
+        t.blocks[idx] = rng.standard_normal(t.block_shape(idx))
+A, B = a.to_dense(), b.to_dense()
+for _ in range(2):                             # dirty the allocator's memory, then use it
+    ca, cb, out = c_bst(a), c_bst(b), cs.BlockSparseTensor()
+    assert lib.ctgpu_block_sparse_tensor_dot(C.byref(ca), 1, C.byref(cb), 0, 1, C.byref(out)) == 0
+    got = cs.read_bst(out).to_dense()
+    bound = 2 * (k + 2) * np.finfo(np.float64).eps * (np.abs(A) @ np.abs(B))
+    assert np.all(np.abs(got - A @ B) <= bound)
+"""
+
+
+def test_large_block_without_terms(gpu):
+    """A product large enough for the largest tiles whose only block of that size has no terms: the block is
+    zeros. (On the FP64 tiles: the digit slices, which such products normally take, are off.)"""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, CTGPU_SLICE_GEMM="0", PYTHONPATH=os.pathsep.join([root, os.path.join(root, "tests")]))
+    r = subprocess.run([sys.executable, "-c", _EMPTY_LARGE], cwd=root, env=env, capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
