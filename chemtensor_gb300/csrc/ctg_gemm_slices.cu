@@ -278,6 +278,13 @@ k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* 
 // the products
 // ------------------------------------------------------------------------------------
 
+// whether the results of two groups with these exponents are zeros: not where a number that is not finite
+// meets them (NaN)
+__device__ __forceinline__ bool zero_result(int e, int f)
+{
+	return (e == 0 && f != 0x7ff) || (f == 0 && e != 0x7ff);
+}
+
 // whether the results of two groups with these exponents are summed in FP64
 __device__ __forceinline__ bool sum_again(int e, int f)
 {
@@ -644,7 +651,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 					}
 					// results in place of the sums; `again`: they are summed in FP64 below
 					const int top = slice_top(tile.e, tile.f);
-					const bool zero = tile.e == 0 || tile.f == 0, again = !zero && sum_again(tile.e, tile.f);
+					const bool zero = zero_result(tile.e, tile.f), again = !zero && sum_again(tile.e, tile.f);
 					int emax = 0;
 					if (zero)
 					{
@@ -748,7 +755,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 							hi += v.x;
 							lo += v.y;
 						}
-						const bool zero = tile.e == 0 || tile.f == 0;
+						const bool zero = zero_result(tile.e, tile.f);
 						const double sum = zero ? 0.0 : __longlong_as_double((long long)slice_value(hi, lo, slice_top(tile.e, tile.f)));
 						C[gemm_out_index(outs[sp.out], sp.m0 + i, sp.n0 + j)] = sum;
 						if (!zero && sum_again(tile.e, tile.f))
