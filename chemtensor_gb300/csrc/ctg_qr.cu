@@ -97,28 +97,37 @@ __device__ __forceinline__ double warp_sum(double v)
 }
 
 // The reflector of (alpha, x), xn2 = |x|^2: H^H (alpha, x) = (beta, 0), H^H = I - f v v^H, v = (v0, x). f = 0: H = I.
-// Squared norms below 1e-290 (of a block whose entries lie in a normal range) are zeros to all purposes,
-// and the reciprocals want normal numbers.
+// Squared norms below 1e-306 (of a block whose entries lie in a normal range) are zeros to all purposes: f,
+// their reciprocal, must stay a number. The functions of ctg_fp64.cuh want normal numbers and their
+// reciprocals: squared norms beyond 1e-290 and 1e290, infinities and NaN (which stay NaN in the factors, as
+// in LAPACK) take the IEEE operations.
+__device__ __forceinline__ bool plain_range(double n2) { return n2 > 1e-290 && n2 < 1e290; }
+__device__ __noinline__ double ieee_sqrt(double x) { return sqrt(x); }
+__device__ __noinline__ double ieee_rcp(double x) { return 1.0 / x; }
 __device__ __forceinline__ void reflector(double alpha, double xn2, double& beta, double& v0, double& f)
 {
 	const double n2 = fma(alpha, alpha, xn2);
 	beta = alpha;
 	v0 = f = 0.0;
-	if (xn2 == 0.0 || n2 <= 1e-290) return;
-	const double nrm = sqrt64(n2);
+	if (xn2 == 0.0 || n2 <= 1e-306) return;
+	const bool plain = plain_range(n2);
+	const double nrm = plain ? sqrt64(n2) : ieee_sqrt(n2);
 	beta = -copysign(nrm, alpha);
 	v0 = alpha - beta;
-	f = rcp64(fma(nrm, fabs(alpha), n2));
+	const double d = fma(nrm, fabs(alpha), n2);
+	f = plain ? rcp64(d) : ieee_rcp(d);
 }
 __device__ __forceinline__ void reflector(double2 alpha, double xn2, double& beta, double2& v0, double2& f)
 {
 	const double n2 = abs2(alpha, xn2);
 	beta = alpha.x;
 	v0 = f = make_double2(0.0, 0.0);
-	if ((xn2 == 0.0 && alpha.y == 0.0) || n2 <= 1e-290) return;
-	beta = -copysign(sqrt64(n2), alpha.x);
+	if ((xn2 == 0.0 && alpha.y == 0.0) || n2 <= 1e-306) return;
+	const bool plain = plain_range(n2);
+	beta = -copysign(plain ? sqrt64(n2) : ieee_sqrt(n2), alpha.x);
 	v0 = make_double2(alpha.x - beta, alpha.y);
-	const double rb = rcp64(beta), rv = rcp64(abs2(v0, 0.0));
+	const double d = abs2(v0, 0.0);
+	const double rb = plain ? rcp64(beta) : ieee_rcp(beta), rv = plain ? rcp64(d) : ieee_rcp(d);
 	f = make_double2(-v0.x * rb * rv, v0.y * rb * rv);
 }
 
