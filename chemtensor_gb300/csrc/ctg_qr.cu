@@ -456,8 +456,9 @@ void launch_qr_blocks(int nblocks, const RqDesc* descs, const RqDesc* host, cons
 		const i64 need = qr_entries(host[b].m, host[b].n, std::min(host[b].m, host[b].n)) * (i64)sizeof(T);
 		if (need <= QR_SMEM_LIMIT) smem = std::max(smem, need);
 	}
-	if (smem > 48 * 1024)
-		CTG_CUDA(cudaFuncSetAttribute(k_qr_householder<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, QR_SMEM_LIMIT));
+	// for every size: the limit that holds without it, 48 KB, counts the kernel's static shared memory too. The
+	// attribute belongs to the current device.
+	CTG_CUDA(cudaFuncSetAttribute(k_qr_householder<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, QR_SMEM_LIMIT));
 	k_qr_householder<T><<<nblocks, QR_THREADS, (size_t)smem, st>>>(descs, (const T*)a, (T*)r, (T*)q, (T*)scratch, (int)smem);
 	CTG_CUDA(cudaGetLastError());
 }
