@@ -449,11 +449,8 @@ struct LocalH {
 	DBufPtr pk_r, pk_w, pk_k, pk_x, pk_t1, pk_t2;   // packed tensor-core operands
 	bool tc1 = false, tc2 = false, tc3 = false;     // product on the tensor cores (else FP64)
 	bool s1 = false, s2 = false, s3 = false;        // FP64 product by digit slices
-	// their packed operands (r, w, k once per bond) and the exponents of the operands' blocks: x's per
-	// application (two arrays in turn: taking one clears the other and those of the intermediates), the
-	// intermediates' from the product that writes them
-	DBufPtr sp_r, sp_w, sp_k, sp_x, sp_t1, sp_t2, exps;
-	int *e_x[2] = {nullptr, nullptr}, *e_t1 = nullptr, *e_t2 = nullptr;
+	// their packed operands: r, w, k once per bond, x and the intermediates per application (turn: DotPlan::slice_pack)
+	DBufPtr sp_r, sp_w, sp_k, sp_x, sp_t1, sp_t2;
 	mutable int turn = 0;
 	bool f1 = false, f2 = false;     // intermediate in FP32 (written and read by tensor-core products only)
 	bool z = false;                  // complex128 entries
@@ -503,41 +500,31 @@ struct LocalH {
 		s1 = d1.nstiles > 0;
 		s2 = d2.nstiles > 0;
 		s3 = d3.nstiles > 0;
-		if (s1 || s2 || s3)
+		auto buf = [&](const DotPlan& d, int s) {
+			DBufPtr p = std::make_shared<DBuf>(&c, (size_t)d.slice_bytes(s));
+			d.slice_clear(c, s, p->ptr);
+			return p;
+		};
+		auto fixed = [&](const DotPlan& d, int s, const double* x) {
+			DBufPtr p = buf(d, s);
+			KScope ks(c, K_GEMM, 2);
+			d.slice_pack(c, s, x, p->ptr, 0);
+			return p;
+		};
+		if (s1)
 		{
-			const size_t nf = std::max({(size_t)r.m().nblocks, (size_t)w.m().nblocks, (size_t)k.m().nblocks}),
-			             nx = (size_t)a.nblocks, n1 = (size_t)d1.out->nblocks, n2 = (size_t)d2.out->nblocks;
-			exps = std::make_shared<DBuf>(&c, (2 * nx + n1 + n2) * sizeof(int));
-			CTG_CUDA(cudaMemsetAsync(exps->ptr, 0, exps->bytes, c.stream()));
-			e_x[0] = (int*)exps->ptr;
-			e_t1 = e_x[0] + nx;
-			e_t2 = e_t1 + n1;
-			e_x[1] = e_t2 + n2;
-			auto buf = [&](const DotPlan& d, int s) { return std::make_shared<DBuf>(&c, (size_t)d.slice_bytes(s)); };
-			DBuf e(&c, 3 * nf * sizeof(int));
-			CTG_CUDA(cudaMemsetAsync(e.ptr, 0, e.bytes, c.stream()));
-			auto fixed = [&](const DotPlan& d, int s, const double* x, int* ex) {
-				DBufPtr p = buf(d, s);
-				KScope ks(c, K_GEMM, 2);
-				d.block_exps(c, s, x, ex);
-				d.slice_pack(c, s, x, ex, p->ptr);
-				return p;
-			};
-			if (s1)
-			{
-				sp_r = fixed(d1, 1, r.data(), (int*)e.ptr);
-				sp_x = buf(d1, 0);
-			}
-			if (s2)
-			{
-				sp_w = fixed(d2, 0, w.data(), (int*)e.ptr + nf);
-				sp_t1 = buf(d2, 1);
-			}
-			if (s3)
-			{
-				sp_k = fixed(d3, 0, k.data(), (int*)e.ptr + 2 * nf);
-				sp_t2 = buf(d3, 1);
-			}
+			sp_r = fixed(d1, 1, r.data());
+			sp_x = buf(d1, 0);
+		}
+		if (s2)
+		{
+			sp_w = fixed(d2, 0, w.data());
+			sp_t1 = buf(d2, 1);
+		}
+		if (s3)
+		{
+			sp_k = fixed(d3, 0, k.data());
+			sp_t2 = buf(d3, 1);
 		}
 		// operands fixed for the bond (r, w, k) are packed once; x and the intermediates per apply
 		auto rec = [&](i64 bytes) { return std::make_shared<DBuf>(&c, (size_t)std::max<i64>(bytes, 16)); };
@@ -581,11 +568,8 @@ struct LocalH {
 		else if (s1)
 		{
 			KScope ks(c, K_GEMM, 3, d1.flops, 0);
-			// cleared: [x0 t1 t2] or [t1 t2 x1]
-			d1.block_exps(c, 0, x, e_x[turn], turn ? e_x[0] : e_t1, (int)(e_x[1] - e_x[0]));
-			d1.slice_pack(c, 0, x, e_x[turn], sp_x->ptr);
-			d1.run_slices(c, x, r.data(), sp_x->ptr, sp_r->ptr, t1, e_t1);
-			turn ^= 1;
+			d1.slice_pack(c, 0, x, sp_x->ptr, turn);
+			d1.run_slices(c, x, r.data(), sp_x->ptr, sp_r->ptr, t1);
 			c.gemm_flops += d1.flops;
 		}
 		else d1.run(c, x, r.data(), t1);
@@ -597,15 +581,9 @@ struct LocalH {
 		}
 		else if (s2)
 		{
-			KScope ks(c, K_GEMM, s1 ? 2 : 3, d2.flops, 0);
-			if (!s1)
-			{
-				// e_t1, e_t2 lie next to each other
-				CTG_CUDA(cudaMemsetAsync(e_t1, 0, (size_t)(e_x[1] - e_t1) * sizeof(int), c.stream()));
-				d2.block_exps(c, 1, t1, e_t1);
-			}
-			d2.slice_pack(c, 1, t1, e_t1, sp_t1->ptr);
-			d2.run_slices(c, w.data(), t1, sp_w->ptr, sp_t1->ptr, t2, e_t2);
+			KScope ks(c, K_GEMM, 3, d2.flops, 0);
+			d2.slice_pack(c, 1, t1, sp_t1->ptr, turn);
+			d2.run_slices(c, w.data(), t1, sp_w->ptr, sp_t1->ptr, t2);
 			c.gemm_flops += d2.flops;
 		}
 		else d2.run(c, w.data(), t1, t2);
@@ -617,17 +595,13 @@ struct LocalH {
 		}
 		else if (s3)
 		{
-			KScope ks(c, K_GEMM, s2 ? 2 : 3, d3.flops, 0);
-			if (!s2)
-			{
-				CTG_CUDA(cudaMemsetAsync(e_t2, 0, (size_t)(e_x[1] - e_t2) * sizeof(int), c.stream()));
-				d3.block_exps(c, 1, t2, e_t2);
-			}
-			d3.slice_pack(c, 1, t2, e_t2, sp_t2->ptr);
-			d3.run_slices(c, k.data(), t2, sp_k->ptr, sp_t2->ptr, y, nullptr);
+			KScope ks(c, K_GEMM, 3, d3.flops, 0);
+			d3.slice_pack(c, 1, t2, sp_t2->ptr, turn);
+			d3.run_slices(c, k.data(), t2, sp_k->ptr, sp_t2->ptr, y);
 			c.gemm_flops += d3.flops;
 		}
 		else d3.run(c, k.data(), t2, y);
+		turn ^= 1;
 	}
 };
 

@@ -477,13 +477,12 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 	const size_t o_tcons = pk.add(l.tcons), o_apacks = pk.add(l.apacks), o_bpacks = pk.add(l.bpacks);
 	const size_t o_st = pk.add(l.stiles);
 	const size_t o_so = pk.add(l.souts);
-	size_t o_side[2][4] = {};
+	size_t o_side[2][3] = {};
 	for (int q = 0; q < 2 && !l.stiles.empty(); q++)
 	{
 		o_side[q][0] = pk.add(l.spack[q].runs);
 		o_side[q][1] = pk.add(l.spack[q].groups);
 		o_side[q][2] = pk.add(l.spack[q].items);
-		o_side[q][3] = pk.add(l.spack[q].chunks);
 	}
 	// at least 16 bytes, from the packer's own storage (a product without output blocks packs nothing)
 	if (pk.bytes.size() < 16) pk.bytes.resize(16);
@@ -498,14 +497,10 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 		d.runs = at<SliceRun>(p.desc, o_side[q][0]);
 		d.groups = at<SliceGroup>(p.desc, o_side[q][1]);
 		d.items = at<SliceItem>(p.desc, o_side[q][2]);
-		d.chunks = at<SliceChunk>(p.desc, o_side[q][3]);
 		d.nitems = (int)l.spack[q].items.size();
-		d.ngroups = (int)l.spack[q].groups.size();
-		d.nchunks = (int)l.spack[q].chunks.size();
-		d.nblocks = l.spack[q].blocks;
+		d.rows = l.spack[q].rows;
 		d.bytes = l.spack[q].bytes;
 	}
-	p.c_blocks = l.out->nblocks;
 	p.tcons = at<TcContrib>(p.desc, o_tcons);
 	p.apacks = at<TcPack>(p.desc, o_apacks);
 	p.bpacks = at<TcPack>(p.desc, o_bpacks);
@@ -562,46 +557,47 @@ void DotPlan::launch_f64(Ctx& c, const double* A, const double* B, double* C) co
 	int* cnt = counters ? (int*)counters->ptr : nullptr;
 	if (nstiles > 0)
 	{
-		DBuf e(&c, (size_t)(side[0].nblocks + side[1].nblocks) * sizeof(int));
-		int *ea = (int*)e.ptr, *eb = ea + side[0].nblocks;
-		CTG_CUDA(cudaMemsetAsync(e.ptr, 0, e.bytes, c.stream()));
 		DBuf pa(&c, (size_t)slice_bytes(0)), pb(&c, (size_t)slice_bytes(1));
-		block_exps(c, 0, A, ea);
-		block_exps(c, 1, B, eb);
-		slice_pack(c, 0, A, ea, pa.ptr);
-		slice_pack(c, 1, B, eb, pb.ptr);
-		run_slices(c, A, B, pa.ptr, pb.ptr, C, nullptr);
+		slice_clear(c, 0, pa.ptr);
+		slice_clear(c, 1, pb.ptr);
+		slice_pack(c, 0, A, pa.ptr, 0);
+		slice_pack(c, 1, B, pb.ptr, 0);
+		run_slices(c, A, B, pa.ptr, pb.ptr, C);
 	}
 	else if (ntiles[0] > 0)
 		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops, large);
 }
 
-// the groups' exponents in front of the digits, which start on a 256-byte boundary
-static size_t slice_head(const DotPlan::Side& d) { return ((size_t)d.ngroups * sizeof(int) + 255) & ~(size_t)255; }
+// a packed operand: two arrays of codes, the exponents, and the digits from a 256-byte boundary on
+static size_t slice_head(const DotPlan::Side& d) { return ((size_t)d.rows * (2 * sizeof(int) + sizeof(short)) + 255) & ~(size_t)255; }
+static int* slice_codes(const DotPlan::Side& d, void* pack, int turn) { return (int*)pack + (turn ? d.rows : 0); }
+static short* slice_exps(const DotPlan::Side& d, const void* pack) { return (short*)((int*)pack + 2 * (size_t)d.rows); }
 
 i64 DotPlan::slice_bytes(int s) const { return (i64)slice_head(side[s]) + std::max<i64>(side[s].bytes, 16); }
 
-void DotPlan::block_exps(Ctx& c, int s, const double* x, int* exps, int* clear, int nclear) const
+void DotPlan::slice_clear(Ctx& c, int s, void* pack) const
 {
-	launch_block_exps(side[s].nchunks, side[s].chunks, x, exps, clear, nclear, c.stream());
+	CTG_CUDA(cudaMemsetAsync(pack, 0, 2 * (size_t)side[s].rows * sizeof(int), c.stream()));
 }
 
-void DotPlan::slice_pack(Ctx& c, int s, const double* x, const int* exps, void* pack) const
+void DotPlan::slice_pack(Ctx& c, int s, const double* x, void* pack, int turn) const
 {
 	const Side& d = side[s];
+	int* codes = slice_codes(d, pack, turn);
+	launch_slice_exps(d.nitems, d.items, d.groups, d.runs, x, codes, slice_codes(d, pack, turn ^ 1), d.rows, c.stream());
 	// orient 0: B lies along the MMA rows
-	launch_slice_pack(d.nitems, d.items, d.groups, d.runs, (orient == 0) == (s == 1), x, exps, (char*)pack + slice_head(d),
-	                  (int*)pack, c.stream());
+	launch_slice_pack(d.nitems, d.items, d.groups, d.runs, (orient == 0) == (s == 1), x, codes, (char*)pack + slice_head(d),
+	                  slice_exps(d, pack), c.stream());
 }
 
-void DotPlan::run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C, int* exp_c) const
+void DotPlan::run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C) const
 {
 	const int x = orient ? 0 : 1;
 	const void* pack[2] = {apack, bpack};
 	launch_gemm_slices(nstiles, stiles, outs, souts, cons, splits, counters ? (int*)counters->ptr : nullptr, orient, A, B,
 	                   (const char*)pack[x] + slice_head(side[x]), (const char*)pack[1 - x] + slice_head(side[1 - x]),
-	                   (const int*)pack[x], (const int*)pack[1 - x], C, exp_c, work ? (double*)work->ptr : nullptr, c.tc_error(),
-	                   c.num_sms(), c.stream());
+	                   slice_exps(side[x], pack[x]), slice_exps(side[1 - x], pack[1 - x]), C, work ? (double*)work->ptr : nullptr,
+	                   c.tc_error(), c.num_sms(), c.stream());
 }
 
 void DotPlan::run_z(Ctx& c, const double* A, const double* B, double* C, bool conj_a, bool conj_b) const

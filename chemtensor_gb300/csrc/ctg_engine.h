@@ -187,11 +187,9 @@ struct DotPlan {
 		const SliceRun* runs = nullptr;
 		const SliceGroup* groups = nullptr;
 		const SliceItem* items = nullptr;
-		const SliceChunk* chunks = nullptr;
-		int nitems = 0, ngroups = 0, nchunks = 0, nblocks = 0;
+		int nitems = 0, rows = 0;
 		i64 bytes = 0;
 	} side[2];
-	int c_blocks = 0;                    // blocks of the result
 	i64 a_entries = 0, b_entries = 0;    // entries of the two operand tensors
 	// tensor-core path: packed operand records (see launch_tc_pack) and per-contribution records
 	const TcContrib* tcons = nullptr;
@@ -207,13 +205,13 @@ struct DotPlan {
 	void run(Ctx& c, const double* A, const double* B, double* C) const;
 	// the FP64 product's launches alone (no counters)
 	void launch_f64(Ctx& c, const double* A, const double* B, double* C) const;
-	// a product by digit slices in parts, so that an operand used by many runs is packed once, and the
-	// exponents of a result's blocks for the next product come from this one. A packed operand is one
-	// buffer: the groups' exponents, then the digits (slice_bytes)
+	// a product by digit slices in parts, so that an operand used by many runs is packed once. A packed operand is
+	// one buffer (slice_bytes): two arrays of its rows' exponent codes, used in turn (a call of slice_pack clears
+	// the other one; both are zero before the first, slice_clear), the rows' exponents and the digits
 	i64 slice_bytes(int s) const;
-	void block_exps(Ctx& c, int s, const double* x, int* exps, int* clear = nullptr, int nclear = 0) const;
-	void slice_pack(Ctx& c, int s, const double* x, const int* exps, void* pack) const;
-	void run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C, int* exp_c) const;
+	void slice_clear(Ctx& c, int s, void* pack) const;
+	void slice_pack(Ctx& c, int s, const double* x, void* pack, int turn) const;
+	void run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C) const;
 	// complex128 entries, operands optionally read conjugated
 	void run_z(Ctx& c, const double* A, const double* B, double* C, bool conj_a, bool conj_b) const;
 	// tensor-core path in parts, so that an operand used by many runs is packed once; src_f32: the

@@ -2,10 +2,10 @@
 //
 // GB300 retires about two FP64 FMAs per clock and SM, its tensor cores about four thousand FP16 ones:
 // the 36 digit products that stand for one FP64 product cost a fiftieth of the FMA. The sums over
-// the digits are exact, so a result carries one rounding and the cut at 2^-62 of its operands' blocks'
-// largest entries, less than the rounding of an FMA chain.
+// the digits are exact, so a result carries one rounding and the cut at 2^-62 of its two rows' largest
+// entries (ctg_slices.h).
 //
-//   k_block_exps   the largest exponent of every block of an operand (the scale of its digits)
+//   k_slice_exps   the largest exponent of every row of an operand (the scale of its digits)
 //   k_slice_pack   cuts an operand into FP16 digits: per group of rows (the blocks with the same free
 //                  indices) the terms of all its blocks one after the other, 16 terms at a time, in the
 //                  canonical K-major core-matrix layout, so that a stage of the GEMM is two bulk copies.
@@ -25,8 +25,8 @@
 // FP64 pipe, 0.62 ms here and 0.24 ms for the digits (1.06 ms with the conversion inside the GEMM). The
 // first two products are bound by the epilogue (integer instructions on 2e7 results, tensor pipe 28 and
 // 37 % busy), the third, with ten times the terms, by the copies out of L2 (46 %).
-// A tile with an operand block that is not finite or tiny, or whose results may leave the normal range,
-// takes its entries from FP64 sums over the operands. Every wait is bounded and ends when another warp
+// Results of a row that is not finite or tiny, and results that may leave the normal range, are FP64 sums
+// over the operands. Every wait is bounded and ends when another warp
 // has failed.
 #include <algorithm>
 #include <mutex>
@@ -64,7 +64,8 @@ struct SliceInfo {
 	int xstep, ystep, xbytes, ybytes;    // digits (bytes) between stages, and of one
 	int nch, halves;
 	int m0, n0, m, n;
-	int split, sp, block, e, f;          // e, f: largest biased exponents of its operand blocks
+	int split, sp;
+	int xe, ye;                          // where the exponents of its rows begin
 };
 constexpr int SL_BARS = 2 * SL_STAGES + 4 + 4 + 1;
 constexpr int SL_SMEM = SL_STAGES * SL_STAGE + SL_EPI_BYTES + 2 * SL_TILES * (int)sizeof(SliceInfo) + SL_BARS * 8 + 32;
@@ -126,89 +127,39 @@ __device__ __forceinline__ int64_t add_order(int64_t acc, int x, int w)
 	return r;
 }
 
-// biased exponent of a number; 1 for denormal numbers, 0 for zero
-__device__ __forceinline__ int exponent_code(double x)
-{
-	const uint32_t hi = (uint32_t)__double2hiint(x) & 0x7fffffffu;
-	return hi >= 0x00100000u ? (int)(hi >> 20) : (hi | (uint32_t)__double2loint(x)) ? 1 : 0;
-}
-
 // ------------------------------------------------------------------------------------
 // exponents and digits of an operand
 // ------------------------------------------------------------------------------------
 
-// largest exponent code of every operand block, SLICE_CHUNK entries per CTA
-__global__ void __launch_bounds__(256)
-k_block_exps(const SliceChunk* __restrict__ chunks, const double* __restrict__ x, int* __restrict__ exps, int* __restrict__ clear,
-             int nclear)
-{
-	pdl_wait();
-	pdl_trigger();
-	const SliceChunk ch = chunks[blockIdx.x];
-	int e = 0;
-	for (int i = threadIdx.x; i < ch.n; i += 256) e = max(e, exponent_code(x[ch.off + i]));
-	e = (int)__reduce_max_sync(0xffffffffu, (unsigned)e);
-	if ((threadIdx.x & 31) == 0 && e > 0) atomicMax(exps + ch.block, e);
-	for (int i = blockIdx.x * 256 + threadIdx.x; i < nclear; i += gridDim.x * 256) clear[i] = 0;
-}
-
-// bytes 0 and 1 (or 2 and 3) of w, biased digits u = d + 128 of two numbers, as FP16 pairs with the
-// numbers' signs: 0x6400 + u is the FP16 pattern of 1024 + u, and sgn (1024 + u) - sgn 1152 = sgn d
-__device__ __forceinline__ uint32_t digits_f16x2(uint32_t w, bool upper, uint32_t sgn, uint32_t off)
-{
-	const uint32_t p = __byte_perm(w, 0x64646464u, upper ? 0x4342 : 0x4140);
-	uint32_t r;
-	asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(p), "r"(sgn), "r"(off));
-	return r;
-}
-
-// One warp per item: 32 rows of a group by SLICE_ITEM stages of its terms, 8 terms at a time (each lane a
-// row: its 8 entries become 16 bytes of each of the 8 digits). The entries of the next 8 terms are on
-// their way while these are cut.
-constexpr int PACK_WARPS = 4;
-__global__ void __launch_bounds__(PACK_WARPS * 32, 8)
-k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups,
-             const SliceRun* __restrict__ runs, int rows8, const double* __restrict__ x, const int* __restrict__ exps,
-             unsigned char* __restrict__ dst, int* __restrict__ gexps)
-{
-	pdl_wait();
-	pdl_trigger();
-	const int item = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-	if (item >= nitems) return;
-	const SliceItem im = items[item];
-	const SliceGroup g = groups[im.group];
-	int E = 0;
-	for (int c = lane; c < g.nrun; c += 32) E = max(E, exps[runs[g.run0 + c].block]);
-	E = (int)__reduce_max_sync(0xffffffffu, (unsigned)E);
-	if (im.row0 == 0 && im.u0 == 0 && lane == 0) gexps[im.group] = E;
-	// blocks with smaller exponents are summed in FP64, or hold zeros only
-	E = max(E, SLICE_EXP_MIN);
-	const int row = im.row0 + lane;
-	const bool valid = row < g.rows;
-	// destination of the lane's row in stage 0, first 8 terms, digit 0; bytes between digits and stages
-	unsigned char* out = dst + g.base + (lane & 7) * 16;
-	const int groups8 = (g.rows + 7) / 8, groups32 = (g.rows + 31) / 32;
-	const int digit = rows8 ? SL_A_DIGIT : SLICE_COL32_BYTES / SLICES;
-	const i64 stage = rows8 ? (i64)groups8 * SLICE_ROW8_BYTES : (i64)groups32 * SLICE_COL32_BYTES;
-	out += rows8 ? (i64)(row >> 3) * SLICE_ROW8_BYTES : (i64)(row >> 5) * SLICE_COL32_BYTES + (lane >> 3) * SL_B_SBO;
-	const bool store = rows8 ? (row >> 3) < groups8 : true;
-	// place in the terms: block c of the group, term kk of it
-	int c = im.run - 1, kk = 0, kend = 0, sk = 0;
-	const double* p = nullptr;
-	auto next = [&]() {
+// The items of an operand (32 rows of a group, a lane each, by SLICE_ITEM stages of its terms), 8 terms at a time.
+struct SliceReader {
+	const SliceRun* __restrict__ runs;   // the group's
+	const double* __restrict__ x;
+	const double* p;
+	int row, nrun;
+	bool valid;
+	int c, kk, kend, sk;                 // place in the terms: block c of the group, term kk of it
+	__device__ SliceReader(const SliceItem& im, const SliceGroup& g, const SliceRun* r, const double* entries, int row_)
+		: runs(r + g.run0), x(entries), p(nullptr), row(row_), nrun(g.nrun), valid(row_ < g.rows), c(im.run - 1), kk(0), kend(0), sk(0)
+	{
+		next();
+		kk = im.kk;
+	}
+	__device__ __forceinline__ void next()
+	{
 		kk = 0;
-		if (++c < g.nrun)
+		if (++c < nrun)
 		{
-			const SliceRun r = runs[g.run0 + c];
+			const SliceRun r = runs[c];
 			kend = r.k;
 			sk = r.sk;
 			p = x + r.off + (i64)(valid ? row : 0) * r.sr;
 		}
-	};
-	next();
-	kk = im.kk;
-	auto read8 = [&](double v[8]) {
-		if (c < g.nrun && kend - kk >= 8)
+	}
+	// the next 8 terms, zeros past the end
+	__device__ __forceinline__ void read8(double v[8])
+	{
+		if (c < nrun && kend - kk >= 8)
 		{
 			const double* s = p + (i64)kk * sk;
 #pragma unroll
@@ -221,18 +172,91 @@ k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* 
 		for (int t = 0; t < 8; t++)
 		{
 			v[t] = 0.0;
-			if (c < g.nrun)
+			if (c < nrun)
 			{
 				if (valid) v[t] = p[(i64)kk * sk];
 				if (++kk == kend) next();
 			}
 		}
-	};
+	}
+};
+
+constexpr int PACK_WARPS = 4;
+
+// Largest exponent code of every row. A pass of its own: the rows' terms are spread over many items, and the
+// digits need the whole row's code. It reads what the product before has just written, mostly from L2.
+__global__ void __launch_bounds__(PACK_WARPS * 32)
+k_slice_exps(int nitems, const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups,
+             const SliceRun* __restrict__ runs, const double* __restrict__ x, int* __restrict__ codes, int* __restrict__ clear,
+             int nclear)
+{
+	pdl_wait();
+	pdl_trigger();
+	for (int i = blockIdx.x * (PACK_WARPS * 32) + threadIdx.x; i < nclear; i += gridDim.x * (PACK_WARPS * 32)) clear[i] = 0;
+	const int item = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	if (item >= nitems) return;
+	const SliceItem im = items[item];
+	const SliceGroup g = groups[im.group];
+	const int row = im.row0 + lane;
+	SliceReader in(im, g, runs, x, row);
+	const int n8 = (min(SLICE_ITEM * SLICE_STAGE_K, g.ktot - im.u0 * SLICE_STAGE_K) + 7) / 8;
+	uint32_t hi = 0, lo = 0;
+	for (int u = 0; u < n8; u++)
+	{
+		double v[8];
+		in.read8(v);
+#pragma unroll
+		for (int t = 0; t < 8; t++)
+		{
+			hi = max(hi, (uint32_t)__double2hiint(v[t]) & 0x7fffffffu);
+			lo |= (uint32_t)__double2loint(v[t]);
+		}
+	}
+	const int code = hi >= 0x00100000u ? (int)(hi >> 20) : (hi | lo) ? 1 : 0;
+	if (code > 0) atomicMax(codes + g.row0 + row, code);
+}
+
+// bytes 0 and 1 (or 2 and 3) of w, biased digits u = d + 128 of two numbers, as FP16 pairs with the
+// numbers' signs: 0x6400 + u is the FP16 pattern of 1024 + u, and sgn (1024 + u) - sgn 1152 = sgn d
+__device__ __forceinline__ uint32_t digits_f16x2(uint32_t w, bool upper, uint32_t sgn, uint32_t off)
+{
+	const uint32_t p = __byte_perm(w, 0x64646464u, upper ? 0x4342 : 0x4140);
+	uint32_t r;
+	asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(p), "r"(sgn), "r"(off));
+	return r;
+}
+
+// One warp per item, each lane a row: its 8 entries become 16 bytes of each of the 8 digits. The entries of the
+// next 8 terms are on their way while these are cut.
+__global__ void __launch_bounds__(PACK_WARPS * 32, 8)
+k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups,
+             const SliceRun* __restrict__ runs, int rows8, const double* __restrict__ x, const int* __restrict__ codes,
+             unsigned char* __restrict__ dst, short* __restrict__ exps)
+{
+	pdl_wait();
+	pdl_trigger();
+	const int item = blockIdx.x * PACK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	if (item >= nitems) return;
+	const SliceItem im = items[item];
+	const SliceGroup g = groups[im.group];
+	const int row = im.row0 + lane;
+	const int code = codes[g.row0 + row];
+	if (im.u0 == 0) exps[g.row0 + row] = (short)slice_exp(code);
+	// rows with smaller exponents are summed in FP64, or hold zeros only
+	const int E = max(code, SLICE_EXP_MIN);
+	// destination of the lane's row in stage 0, first 8 terms, digit 0; bytes between digits and stages
+	unsigned char* out = dst + g.base + (lane & 7) * 16;
+	const int groups8 = (g.rows + 7) / 8, groups32 = (g.rows + 31) / 32;
+	const int digit = rows8 ? SL_A_DIGIT : SLICE_COL32_BYTES / SLICES;
+	const i64 stage = rows8 ? (i64)groups8 * SLICE_ROW8_BYTES : (i64)groups32 * SLICE_COL32_BYTES;
+	out += rows8 ? (i64)(row >> 3) * SLICE_ROW8_BYTES : (i64)(row >> 5) * SLICE_COL32_BYTES + (lane >> 3) * SL_B_SBO;
+	const bool store = rows8 ? (row >> 3) < groups8 : true;
+	SliceReader in(im, g, runs, x, row);
 	const int stages = (g.ktot + SLICE_STAGE_K - 1) / SLICE_STAGE_K;
 	const int n8 = 2 * min(SLICE_ITEM, stages - im.u0);
 	out += (i64)im.u0 * stage;
 	double v[8];
-	read8(v);
+	in.read8(v);
 	for (int u = 0; u < n8; u++)
 	{
 		uint32_t dig[8][2], sgn[4], off[4];
@@ -251,7 +275,7 @@ k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* 
 			sgn[q] = s2 | 0x3c003c00u;
 			off[q] = s2 ^ 0xe480e480u;
 		}
-		if (u + 1 < n8) read8(v);
+		if (u + 1 < n8) in.read8(v);
 		unsigned char* d = out + (i64)(u >> 1) * stage + (u & 1) * SL_LBO;
 #pragma unroll
 		for (int h = 0; h < 4; h++)
@@ -278,42 +302,25 @@ k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* 
 // the products
 // ------------------------------------------------------------------------------------
 
-// whether the results of two groups with these exponents are zeros: not where a number that is not finite
-// meets them (NaN)
-__device__ __forceinline__ bool zero_result(int e, int f)
+// entry (i, j) of an output block, by FP64 sums
+__device__ __noinline__ void slice_entry_f64(const GemmOut& o, const GemmContrib* cons, const double* A, const double* B, int i,
+                                             int j, double* C)
 {
-	return (e == 0 && f != 0x7ff) || (f == 0 && e != 0x7ff);
-}
-
-// whether the results of two groups with these exponents are summed in FP64
-__device__ __forceinline__ bool sum_again(int e, int f)
-{
-	return e == 0x7ff || f == 0x7ff || e < SLICE_EXP_MIN || f < SLICE_EXP_MIN || !slice_in_range(slice_top(e, f));
-}
-
-// n entries of an output block from (i, j) on, along its columns (along = 1) or rows, by FP64 sums
-__device__ __noinline__ void slice_entries_f64(const GemmOut& o, const GemmContrib* cons, const double* A, const double* B, int i,
-                                               int j, int along, int n, double* C, int* exp_c)
-{
-	for (; n > 0; n--, along ? j++ : i++)
+	double s = 0.0;
+	for (int c = o.c0; c < o.c0 + o.nc; c++)
 	{
-		double s = 0.0;
-		for (int c = o.c0; c < o.c0 + o.nc; c++)
-		{
-			const GemmContrib g = cons[c];
-			const double* a = A + g.a_off + (i64)i * g.sAm;
-			const double* b = B + g.b_off + (i64)j * g.sBn;
-			for (int kk = 0; kk < g.k; kk++) s = fma(a[(i64)kk * g.sAk], b[(i64)kk * g.sBk], s);
-		}
-		C[gemm_out_index(o, i, j)] = s;
-		if (exp_c && exponent_code(s)) atomicMax(exp_c + o.block, exponent_code(s));
+		const GemmContrib g = cons[c];
+		const double* a = A + g.a_off + (i64)i * g.sAm;
+		const double* b = B + g.b_off + (i64)j * g.sBn;
+		for (int kk = 0; kk < g.k; kk++) s = fma(a[(i64)kk * g.sAk], b[(i64)kk * g.sBk], s);
 	}
+	C[gemm_out_index(o, i, j)] = s;
 }
 
 __global__ void __launch_bounds__(SL_THREADS, 1)
 k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
               const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const unsigned char* xpack,
-              const unsigned char* ypack, const int* xexps, const int* yexps, double* C, int* exp_c, double* work, int* error)
+              const unsigned char* ypack, const short* xexps, const short* yexps, double* C, double* work, int* error)
 {
 	extern __shared__ __align__(1024) unsigned char smem[];
 	double* stage_out = (double*)(smem + SL_STAGES * SL_STAGE);
@@ -501,7 +508,6 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 				f.c1 = o.c1;
 				f.split = t.split;
 				f.sp = t.sp;
-				f.block = o.block;
 				if (f.nch > 0)
 				{
 					const SliceOut s = souts[t.out];
@@ -512,8 +518,8 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 					f.ybytes = min(2, s.y32 - y32) * SLICE_COL32_BYTES;
 					f.xs = s.xbase + (i64)t.u0 * f.xstep + (i64)x8 * SLICE_ROW8_BYTES;
 					f.ys = s.ybase + (i64)t.u0 * f.ystep + (i64)y32 * SLICE_COL32_BYTES;
-					f.e = xexps[s.xgroup];
-					f.f = yexps[s.ygroup];
+					f.xe = s.xrow + x8 * 8;
+					f.ye = s.yrow + y32 * 32;
 				}
 			}
 			infos[batch * SL_TILES + lane] = f;
@@ -583,6 +589,14 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 							lo[c] = kept[h * 16 + 8 + c];
 						}
 					}
+					// exponents of the lane's row and of the 8 columns, for the results
+					int e = 0;
+					int4 ys = make_int4(0, 0, 0, 0);
+					if (fl == nfl - 1 && tile.split < 0 && nch > 0 && active)
+					{
+						if (lane < rows) e = xexps[tile.xe + gr];
+						ys = *(const int4*)(yexps + tile.ye + gc);
+					}
 					if (nch > 0)
 					{
 						const int b = f & 1;
@@ -649,28 +663,15 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 						}
 						continue;
 					}
-					// results in place of the sums; `again`: they are summed in FP64 below
-					const int top = slice_top(tile.e, tile.f);
-					const bool zero = zero_result(tile.e, tile.f), again = !zero && sum_again(tile.e, tile.f);
-					int emax = 0;
-					if (zero)
-					{
+					// results in place of the sums; `again`: columns that are summed in FP64 below
+					unsigned again = 0;
 #pragma unroll
-						for (int c = 0; c < 8; c++) hi[c] = 0;
-					}
-					else
+					for (int c = 0; c < 8; c++)
 					{
-#pragma unroll
-						for (int c = 0; c < 8; c++) hi[c] = (int64_t)slice_value(hi[c], lo[c], top);
-					}
-					// columns past the block's end have zero digits
-#pragma unroll
-					for (int c = 0; c < 8; c++) emax = max(emax, (int)((uint32_t)((uint64_t)hi[c] >> 32) & 0x7fffffffu));
-					emax = again || lane >= rows ? 0 : emax >> 20;
-					if (exp_c)
-					{
-						emax = (int)__reduce_max_sync(0xffffffffu, (unsigned)emax);
-						if (lane == 0 && emax > 0) atomicMax(exp_c + tile.block, emax);
+						const int w = c < 2 ? ys.x : c < 4 ? ys.y : c < 6 ? ys.z : ys.w;
+						const int fc = (c & 1) ? w >> 16 : (int)(short)w;
+						hi[c] = nch > 0 ? (int64_t)slice_value(hi[c], lo[c], slice_top(e, fc)) : 0;
+						if (nch > 0 && slice_sum_fp64(e, fc)) again |= 1u << c;
 					}
 					if (orient == 0)
 					{
@@ -720,7 +721,11 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 						}
 					}
 					__syncwarp();
-					if (again && lane < rows) slice_entries_f64(outs[tiles[tile.tile].out], cons, A, B, orient ? tile.m0 + gr : tile.m0 + gc, orient ? tile.n0 + gc : tile.n0 + gr, orient, cols, C, exp_c);
+					if (again && lane < rows)
+						for (int c = 0; c < cols; c++)
+							if (again >> c & 1)
+								slice_entry_f64(outs[tiles[tile.tile].out], cons, A, B, orient ? tile.m0 + gr : tile.m0 + gc + c,
+								                orient ? tile.n0 + gc + c : tile.n0 + gr, C);
 				}
 			}
 			if (!ok) break;
@@ -743,10 +748,9 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 				if (*last_share)
 				{
 					__threadfence();
-					int emax = 0;
-					for (int e = tid - 32 * SL_EPI_WARP0; e < sp.rows * sp.cols; e += 32 * SL_EPI)
+					for (int q = tid - 32 * SL_EPI_WARP0; q < sp.rows * sp.cols; q += 32 * SL_EPI)
 					{
-						const int i = e / sp.cols, j = e - i * sp.cols;
+						const int i = q / sp.cols, j = q - i * sp.cols;
 						const longlong2* pw = (const longlong2*)(work + sp.part) + (i64)i * sp.ld + j;
 						int64_t hi = 0, lo = 0;
 						for (int p = 0; p < sp.nsplit; p++)
@@ -755,14 +759,10 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 							hi += v.x;
 							lo += v.y;
 						}
-						const bool zero = zero_result(tile.e, tile.f);
-						const double sum = zero ? 0.0 : __longlong_as_double((long long)slice_value(hi, lo, slice_top(tile.e, tile.f)));
-						C[gemm_out_index(outs[sp.out], sp.m0 + i, sp.n0 + j)] = sum;
-						if (!zero && sum_again(tile.e, tile.f))
-							slice_entries_f64(outs[sp.out], cons, A, B, sp.m0 + i, sp.n0 + j, 0, 1, C, exp_c);
-						else emax = max(emax, exponent_code(sum));
+						const int e = xexps[tile.xe + (orient ? i : j)], fc = yexps[tile.ye + (orient ? j : i)];
+						if (slice_sum_fp64(e, fc)) slice_entry_f64(outs[sp.out], cons, A, B, sp.m0 + i, sp.n0 + j, C);
+						else C[gemm_out_index(outs[sp.out], sp.m0 + i, sp.n0 + j)] = __longlong_as_double((long long)slice_value(hi, lo, slice_top(e, fc)));
 					}
-					if (exp_c && emax > 0) atomicMax(exp_c + tile.block, emax);
 					if (tid == 32 * SL_EPI_WARP0) counters[tile.split] = 0;
 				}
 				// nobody overwrites *last_share before every warp has read it
@@ -788,28 +788,26 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 
 }  // namespace
 
-void launch_block_exps(int nchunks, const SliceChunk* chunks, const double* x, int* exps, int* clear, int nclear, cudaStream_t st)
+void launch_slice_exps(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, const double* x,
+                       int* codes, int* clear, int nclear, cudaStream_t st)
 {
-	if (nchunks <= 0)
-	{
-		if (nclear > 0) CTG_CUDA(cudaMemsetAsync(clear, 0, (size_t)nclear * sizeof(int), st));
-		return;
-	}
-	launch_pdl(launch_config(dim3(nchunks), dim3(256), 0, st), k_block_exps, chunks, x, exps, clear, nclear);
+	if (nitems <= 0) return;
+	launch_pdl(launch_config(dim3((nitems + PACK_WARPS - 1) / PACK_WARPS), dim3(PACK_WARPS * 32), 0, st), k_slice_exps, nitems, items,
+	           groups, runs, x, codes, clear, nclear);
 }
 
 void launch_slice_pack(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, bool rows8,
-                       const double* x, const int* exps, void* dst, int* gexps, cudaStream_t st)
+                       const double* x, const int* codes, void* dst, short* exps, cudaStream_t st)
 {
 	if (nitems <= 0) return;
 	launch_pdl(launch_config(dim3((nitems + PACK_WARPS - 1) / PACK_WARPS), dim3(PACK_WARPS * 32), 0, st), k_slice_pack, nitems, items,
-	           groups, runs, rows8 ? 1 : 0, x, exps, (unsigned char*)dst, gexps);
+	           groups, runs, rows8 ? 1 : 0, x, codes, (unsigned char*)dst, exps);
 }
 
 void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
                         const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const void* xpack,
-                        const void* ypack, const int* xexps, const int* yexps, double* C, int* exp_c, double* work, int* error,
-                        int num_sms, cudaStream_t st)
+                        const void* ypack, const short* xexps, const short* yexps, double* C, double* work, int* error, int num_sms,
+                        cudaStream_t st)
 {
 	if (ntiles <= 0) return;
 	static std::once_flag attr_once;
@@ -819,7 +817,7 @@ void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs,
 	// persistent: one CTA per SM (its shared memory admits one)
 	const cudaLaunchConfig_t cfg = launch_config(dim3(std::min(ntiles, num_sms)), dim3(SL_THREADS), SL_SMEM, st);
 	launch_pdl(cfg, k_gemm_slices, ntiles, tiles, outs, souts, cons, splits, counters, orient, A, B, (const unsigned char*)xpack,
-	           (const unsigned char*)ypack, xexps, yexps, C, exp_c, work, error);
+	           (const unsigned char*)ypack, xexps, yexps, C, work, error);
 }
 
 }  // namespace ctg

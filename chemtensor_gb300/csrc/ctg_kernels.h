@@ -24,7 +24,6 @@ struct GemmOut {
 	// of column axes rearranged, the last column run innermost), so that no transpose pass is needed.
 	int r1, c1;
 	i64 sr0, sr1, sc0;
-	int block, pad;    // the block's number in the result's (transposed) structure
 };
 
 __host__ __device__ inline i64 gemm_out_index(const GemmOut& o, int i, int j)
@@ -95,42 +94,39 @@ struct SliceTile {
 	int halves;        // 1 or 2
 	int split, sp;     // share of a split tile (GemmSplit, counters; two integers per entry in the work space)
 };
-struct SliceOut {      // an output block's groups: packed digits (bytes), rows / 8 of x, rows / 32 of y, numbers
+struct SliceOut {      // an output block's groups: packed digits (bytes), rows / 8 of x, rows / 32 of y, numbers, rows
 	i64 xbase, ybase;
 	int x8, y32;
 	int xgroup, ygroup;
+	int xrow, yrow;
 };
-struct SliceRun {      // one block of a group: first entry, terms, strides of rows and terms, its number
+struct SliceRun {      // one block of a group: first entry, terms, strides of rows and terms
 	i64 off;
-	int k, sr, sk, block;
+	int k, sr, sk, pad;
 };
 struct SliceGroup {
 	i64 base;          // packed digits (bytes)
 	int run0, nrun;
 	int rows, ktot;
+	int row0, pad;     // first of its rows among those of the operand (each group's padded to 32)
 };
 constexpr int SLICE_ITEM = 4;                                       // stages of an item at most
 struct SliceItem {     // 32 rows of a group, stages from u0 on: they begin in block run of the group, at its term kk
 	int group, row0, u0;
 	int run, kk;
 };
-// largest biased exponent of every block of an operand into exps (zero before the launch): 0 a block of
-// zeros, 1 denormal numbers at most, 0x7ff a number that is not finite. Also sets clear[0 .. nclear) to zero.
-constexpr int SLICE_CHUNK = 4096;
-struct SliceChunk {
-	i64 off;
-	int n, block;
-};
-void launch_block_exps(int nchunks, const SliceChunk* chunks, const double* x, int* exps, int* clear, int nclear, cudaStream_t st);
-// digits of an operand (rows8: as x, else as y) from its blocks' exponents; gexps receives the groups'
+// largest biased exponent of every row of an operand into codes (zero before the launch): 0 a row of zeros, 1
+// denormal numbers at most, 0x7ff a number that is not finite. Also sets clear[0 .. nclear) to zero.
+void launch_slice_exps(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, const double* x,
+                       int* codes, int* clear, int nclear, cudaStream_t st);
+// digits of an operand (rows8: as x, else as y) from its rows' codes; exps receives the rows' slice_exp
 void launch_slice_pack(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, bool rows8,
-                       const double* x, const int* exps, void* dst, int* gexps, cudaStream_t st);
-// tiles are listed by falling work; exp_c (optional, zero before the launch) receives the largest biased
-// exponents of the result's blocks; *error becomes 1 if a bounded wait ran out
+                       const double* x, const int* codes, void* dst, short* exps, cudaStream_t st);
+// tiles are listed by falling work; *error becomes 1 if a bounded wait ran out
 void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
                         const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const void* xpack,
-                        const void* ypack, const int* xexps, const int* yexps, double* C, int* exp_c, double* work, int* error,
-                        int num_sms, cudaStream_t st);
+                        const void* ypack, const short* xexps, const short* yexps, double* C, double* work, int* error, int num_sms,
+                        cudaStream_t st);
 
 // Same work lists on the tcgen05 tensor cores with FP32 accumulation, output tiles of
 // tc_tile_rows() x BN (BN = 64, 128 or 256, chosen per product). Operand formats (TcFormat):

@@ -166,10 +166,6 @@ struct SliceKey {
 void slice_pack(const Meta& m, const std::vector<SliceKey>& keys, const std::vector<char>& used, bool leading,
                 const std::vector<i64>& lead, const std::vector<i64>& trail, bool rows8, SlicePack& p, std::vector<int>& group_at)
 {
-	p.blocks = m.nblocks;
-	for (int b = 0; b < m.nblocks; b++)
-		for (i64 e = 0, n = m.block_size(b); e < n; e += SLICE_CHUNK)
-			p.chunks.push_back(SliceChunk{m.boff[b] + e, (int)std::min<i64>(SLICE_CHUNK, n - e), b});
 	group_at.assign(keys.size(), -1);
 	for (size_t x = 0; x < keys.size();)
 	{
@@ -190,13 +186,14 @@ void slice_pack(const Meta& m, const std::vector<SliceKey>& keys, const std::vec
 				r.k = (int)(leading ? l : t);
 				r.sr = (int)(leading ? 1 : t);
 				r.sk = (int)(leading ? t : 1);
-				r.block = b;
 				p.runs.push_back(r);
 				g.ktot += r.k;
 				g.rows = (int)(leading ? t : l);
 				CTG_CHECK(r.off + (i64)(g.rows - 1) * r.sr + (i64)(r.k - 1) * r.sk < m.nnz, "dot: operand out of range");
 			}
 			const i64 stages = (g.ktot + SLICE_STAGE_K - 1) / SLICE_STAGE_K;
+			g.row0 = p.rows;
+			p.rows += (g.rows + 31) / 32 * 32;
 			p.bytes += stages * (rows8 ? (i64)((g.rows + 7) / 8) * SLICE_ROW8_BYTES : (i64)((g.rows + 31) / 32) * SLICE_COL32_BYTES);
 			group_at[x] = (int)p.groups.size();
 			int run = 0, kk = 0;                  // first term of the item's stages
@@ -392,7 +389,6 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			o.sr1 = o.n;
 			o.c1 = o.n;
 			o.sc0 = 0;
-			o.block = b;
 			o.c0 = (int)R.cons.size();             // range-local until the join
 			i64 fs = 0, ft = 0;
 			for (int i = 0; i < nfs; i++) fs = fs * r.nb[i] + ir[i];
@@ -596,7 +592,6 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			}
 			GemmOut& o = outs[(size_t)b];
 			o.c_off = outp->boff[bp];
-			o.block = bp;
 			o.r1 = (int)size[1];
 			o.sr0 = stride[0];
 			o.sr1 = stride[1];
@@ -632,7 +627,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			CTG_CHECK(gx.ktot == ksum[b] && gy.ktot == ksum[b] && gx.rows == (x ? outs[b].n : outs[b].m) &&
 			              gy.rows == (x ? outs[b].m : outs[b].n),
 			          "dot: groups of an output block");
-			p.souts[b] = SliceOut{gx.base, gy.base, (gx.rows + 7) / 8, (gy.rows + 31) / 32, gi[x], gi[1 - x]};
+			p.souts[b] = SliceOut{gx.base, gy.base, (gx.rows + 7) / 8, (gy.rows + 31) / 32, gi[x], gi[1 - x], gx.row0, gy.row0};
 		}
 		slice_tiles(outs, ksum, num_sms, p);
 		p.outs = std::move(outs);

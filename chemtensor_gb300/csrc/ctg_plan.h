@@ -18,9 +18,8 @@ struct SlicePack {
 	std::vector<SliceRun> runs;
 	std::vector<SliceGroup> groups;
 	std::vector<SliceItem> items;
-	std::vector<SliceChunk> chunks;      // pieces of its blocks, for their exponents
 	i64 bytes = 0;                       // of the packed digits
-	int blocks = 0;
+	int rows = 0;                        // of all groups, each padded to 32
 };
 
 // block_sparse_tensor_dot (block_sparse_tensor.c:1826-2001) as GEMM work lists

@@ -7,8 +7,8 @@
 // 2^24 / (8 * 2^14) = 128 terms of one order s + t are exact in FP32, so the tensor cores form
 //   acc_o = sum_{s + t = o} sum_k d_s(k) d'_t(k),  o = 0 .. 7
 // without any rounding, and sum_k x(k) y(k) = 2^(e + f - 68) sum_o acc_o 2^(56 - 8 o) up to the orders
-// o >= 8, which lie below 2^-64 of the largest product (the error-free splitting of K. Ozaki, T. Ogita,
-// S. Oishi, S. M. Rump, Numer. Algorithms 59, 2012, with integer digits).
+// o >= 8, which lie below 2^-59 2^(e + f) for each term (2^-62 in the root mean square) (the error-free
+// splitting of K. Ozaki, T. Ogita, S. Oishi, S. M. Rump, Numer. Algorithms 59, 2012, with integer digits).
 // The sum over o is an integer, accumulated over the whole contraction and rounded once.
 #pragma once
 
@@ -22,6 +22,8 @@ constexpr int SLICES = 8;                  // digits of an entry
 constexpr int SLICE_K = 128;               // terms summed in FP32 before the sums move to integers
 constexpr int SLICE_EXP_MIN = 128;         // rows whose largest entry has a smaller biased exponent (or holds a
                                            // number that is not finite) are summed in FP64 instead
+constexpr int SLICE_EXP_ZERO = -4000;      // in place of the exponent: a row of zeros
+constexpr int SLICE_EXP_FP64 = 20000;      // a row that is summed in FP64
 constexpr uint64_t SLICE_BIAS = 0x8080808080808080ull;
 
 // magnitude of the number with the bits (hi, lo) in a row whose largest biased exponent is
@@ -41,6 +43,20 @@ __host__ __device__ inline uint64_t slice_digits(uint32_t hi, uint32_t lo, int E
 // the normal range if slice_in_range.
 __host__ __device__ inline int slice_top(int E, int F) { return E + F - 2112 + 1023 + 95; }
 __host__ __device__ inline bool slice_in_range(int top) { return top - 96 >= 1 && top + 1 <= 2046; }
+
+// the exponent of a row as the product reads it, from its largest biased exponent (0: zeros only, 1: denormal
+// numbers at most, 0x7ff: a number that is not finite)
+__host__ __device__ inline int slice_exp(int code)
+{
+	return code == 0 ? SLICE_EXP_ZERO : code < SLICE_EXP_MIN || code == 0x7ff ? SLICE_EXP_FP64 : code;
+}
+
+// whether the result of two rows with these exponents is summed in FP64. That of a row of zeros is not, unless it
+// meets a row that is: a number that is not finite makes NaN of it.
+__host__ __device__ inline bool slice_sum_fp64(int e, int f)
+{
+	return e + f >= SLICE_EXP_ZERO / 2 && !slice_in_range(slice_top(e, f));
+}
 
 // bits of the FP64 number nearest to (h 2^32 + l) 2^(E + F - 2112) (ties away from zero), the value of a
 // sum over the orders with weights 2^(56 - 8 o): h the orders 0 .. 3 (units of 2^32), l the orders 4 .. 7,
