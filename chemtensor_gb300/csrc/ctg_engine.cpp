@@ -499,8 +499,15 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 		d.items = at<SliceItem>(p.desc, o_side[q][2]);
 		d.nitems = (int)l.spack[q].items.size();
 		d.rows = l.spack[q].rows;
+		d.terms = l.spack[q].terms;
 		d.bytes = l.spack[q].bytes;
 	}
+	// lists for the smaller operand (an MPO tensor, whose rows are mostly zeros) where they take less memory than
+	// the other operand has
+	const int small = l.b_entries < l.a_entries ? 1 : 0;
+	p.side[1 - small].terms = 0;
+	if (2 * p.side[small].terms > std::max(l.a_entries, l.b_entries)) p.side[small].terms = 0;
+	for (const SliceOut& o : l.souts) p.max_k = std::max(p.max_k, o.k);
 	p.tcons = at<TcContrib>(p.desc, o_tcons);
 	p.apacks = at<TcPack>(p.desc, o_apacks);
 	p.bpacks = at<TcPack>(p.desc, o_bpacks);
@@ -545,7 +552,7 @@ void DotPlan::run(Ctx& c, const double* A, const double* B, double* C) const
 	}
 	if (ntiles[0] > 0 || nstiles > 0)
 	{
-		KScope ks(c, K_GEMM, 1, flops, 0);
+		KScope ks(c, K_GEMM, nstiles > 0 ? 7 : 1, flops, 0);
 		launch_f64(c, A, B, C);
 	}
 	c.gemm_flops += flops;
@@ -568,12 +575,20 @@ void DotPlan::launch_f64(Ctx& c, const double* A, const double* B, double* C) co
 		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops, large);
 }
 
-// a packed operand: two arrays of codes, the exponents, and the digits from a 256-byte boundary on
-static size_t slice_head(const DotPlan::Side& d) { return ((size_t)d.rows * (2 * sizeof(int) + sizeof(short)) + 255) & ~(size_t)255; }
+// a packed operand: two arrays of codes, the list lengths, the exponents; the digits; the lists
+static size_t slice_head(const DotPlan::Side& d) { return ((size_t)d.rows * (3 * sizeof(int) + sizeof(short)) + 255) & ~(size_t)255; }
 static int* slice_codes(const DotPlan::Side& d, void* pack, int turn) { return (int*)pack + (turn ? d.rows : 0); }
-static short* slice_exps(const DotPlan::Side& d, const void* pack) { return (short*)((int*)pack + 2 * (size_t)d.rows); }
+static int* slice_counts(const DotPlan::Side& d, const void* pack) { return (int*)pack + 2 * (size_t)d.rows; }
+static short* slice_exps(const DotPlan::Side& d, const void* pack) { return (short*)((int*)pack + 3 * (size_t)d.rows); }
+static SliceTerm* slice_lists(const DotPlan::Side& d, const void* pack)
+{
+	return d.terms > 0 ? (SliceTerm*)((char*)pack + slice_head(d) + (size_t)d.bytes) : nullptr;
+}
 
-i64 DotPlan::slice_bytes(int s) const { return (i64)slice_head(side[s]) + std::max<i64>(side[s].bytes, 16); }
+i64 DotPlan::slice_bytes(int s) const
+{
+	return (i64)slice_head(side[s]) + std::max<i64>(side[s].bytes, 16) + side[s].terms * (i64)sizeof(SliceTerm);
+}
 
 void DotPlan::slice_clear(Ctx& c, int s, void* pack) const
 {
@@ -588,16 +603,22 @@ void DotPlan::slice_pack(Ctx& c, int s, const double* x, void* pack, int turn) c
 	// orient 0: B lies along the MMA rows
 	launch_slice_pack(d.nitems, d.items, d.groups, d.runs, (orient == 0) == (s == 1), x, codes, (char*)pack + slice_head(d),
 	                  slice_exps(d, pack), c.stream());
+	if (d.terms > 0) launch_slice_lists(d.nitems, d.items, d.groups, d.runs, x, slice_lists(d, pack), slice_counts(d, pack), c.stream());
 }
 
 void DotPlan::run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C) const
 {
 	const int x = orient ? 0 : 1;
 	const void* pack[2] = {apack, bpack};
-	launch_gemm_slices(nstiles, stiles, outs, souts, cons, splits, counters ? (int*)counters->ptr : nullptr, orient, A, B,
-	                   (const char*)pack[x] + slice_head(side[x]), (const char*)pack[1 - x] + slice_head(side[1 - x]),
-	                   slice_exps(side[x], pack[x]), slice_exps(side[1 - x], pack[1 - x]), C, work ? (double*)work->ptr : nullptr,
-	                   c.tc_error(), c.num_sms(), c.stream());
+	const short *xe = slice_exps(side[x], pack[x]), *ye = slice_exps(side[1 - x], pack[1 - x]);
+	DBuf check(&c, (size_t)slice_check_bytes(nstiles, nsplits, max_k));
+	launch_gemm_slices(nstiles, stiles, outs, souts, cons, nsplits, splits, counters ? (int*)counters->ptr : nullptr, orient, A, B,
+	                   (const char*)pack[x] + slice_head(side[x]), (const char*)pack[1 - x] + slice_head(side[1 - x]), xe, ye, C,
+	                   max_k, check.ptr, work ? (double*)work->ptr : nullptr, c.tc_error(), c.num_sms(), c.stream());
+	const int small = b_entries < a_entries ? 1 : 0;
+	launch_slice_check(nstiles, nsplits, stiles, outs, souts, cons, splits, orient, small == 1, side[small].groups,
+	                   slice_lists(side[small], pack[small]), slice_counts(side[small], pack[small]), A, B, xe, ye, C, max_k, check.ptr,
+	                   c.num_sms(), c.stream());
 }
 
 void DotPlan::run_z(Ctx& c, const double* A, const double* B, double* C, bool conj_a, bool conj_b) const

@@ -180,7 +180,7 @@ struct DotPlan {
 	DBufPtr work;                        // their partial sums
 	DBufPtr counters;                    // their completion counters (one int per split tile)
 	// FP64 on the tensor cores by digit slices (then ntiles is 0); side 0 is operand A, 1 is B
-	int nstiles = 0, orient = 0;
+	int nstiles = 0, orient = 0, max_k = 0;
 	const SliceTile* stiles = nullptr;
 	const SliceOut* souts = nullptr;
 	struct Side {
@@ -189,6 +189,7 @@ struct DotPlan {
 		const SliceItem* items = nullptr;
 		int nitems = 0, rows = 0;
 		i64 bytes = 0;
+		i64 terms = 0;                   // of its rows' lists (0: none)
 	} side[2];
 	i64 a_entries = 0, b_entries = 0;    // entries of the two operand tensors
 	// tensor-core path: packed operand records (see launch_tc_pack) and per-contribution records
@@ -207,7 +208,8 @@ struct DotPlan {
 	void launch_f64(Ctx& c, const double* A, const double* B, double* C) const;
 	// a product by digit slices in parts, so that an operand used by many runs is packed once. A packed operand is
 	// one buffer (slice_bytes): two arrays of its rows' exponent codes, used in turn (a call of slice_pack clears
-	// the other one; both are zero before the first, slice_clear), the rows' exponents and the digits
+	// the other one; both are zero before the first, slice_clear), the rows' exponents, the digits and, for a small
+	// operand, lists of its rows' nonzero terms
 	i64 slice_bytes(int s) const;
 	void slice_clear(Ctx& c, int s, void* pack) const;
 	void slice_pack(Ctx& c, int s, const double* x, void* pack, int turn) const;

@@ -13,7 +13,9 @@
 //                  warps of the GEMM converting, its MMAs waited for them three quarters of the time
 //   k_gemm_slices  persistent, one CTA per SM, output tiles of 128 x 64 (SliceTile): warp 0 copies the
 //                  digits of 16 terms per stage (up to 32 + 16 KiB), warp 1 issues the MMAs, warps 4-19 add
-//                  the orders up and write.
+//                  the orders up and write, and mark the results whose digits may not be enough
+//   k_slice_find, k_slice_check   look at the marked results and sum those in FP64 that need it; k_slice_lists
+//                  makes lists of the nonzero terms of a small operand for them
 // The 64 columns of a tile are two halves of 32 with an accumulator each in tensor memory: columns 32 o ..
 // 32 o + 31 of it hold order o. Digit s of the 128 rows meets the digits 0 .. 7 - s of the 32 columns,
 // which lie one after the other as rows of one B operand, in one MMA of N = 32 (8 - s) that writes
@@ -22,12 +24,12 @@
 // cycle and SM out of L2; 66 with 32 columns), and tensor memory holds no more. Every 128 terms the
 // epilogue takes the sums over: half 0 while the MMAs of half 1 run, and conversely.
 // Measured, three products of a local-Hamiltonian application at D = 1024 (4.1e9 FMAs): 7.65 ms on the
-// FP64 pipe, 0.62 ms here and 0.24 ms for the digits (1.06 ms with the conversion inside the GEMM). The
-// first two products are bound by the epilogue (integer instructions on 2e7 results, tensor pipe 28 and
-// 37 % busy), the third, with ten times the terms, by the copies out of L2 (46 %).
-// Results of a row that is not finite or tiny, and results that may leave the normal range, are FP64 sums
-// over the operands. Every wait is bounded and ends when another warp
-// has failed.
+// FP64 pipe; 0.65 ms here (1.06 ms with the conversion inside the GEMM), 0.30 ms for the digits, 0.13 ms for the
+// exponents and 0.25 ms for the marked results. The first two products are bound by the epilogue (integer
+// instructions on 2e7 results, tensor pipe 28 and 37 % busy), the third, with ten times the terms, by the copies out
+// of L2 (46 %). A molecular search (n = 16, D = 256): 1054 ms on the FP64 pipe, 214 ms here, 152 without the
+// marked results.
+// Every wait is bounded and ends when another warp has failed.
 #include <algorithm>
 #include <mutex>
 
@@ -55,6 +57,7 @@ constexpr int SL_FLUSH = SLICE_K / SLICE_STAGE_K;                // stages betwe
 constexpr int SL_LD = 5;                        // staging row of the epilogue (4 columns)
 constexpr int SL_EPI_BYTES = SL_EPI * 32 * SL_LD * 8;
 constexpr int SL_TILES = 32;                    // tiles described at a time (twice)
+constexpr int SL_MASKS = SLICE_TILE_COLS * SL_M / 32;            // words of a tile's mask of suspect results
 // one tile, as the other warps need it
 struct SliceInfo {
 	i64 xs, ys;                          // digits of its first stage (bytes)
@@ -199,14 +202,15 @@ k_slice_exps(int nitems, const SliceItem* __restrict__ items, const SliceGroup* 
 	const SliceGroup g = groups[im.group];
 	const int row = im.row0 + lane;
 	SliceReader in(im, g, runs, x, row);
-	const int n8 = (min(SLICE_ITEM * SLICE_STAGE_K, g.ktot - im.u0 * SLICE_STAGE_K) + 7) / 8;
+	const int n8 = 2 * min(SLICE_ITEM, (g.ktot + SLICE_STAGE_K - 1) / SLICE_STAGE_K - im.u0);
 	uint32_t hi = 0, lo = 0;
-	for (int u = 0; u < n8; u++)
+	for (int u = 0; u < n8; u += 2)
 	{
-		double v[8];
+		double v[16];
 		in.read8(v);
+		in.read8(v + 8);
 #pragma unroll
-		for (int t = 0; t < 8; t++)
+		for (int t = 0; t < 16; t++)
 		{
 			hi = max(hi, (uint32_t)__double2hiint(v[t]) & 0x7fffffffu);
 			lo |= (uint32_t)__double2loint(v[t]);
@@ -298,29 +302,44 @@ k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* 
 	}
 }
 
+// the nonzero terms of every row (a warp) of an item's 32
+__global__ void __launch_bounds__(1024)
+k_slice_lists(const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups, const SliceRun* __restrict__ runs,
+              const double* __restrict__ x, SliceTerm* __restrict__ terms, int* __restrict__ counts)
+{
+	pdl_wait();
+	pdl_trigger();
+	const SliceItem im = items[blockIdx.x];
+	if (im.u0 != 0) return;
+	const SliceGroup g = groups[im.group];
+	const int row = im.row0 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+	if (row >= g.rows) return;
+	SliceTerm* list = terms + g.list + (i64)row * g.ktot;
+	int n = 0;
+	for (int c = 0; c < g.nrun; c++)
+	{
+		const SliceRun r = runs[g.run0 + c];
+		const double* p = x + r.off + (i64)row * r.sr;
+		for (int k0 = 0; k0 < r.k; k0 += 32)
+		{
+			const int k = k0 + lane;
+			const double v = k < r.k ? p[(i64)k * r.sk] : 0.0;
+			const unsigned some = __ballot_sync(0xffffffffu, v != 0.0);
+			if (v != 0.0) list[n + __popc(some & ((1u << lane) - 1))] = SliceTerm{v, c, k};
+			n += __popc(some);
+		}
+	}
+	if (lane == 0) counts[g.row0 + row] = n;
+}
+
 // ------------------------------------------------------------------------------------
 // the products
 // ------------------------------------------------------------------------------------
 
-// entry (i, j) of an output block, by FP64 sums
-__device__ __noinline__ void slice_entry_f64(const GemmOut& o, const GemmContrib* cons, const double* A, const double* B, int i,
-                                             int j, double* C)
-{
-	double s = 0.0;
-	for (int c = o.c0; c < o.c0 + o.nc; c++)
-	{
-		const GemmContrib g = cons[c];
-		const double* a = A + g.a_off + (i64)i * g.sAm;
-		const double* b = B + g.b_off + (i64)j * g.sBn;
-		for (int kk = 0; kk < g.k; kk++) s = fma(a[(i64)kk * g.sAk], b[(i64)kk * g.sBk], s);
-	}
-	C[gemm_out_index(o, i, j)] = s;
-}
-
 __global__ void __launch_bounds__(SL_THREADS, 1)
 k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
               const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const unsigned char* xpack,
-              const unsigned char* ypack, const short* xexps, const short* yexps, double* C, double* work, int* error)
+              const unsigned char* ypack, const short* xexps, const short* yexps, double* C, uint2* list, unsigned* masks, double* work, int* error)
 {
 	extern __shared__ __align__(1024) unsigned char smem[];
 	double* stage_out = (double*)(smem + SL_STAGES * SL_STAGE);
@@ -367,6 +386,8 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 	const uint32_t tmem = *tmem_slot;
 	// everything up to here overlaps the tail of the previous kernel in the stream
 	pdl_wait();
+	// the list of k_slice_find, empty
+	if (blockIdx.x == 0 && tid == 0) list[0] = make_uint2(0, 0);
 
 	// the description of the CTA's tile number it (every lane of a warp, in order): null at the end
 	auto tile_info = [&](int it, bool& ok) -> const SliceInfo* {
@@ -659,20 +680,22 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 						{
 #pragma unroll
 							for (int c = 0; c < 8; c++)
-								if (c < cols) *(longlong2*)(w + 2 * (orient ? gr * sp.ld + gc + c : (gc + c) * sp.ld + gr)) = make_longlong2(hi[c], lo[c]);
+								if (c < cols) *(longlong2*)(w + 2 * ((gc + c) * SL_M + gr)) = make_longlong2(hi[c], lo[c]);
 						}
 						continue;
 					}
-					// results in place of the sums; `again`: columns that are summed in FP64 below
-					unsigned again = 0;
+					// results in place of the sums, and which of them k_slice_check has to look at
+					unsigned mask = 0;
 #pragma unroll
 					for (int c = 0; c < 8; c++)
 					{
 						const int w = c < 2 ? ys.x : c < 4 ? ys.y : c < 6 ? ys.z : ys.w;
 						const int fc = (c & 1) ? w >> 16 : (int)(short)w;
 						hi[c] = nch > 0 ? (int64_t)slice_value(hi[c], lo[c], slice_top(e, fc)) : 0;
-						if (nch > 0 && slice_sum_fp64(e, fc)) again |= 1u << c;
+						const unsigned m = __ballot_sync(0xffffffffu, lane < rows && slice_suspect(e, fc, (int)(hi[c] >> 52) & 0x7ff));
+						if (lane == c) mask = m;
 					}
+					if (lane < 8) masks[(i64)tile.tile * SL_MASKS + (gc + lane) * 4 + q] = mask;
 					if (orient == 0)
 					{
 						// lanes are neighbouring columns of the output block: coalesced
@@ -721,11 +744,6 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 						}
 					}
 					__syncwarp();
-					if (again && lane < rows)
-						for (int c = 0; c < cols; c++)
-							if (again >> c & 1)
-								slice_entry_f64(outs[tiles[tile.tile].out], cons, A, B, orient ? tile.m0 + gr : tile.m0 + gc + c,
-								                orient ? tile.n0 + gc + c : tile.n0 + gr, C);
 				}
 			}
 			if (!ok) break;
@@ -748,20 +766,32 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 				if (*last_share)
 				{
 					__threadfence();
-					for (int q = tid - 32 * SL_EPI_WARP0; q < sp.rows * sp.cols; q += 32 * SL_EPI)
+					// a warp per column and 32 rows of the MMA tile
+					const GemmOut o = outs[sp.out];
+					const int mr = orient ? sp.rows : sp.cols, mc = orient ? sp.cols : sp.rows;
+					unsigned* mask = masks + (i64)(ntiles + tile.split) * SL_MASKS;
+					for (int wd = warp - SL_EPI_WARP0; wd < 4 * mc; wd += SL_EPI)
 					{
-						const int i = q / sp.cols, j = q - i * sp.cols;
-						const longlong2* pw = (const longlong2*)(work + sp.part) + (i64)i * sp.ld + j;
-						int64_t hi = 0, lo = 0;
-						for (int p = 0; p < sp.nsplit; p++)
+						const int col = wd >> 2, row = (wd & 3) * 32 + lane;
+						if ((wd & 3) * 32 >= mr) continue;
+						bool look = false;
+						if (row < mr)
 						{
-							const longlong2 v = __ldcg(pw + (i64)p * (sp.stride / 2));
-							hi += v.x;
-							lo += v.y;
+							const longlong2* pw = (const longlong2*)(work + sp.part) + col * SL_M + row;
+							int64_t hi = 0, lo = 0;
+							for (int p = 0; p < sp.nsplit; p++)
+							{
+								const longlong2 v = __ldcg(pw + (i64)p * (sp.stride / 2));
+								hi += v.x;
+								lo += v.y;
+							}
+							const int e = xexps[tile.xe + row], fc = yexps[tile.ye + col];
+							const uint64_t r = slice_value(hi, lo, slice_top(e, fc));
+							look = slice_suspect(e, fc, (int)(r >> 52) & 0x7ff);
+							C[gemm_out_index(o, sp.m0 + (orient ? row : col), sp.n0 + (orient ? col : row))] = __longlong_as_double((long long)r);
 						}
-						const int e = xexps[tile.xe + (orient ? i : j)], fc = yexps[tile.ye + (orient ? j : i)];
-						if (slice_sum_fp64(e, fc)) slice_entry_f64(outs[sp.out], cons, A, B, sp.m0 + i, sp.n0 + j, C);
-						else C[gemm_out_index(outs[sp.out], sp.m0 + i, sp.n0 + j)] = __longlong_as_double((long long)slice_value(hi, lo, slice_top(e, fc)));
+						const unsigned m = __ballot_sync(0xffffffffu, look);
+						if (lane == 0) mask[wd] = m;
 					}
 					if (tid == 32 * SL_EPI_WARP0) counters[tile.split] = 0;
 				}
@@ -786,7 +816,261 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 	}
 }
 
+// ------------------------------------------------------------------------------------
+// the results whose digits may not be enough
+// ------------------------------------------------------------------------------------
+
+// Results of rows that are not finite, tiny or out of range are FP64 sums over the operands. A small result keeps
+// its value if one of its terms is large (terms that cancel); if none is (a graded row times a column that is small
+// where the row is large), it is an FP64 sum too, so that every entry has the accuracy of the FP64 pipe.
+// k_slice_find lists the mask words with suspects, so that the few tiles that hold many are shared out;
+// k_slice_check takes the words in turn, a warp each, its lanes divided among the word's suspects.
+// Suspect: 0.6 % of random operands (all of them cleared by their first terms), 5 % in a molecular search at
+// D = 256, of which 3 % are summed: there the MPO tensor's rows have ten nonzero terms of four hundred, and the lists
+// of these (k_slice_lists) stand for the row.
+constexpr int CHECK_WARPS = 4, CHECK_UNROLL = 4;
+// rows per listed word, 32 or fewer where the sums are long (max_k is the longest one of the product)
+__host__ __device__ inline int check_rows(int k) { return k >= 2048 ? 1 : k >= 512 ? 8 : 32; }
+
+__device__ __forceinline__ int biased_exponent(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
+// rows and columns of the MMA tile of a mask (numbers below ntiles: tiles that are not split; then split tiles)
+struct MaskTile {
+	int out, m0, n0, mr, mc;
+	__device__ MaskTile(int id, int ntiles, const SliceTile* tiles, const GemmSplit* splits, const GemmOut* outs, int orient)
+	{
+		mr = mc = 0;
+		if (id < ntiles)
+		{
+			const SliceTile t = tiles[id];
+			if (t.split >= 0 || t.u0 == t.u1) return;
+			out = t.out;
+			m0 = t.m0;
+			n0 = t.n0;
+		}
+		else
+		{
+			const GemmSplit t = splits[id - ntiles];
+			out = t.out;
+			m0 = t.m0;
+			n0 = t.n0;
+		}
+		const int m = outs[out].m - m0, n = outs[out].n - n0;
+		mr = min(SL_M, orient ? m : n);
+		mc = min(SLICE_TILE_COLS, orient ? n : m);
+	}
+};
+
+// list: its length (zero before the launch), then (mask word, its bits)
+__global__ void __launch_bounds__(CHECK_WARPS * 32)
+k_slice_find(int ntiles, int nsplits, const SliceTile* __restrict__ tiles, const GemmOut* __restrict__ outs,
+             const SliceOut* __restrict__ souts, const GemmSplit* __restrict__ splits, int orient, const unsigned* __restrict__ masks,
+             uint2* __restrict__ list)
+{
+	pdl_wait();
+	pdl_trigger();
+	const int lane = threadIdx.x & 31, units = (ntiles + nsplits) * 8;
+	for (int unit = blockIdx.x * CHECK_WARPS + (threadIdx.x >> 5); unit < units; unit += gridDim.x * CHECK_WARPS)
+	{
+		const int id = unit >> 3, col = (unit & 7) * 8 + (lane >> 2), row0 = (lane & 3) * 32;
+		const MaskTile t(id, ntiles, tiles, splits, outs, orient);
+		const unsigned at = (unsigned)id * SL_MASKS + (unit & 7) * 32 + lane;
+		unsigned word = col < t.mc && row0 < t.mr ? masks[at] : 0;
+		if (t.mr - row0 < 32) word &= (1u << max(t.mr - row0, 0)) - 1;
+		if (!__any_sync(0xffffffffu, word != 0)) continue;
+		const int width = check_rows(souts[t.out].k);
+		int n = 0;
+		for (int q = 0; q < 32; q += width) n += (word >> q & (0xffffffffu >> (32 - width))) != 0;
+		int end = n;
+#pragma unroll
+		for (int q = 1; q < 32; q <<= 1)
+		{
+			const int v = __shfl_up_sync(0xffffffffu, end, q);
+			if (lane >= q) end += v;
+		}
+		unsigned base = 0;
+		if (lane == 31) base = atomicAdd(&list[0].x, (unsigned)end);
+		base = __shfl_sync(0xffffffffu, base, 31) + 1 + end - n;
+		for (int q = 0; q < 32; q += width)
+		{
+			const unsigned part = word & (0xffffffffu >> (32 - width)) << q;
+			if (part) list[base++] = make_uint2(at, part);
+		}
+	}
+}
+
+// use(a, b) for the terms of an entry that are the lane's (sub, sub + lanes, ..), for all lanes of a warp at once,
+// until done() holds in all of them. x is the operand with fewer entries (i its row: an MPO tensor, whose rows are
+// mostly zeros) and read first: unless all terms are asked for, y is read where x is not zero, and terms that
+// are zero in every lane are left out. Contributions of more terms than an entry has lanes are taken one by one;
+// those of shorter ones, 32 at a time, are one list.
+template <bool ALL, class Use, class Done>
+__device__ __forceinline__ void entry_terms(const GemmOut& o, const GemmContrib* cons, bool swap, const double* x, const double* y, int i,
+                                            int j, int sub, int lanes, bool on, const Use& use, const Done& done)
+{
+	constexpr unsigned FULL = 0xffffffffu;
+	const int lane = threadIdx.x & 31;
+	for (int c0 = 0; c0 < o.nc; c0 += 32)
+	{
+		const int nb = min(32, o.nc - c0);
+		GemmContrib g = {};
+		if (lane < nb) g = cons[o.c0 + c0 + lane];
+		if (swap) g = GemmContrib{g.b_off, g.a_off, g.k, g.sBn, g.sBk, g.sAk, g.sAm};
+		int end = g.k;
+#pragma unroll
+		for (int q = 1; q < 32; q <<= 1)
+		{
+			const int v = __shfl_up_sync(FULL, end, q);
+			if (lane >= q) end += v;
+		}
+		const int start = end - g.k, total = __shfl_sync(FULL, end, 31);
+		const bool list = total < nb * lanes;
+		for (int c = 0; c < (list ? 1 : nb); c++)
+		{
+			const int n = list ? total : __shfl_sync(FULL, g.k, c);
+			int d = c;
+			auto first = [&] { return x + __shfl_sync(FULL, g.a_off, d) + (i64)i * __shfl_sync(FULL, g.sAm, d); };
+			auto second = [&] { return y + __shfl_sync(FULL, g.b_off, d) + (i64)j * __shfl_sync(FULL, g.sBn, d); };
+			const double *px = first(), *py = second();
+			int kx = __shfl_sync(FULL, g.sAk, d), ky = __shfl_sync(FULL, g.sBk, d);
+			for (int t0 = 0; t0 < n; t0 += CHECK_UNROLL * lanes)
+			{
+				double a[CHECK_UNROLL], b[CHECK_UNROLL];
+				const double* pb[CHECK_UNROLL];
+#pragma unroll
+				for (int u = 0; u < CHECK_UNROLL; u++)
+				{
+					int t = t0 + u * lanes + sub;
+					const bool in = on && t < n;
+					if (list)
+					{
+						d = 0;
+#pragma unroll
+						for (int step = 16; step > 0; step >>= 1)
+							if (__shfl_sync(FULL, start, d + step) <= t) d += step;
+						px = first();
+						py = second();
+						kx = __shfl_sync(FULL, g.sAk, d);
+						ky = __shfl_sync(FULL, g.sBk, d);
+						t -= __shfl_sync(FULL, start, d);
+					}
+					pb[u] = in ? py + (i64)t * ky : nullptr;
+					a[u] = in ? px[(i64)t * kx] : 0.0;
+				}
+#pragma unroll
+				for (int u = 0; u < CHECK_UNROLL; u++) b[u] = pb[u] && (ALL || a[u] != 0.0) ? *pb[u] : 0.0;
+#pragma unroll
+				for (int u = 0; u < CHECK_UNROLL; u++)
+					if (ALL || __any_sync(FULL, a[u] != 0.0)) use(a[u], b[u]);
+				if (done()) return;
+			}
+		}
+	}
+}
+
+__global__ void __launch_bounds__(CHECK_WARPS * 32)
+k_slice_check(int ntiles, const SliceTile* __restrict__ tiles, const GemmOut* __restrict__ outs, const SliceOut* __restrict__ souts,
+              const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits, int orient, int swap,
+              const SliceGroup* __restrict__ groups, const SliceTerm* __restrict__ terms, const int* __restrict__ counts,
+              const double* __restrict__ A, const double* __restrict__ B, const short* __restrict__ xexps,
+              const short* __restrict__ yexps, double* __restrict__ C, uint2* list)
+{
+	pdl_wait();
+	pdl_trigger();
+	const int lane = threadIdx.x & 31;
+	const unsigned n = list[0].x;
+	// the smaller operand, and the other one
+	const double *x = swap ? B : A, *y = swap ? A : B;
+	unsigned item = blockIdx.x * CHECK_WARPS + (threadIdx.x >> 5);
+	uint2 next = item < n ? list[1 + item] : make_uint2(0, 0);
+	for (; item < n; item += gridDim.x * CHECK_WARPS)
+	{
+		const uint2 w = next;
+		if (item + gridDim.x * CHECK_WARPS < n) next = list[1 + item + gridDim.x * CHECK_WARPS];
+		const int wd = (int)(w.x % SL_MASKS), col = wd >> 2;
+		const MaskTile t((int)(w.x / SL_MASKS), ntiles, tiles, splits, outs, orient);
+		const GemmOut o = outs[t.out];
+		const SliceOut so = souts[t.out];
+		// the suspects get 32, 16, .. 1 lanes each
+		const int count = __popc(w.y), lanes = 32 >> (count > 1 ? 32 - __clz(count - 1) : 0);
+		const int which = lane / lanes, sub = lane % lanes;
+		unsigned left = w.y;
+		for (int q = 0; q < which && q + 1 < count; q++) left &= left - 1;
+		const int row = (wd & 3) * 32 + __ffs(left) - 1;
+		const int i = orient ? t.m0 + row : t.m0 + col, j = orient ? t.n0 + col : t.n0 + row;
+		const int ix = swap ? j : i, iy = swap ? i : j;
+		const int e = xexps[so.xrow + (orient ? i : j)], f = yexps[so.yrow + (orient ? j : i)], limit = slice_term_limit(e, f);
+		const unsigned mine = (lanes == 32 ? 0xffffffffu : (1u << lanes) - 1) << (which * lanes);
+		const bool on = which < count, look = on && slice_in_range(slice_top(e, f));
+		bool enough = false;
+		double s = 0.0;
+		if (terms)
+		{
+			// test and sum in one
+			const SliceGroup g = groups[swap == orient ? so.ygroup : so.xgroup];
+			const SliceTerm* p = terms + g.list + (i64)ix * g.ktot;
+			const int k = look ? counts[g.row0 + ix] : 0;
+			for (int t0 = sub; __any_sync(0xffffffffu, t0 < k && !enough); t0 += CHECK_UNROLL * lanes)
+			{
+				SliceTerm z[CHECK_UNROLL];
+				double v[CHECK_UNROLL];
+#pragma unroll
+				for (int u = 0; u < CHECK_UNROLL; u++) z[u] = t0 + u * lanes < k ? p[t0 + u * lanes] : SliceTerm{0.0, 0, 0};
+#pragma unroll
+				for (int u = 0; u < CHECK_UNROLL; u++)
+				{
+					v[u] = 0.0;
+					if (t0 + u * lanes >= k) continue;
+					const GemmContrib h = cons[o.c0 + z[u].run];
+					v[u] = swap ? y[h.a_off + (i64)iy * h.sAm + (i64)z[u].k * h.sAk] : y[h.b_off + (i64)iy * h.sBn + (i64)z[u].k * h.sBk];
+				}
+#pragma unroll
+				for (int u = 0; u < CHECK_UNROLL; u++)
+				{
+					enough |= biased_exponent(z[u].v) + biased_exponent(v[u]) >= limit;
+					s = fma(z[u].v, v[u], s);
+				}
+				enough = (__ballot_sync(0xffffffffu, enough && look) & mine) != 0;
+			}
+		}
+		else if (__any_sync(0xffffffffu, look))
+			entry_terms<false>(o, cons, swap, x, y, ix, iy, sub, lanes, look,
+			                   [&](double a, double b) { enough |= biased_exponent(a) + biased_exponent(b) >= limit; },
+			                   [&] {
+				                   enough = (__ballot_sync(0xffffffffu, enough && look) & mine) != 0;
+				                   return !__any_sync(0xffffffffu, look && !enough);
+			                   });
+		const auto all = [] { return false; };
+		const bool sum = look && !enough;
+		if (__any_sync(0xffffffffu, sum))
+		{
+			if (!terms)
+				entry_terms<false>(o, cons, swap, x, y, ix, iy, sub, lanes, sum, [&](double a, double b) { s = fma(a, b, s); }, all);
+			for (int q = lanes >> 1; q > 0; q >>= 1) s += __shfl_xor_sync(0xffffffffu, s, q);
+		}
+		// a sum that may overflow in one chain: infinities of both signs would make NaN of partial sums
+		const bool chain = on && !look && sub == 0;
+		if (__any_sync(0xffffffffu, chain))
+		{
+			if (chain) s = 0.0;
+			entry_terms<true>(o, cons, swap, x, y, ix, iy, 0, 1, chain, [&](double a, double b) { if (chain) s = fma(a, b, s); }, all);
+		}
+		if ((sum && sub == 0) || chain) C[gemm_out_index(o, i, j)] = s;
+	}
+}
+
 }  // namespace
+
+// the list, then the masks
+i64 slice_check_bytes(int ntiles, int nsplits, int max_k)
+{
+	return 8 + (i64)(ntiles + nsplits) * SL_MASKS * (32 / check_rows(max_k) * (i64)sizeof(uint2) + (i64)sizeof(unsigned));
+}
+
+static unsigned* check_masks(void* check, int ntiles, int nsplits, int max_k)
+{
+	return (unsigned*)((uint2*)check + 1 + (i64)(ntiles + nsplits) * SL_MASKS * (32 / check_rows(max_k)));
+}
 
 void launch_slice_exps(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, const double* x,
                        int* codes, int* clear, int nclear, cudaStream_t st)
@@ -804,10 +1088,16 @@ void launch_slice_pack(int nitems, const SliceItem* items, const SliceGroup* gro
 	           groups, runs, rows8 ? 1 : 0, x, codes, (unsigned char*)dst, exps);
 }
 
+void launch_slice_lists(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, const double* x,
+                        SliceTerm* terms, int* counts, cudaStream_t st)
+{
+	if (nitems > 0) launch_pdl(launch_config(dim3(nitems), dim3(1024), 0, st), k_slice_lists, items, groups, runs, x, terms, counts);
+}
+
 void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
-                        const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const void* xpack,
-                        const void* ypack, const short* xexps, const short* yexps, double* C, double* work, int* error, int num_sms,
-                        cudaStream_t st)
+                        int nsplits, const GemmSplit* splits, int* counters, int orient, const double* A, const double* B,
+                        const void* xpack, const void* ypack, const short* xexps, const short* yexps, double* C, int max_k,
+                        void* check, double* work, int* error, int num_sms, cudaStream_t st)
 {
 	if (ntiles <= 0) return;
 	static std::once_flag attr_once;
@@ -817,7 +1107,21 @@ void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs,
 	// persistent: one CTA per SM (its shared memory admits one)
 	const cudaLaunchConfig_t cfg = launch_config(dim3(std::min(ntiles, num_sms)), dim3(SL_THREADS), SL_SMEM, st);
 	launch_pdl(cfg, k_gemm_slices, ntiles, tiles, outs, souts, cons, splits, counters, orient, A, B, (const unsigned char*)xpack,
-	           (const unsigned char*)ypack, xexps, yexps, C, work, error);
+	           (const unsigned char*)ypack, xexps, yexps, C, (uint2*)check, check_masks(check, ntiles, nsplits, max_k), work, error);
+}
+
+void launch_slice_check(int ntiles, int nsplits, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts,
+                        const GemmContrib* cons, const GemmSplit* splits, int orient, bool b_smaller, const SliceGroup* groups,
+                        const SliceTerm* terms, const int* counts, const double* A, const double* B, const short* xexps,
+                        const short* yexps, double* C, int max_k, void* check, int num_sms, cudaStream_t st)
+{
+	if (ntiles <= 0) return;
+	uint2* list = (uint2*)check;
+	const int all = num_sms * 8;
+	launch_pdl(launch_config(dim3(std::min((ntiles + nsplits) * 8 / CHECK_WARPS, 2 * all)), dim3(CHECK_WARPS * 32), 0, st), k_slice_find,
+	           ntiles, nsplits, tiles, outs, souts, splits, orient, check_masks(check, ntiles, nsplits, max_k), list);
+	launch_pdl(launch_config(dim3(all), dim3(CHECK_WARPS * 32), 0, st), k_slice_check, ntiles, tiles, outs, souts, cons, splits, orient,
+	           b_smaller ? 1 : 0, groups, terms, counts, A, B, xexps, yexps, C, list);
 }
 
 }  // namespace ctg

@@ -94,11 +94,12 @@ struct SliceTile {
 	int halves;        // 1 or 2
 	int split, sp;     // share of a split tile (GemmSplit, counters; two integers per entry in the work space)
 };
-struct SliceOut {      // an output block's groups: packed digits (bytes), rows / 8 of x, rows / 32 of y, numbers, rows
-	i64 xbase, ybase;
+struct SliceOut {      // an output block's groups: packed digits (bytes), rows / 8 of x, rows / 32 of y, numbers, rows;
+	i64 xbase, ybase;  // its terms
 	int x8, y32;
 	int xgroup, ygroup;
 	int xrow, yrow;
+	int k, pad;
 };
 struct SliceRun {      // one block of a group: first entry, terms, strides of rows and terms
 	i64 off;
@@ -109,6 +110,11 @@ struct SliceGroup {
 	int run0, nrun;
 	int rows, ktot;
 	int row0, pad;     // first of its rows among those of the operand (each group's padded to 32)
+	i64 list;          // where its rows' lists of nonzero terms begin (ktot apart)
+};
+struct SliceTerm {     // a term of a row: its entry, its block in the group and place in it
+	double v;
+	int run, k;
 };
 constexpr int SLICE_ITEM = 4;                                       // stages of an item at most
 struct SliceItem {     // 32 rows of a group, stages from u0 on: they begin in block run of the group, at its term kk
@@ -122,11 +128,21 @@ void launch_slice_exps(int nitems, const SliceItem* items, const SliceGroup* gro
 // digits of an operand (rows8: as x, else as y) from its rows' codes; exps receives the rows' slice_exp
 void launch_slice_pack(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, bool rows8,
                        const double* x, const int* codes, void* dst, short* exps, cudaStream_t st);
-// tiles are listed by falling work; *error becomes 1 if a bounded wait ran out
+// tiles are listed by falling work; check (slice_check_bytes) receives the suspect results, which
+// launch_slice_check then looks at; *error becomes 1 if a bounded wait ran out
 void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
-                        const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const void* xpack,
-                        const void* ypack, const short* xexps, const short* yexps, double* C, double* work, int* error, int num_sms,
-                        cudaStream_t st);
+                        int nsplits, const GemmSplit* splits, int* counters, int orient, const double* A, const double* B,
+                        const void* xpack, const void* ypack, const short* xexps, const short* yexps, double* C, int max_k,
+                        void* check, double* work, int* error, int num_sms, cudaStream_t st);
+// the nonzero terms of every row of an operand, and their number
+void launch_slice_lists(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, const double* x,
+                        SliceTerm* terms, int* counts, cudaStream_t st);
+i64 slice_check_bytes(int ntiles, int nsplits, int max_k);     // max_k: most terms of an output block
+// terms (may be null), counts, groups: of the operand with fewer entries, which is B if b_smaller
+void launch_slice_check(int ntiles, int nsplits, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts,
+                        const GemmContrib* cons, const GemmSplit* splits, int orient, bool b_smaller, const SliceGroup* groups,
+                        const SliceTerm* terms, const int* counts, const double* A, const double* B, const short* xexps,
+                        const short* yexps, double* C, int max_k, void* check, int num_sms, cudaStream_t st);
 
 // Same work lists on the tcgen05 tensor cores with FP32 accumulation, output tiles of
 // tc_tile_rows() x BN (BN = 64, 128 or 256, chosen per product). Operand formats (TcFormat):

@@ -133,16 +133,17 @@ int slice_orient(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum,
 	return clocks[1] < clocks[0] ? 1 : 0;
 }
 
-// SM clocks of the three launches that a product by digit slices has besides the GEMM (exponents, digits)
-constexpr double SLICE_OVERHEAD = 50000;
+// SM clocks of the five launches that a product by digit slices has besides the GEMM (exponents, digits, the
+// results to look at again), and of those for an entry of an operand and of the result
+constexpr double SLICE_OVERHEAD = 75000, SLICE_ENTRY = 3.0, SLICE_RESULT = 4.0;
 
 // Digit slices or the FP64 pipe, by the SM clocks that each takes: the FP64 tiles at 2.1 FMAs a clock
-// (padding included), against the MMAs, the conversion of the operands' entries and the launches. Both
-// sides measured: a D = 1024 local-Hamiltonian product of 1.1e9 FMAs 2.0 ms against 0.2 ms, the
+// (padding included), against the MMAs, the conversion of the operands' entries, the check of the results and
+// the launches. Both sides measured: a D = 1024 local-Hamiltonian product of 1.1e9 FMAs 2.0 ms against 0.3 ms, the
 // products of a Hubbard chain at D = 256 (3e6 .. 9e6 FMAs in 300 .. 1500 output blocks) 15 .. 60 us
-// against 40 .. 55 us.
+// against 50 .. 70 us.
 bool use_slices(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum, const std::vector<GemmTile>* tiles, i64 entries,
-                int num_sms)
+                i64 results, int num_sms)
 {
 	static const int forced = [] {
 		const char* e = getenv("CTGPU_SLICE_GEMM");
@@ -155,7 +156,7 @@ bool use_slices(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum, 
 	for (int k = 0; k < NUM_TILE_CLASSES; k++)
 		for (const GemmTile& t : tiles[k])
 			f64 += (double)TILE_ROWS[k] * TILE_COLS[k] * (double)ksum[(size_t)t.out] / 2.1;
-	return (clocks[o] + 2.0 * (double)entries) / num_sms + SLICE_OVERHEAD < f64 / num_sms;
+	return (clocks[o] + SLICE_ENTRY * (double)entries + SLICE_RESULT * (double)results) / num_sms + SLICE_OVERHEAD < f64 / num_sms;
 }
 
 // how an operand is packed: the groups (runs of `keys` with one free index) that some output block uses
@@ -194,6 +195,8 @@ void slice_pack(const Meta& m, const std::vector<SliceKey>& keys, const std::vec
 			const i64 stages = (g.ktot + SLICE_STAGE_K - 1) / SLICE_STAGE_K;
 			g.row0 = p.rows;
 			p.rows += (g.rows + 31) / 32 * 32;
+			g.list = p.terms;
+			p.terms += (i64)g.rows * g.ktot;
 			p.bytes += stages * (rows8 ? (i64)((g.rows + 7) / 8) * SLICE_ROW8_BYTES : (i64)((g.rows + 31) / 32) * SLICE_COL32_BYTES);
 			group_at[x] = (int)p.groups.size();
 			int run = 0, kk = 0;                  // first term of the item's stages
@@ -602,7 +605,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 		}
 		p.out = outp;
 	}
-	if (slices && precision == GEMM_FP64 && use_slices(outs, ksum, tiles, s.nnz + t.nnz, num_sms))
+	if (slices && precision == GEMM_FP64 && use_slices(outs, ksum, tiles, s.nnz + t.nnz, r.nnz, num_sms))
 	{
 		g_plan_stage[1] += host_seconds() - ts0;
 		double clocks[2];
@@ -627,7 +630,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 			CTG_CHECK(gx.ktot == ksum[b] && gy.ktot == ksum[b] && gx.rows == (x ? outs[b].n : outs[b].m) &&
 			              gy.rows == (x ? outs[b].m : outs[b].n),
 			          "dot: groups of an output block");
-			p.souts[b] = SliceOut{gx.base, gy.base, (gx.rows + 7) / 8, (gy.rows + 31) / 32, gi[x], gi[1 - x], gx.row0, gy.row0};
+			p.souts[b] = SliceOut{gx.base, gy.base, (gx.rows + 7) / 8, (gy.rows + 31) / 32, gi[x], gi[1 - x], gx.row0, gy.row0, gx.ktot, 0};
 		}
 		slice_tiles(outs, ksum, num_sms, p);
 		p.outs = std::move(outs);

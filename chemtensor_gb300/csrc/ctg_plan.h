@@ -20,6 +20,7 @@ struct SlicePack {
 	std::vector<SliceItem> items;
 	i64 bytes = 0;                       // of the packed digits
 	int rows = 0;                        // of all groups, each padded to 32
+	i64 terms = 0;                       // of all rows
 };
 
 // block_sparse_tensor_dot (block_sparse_tensor.c:1826-2001) as GEMM work lists

@@ -51,11 +51,20 @@ __host__ __device__ inline int slice_exp(int code)
 	return code == 0 ? SLICE_EXP_ZERO : code < SLICE_EXP_MIN || code == 0x7ff ? SLICE_EXP_FP64 : code;
 }
 
-// whether the result of two rows with these exponents is summed in FP64. That of a row of zeros is not, unless it
-// meets a row that is: a number that is not finite makes NaN of it.
-__host__ __device__ inline bool slice_sum_fp64(int e, int f)
+// The digits that are cut off (2^-62, and the orders o >= 8, 2^-59.2 at most, 2^-62.2 in the root mean square, of
+// 2^(e + f) for each term) lie within the rounding of an FP64 sum if some term is not much smaller than the product
+// of its rows' largest entries: if the biased exponents of its factors add up to slice_term_limit at least, k
+// terms are off by sqrt(k) 2^-53.2 of that term (k 2^-50.2 for the worst digits), an FP64 sum by up to k 2^-53 of
+// the sum of all magnitudes.
+constexpr int SLICE_TERM = 7;
+__host__ __device__ inline int slice_term_limit(int e, int f) { return e + f - SLICE_TERM; }
+
+// Whether a result with the biased exponent r of two rows with these exponents has to be looked at again: it may
+// leave the normal range, a row is not finite or tiny, or the result is so small that it does not itself show
+// that it has such a term. That of a row of zeros only if it meets a row that is not finite (NaN) or tiny.
+__host__ __device__ inline bool slice_suspect(int e, int f, int r)
 {
-	return e + f >= SLICE_EXP_ZERO / 2 && !slice_in_range(slice_top(e, f));
+	return e + f >= SLICE_EXP_ZERO / 2 && (!slice_in_range(slice_top(e, f)) || r < slice_term_limit(e, f) - 1023);
 }
 
 // bits of the FP64 number nearest to (h 2^32 + l) 2^(E + F - 2112) (ties away from zero), the value of a
