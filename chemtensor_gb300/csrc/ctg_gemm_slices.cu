@@ -1100,8 +1100,11 @@ void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs,
                         void* check, double* work, int* error, int num_sms, cudaStream_t st)
 {
 	if (ntiles <= 0) return;
-	static std::once_flag attr_once;
-	std::call_once(attr_once, [] {
+	// the attribute belongs to the device
+	static std::once_flag attr_once[64];
+	int dev = 0;
+	CTG_CUDA(cudaGetDevice(&dev));
+	std::call_once(attr_once[dev & 63], [] {
 		CTG_CUDA(cudaFuncSetAttribute(k_gemm_slices, cudaFuncAttributeMaxDynamicSharedMemorySize, SL_SMEM));
 	});
 	// persistent: one CTA per SM (its shared memory admits one)
