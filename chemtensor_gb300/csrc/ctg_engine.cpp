@@ -251,6 +251,7 @@ void Ctx::sync()
 		if (flag != 0)
 		{
 			CTG_CUDA(cudaMemset(tc_error_, 0, sizeof(int)));
+			clear_plans();                     // a product that gave up leaves its plan's split counters as they were
 			throw std::runtime_error("ctgpu: a tensor-core GEMM timed out waiting for its MMAs");
 		}
 	}

@@ -73,6 +73,9 @@ struct SliceInfo {
 constexpr int SL_BARS = 2 * SL_STAGES + 4 + 4 + 1;
 constexpr int SL_SMEM = SL_STAGES * SL_STAGE + SL_EPI_BYTES + 2 * SL_TILES * (int)sizeof(SliceInfo) + SL_BARS * 8 + 32;
 constexpr int SL_WAIT = 1 << 21;                // polls before a wait is declared failed
+// A description of 32 tiles lasts until the slowest warp has passed all of them; should one hang, its own wait
+// ends first and sets the abort flag
+constexpr int SL_INFO_WAITS = 2 * SL_TILES;
 constexpr uint32_t SL_POLL_NS = 1000;           // longest a poll suspends its warp
 static_assert(SL_SMEM <= 227 * 1024, "shared memory per CTA");
 static_assert(2 * SL_ACC <= 512, "tensor memory");
@@ -101,11 +104,12 @@ __device__ __forceinline__ void slice_mma(uint32_t d, uint64_t a, uint64_t b, ui
 		: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"((uint32_t)accumulate));
 }
 
-// bounded wait for the given phase parity; false after SL_WAIT polls, or when *abort is set
-__device__ __forceinline__ bool slice_wait(uint64_t* bar, uint32_t parity, const volatile int* abort)
+// bounded wait for the given phase parity; false after `limit` polls, or when *abort is set. Lanes may differ in
+// what they see last: a warp that goes on together votes.
+__device__ __forceinline__ bool slice_wait(uint64_t* bar, uint32_t parity, const volatile int* abort, int limit)
 {
 	const uint32_t mbar = smem_u32(bar);
-	for (int it = 0; it < SL_WAIT; it++)
+	for (int it = 0; it < limit; it++)
 	{
 		uint32_t done;
 		asm volatile(
@@ -339,7 +343,7 @@ k_slice_lists(const SliceItem* __restrict__ items, const SliceGroup* __restrict_
 __global__ void __launch_bounds__(SL_THREADS, 1)
 k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts, const GemmContrib* cons,
               const GemmSplit* splits, int* counters, int orient, const double* A, const double* B, const unsigned char* xpack,
-              const unsigned char* ypack, const short* xexps, const short* yexps, double* C, uint2* list, unsigned* masks, double* work, int* error)
+              const unsigned char* ypack, const short* xexps, const short* yexps, double* C, uint2* list, unsigned* masks, double* work, int* error, int limit)
 {
 	extern __shared__ __align__(1024) unsigned char smem[];
 	double* stage_out = (double*)(smem + SL_STAGES * SL_STAGE);
@@ -392,7 +396,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 	// the description of the CTA's tile number it (every lane of a warp, in order): null at the end
 	auto tile_info = [&](int it, bool& ok) -> const SliceInfo* {
 		const int batch = (it / SL_TILES) & 1;
-		if (it % SL_TILES == 0) ok = __all_sync(0xffffffffu, slice_wait(info_full + batch, (uint32_t)((it / (2 * SL_TILES)) & 1), abort));
+		if (it % SL_TILES == 0) ok = __all_sync(0xffffffffu, slice_wait(info_full + batch, (uint32_t)((it / (2 * SL_TILES)) & 1), abort, SL_INFO_WAITS * limit));
 		const SliceInfo* f = infos + batch * SL_TILES + it % SL_TILES;
 		return ok && f->tile >= 0 ? f : nullptr;
 	};
@@ -418,7 +422,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 			for (int u = 0; u < nch; u++, g++, xs += xstep, ys += ystep)
 			{
 				const int st = g % SL_STAGES;
-				if (g >= SL_STAGES) ok = slice_wait(empty + st, (uint32_t)(((g / SL_STAGES) - 1) & 1), abort);
+				if (g >= SL_STAGES) ok = slice_wait(empty + st, (uint32_t)(((g / SL_STAGES) - 1) & 1), abort, limit);
 				ok = __all_sync(0xffffffffu, ok);
 				if (!ok) break;
 				if (lane == 0)
@@ -438,7 +442,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 			atomicExch(error, 1);
 		}
 		// the copies of the last stages must land before shared memory is released
-		for (int u = max(g - SL_STAGES, 0); u < g; u++) slice_wait(full + u % SL_STAGES, (uint32_t)((u / SL_STAGES) & 1), nullptr);
+		for (int u = max(g - SL_STAGES, 0); u < g; u++) slice_wait(full + u % SL_STAGES, (uint32_t)((u / SL_STAGES) & 1), nullptr, SL_WAIT);
 	}
 	else if (warp == 1)
 	{
@@ -452,19 +456,25 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 			const SliceInfo* info = tile_info(it, ok);
 			if (!info) break;
 			const int nch = info->nch, halves = info->halves;
-			for (int u = 0; u < nch && ok; u++, g++)
+			for (int u = 0; u < nch && ok; u++)
 			{
 				const int st = g % SL_STAGES;
 				const bool first = u % SL_FLUSH == 0, last = u % SL_FLUSH == SL_FLUSH - 1 || u == nch - 1;
-				ok = slice_wait(full + st, (uint32_t)((g / SL_STAGES) & 1), abort);
+				ok = __all_sync(0xffffffffu, slice_wait(full + st, (uint32_t)((g / SL_STAGES) & 1), abort, limit));
 				if (!ok) break;
 				for (int h = 0; h < halves; h++)
 				{
 					const int fh = f + h, b = fh & 1;
 					if (first && fh >= 2)
 					{
-						ok = slice_wait(acc_empty + b, (uint32_t)(((fh >> 1) - 1) & 1), abort);
-						if (!ok) break;
+						ok = __all_sync(0xffffffffu, slice_wait(acc_empty + b, (uint32_t)(((fh >> 1) - 1) & 1), abort, limit));
+						if (!ok)
+						{
+							// what has been issued of the stage still ends in its commit
+							if (h > 0 && one) mma_commit(smem_u32(empty + st));
+							if (h > 0) g++;
+							break;
+						}
 					}
 					tc_fence_after();
 					if (one)
@@ -482,6 +492,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 					__syncwarp();
 				}
 				if (last) f += halves;
+				if (ok) g++;
 			}
 			tile_done(it);
 		}
@@ -491,7 +502,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 			atomicExch(error, 1);
 		}
 		// no MMA may still run when tensor memory is freed
-		if (g > 0) slice_wait(empty + (g - 1) % SL_STAGES, (uint32_t)(((g - 1) / SL_STAGES) & 1), nullptr);
+		if (g > 0) slice_wait(empty + (g - 1) % SL_STAGES, (uint32_t)(((g - 1) / SL_STAGES) & 1), nullptr, SL_WAIT);
 		pdl_trigger();
 	}
 	else if (warp == 2)
@@ -505,7 +516,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 		{
 			const int batch = (p0 / SL_TILES) & 1;
 			if (p0 >= 2 * SL_TILES)
-				ok = __all_sync(0xffffffffu, slice_wait(info_empty + batch, (uint32_t)((p0 / (2 * SL_TILES) - 1) & 1), abort));
+				ok = __all_sync(0xffffffffu, slice_wait(info_empty + batch, (uint32_t)((p0 / (2 * SL_TILES) - 1) & 1), abort, SL_INFO_WAITS * limit));
 			if (!ok) break;
 			const int pass = p0 + lane, ti = pass * grid + ((pass & 1) ? grid - 1 - me : me);
 			SliceInfo f = {};
@@ -621,7 +632,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 					if (nch > 0)
 					{
 						const int b = f & 1;
-						ok = __all_sync(0xffffffffu, slice_wait(acc_full + b, (uint32_t)((f >> 1) & 1), abort));
+						ok = __all_sync(0xffffffffu, slice_wait(acc_full + b, (uint32_t)((f >> 1) & 1), abort, limit));
 						f++;
 						if (!ok) break;
 						if (active)
@@ -754,7 +765,7 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 				auto step = [&]() {
 					__syncwarp();
 					if (lane == 0) mbar_arrive(smem_u32(split_bar));
-					ok = __all_sync(0xffffffffu, slice_wait(split_bar, (uint32_t)(nsp & 1), abort));
+					ok = __all_sync(0xffffffffu, slice_wait(split_bar, (uint32_t)(nsp & 1), abort, limit));
 					nsp++;
 				};
 				__threadfence();
@@ -1110,7 +1121,8 @@ void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs,
 	// persistent: one CTA per SM (its shared memory admits one)
 	const cudaLaunchConfig_t cfg = launch_config(dim3(std::min(ntiles, num_sms)), dim3(SL_THREADS), SL_SMEM, st);
 	launch_pdl(cfg, k_gemm_slices, ntiles, tiles, outs, souts, cons, splits, counters, orient, A, B, (const unsigned char*)xpack,
-	           (const unsigned char*)ypack, xexps, yexps, C, (uint2*)check, check_masks(check, ntiles, nsplits, max_k), work, error);
+	           (const unsigned char*)ypack, xexps, yexps, C, (uint2*)check, check_masks(check, ntiles, nsplits, max_k), work, error,
+	           (int)std::min<long long>(tc_wait_limit(), SL_WAIT));
 }
 
 void launch_slice_check(int ntiles, int nsplits, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts,

@@ -537,6 +537,8 @@ int tc_k_chunk(int fmt)
 i64 tc_a_rec_bytes(int fmt) { return (i64)tc_parts(fmt) * A_PART_BYTES; }
 i64 tc_b_rec_bytes(int fmt) { return (i64)tc_parts(fmt) * B_PART_BYTES; }
 
+long long tc_wait_limit() { return g_wait_limit; }
+
 void set_tc_wait_limit(long long polls)
 {
 	g_wait_limit = polls > 0 ? polls : TC_WAIT_LIMIT_DEFAULT;

@@ -164,6 +164,7 @@ constexpr int TC_A_ROWS = 128, TC_B_ROWS = 64, TC_KB = 64;
 i64 tc_a_rec_bytes(int fmt);
 i64 tc_b_rec_bytes(int fmt);
 void set_tc_wait_limit(long long polls);
+long long tc_wait_limit();
 struct TcPack {
 	i64 src;           // element offset of (row 0, k 0) of the block in the operand
 	int rows, k;       // block extent

@@ -172,7 +172,7 @@ int ctgpu_inject_failure(int which, int count);
 int ctgpu_set_tc_tile_width(int bn);
 
 /* Number of polls after which a bounded mbarrier wait inside the tensor-core GEMM gives up
- * (0 restores the default, 2^26). A wait that runs out makes the kernel record an error flag,
+ * (0 restores the default, 2^26; the FP64 product by digit slices takes at most 2^21). A wait that runs out makes the kernel record an error flag,
  * let its copies in flight land, free its tensor memory and return; the call that launched it
  * then returns -5. For tests of that error path; process-wide. No counterpart in the reference. */
 void ctgpu_set_tc_wait_limit(long long polls);
