@@ -450,7 +450,7 @@ struct LocalH {
 	bool tc1 = false, tc2 = false, tc3 = false;     // product on the tensor cores (else FP64)
 	bool s1 = false, s2 = false, s3 = false;        // FP64 product by digit slices
 	// their packed operands: r, w, k once per bond, x and the intermediates per application (turn: DotPlan::slice_pack)
-	DBufPtr sp_r, sp_w, sp_k, sp_x, sp_t1, sp_t2;
+	DBufPtr sp_r, sp_w, sp_k, sp_x, sp_t1, sp_t2, check;
 	mutable int turn = 0;
 	bool f1 = false, f2 = false;     // intermediate in FP32 (written and read by tensor-core products only)
 	bool z = false;                  // complex128 entries
@@ -470,10 +470,13 @@ struct LocalH {
 		const int p0[5] = {1, 2, 0, 3, 4};
 		const int p1[5] = {2, 0, 1, 3, 4};
 		const int p2[4] = {0, 3, 1, 2};
-		d1 = make_dot_plan(c, a, AX_TRAILING, r.m(), AX_LEADING, 1, precision, p0);
-		d2 = make_dot_plan(c, w.m(), AX_TRAILING, *d1.out, AX_LEADING, 2, precision, p1);
 		k = op_transpose(c, l, p2);
-		d3 = make_dot_plan(c, k.m(), AX_TRAILING, *d2.out, AX_LEADING, 2, precision);
+		auto plan = [&](bool slices) {
+			d1 = make_dot_plan(c, a, AX_TRAILING, r.m(), AX_LEADING, 1, precision, p0, slices);
+			d2 = make_dot_plan(c, w.m(), AX_TRAILING, *d1.out, AX_LEADING, 2, precision, p1, slices);
+			d3 = make_dot_plan(c, k.m(), AX_TRAILING, *d2.out, AX_LEADING, 2, precision, nullptr, slices);
+		};
+		plan(true);
 		// the cyclic partial trace of the unit outer bonds keeps blocks and entries (view_trace_unit):
 		// with outer axes of dimension 1, equal quantum numbers and opposite directions, the inner
 		// axes obey the conservation law of a, so equal inner axes mean an equal block structure
@@ -486,46 +489,38 @@ struct LocalH {
 			       o.ql[(size_t)i + 1] == a.ql[(size_t)i];
 		CTG_CHECK(same, "local Hamiltonian output structure differs from the input");
 		const size_t wz = z ? 2 : 1;
-		// each product runs where its plan says: the autotuner keeps small products on FP64
-		tc1 = is_tc_precision(d1.precision);
-		tc2 = is_tc_precision(d2.precision);
-		tc3 = is_tc_precision(d3.precision);
-		// an intermediate that only feeds a tensor-core product from a tensor-core product is FP32
-		// (which keeps all the bits the operand formats use): half the traffic
-		f1 = tc1 && tc2;
-		f2 = tc2 && tc3;
-		tt1 = std::make_shared<DBuf>(&c, (size_t)std::max<i64>(d1.out->nnz, 1) * wz * (f1 ? sizeof(float) : sizeof(double)));
-		tt2 = std::make_shared<DBuf>(&c, (size_t)std::max<i64>(d2.out->nnz, 1) * wz * (f2 ? sizeof(float) : sizeof(double)));
+		auto layout = [&] {
+			// each product runs where its plan says: the autotuner keeps small products on FP64
+			tc1 = is_tc_precision(d1.precision);
+			tc2 = is_tc_precision(d2.precision);
+			tc3 = is_tc_precision(d3.precision);
+			// an intermediate that only feeds a tensor-core product from a tensor-core product is FP32
+			// (which keeps all the bits the operand formats use): half the traffic
+			f1 = tc1 && tc2;
+			f2 = tc2 && tc3;
+			tt1.reset();
+			tt2.reset();
+			tt1 = std::make_shared<DBuf>(&c, (size_t)std::max<i64>(d1.out->nnz, 1) * wz * (f1 ? sizeof(float) : sizeof(double)));
+			tt2 = std::make_shared<DBuf>(&c, (size_t)std::max<i64>(d2.out->nnz, 1) * wz * (f2 ? sizeof(float) : sizeof(double)));
+		};
+		layout();
 		flops = (z ? 4.0 : 1.0) * (d1.flops + d2.flops + d3.flops);
+		// where the digits do not fit beside everything else, the FP64 products run on the FP64 pipe
+		if (!reserve_slices(c))
+		{
+			plan(false);
+			layout();
+		}
 		s1 = d1.nstiles > 0;
 		s2 = d2.nstiles > 0;
 		s3 = d3.nstiles > 0;
-		auto buf = [&](const DotPlan& d, int s) {
-			DBufPtr p = std::make_shared<DBuf>(&c, (size_t)d.slice_bytes(s));
-			d.slice_clear(c, s, p->ptr);
-			return p;
-		};
-		auto fixed = [&](const DotPlan& d, int s, const double* x) {
-			DBufPtr p = buf(d, s);
+		auto fixed = [&](const DotPlan& d, int s, const double* x, const DBufPtr& p) {
 			KScope ks(c, K_GEMM, 2);
 			d.slice_pack(c, s, x, p->ptr, 0);
-			return p;
 		};
-		if (s1)
-		{
-			sp_r = fixed(d1, 1, r.data());
-			sp_x = buf(d1, 0);
-		}
-		if (s2)
-		{
-			sp_w = fixed(d2, 0, w.data());
-			sp_t1 = buf(d2, 1);
-		}
-		if (s3)
-		{
-			sp_k = fixed(d3, 0, k.data());
-			sp_t2 = buf(d3, 1);
-		}
+		if (s1) fixed(d1, 1, r.data(), sp_r);
+		if (s2) fixed(d2, 0, w.data(), sp_w);
+		if (s3) fixed(d3, 0, k.data(), sp_k);
 		// operands fixed for the bond (r, w, k) are packed once; x and the intermediates per apply
 		auto rec = [&](i64 bytes) { return std::make_shared<DBuf>(&c, (size_t)std::max<i64>(bytes, 16)); };
 		if (tc1)
@@ -546,6 +541,38 @@ struct LocalH {
 			pk_t2 = rec(d3.b_rec_bytes());
 			d3.pack_a(c, k.data(), pk_k->ptr);
 		}
+	}
+
+	// buffers of the products by digit slices; false (and none kept) if there is no room for all of them
+	bool reserve_slices(Ctx& c)
+	{
+		bool ok = true;
+		size_t most = 0;
+		auto buf = [&](const DotPlan& d, int s) -> DBufPtr {
+			if (!ok) return nullptr;
+			DBufPtr p = DBuf::try_make(&c, (size_t)d.slice_bytes(s));
+			ok = p != nullptr;
+			if (ok) d.slice_clear(c, s, p->ptr);
+			return p;
+		};
+		auto pair = [&](const DotPlan& d, DBufPtr& fixed, int sf, DBufPtr& other) {
+			if (d.nstiles == 0) return;
+			ok = ok && d.slice_room(c);
+			fixed = buf(d, sf);
+			other = buf(d, 1 - sf);
+			most = std::max(most, (size_t)d.check_bytes());
+		};
+		pair(d1, sp_r, 1, sp_x);
+		pair(d2, sp_w, 0, sp_t1);
+		pair(d3, sp_k, 0, sp_t2);
+		if (ok && most > 0)
+		{
+			check = DBuf::try_make(&c, most);
+			ok = check != nullptr;
+		}
+		if (!ok)
+			for (DBufPtr* p : {&sp_r, &sp_w, &sp_k, &sp_x, &sp_t1, &sp_t2, &check}) p->reset();
+		return ok;
 	}
 
 	void apply(Ctx& c, const double* x, double* y) const
@@ -569,7 +596,7 @@ struct LocalH {
 		{
 			KScope ks(c, K_GEMM, 5, d1.flops, 0);
 			d1.slice_pack(c, 0, x, sp_x->ptr, turn);
-			d1.run_slices(c, x, r.data(), sp_x->ptr, sp_r->ptr, t1);
+			d1.run_slices(c, x, r.data(), sp_x->ptr, sp_r->ptr, t1, check->ptr);
 			c.gemm_flops += d1.flops;
 		}
 		else d1.run(c, x, r.data(), t1);
@@ -583,7 +610,7 @@ struct LocalH {
 		{
 			KScope ks(c, K_GEMM, 5, d2.flops, 0);
 			d2.slice_pack(c, 1, t1, sp_t1->ptr, turn);
-			d2.run_slices(c, w.data(), t1, sp_w->ptr, sp_t1->ptr, t2);
+			d2.run_slices(c, w.data(), t1, sp_w->ptr, sp_t1->ptr, t2, check->ptr);
 			c.gemm_flops += d2.flops;
 		}
 		else d2.run(c, w.data(), t1, t2);
@@ -597,7 +624,7 @@ struct LocalH {
 		{
 			KScope ks(c, K_GEMM, 5, d3.flops, 0);
 			d3.slice_pack(c, 1, t2, sp_t2->ptr, turn);
-			d3.run_slices(c, k.data(), t2, sp_k->ptr, sp_t2->ptr, y);
+			d3.run_slices(c, k.data(), t2, sp_k->ptr, sp_t2->ptr, y, check->ptr);
 			c.gemm_flops += d3.flops;
 		}
 		else d3.run(c, k.data(), t2, y);
@@ -612,18 +639,20 @@ thread_local double g_host_detail[4];       // host time: local-H setup, matvecs
 int minimize_local_energy(Ctx& c, const DTensor& w, const DTensor& l, const DTensor& r, const DTensor& a_start, int maxiter,
                           LanczosScalars* d_sc, DTensor& a_opt, DmrgStats* st, int precision)
 {
-	double hz = now_s();
-	LocalH h(c, a_start.m(), w, l, r, precision);
-	g_host_detail[0] += now_s() - hz;
-	CTG_CHECK(a_start.cplx == h.z, "local eigenproblem: start vector and operator of different numeric types");
 	// the vector as doubles (a complex128 vector is its real and imaginary parts: the Lanczos
 	// scalars alpha = Re <v, w> and beta = ||w|| of lanczos_iteration_z are the real ones of
-	// that vector, krylov.c:96-165); the breakdown test counts entries
+	// that vector, krylov.c:96-165); the breakdown test counts entries. Allocated first: the local
+	// Hamiltonian takes what memory is left.
 	const i64 nent = a_start.m().nnz;
 	const i64 n = nent * a_start.width();
 	DBuf V(&c, (size_t)maxiter * n * sizeof(double));
 	DBuf wv(&c, (size_t)n * sizeof(double));
 	DBuf partial(&c, 2 * RED_BLOCKS * sizeof(double));
+	a_opt = c.empty(a_start.meta, a_start.cplx);
+	double hz = now_s();
+	LocalH h(c, a_start.m(), w, l, r, precision);
+	g_host_detail[0] += now_s() - hz;
+	CTG_CHECK(a_start.cplx == h.z, "local eigenproblem: start vector and operator of different numeric types");
 	double* Vp = (double*)V.ptr;
 	double* wp = (double*)wv.ptr;
 	double* pp = (double*)partial.ptr;
@@ -640,7 +669,6 @@ int minimize_local_energy(Ctx& c, const DTensor& w, const DTensor& l, const DTen
 		KScope ks(c, K_LANCZOS, 1, 3.0 * dn, 24.0 * dn);
 		launch_lz_start(a_start.data(), Vp, n, pp, d_sc, c.steady, s);
 	}
-	a_opt = c.empty(a_start.meta, a_start.cplx);
 	for (int j = 0; j < maxiter; j++)
 	{
 		hz = now_s();
@@ -674,8 +702,8 @@ int minimize_local_energy(Ctx& c, const DTensor& w, const DTensor& l, const DTen
 DTensor apply_local_hamiltonian_once(Ctx& c, const DTensor& a, const DTensor& w, const DTensor& l, const DTensor& r,
                                      int precision)
 {
-	LocalH h(c, a.m(), w, l, r, precision);
 	DTensor out = c.empty(a.meta);
+	LocalH h(c, a.m(), w, l, r, precision);
 	h.apply(c, a.data(), out.data());
 	return out;
 }
@@ -683,8 +711,8 @@ DTensor apply_local_hamiltonian_once(Ctx& c, const DTensor& a, const DTensor& w,
 double time_local_hamiltonian(Ctx& c, const DTensor& a, const DTensor& w, const DTensor& l, const DTensor& r,
                               int precision, int nmatvec, double* flops)
 {
-	LocalH h(c, a.m(), w, l, r, precision);
 	DTensor out = c.empty(a.meta);
+	LocalH h(c, a.m(), w, l, r, precision);
 	for (int i = 0; i < 3; i++) h.apply(c, a.data(), out.data());
 	cudaEvent_t e[2];
 	for (auto& x : e) CTG_CUDA(cudaEventCreate(&x));

@@ -21,6 +21,17 @@ namespace ctg {
 // ------------------------------------------------------------------------------------
 
 DBuf::DBuf(Ctx* c, size_t n) : ctx(c), bytes(n) { ptr = c->alloc(n); }
+DBufPtr DBuf::try_make(Ctx* c, size_t n)
+{
+	void* p = c->try_alloc(n);
+	if (!p) return nullptr;
+	DBufPtr b(new DBuf());
+	b->ctx = c;
+	b->ptr = p;
+	b->bytes = n;
+	return b;
+}
+
 DBuf::~DBuf()
 {
 	if (ptr && ctx) ctx->free(ptr);
@@ -84,6 +95,7 @@ void Ctx::clear_plans()
 {
 	plans_->map.clear();
 	plans_->bytes = 0;
+	split_work_.reset();
 }
 
 static void plan_insert(Ctx& c, uint64_t key, PlanEntry&& e, size_t bytes)
@@ -191,6 +203,7 @@ Ctx::~Ctx()
 		if (join_ev_[i]) cudaEventDestroy(join_ev_[i]);
 	}
 	delete plans_;
+	split_work_.reset();
 	if (pinned_) cudaFreeHost(pinned_);
 	if (pinned_d_) cudaFreeHost(pinned_d_);
 	if (fork_ev_) cudaEventDestroy(fork_ev_);
@@ -214,14 +227,42 @@ Ctx& context_for_device(int device)
 	return *ctxs.back();
 }
 
-void* Ctx::alloc(size_t bytes)
+void* Ctx::try_alloc(size_t bytes)
 {
 	const double t0 = host_seconds();
 	void* p = nullptr;
 	if (bytes == 0) bytes = 16;
-	CTG_CUDA(cudaMallocFromPoolAsync(&p, (bytes + 255) & ~(size_t)255, pool_, st_));
+	const cudaError_t e = cudaMallocFromPoolAsync(&p, (bytes + 255) & ~(size_t)255, pool_, st_);
 	host_alloc_s += host_seconds() - t0;
+	if (e == cudaErrorMemoryAllocation)
+	{
+		cudaGetLastError();
+		return nullptr;
+	}
+	CTG_CUDA(e);
 	return p;
+}
+
+void* Ctx::alloc(size_t bytes)
+{
+	void* p = try_alloc(bytes);
+	if (!p) CTG_CUDA(cudaErrorMemoryAllocation);
+	return p;
+}
+
+bool Ctx::reserve_split_work(size_t bytes)
+{
+	if (split_work_ && split_work_->bytes >= bytes) return true;
+	split_work_.reset();
+	split_work_ = DBuf::try_make(this, bytes);
+	return split_work_ != nullptr;
+}
+
+double* Ctx::split_work(size_t bytes)
+{
+	if (bytes == 0) return nullptr;
+	if (!reserve_split_work(bytes)) CTG_CUDA(cudaErrorMemoryAllocation);
+	return (double*)split_work_->ptr;
 }
 
 void Ctx::free(void* p)
@@ -444,7 +485,7 @@ static int tuned_tile_width(Ctx& c, const Meta& s, int axs, const Meta& t, int a
                             const int* out_perm, const DotLowering& l64);
 
 static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision,
-                              const int* out_perm)
+                              const int* out_perm, bool slices)
 {
 	// complex128: the FP64 lists and tiles, over complex entries
 	const bool z = precision == GEMM_Z64;
@@ -454,12 +495,12 @@ static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int
 		// cores to pay for their operand packing (FP64 is then both faster and exact). Its key comes
 		// from the output blocks and contributions, which the FP64 lowering has too: a product that
 		// stays on FP64 is lowered once, one on the tensor cores twice
-		DotLowering l = lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm, 64, true, c.steady);
+		DotLowering l = lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm, 64, slices, c.steady);
 		const int bn = tuned_tile_width(c, s, axs, t, axt, nmult, precision, out_perm, l);
 		if (bn == 0) return upload_dot_plan(c, std::move(l), GEMM_FP64, 64);
 		return upload_dot_plan(c, lower_dot(s, axs, t, axt, nmult, precision, c.num_sms(), out_perm, bn), precision, bn);
 	}
-	DotLowering l = lower_dot(s, axs, t, axt, nmult, z ? (int)GEMM_FP64 : precision, c.num_sms(), out_perm, 64, !z, c.steady);
+	DotLowering l = lower_dot(s, axs, t, axt, nmult, z ? (int)GEMM_FP64 : precision, c.num_sms(), out_perm, 64, slices && !z, c.steady);
 	return upload_dot_plan(c, std::move(l), precision, 64);
 }
 
@@ -519,7 +560,7 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 	p.splits = at<GemmSplit>(p.desc, o_splits);
 	p.nsplits = (int)l.splits.size();
 	const size_t entry = precision == GEMM_Z64 ? 2 * sizeof(double) : sizeof(double);
-	if (l.work_doubles > 0) p.work = std::make_shared<DBuf>(&c, (size_t)l.work_doubles * entry);
+	p.work_bytes = (size_t)l.work_doubles * entry;
 	if (!l.splits.empty())
 	{
 		// completion counters of the split tiles: zero now, and reset by the kernel after each use
@@ -536,7 +577,7 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 	return p;
 }
 
-void DotPlan::run(Ctx& c, const double* A, const double* B, double* C) const
+bool DotPlan::run(Ctx& c, const double* A, const double* B, double* C) const
 {
 	if (is_tc_precision(precision))
 	{
@@ -549,31 +590,35 @@ void DotPlan::run(Ctx& c, const double* A, const double* B, double* C) const
 			run_packed(c, apk.ptr, bpk.ptr, C);
 		}
 		c.gemm_flops += flops;
-		return;
+		return true;
 	}
 	if (ntiles[0] > 0 || nstiles > 0)
 	{
 		KScope ks(c, K_GEMM, nstiles > 0 ? 7 : 1, flops, 0);
-		launch_f64(c, A, B, C);
+		if (!launch_f64(c, A, B, C)) return false;
 	}
 	c.gemm_flops += flops;
+	return true;
 }
 
-void DotPlan::launch_f64(Ctx& c, const double* A, const double* B, double* C) const
+bool DotPlan::launch_f64(Ctx& c, const double* A, const double* B, double* C) const
 {
-	double* w = work ? (double*)work->ptr : nullptr;
 	int* cnt = counters ? (int*)counters->ptr : nullptr;
 	if (nstiles > 0)
 	{
-		DBuf pa(&c, (size_t)slice_bytes(0)), pb(&c, (size_t)slice_bytes(1));
-		slice_clear(c, 0, pa.ptr);
-		slice_clear(c, 1, pb.ptr);
-		slice_pack(c, 0, A, pa.ptr, 0);
-		slice_pack(c, 1, B, pb.ptr, 0);
-		run_slices(c, A, B, pa.ptr, pb.ptr, C);
+		if (!slice_room(c)) return false;
+		const DBufPtr pa = DBuf::try_make(&c, (size_t)slice_bytes(0)), pb = pa ? DBuf::try_make(&c, (size_t)slice_bytes(1)) : nullptr,
+		              check = pb ? DBuf::try_make(&c, (size_t)check_bytes()) : nullptr;
+		if (!check) return false;
+		slice_clear(c, 0, pa->ptr);
+		slice_clear(c, 1, pb->ptr);
+		slice_pack(c, 0, A, pa->ptr, 0);
+		slice_pack(c, 1, B, pb->ptr, 0);
+		run_slices(c, A, B, pa->ptr, pb->ptr, C, check->ptr);
 	}
 	else if (ntiles[0] > 0)
-		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, w, c.stream(), flops, large);
+		launch_gemm_f64(ntiles[0], tiles[0], outs, cons, splits, cnt, A, B, C, c.split_work(work_bytes), c.stream(), flops, large);
+	return true;
 }
 
 // a packed operand: two arrays of codes, the list lengths, the exponents; the digits; the lists
@@ -589,6 +634,17 @@ static SliceTerm* slice_lists(const DotPlan::Side& d, const void* pack)
 i64 DotPlan::slice_bytes(int s) const
 {
 	return (i64)slice_head(side[s]) + std::max<i64>(side[s].bytes, 16) + side[s].terms * (i64)sizeof(SliceTerm);
+}
+
+i64 DotPlan::check_bytes() const { return slice_check_bytes(nstiles, nsplits, max_k); }
+
+bool DotPlan::slice_room(Ctx& c) const
+{
+	static const i64 most = [] {
+		const char* e = getenv("CTGPU_SLICE_BYTES");
+		return e ? (i64)atoll(e) : INT64_MAX;
+	}();
+	return slice_bytes(0) + slice_bytes(1) <= most && (work_bytes == 0 || c.reserve_split_work(work_bytes));
 }
 
 void DotPlan::slice_clear(Ctx& c, int s, void* pack) const
@@ -607,18 +663,17 @@ void DotPlan::slice_pack(Ctx& c, int s, const double* x, void* pack, int turn) c
 	if (d.terms > 0) launch_slice_lists(d.nitems, d.items, d.groups, d.runs, x, slice_lists(d, pack), slice_counts(d, pack), c.stream());
 }
 
-void DotPlan::run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C) const
+void DotPlan::run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C, void* check) const
 {
 	const int x = orient ? 0 : 1;
 	const void* pack[2] = {apack, bpack};
 	const short *xe = slice_exps(side[x], pack[x]), *ye = slice_exps(side[1 - x], pack[1 - x]);
-	DBuf check(&c, (size_t)slice_check_bytes(nstiles, nsplits, max_k));
 	launch_gemm_slices(nstiles, stiles, outs, souts, cons, nsplits, splits, counters ? (int*)counters->ptr : nullptr, orient, A, B,
 	                   (const char*)pack[x] + slice_head(side[x]), (const char*)pack[1 - x] + slice_head(side[1 - x]), xe, ye, C,
-	                   max_k, check.ptr, work ? (double*)work->ptr : nullptr, c.tc_error(), c.num_sms(), c.stream());
+	                   max_k, check, c.split_work(work_bytes), c.tc_error(), c.num_sms(), c.stream());
 	const int small = b_entries < a_entries ? 1 : 0;
 	launch_slice_check(nstiles, nsplits, stiles, outs, souts, cons, splits, orient, small == 1, side[small].groups,
-	                   slice_lists(side[small], pack[small]), slice_counts(side[small], pack[small]), A, B, xe, ye, C, max_k, check.ptr,
+	                   slice_lists(side[small], pack[small]), slice_counts(side[small], pack[small]), A, B, xe, ye, C, max_k, check,
 	                   c.num_sms(), c.stream());
 }
 
@@ -627,7 +682,7 @@ void DotPlan::run_z(Ctx& c, const double* A, const double* B, double* C, bool co
 	CTG_CHECK(precision == GEMM_Z64, "complex GEMM on a real plan");
 	KScope ks(c, K_GEMM, 1, 4.0 * flops, 0);
 	launch_gemm_z(ntiles[0], tiles[0], outs, cons, splits, counters ? (int*)counters->ptr : nullptr, A, B, C,
-	              work ? (double*)work->ptr : nullptr, conj_a, conj_b, c.stream(), 4.0 * flops);
+	              c.split_work(work_bytes), conj_a, conj_b, c.stream(), 4.0 * flops);
 	c.gemm_flops += 4.0 * flops;
 }
 
@@ -762,7 +817,7 @@ double time_tc_variant(Ctx& c, DotLowering&& l, int precision, int bn, const Met
 		for (int rep = 0; rep < 3; rep++)
 		{
 			CTG_CUDA(cudaEventRecord(e[0], c.stream()));
-			p.launch_f64(c, (const double*)A.ptr, (const double*)B.ptr, (double*)C.ptr);
+			if (!p.launch_f64(c, (const double*)A.ptr, (const double*)B.ptr, (double*)C.ptr)) break;    // no room: not chosen
 			CTG_CUDA(cudaEventRecord(e[1], c.stream()));
 			CTG_CUDA(cudaEventSynchronize(e[1]));
 			float ms = 0;
@@ -935,13 +990,13 @@ static void dump_plan_request(int kind, const std::vector<i64>& params, const Me
 	fflush(f);
 }
 
-constexpr i64 PLAN_STEADY = 1 << 16;      // beside the precision in a plan's key
+constexpr i64 PLAN_STEADY = 1 << 16, PLAN_TILES = 1 << 17;      // beside the precision in a plan's key
 
 DotPlan make_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision,
-                      const int* out_perm)
+                      const int* out_perm, bool slices)
 {
 	PlanTimer plan_timer(c);
-	std::vector<i64> params = {axs, axt, nmult, precision + (c.steady ? PLAN_STEADY : 0)};
+	std::vector<i64> params = {axs, axt, nmult, precision + (c.steady ? PLAN_STEADY : 0) + (slices ? 0 : PLAN_TILES)};
 	if (out_perm)
 		for (int i = 0; i < s.ndim + t.ndim - 2 * nmult; i++) params.push_back(out_perm[i]);
 	const uint64_t key = plan_key(0, params, s, &t);
@@ -952,7 +1007,7 @@ DotPlan make_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, in
 	e.params = params;
 	e.s = StructSig(s);
 	e.t = StructSig(t);
-	e.dot = build_dot_plan(c, s, axs, t, axt, nmult, precision, out_perm);
+	e.dot = build_dot_plan(c, s, axs, t, axt, nmult, precision, out_perm, slices);
 	const size_t bytes = e.dot.desc ? e.dot.desc->bytes : 0;
 	DotPlan p = e.dot;
 	plan_insert(c, key, std::move(e), bytes);
@@ -1024,7 +1079,8 @@ DTensor op_dot(Ctx& c, const DTensor& s, int axs, const DTensor& t, int axt, int
 	DTensor r;
 	r.meta = p.out;
 	r.buf = std::make_shared<DBuf>(&c, (size_t)std::max<i64>(p.out->nnz, 1) * sizeof(double));
-	p.run(c, s.data(), t.data(), r.data());
+	if (!p.run(c, s.data(), t.data(), r.data()))
+		make_dot_plan(c, s.m(), axs, t.m(), axt, nmult, precision, nullptr, false).run(c, s.data(), t.data(), r.data());
 	return r;
 }
 

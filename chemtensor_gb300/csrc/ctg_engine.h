@@ -42,8 +42,13 @@ struct DBuf {
 	size_t bytes = 0;
 	DBuf(Ctx* c, size_t n);
 	~DBuf();
+	// null where the device has no room for it
+	static std::shared_ptr<DBuf> try_make(Ctx* c, size_t n);
 	DBuf(const DBuf&) = delete;
 	DBuf& operator=(const DBuf&) = delete;
+
+private:
+	DBuf() = default;
 };
 using DBufPtr = std::shared_ptr<DBuf>;
 
@@ -72,7 +77,12 @@ public:
 	void fork(int n);
 	void join(int n);
 	void* alloc(size_t bytes);
+	void* try_alloc(size_t bytes);   // null where the device has no room for it
 	void free(void* p);
+	// Partial sums of split tiles: one work space for the products of all plans, which follow one another on
+	// stream(). false: no room for it.
+	bool reserve_split_work(size_t bytes);
+	double* split_work(size_t bytes);
 	// make the private pool hold at least this many bytes, so that later allocations are served
 	// without growing it (growing maps new physical memory, which costs milliseconds)
 	void reserve(size_t bytes);
@@ -138,6 +148,7 @@ private:
 	cudaEvent_t get_event();
 	int dev_;
 	int sms_ = 1;
+	DBufPtr split_work_;
 	int* tc_error_ = nullptr;
 	bool tc_used_ = false;
 	struct PlanCache* plans_ = nullptr;
@@ -177,7 +188,7 @@ struct DotPlan {
 	const GemmContrib* cons = nullptr;
 	const GemmSplit* splits = nullptr;   // tiles whose sum is split over several CTAs
 	int nsplits = 0;
-	DBufPtr work;                        // their partial sums
+	size_t work_bytes = 0;               // their partial sums (Ctx::split_work)
 	DBufPtr counters;                    // their completion counters (one int per split tile)
 	// FP64 on the tensor cores by digit slices (then ntiles is 0); side 0 is operand A, 1 is B
 	int nstiles = 0, orient = 0, max_k = 0;
@@ -203,17 +214,23 @@ struct DotPlan {
 	double flops_cls[NUM_TILE_CLASSES] = {};
 	bool large = false;                  // some FP64 tile is a TILE_L (also one without terms)
 	int precision = GEMM_FP64;
-	void run(Ctx& c, const double* A, const double* B, double* C) const;
+	// false, and nothing done, if the product runs by digit slices and there is no room for the digits: the caller then
+	// makes a plan without them
+	bool run(Ctx& c, const double* A, const double* B, double* C) const;
 	// the FP64 product's launches alone (no counters)
-	void launch_f64(Ctx& c, const double* A, const double* B, double* C) const;
+	bool launch_f64(Ctx& c, const double* A, const double* B, double* C) const;
 	// a product by digit slices in parts, so that an operand used by many runs is packed once. A packed operand is
 	// one buffer (slice_bytes): two arrays of its rows' exponent codes, used in turn (a call of slice_pack clears
 	// the other one; both are zero before the first, slice_clear), the rows' exponents, the digits and, for a small
 	// operand, lists of its rows' nonzero terms
+	// check: check_bytes. slice_room: whether the digits of both operands may be held at all (CTGPU_SLICE_BYTES), and the
+	// partial sums of split tiles have room.
 	i64 slice_bytes(int s) const;
+	i64 check_bytes() const;
+	bool slice_room(Ctx& c) const;
 	void slice_clear(Ctx& c, int s, void* pack) const;
 	void slice_pack(Ctx& c, int s, const double* x, void* pack, int turn) const;
-	void run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C) const;
+	void run_slices(Ctx& c, const double* A, const double* B, const void* apack, const void* bpack, double* C, void* check) const;
 	// complex128 entries, operands optionally read conjugated
 	void run_z(Ctx& c, const double* A, const double* B, double* C, bool conj_a, bool conj_b) const;
 	// tensor-core path in parts, so that an operand used by many runs is packed once; src_f32: the
@@ -226,9 +243,9 @@ struct DotPlan {
 	void run_packed(Ctx& c, const void* apack, const void* bpack, void* C, bool out_f32 = false) const;
 };
 // out_perm (every precision): the result is written straight in the layout of its transpose by out_perm
-// (see lower_dot), and the plan's `out` is that transposed structure
+// (see lower_dot), and the plan's `out` is that transposed structure. slices: an FP64 product may run by digit slices.
 DotPlan make_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision = GEMM_FP64,
-                      const int* out_perm = nullptr);
+                      const int* out_perm = nullptr, bool slices = true);
 
 // Tile autotuner of the reduced-precision GEMMs: the column width (64, 128 or 256) of a product's
 // tensor-core tiles, or FP64 (0) where the product is too small for the tensor cores to pay for the
