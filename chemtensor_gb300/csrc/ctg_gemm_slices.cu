@@ -590,7 +590,9 @@ k_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs, const Sli
 			// (the sums of the orders 0 .. 2 stay below 2^22 for 128 terms, and always go that way: the integer
 			// conversion runs at an eighth of the rate)
 			const bool few_last = nch > 0 && (nch - 1) % SL_FLUSH < 2;
-			const int64_t start_hi = -0x4b400000ll * ((int64_t)nfl * 0x01010100ll + (few_last ? 1 : 0));
+			// (modulo 2^64, as the sums: the offsets pass 63 bits at 437 flushes, the orders themselves do not before
+			// SLICE_TERMS_MAX terms)
+			const int64_t start_hi = (int64_t)(0ull - 0x4b400000ull * ((uint64_t)nfl * 0x01010100ull + (few_last ? 1 : 0)));
 			const int64_t start_lo = few_last ? -0x4b400000ll * 0x01010101ll : 0;
 			for (int fl = 0; fl < nfl && ok; fl++)
 			{

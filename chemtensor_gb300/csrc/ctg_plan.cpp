@@ -1,6 +1,7 @@
 // ctg_plan.cpp - lowering of block-sparse operations into descriptor lists (host only).
 #include "ctg_plan.h"
 #include "ctg_pool.h"
+#include "ctg_slices.h"
 
 #include <algorithm>
 #include <chrono>
@@ -150,6 +151,8 @@ bool use_slices(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum, 
 		return e ? atoi(e) : -1;
 	}();
 	if (forced == 0) return false;
+	for (i64 k : ksum)
+		if (k > SLICE_TERMS_MAX) return false;
 	if (forced == 1) return true;
 	double clocks[2], f64 = 0;
 	const int o = slice_orient(outs, ksum, clocks);

@@ -20,6 +20,7 @@ namespace ctg {
 
 constexpr int SLICES = 8;                  // digits of an entry
 constexpr int SLICE_K = 128;               // terms summed in FP32 before the sums move to integers
+constexpr int SLICE_TERMS_MAX = 1 << 21;   // most terms of a result: its low orders, below 2^48 per 128 terms, stay in 63 bits
 constexpr int SLICE_EXP_MIN = 128;         // rows whose largest entry has a smaller biased exponent (or holds a
                                            // number that is not finite) are summed in FP64 instead
 constexpr int SLICE_EXP_ZERO = -4000;      // in place of the exponent: a row of zeros
