@@ -388,8 +388,6 @@ void launch_gemm_z(int ntiles, const GemmTile* tiles, const GemmOut* outs, const
 // entries at a time, their divisions and loads side by side. Hubbard chain at D = 256, per launch: permutations
 // 11.6 -> 6.9 us, row maps 6.4 -> 4.5; the two-site search 251 -> 248.5 ms, the one-site search 59.5 -> 57.7, energy and
 // norm 4.45 -> 4.2. Chunks of 1024 instead of 4096 entries: 5.8 and 3.7 us, the searches within their noise.
-constexpr int COPY_BATCH = 4;
-
 // the block's descriptor to shared memory, by all threads
 template <class D>
 __device__ __forceinline__ void copy_desc(D* to, const D* __restrict__ from)
@@ -417,7 +415,7 @@ k_permute(const Chunk* __restrict__ chunks, const PermDesc* __restrict__ descs, 
 		const int nd = d.ndim;
 		const T* s = src + d.src_off;
 		T* t = dst + d.dst_off;
-		for (int e0 = (int)ch.start + threadIdx.x; e0 < (int)end; e0 += COPY_BATCH * blockDim.x)
+		for (unsigned e0 = copy_first(ch.start, threadIdx.x); e0 < (unsigned)end; e0 = copy_next(e0, blockDim.x))
 		{
 			unsigned r[COPY_BATCH];
 			i64 so[COPY_BATCH];
@@ -425,7 +423,7 @@ k_permute(const Chunk* __restrict__ chunks, const PermDesc* __restrict__ descs, 
 #pragma unroll
 			for (int u = 0; u < COPY_BATCH; u++)
 			{
-				r[u] = (unsigned)e0 + u * blockDim.x;
+				r[u] = copy_entry(e0, u, blockDim.x);
 				so[u] = 0;
 			}
 			for (int i = nd - 1; i > 0; i--)
@@ -443,10 +441,10 @@ k_permute(const Chunk* __restrict__ chunks, const PermDesc* __restrict__ descs, 
 			const i64 st0 = d.sstr[0];
 #pragma unroll
 			for (int u = 0; u < COPY_BATCH; u++)
-				if (e0 + u * (int)blockDim.x < (int)end) v[u] = s[so[u] + (i64)r[u] * st0];
+				if (copy_entry(e0, u, blockDim.x) < (unsigned)end) v[u] = s[so[u] + (i64)r[u] * st0];
 #pragma unroll
 			for (int u = 0; u < COPY_BATCH; u++)
-				if (e0 + u * (int)blockDim.x < (int)end) t[e0 + u * blockDim.x] = v[u];
+				if (copy_entry(e0, u, blockDim.x) < (unsigned)end) t[copy_entry(e0, u, blockDim.x)] = v[u];
 		}
 		return;
 	}
@@ -498,7 +496,7 @@ k_rowmap(const Chunk* __restrict__ chunks, const RowDesc* __restrict__ descs, co
 		const i64 srows = d.src_rows, drows = d.dst_rows;
 		const T* s = src + d.src_off;
 		T* o = dst + d.dst_off;
-		for (unsigned e0 = (unsigned)ch.start + threadIdx.x; e0 < (unsigned)end; e0 += COPY_BATCH * blockDim.x)
+		for (unsigned e0 = copy_first(ch.start, threadIdx.x); e0 < (unsigned)end; e0 = copy_next(e0, blockDim.x))
 		{
 			unsigned t[COPY_BATCH], lead[COPY_BATCH], j[COPY_BATCH];
 			i64 mj[COPY_BATCH];
@@ -506,7 +504,7 @@ k_rowmap(const Chunk* __restrict__ chunks, const RowDesc* __restrict__ descs, co
 #pragma unroll
 			for (int u = 0; u < COPY_BATCH; u++)
 			{
-				const unsigned e = e0 + u * blockDim.x;
+				const unsigned e = copy_entry(e0, u, blockDim.x);
 				const unsigned lj = e / nt;
 				t[u] = e - lj * nt;
 				lead[u] = lj / nr;
@@ -515,11 +513,11 @@ k_rowmap(const Chunk* __restrict__ chunks, const RowDesc* __restrict__ descs, co
 			}
 #pragma unroll
 			for (int u = 0; u < COPY_BATCH; u++)
-				if (e0 + u * blockDim.x < (unsigned)end)
+				if (copy_entry(e0, u, blockDim.x) < (unsigned)end)
 					v[u] = s[((i64)lead[u] * srows + (scatter ? (i64)j[u] : mj[u])) * nt + t[u]];
 #pragma unroll
 			for (int u = 0; u < COPY_BATCH; u++)
-				if (e0 + u * blockDim.x < (unsigned)end)
+				if (copy_entry(e0, u, blockDim.x) < (unsigned)end)
 					o[((i64)lead[u] * drows + (scatter ? mj[u] : (i64)j[u])) * nt + t[u]] = v[u];
 		}
 		return;

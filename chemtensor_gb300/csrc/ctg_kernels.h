@@ -213,6 +213,12 @@ struct Chunk {
 };
 
 constexpr int COPY_CHUNK = 4096;
+// The entries of a chunk that a thread copies: COPY_BATCH at a time, `threads` apart. In unsigned 32 bits, which
+// hold every index that is formed (past the end by up to a batch) for blocks of fewer than 2^31 entries.
+constexpr int COPY_BATCH = 4;
+__host__ __device__ inline unsigned copy_first(i64 start, unsigned thread) { return (unsigned)start + thread; }
+__host__ __device__ inline unsigned copy_entry(unsigned e0, int u, unsigned threads) { return e0 + (unsigned)u * threads; }
+__host__ __device__ inline unsigned copy_next(unsigned e0, unsigned threads) { return e0 + COPY_BATCH * threads; }
 
 // cplx: entries are complex128 (two doubles each); descriptors count entries
 void launch_permute(int nchunks, const Chunk* chunks, const PermDesc* descs, const double* src, double* dst, cudaStream_t st,
