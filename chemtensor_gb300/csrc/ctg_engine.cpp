@@ -775,7 +775,10 @@ void tune_load(TuneTable& t)
 
 // flop-weighted histogram of a product's output blocks by column extent (<= 64, 128, 256, 512,
 // more) and summed contracted extent (<= 64, 256, more), shares rounded to eighths; with the
-// precision and the log4 of the total work
+// precision and the log4 of the total work. At the end whether the FP64 product runs by digit slices, and a version
+// that is raised whenever a timed kernel changes its speed: lines of a file that were timed against others
+// are not taken
+constexpr int TUNE_VERSION = 2;
 std::string tune_key(const DotLowering& l, int precision)
 {
 	double hn[5] = {0, 0, 0, 0, 0}, hk[3] = {0, 0, 0}, total = 0;
@@ -792,9 +795,9 @@ std::string tune_key(const DotLowering& l, int precision)
 	}
 	char buf[160];
 	auto q = [&](double x) { return total > 0 ? (int)std::lround(8.0 * x / total) : 0; };
-	snprintf(buf, sizeof buf, "p%d_w%d_n%d.%d.%d.%d.%d_k%d.%d.%d", precision,
+	snprintf(buf, sizeof buf, "p%d_w%d_n%d.%d.%d.%d.%d_k%d.%d.%d_s%d_v%d", precision,
 	         total > 0 ? (int)std::floor(std::log(total) / std::log(4.0)) : 0, q(hn[0]), q(hn[1]), q(hn[2]), q(hn[3]),
-	         q(hn[4]), q(hk[0]), q(hk[1]), q(hk[2]));
+	         q(hn[4]), q(hk[0]), q(hk[1]), q(hk[2]), l.stiles.empty() ? 0 : 1, TUNE_VERSION);
 	return buf;
 }
 
