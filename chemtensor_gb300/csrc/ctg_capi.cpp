@@ -343,6 +343,29 @@ int ctgpu_block_sparse_tensor_svd_values(const struct block_sparse_tensor* a, do
 	});
 }
 
+int ctgpu_block_sparse_tensor_svd(const struct block_sparse_tensor* a, double discard_weight, struct block_sparse_tensor* u,
+                                  double* sigma, ct_long* ns, struct block_sparse_tensor* vh)
+{
+	return guarded([&] {
+		CTG_CHECK(a && u && sigma && ns && vh, "null argument");
+		CTG_CHECK(discard_weight >= 0, "discard_weight must be non-negative");
+		ctg::Ctx& c = ctg::context_for_device(g_opts.device);
+		ctg::DTensor da = ctg::tensor_from_struct(c, a);
+		ctg::SvdResult sv;
+		ctg::SvdPending pend;
+		int ret = ctg::op_svd_launch(c, da, sv, pend, discard_weight);
+		if (ret < 0) return ret;
+		c.sync();
+		ret = ctg::op_svd_finish(c, pend);
+		if (ret < 0) return ret;
+		CTG_CUDA(cudaMemcpy(sigma, sv.s->ptr, (size_t)sv.ns * sizeof(double), cudaMemcpyDeviceToHost));
+		*ns = sv.ns;
+		ctg::tensor_to_struct(c, sv.u, u);
+		ctg::tensor_to_struct(c, sv.vh, vh);
+		return 0;
+	});
+}
+
 int ctgpu_device_memory(int device, size_t* free_bytes, size_t* total_bytes)
 {
 	return guarded([&] {

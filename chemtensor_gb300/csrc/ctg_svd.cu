@@ -1879,9 +1879,6 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	// FP64 steps (or the refinement), FP64 sweeps, FP32 sweeps, exchanges, FP32 cycles, hand-over cycles;
 	// refinement cycles: Gram matrices, analysis (cosines, tail, clusters, generator), updates, clusters
 	long long cyc_acc[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-	// counted on the second CTA: the first one holds the last column group, often short or empty
-	const bool count = phase_ts && tid == 0 && rank == (cl > 1 ? 1 : 0);
-	long long* cyc = count ? cyc_acc : nullptr;
 	// FP32 sub-cluster: the requested size, or larger until its column groups fit
 	int cf = f32_cl < cl ? f32_cl : cl;
 	if (!full)
@@ -1889,6 +1886,10 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	while (cf < cl && f32_tour_bytes(N, r, cf) > (i64)smem_bytes) cf *= 2;
 	const bool mixed = f32_min > 0 && r >= f32_min && 8 * refine_doubles(N, cl) <= (i64)smem_bytes &&
 	                   f32_tour_bytes(N, r, cf) <= (i64)smem_bytes;
+	// counted on the second CTA (the first one holds the last column group, often short or empty), but FP32 sweeps
+	// on one CTA alone on that one
+	const bool count = phase_ts && tid == 0 && rank == (cl > 1 && !(mixed && cf == 1) ? 1 : 0);
+	long long* cyc = count ? cyc_acc : nullptr;
 	bool refined = false;
 	int rf_iters = 0;
 	if (mixed)

@@ -35,6 +35,7 @@ EXPORTS = [
     "ctgpu_contraction_operator_step_left",
     "ctgpu_contraction_operator_step_right",
     "ctgpu_block_sparse_tensor_svd_values",
+    "ctgpu_block_sparse_tensor_svd",
     "ctgpu_block_sparse_tensor_qr",
     "ctgpu_construct_spin_molecular_mpo",
     "ctgpu_mps_vdot",
@@ -106,6 +107,7 @@ def load(path: str = LIB_PATH) -> C.CDLL:
     lib.ctgpu_contraction_operator_step_left.argtypes = [P] * 4
     lib.ctgpu_contraction_operator_step_right.argtypes = [P] * 4
     lib.ctgpu_block_sparse_tensor_svd_values.argtypes = [P, P, P]
+    lib.ctgpu_block_sparse_tensor_svd.argtypes = [P, C.c_double, P, P, P, P]
     lib.ctgpu_block_sparse_tensor_qr.argtypes = [P, C.c_int, P, P]
     lib.ctgpu_construct_spin_molecular_mpo.argtypes = [C.c_int, P, P, P]
     lib.ctgpu_mps_vdot.argtypes = [P, P, P]

@@ -251,6 +251,13 @@ int ctgpu_contraction_operator_step_right(const struct block_sparse_tensor* a, c
  * *ns receives the count */
 int ctgpu_block_sparse_tensor_svd_values(const struct block_sparse_tensor* a, double* sigma, ct_long* ns);
 
+/* block_sparse_tensor_svd (src/tensor/block_sparse_tensor.c:2686-2848): a = u diag(sigma) vh; sigma must hold
+ * min(dim0, dim1) entries, *ns receives the count. discard_weight: the caller discards the smallest singular
+ * values whose squares sum to at most this (0: keeps all), as the split of a two-site tensor does; their
+ * columns of u and vh then need not be orthogonal to each other. */
+int ctgpu_block_sparse_tensor_svd(const struct block_sparse_tensor* a, double discard_weight, struct block_sparse_tensor* u,
+	double* sigma, ct_long* ns, struct block_sparse_tensor* vh);
+
 /* block_sparse_tensor_qr / block_sparse_tensor_rq (src/tensor/block_sparse_tensor.c:2402-2540 /
  * :2544-2676), mode QR_REDUCED (= 0) only; blocks factored with the conventions of LAPACK
  * dgeqrf + dorgqr and dgerqf + dorgrq (dense_tensor.c:2253-2651 / :2680-2880). Other modes
