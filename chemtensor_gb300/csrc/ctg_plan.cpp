@@ -135,14 +135,18 @@ int slice_orient(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum,
 }
 
 // SM clocks of the five launches that a product by digit slices has besides the GEMM (exponents, digits, the
-// results to look at again), and of those for an entry of an operand and of the result
-constexpr double SLICE_OVERHEAD = 75000, SLICE_ENTRY = 3.0, SLICE_RESULT = 4.0;
+// results to look at again, of which graded states have many), and of those for an entry of an operand and of
+// the result
+constexpr double SLICE_OVERHEAD = 150000, SLICE_ENTRY = 3.0, SLICE_RESULT = 4.0;
 
 // Digit slices or the FP64 pipe, by the SM clocks that each takes: the FP64 tiles at 2.1 FMAs a clock
 // (padding included), against the MMAs, the conversion of the operands' entries, the check of the results and
-// the launches. Both sides measured: a D = 1024 local-Hamiltonian product of 1.1e9 FMAs 2.0 ms against 0.3 ms, the
+// the launches. Both sides measured: a D = 1024 local-Hamiltonian product of 1.1e9 FMAs 2.0 ms against 0.4 ms, the
 // products of a Hubbard chain at D = 256 (3e6 .. 9e6 FMAs in 300 .. 1500 output blocks) 15 .. 60 us
-// against 50 .. 70 us.
+// against 60 .. 90 us. Searches (ms) on the FP64 pipe, with an overhead of 75000 clocks, with this one and with
+// 300000: molecular n = 8, D = 128 11.1, 11.3, 10.8, 11.0; n = 10, D = 128 36.4, 26.0, 24.2, 24.1; n = 14,
+// D = 256 544, 139, 138, 138; one-site Hubbard L = 20, D = 800 204, 222, 204, 204; spin chain L = 24,
+// D = 600 275, 279, 276, 272.
 bool use_slices(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum, const std::vector<GemmTile>* tiles, i64 entries,
                 i64 results, int num_sms)
 {
