@@ -21,6 +21,7 @@
 // D = 64 211 -> 37 us. (Before: one warp per column with a reduction each, matrix in global memory, three to
 // four barriers and FP64 divisions per column, Q over all columns.)
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 
 #include "ctg_fp64.cuh"
@@ -44,18 +45,19 @@ __device__ __forceinline__ double2 mul(double2 a, double2 b)
 {
 	return make_double2(fma(a.x, b.x, -(a.y * b.y)), fma(a.x, b.y, a.y * b.x));
 }
-// s += conj(x) b
+// s += conj(x) b. Complex products are rounded by themselves and then added: one rounding of the size of the
+// sum (or of b) instead of two
 __device__ __forceinline__ void add_dot(double& s, double x, double b) { s = fma(x, b, s); }
 __device__ __forceinline__ void add_dot(double2& s, double2 x, double2 b)
 {
-	s.x = fma(x.x, b.x, fma(x.y, b.y, s.x));
-	s.y = fma(x.x, b.y, fma(-x.y, b.x, s.y));
+	s.x += fma(x.x, b.x, x.y * b.y);
+	s.y += fma(x.x, b.y, -(x.y * b.x));
 }
 // b - t x
 __device__ __forceinline__ double sub_mul(double b, double t, double x) { return fma(-t, x, b); }
 __device__ __forceinline__ double2 sub_mul(double2 b, double2 t, double2 x)
 {
-	return make_double2(fma(-t.x, x.x, fma(t.y, x.y, b.x)), fma(-t.x, x.y, fma(-t.y, x.x, b.y)));
+	return make_double2(b.x - fma(t.x, x.x, -(t.y * x.y)), b.y - fma(t.x, x.y, t.y * x.x));
 }
 __device__ __forceinline__ double abs2(double x, double s) { return fma(x, x, s); }
 __device__ __forceinline__ double abs2(double2 x, double s) { return fma(x.x, x.x, fma(x.y, x.y, s)); }
@@ -97,6 +99,10 @@ __device__ __forceinline__ double warp_sum(double v)
 }
 
 // The reflector of (alpha, x), xn2 = |x|^2: H^H (alpha, x) = (beta, 0), H^H = I - f v v^H, v = (v0, x). f = 0: H = I.
+// H is as orthogonal as f is accurate for the v0 that is used, rounding and all: f = 2 / (v0^2 + xn2), and for complex
+// entries f = 2 Re v0 conj(v0) / (|v0|^2 (|v0|^2 + xn2)), whose five roundings would make it 1.5 times as far off as
+// LAPACK's scaled vectors and which is therefore formed in pairs of numbers (after an exact scaling that keeps
+// the products in range).
 // Squared norms below 1e-306 (of a block whose entries lie in a normal range) are zeros to all purposes: f,
 // their reciprocal, must stay a number. The functions of ctg_fp64.cuh want normal numbers and their
 // reciprocals: squared norms beyond 1e-290 and 1e290, infinities and NaN (which stay NaN in the factors, as
@@ -111,11 +117,10 @@ __device__ __forceinline__ void reflector(double alpha, double xn2, double& beta
 	v0 = f = 0.0;
 	if (xn2 == 0.0 || n2 <= 1e-306) return;
 	const bool plain = plain_range(n2);
-	const double nrm = plain ? sqrt64(n2) : ieee_sqrt(n2);
-	beta = -copysign(nrm, alpha);
+	beta = -copysign(plain ? sqrt64(n2) : ieee_sqrt(n2), alpha);
 	v0 = alpha - beta;
-	const double d = fma(nrm, fabs(alpha), n2);
-	f = plain ? rcp64(d) : ieee_rcp(d);
+	const double d = fma(v0, v0, xn2);
+	f = 2.0 * (plain ? rcp64(d) : ieee_rcp(d));
 }
 __device__ __forceinline__ void reflector(double2 alpha, double xn2, double& beta, double2& v0, double2& f)
 {
@@ -126,9 +131,29 @@ __device__ __forceinline__ void reflector(double2 alpha, double xn2, double& bet
 	const bool plain = plain_range(n2);
 	beta = -copysign(plain ? sqrt64(n2) : ieee_sqrt(n2), alpha.x);
 	v0 = make_double2(alpha.x - beta, alpha.y);
-	const double d = abs2(v0, 0.0);
-	const double rb = plain ? rcp64(beta) : ieee_rcp(beta), rv = plain ? rcp64(d) : ieee_rcp(d);
-	f = make_double2(-v0.x * rb * rv, v0.y * rb * rv);
+	if (!(n2 <= DBL_MAX))
+	{
+		f.x = f.y = 0.0 * n2;
+		return;
+	}
+	// |Re v0| is the largest of the entries' magnitudes, up to a factor: scaled to [1, 2)
+	const double sc = __hiloint2double((2046 - ((__double2hiint(v0.x) >> 20) & 0x7ff)) << 20, 0);
+	const double vx = v0.x * sc, vy = v0.y * sc;
+	// |v0|^2 = a + al, |v0|^2 + xn2 = b + bl
+	const double p = vx * vx, pe = fma(vx, vx, -p), q = vy * vy, qe = fma(vy, vy, -q);
+	const double a = p + q, al = (q - (a - p)) + (pe + qe);              // p >= q
+	const double x2 = xn2 * sc * sc, b = a + x2, bb = b - a;
+	const double bl = ((a - (b - bb)) + (x2 - bb)) + al;
+	// 1 / ((a + al) (b + bl)) = y + yl
+	const double y = rcp64(a * b), t = a * y, te = fma(a, y, -t);
+	double r = fma(-b, t, 1.0);
+	r = fma(-b, te, r);
+	r = fma(-bl, t, r);
+	r = fma(-b * al, y, r);
+	const double yl = y * r;
+	const double m = vx * vy, me = fma(vx, vy, -m), s2 = 2.0 * sc;
+	f.x = s2 * (fma(p, y, fma(p, yl, pe * y)) * sc);
+	f.y = -s2 * (fma(m, y, fma(m, yl, me * y)) * sc);
 }
 
 template <class T>
