@@ -129,14 +129,30 @@ __device__ __forceinline__ double2 gemm_entry(double2 x, unsigned flip)
 {
 	return make_double2(x.x, __hiloint2double(__double2hiint(x.y) ^ (int)flip, __double2loint(x.y)));
 }
+// A complex sum is kept as the sums of Re a times b and of Im a times b, so that a pair of entries takes four FMAs
+// and the sum no more rounding than with products that are rounded by themselves; where the accumulators of a tile
+// would not fit (SMALL = false), those take six instructions.
+struct GemmPair {
+	double2 p, q;
+};
+template <class T, bool SMALL> struct GemmAcc { using type = T; };
+template <> struct GemmAcc<double2, true> { using type = GemmPair; };
 __device__ __forceinline__ void gemm_mac(double& c, double a, double b) { c = fma(a, b, c); }
 __device__ __forceinline__ void gemm_mac(double2& c, double2 a, double2 b)
 {
-	c.x = fma(a.x, b.x, c.x);
-	c.y = fma(a.x, b.y, c.y);
-	c.x = fma(-a.y, b.y, c.x);
-	c.y = fma(a.y, b.x, c.y);
+	c.x += fma(a.x, b.x, -(a.y * b.y));
+	c.y += fma(a.x, b.y, a.y * b.x);
 }
+__device__ __forceinline__ void gemm_mac(GemmPair& c, double2 a, double2 b)
+{
+	c.p.x = fma(a.x, b.x, c.p.x);
+	c.p.y = fma(a.x, b.y, c.p.y);
+	c.q.x = fma(a.y, b.x, c.q.x);
+	c.q.y = fma(a.y, b.y, c.q.y);
+}
+__device__ __forceinline__ double gemm_value(double c) { return c; }
+__device__ __forceinline__ double2 gemm_value(double2 c) { return c; }
+__device__ __forceinline__ double2 gemm_value(const GemmPair& c) { return make_double2(c.p.x - c.q.y, c.p.y + c.q.x); }
 __device__ __forceinline__ void gemm_add(double& c, double x) { c += x; }
 __device__ __forceinline__ void gemm_add(double2& c, double2 x)
 {
@@ -157,11 +173,12 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 	const GemmOut o = outs[tile.out];
 	const int tid = threadIdx.x;
 	const int tx = tid % NTX, ty = tid / NTX;
-	T acc[TM][TN];
+	using Acc = typename GemmAcc<T, TM * TN <= 4>::type;
+	Acc acc[TM][TN];
 #pragma unroll
 	for (int i = 0; i < TM; i++)
 #pragma unroll
-		for (int j = 0; j < TN; j++) acc[i][j] = T();
+		for (int j = 0; j < TN; j++) acc[i][j] = Acc();
 
 	// rows and columns beyond the block and terms beyond the table stay unset: what they give is not stored
 	auto load = [&](int st) {
@@ -235,13 +252,13 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 	if (tile.split >= 0)
 	{
 		// partial sum of a split tile (full BM x BN, leading dimension BN); the CTA that completes
-		// the split last adds the partial sums in share order (deterministic) and writes C
+		// the split last adds the partial sums in a fixed order (deterministic) and writes C
 		const GemmSplit sp = splits[tile.split];
 		T* part = work + sp.part + (i64)tile.sp * sp.stride;
 #pragma unroll
 		for (int i = 0; i < TM; i++)
 #pragma unroll
-			for (int j = 0; j < TN; j++) part[(ty + i * NTY) * BN + tx + j * NTX] = acc[i][j];
+			for (int j = 0; j < TN; j++) part[(ty + i * NTY) * BN + tx + j * NTX] = gemm_value(acc[i][j]);
 		__threadfence();
 		__syncthreads();
 		__shared__ int last;
@@ -253,10 +270,24 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 		{
 			const int i = e / sp.cols, j = e - i * sp.cols;
 			const T* pw = work + sp.part + (i64)i * sp.ld + j;
-			T sum = T();
+			// four sums side by side: a fraction of the rounding of one chain
+			T sum[4] = {T(), T(), T(), T()};
+			if (sp.chain)
+			{
 #pragma unroll 4
-			for (int q = 0; q < sp.nsplit; q++) gemm_add(sum, __ldcg(pw + (i64)q * sp.stride));
-			C[gemm_out_index(o, sp.m0 + i, sp.n0 + j)] = sum;
+				for (int q = 0; q < sp.nsplit; q++) gemm_add(sum[0], __ldcg(pw + (i64)q * sp.stride));
+			}
+			else
+			{
+				for (int q = 0; q < sp.nsplit; q += 4)
+#pragma unroll
+					for (int u = 0; u < 4; u++)
+						if (q + u < sp.nsplit) gemm_add(sum[u], __ldcg(pw + (i64)(q + u) * sp.stride));
+				gemm_add(sum[0], sum[1]);
+				gemm_add(sum[2], sum[3]);
+				gemm_add(sum[0], sum[2]);
+			}
+			C[gemm_out_index(o, sp.m0 + i, sp.n0 + j)] = sum[0];
 		}
 		if (tid == 0) counters[tile.split] = 0;
 		return;
@@ -270,7 +301,7 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 		for (int j = 0; j < TN; j++)
 		{
 			const int gj = tile.n0 + tx + j * NTX;
-			if (gj < o.n) C[gemm_out_index(o, gi, gj)] = acc[i][j];
+			if (gj < o.n) C[gemm_out_index(o, gi, gj)] = gemm_value(acc[i][j]);
 		}
 	}
 }

@@ -41,7 +41,7 @@ struct GemmContrib {
 // k = k1 exclusive) of the tile's sum over its contributions and their inner index k, in order.
 // split < 0: the share is the whole sum and goes to C; otherwise the CTA is share sp of GemmSplit
 // entry `split`: it writes its partial sum to work[part + sp * stride + i * ld + j], and the CTA
-// that finishes its split last adds the partial sums in order of sp and writes C.
+// that finishes its split last adds the partial sums in a fixed order and writes C.
 struct GemmTile {
 	int out;           // output block
 	int m0, n0;        // tile origin inside the output block
@@ -56,6 +56,7 @@ struct GemmTile {
 struct GemmSplit {
 	int out, m0, n0, rows, cols, nsplit, ld, stride;
 	i64 part;
+	int chain, pad;    // the shares are added one after the other (see Ctx::steady), else in four sums
 };
 
 // tile classes (rows x cols of C per CTA of 256 threads): 256 outputs, one per thread (S 16 x 16,

@@ -721,6 +721,7 @@ DotLowering lower_dot(const Meta& s, int axs, const Meta& t, int axt, int nmult,
 				g.rows = std::min(tr, o.m - t.m0);
 				g.cols = std::min(tc, o.n - t.n0);
 				g.nsplit = S;
+				g.chain = steady ? 1 : 0;
 				g.ld = tc;
 				g.stride = tr * tc;
 				g.part = wsz;
