@@ -50,7 +50,8 @@ __device__ __forceinline__ double sqrt64(double x)
 
 
 // sqrt(x) and 1 / sqrt(x) together for a positive normal double (the reciprocal comes with the
-// square root: one Newton sequence for both, accurate to about one unit in the last place)
+// square root: one Newton sequence for both; the square root is accurate to half a unit in the last place, its
+// reciprocal to three, 0.4 in the mean)
 __device__ __forceinline__ void sqrt_rsqrt64(double x, double& sq, double& rsq)
 {
 	const int hi = __double2hiint(x), lo = __double2loint(x);

@@ -159,7 +159,12 @@ struct ClusterReduce {
 		if (threadIdx.x < 32)
 		{
 			double b, r;
-			if (v > 1e-290 && v < 1e290) sqrt_rsqrt64(v, b, r);
+			if (v > 1e-290 && v < 1e290)
+			{
+				sqrt_rsqrt64(v, b, r);
+				// the reciprocal of the norm as it was rounded, to half a unit in the last place
+				r = fma(r, fma(-b, r, 1.0), r);
+			}
 			else
 			{
 				b = sqrt(v);
