@@ -281,7 +281,8 @@ SvdLaunch svd_launch_for(int m, int n, int want, int max_cluster);
 // cluster exchanges to phase_ts[8 block + 4 ..].
 // discard2: the caller discards every singular value whose square is below it (0: none); the
 // refinement of the mixed path then leaves the mutual rotations of those columns out.
-// steady (see Ctx::steady): five FP32 sweeps from rank 32 on and 256 threads, whatever the angles and the size.
+// steady (see Ctx::steady): five FP32 sweeps from rank 32 on and 256 threads, whatever the angles and the size,
+// and the refinement's rounding as it was.
 void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* descs, const double* a, double* u,
                       double* s, double* vh, double* scratch, int* status, double* flops, cudaStream_t st,
                       unsigned long long* phase_ts = nullptr, double discard2 = 0.0, bool steady = false);

@@ -1060,8 +1060,10 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 //   2. T = R^T V (FP64);
 //   3. G = T^T T (FP64 inner products, each pair once). For columns i, j whose squared norms lie
 //      apart, the first-order generator X_ij = G_ij / (G_jj - G_ii) (antisymmetric) removes the
-//      cosine of the pair to second order; T and V are multiplied by I + X + X^2 / 2, which is
-//      orthogonal to O(X^4). Columns whose squared norms lie within a relative gap gamma of their
+//      cosine of the pair to second order; T and V are multiplied by I + X + X^2 / 2 + X^3 / 8, which is
+//      orthogonal to X^6 / 64 (without the last term to X^4 / 4: at 190 x 150 and a flat spectrum that, and X^2
+//      rounded to FP32, left 3e-14 in the residual and the singular values where FP64 sweeps leave 2e-15;
+//      X^2 is summed in double-float; both only where X is large enough to matter). Columns whose squared norms lie within a relative gap gamma of their
 //      neighbours (a cluster, where the first-order angle would not be small) get X = 0 and are
 //      rotated afterwards among themselves by exact one-sided Jacobi rotations (one warp per
 //      cluster). gamma = c_max / (2 delta) keeps every first-order angle below delta = 3e-4 for
@@ -1074,6 +1076,7 @@ __device__ void precondition_f32(cg::cluster_group& cluster, const Tour& t, doub
 
 constexpr int RF_MAX_IT = 6;              // refinement iterations before the FP64 sweeps take over
 constexpr float RF_DELTA = 3e-4f;         // largest first-order angle outside a cluster
+constexpr float RF_LARGE_X2 = 1e-9f;      // r x^2 of a generator whose square FP32 rounds by more than 6e-17
 constexpr int RF_CLUSTER_MAX = 16;        // most columns of one cluster
 constexpr int RF_CLUSTER_SWEEPS = 8;      // most Jacobi sweeps inside one cluster
 constexpr int RF_EDGES_PER_COL = 4;       // capacity of the cluster-edge list, per column
@@ -1138,7 +1141,7 @@ struct Refine {
 	double* Vr;       // V row-major (the scratch V area)
 	float2* Th;       // T column-major as (hi, lo) pairs, entry (k, i) at Th + i N + k
 	float2* Vh;       // V column-major as (hi, lo) pairs, entry (k, i) at Vh + i r + k
-	int* gfail;       // per iteration: a first-order angle came out too large
+	int* gx;          // per iteration: largest first-order angle (bits of a non-negative float)
 	int* gc2;         // per iteration: largest cos^2 (bits of a non-negative float)
 	int* gne;         // per iteration: cluster edges found
 	int2* gedges;     // the cluster edges of the current iteration
@@ -1417,7 +1420,8 @@ __device__ double rf_cluster_jacobi(const Tour& t, const Refine& rf, int cl, int
 // CTA's round-0 records [T | V]; the return value says whether the refinement converged (the same
 // on every CTA of the cluster); if not, the FP64 sweeps continue from those records.
 __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* smem, const SvdScratch& xs, int M,
-                             int cl, int rank, bool refine, float tail2, double& flops, long long* cyc, int& iters)
+                             int cl, int rank, bool refine, bool steady, float tail2, double& flops, long long* cyc,
+                             int& iters)
 {
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	const int N = t.N, r = t.r;
@@ -1430,10 +1434,10 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 	rf.X = (float*)(xs.G + (i64)N * N);
 	rf.Th = (float2*)(xs.G + (i64)N * N + ((i64)N * N + 1) / 2);
 	rf.Vh = rf.Th + (i64)N * N;
-	rf.gfail = (int*)(rf.Vh + (i64)N * N);
-	rf.gc2 = rf.gfail + 8;
-	rf.gne = rf.gfail + 16;
-	rf.gedges = (int2*)(rf.gfail + 24);
+	rf.gx = (int*)(rf.Vh + (i64)N * N);
+	rf.gc2 = rf.gx + 8;
+	rf.gne = rf.gx + 16;
+	rf.gedges = (int2*)(rf.gx + 24);
 	rf.Tr = xs.T;
 	rf.Vr = xs.V;
 	{
@@ -1474,7 +1478,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 		const int jj = e / N, k = e % N;
 		rf_rec(t, rf, jj)[N + k] = k < r ? __ldcg(xs.V + (i64)rf_col(t, rf, jj) * r + k) : 0.0;
 	}
-	if (rank == 0 && tid < 24) rf.gfail[tid] = 0;        // failure flags, cosines, edge counts
+	if (rank == 0 && tid < 24) rf.gx[tid] = 0;           // angles, cosines, edge counts
 	cluster.sync();                              // xs.V is read before its row-major overwrite
 	for (int step = 0; step < 2; step++)
 	{
@@ -1695,6 +1699,7 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 			break;
 		}
 		// first-order generator, own columns (zero inside a cluster and between tail columns)
+		float xmax = 0.0f;
 		for (int e = tid; e < rf.nown * r; e += svd_threads())
 		{
 			const int jj = e / r, i = e % r, g = rf_col(t, rf, jj);
@@ -1703,23 +1708,88 @@ __device__ bool finish_mixed(cg::cluster_group& cluster, const Tour& t, double* 
 			{
 				const double den = rf.D[g] - rf.D[i];
 				x = den != 0.0 ? ratio_f32(__ldcg(rf.G + (i64)g * r + i), den) : 2.0f;
-				// should have been an edge (float rounding of the edge test): the FP64 sweeps take over
-				if (fabsf(x) > 4.0f * RF_DELTA) atomicOr(rf.gfail + it, 1);
+				xmax = fmaxf(xmax, fabsf(x));
 			}
 			rf.Xo[jj * r + i] = x;
 			rf.X[(i64)g * r + i] = x;
 		}
+		for (int o = 16; o > 0; o >>= 1) xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o));
+		if (lane == 0 && xmax > 0.0f) atomicMax(rf.gx + it, __float_as_int(xmax));
 		cluster.sync();
 		lap(7);
-		if (__ldcg(rf.gfail + it))
+		xmax = __int_as_float(__ldcg(rf.gx + it));
+		// should have been an edge (float rounding of the edge test): the FP64 sweeps take over
+		if (xmax > 4.0f * RF_DELTA)
 		{
 			fail = 4;
 			break;
 		}
 		// F + Fl = X + X^2 / 2 exactly (two-sum) for the own columns ((X^2)_ij = sum_k X_ik X_kj,
-		// X_ik at X + k r + i): the antisymmetric X stays exact in F + Fl
+		// X_ik at X + k r + i): the antisymmetric X stays exact in F + Fl. An entry of X^2 rounds by up to
+		// r xmax^2 eps_32
+		const bool large = !steady && (float)r * xmax * xmax > RF_LARGE_X2;
+		if (large)
+		{
+			// X^2 in double-float, then X^3 from it (its leading floats lie where the clusters are rotated later)
+			constexpr int XB = 4;
+			float* Y = (float*)rf.cstage;
+			const int nb = (rf.nown + XB - 1) / XB;
+			for (int e = tid; e < nb * r; e += svd_threads())
+			{
+				const int b = e / r, i = e % r, j0 = b * XB, nj = min(XB, rf.nown - j0);
+				float sh[XB], sl[XB];
+#pragma unroll
+				for (int q = 0; q < XB; q++) sh[q] = sl[q] = 0.0f;
+#pragma unroll 4
+				for (int k = 0; k < r; k++)
+				{
+					const float xv = __ldcg(rf.X + (i64)k * r + i);
+#pragma unroll
+					for (int q = 0; q < XB; q++)
+					{
+						if (q >= nj) break;
+						const float y = rf.Xo[(j0 + q) * r + k], p = xv * y, s = sh[q] + p, bp = s - sh[q];
+						sl[q] += ((sh[q] - (s - bp)) + (p - bp)) + fmaf(xv, y, -p);
+						sh[q] = s;
+					}
+				}
+				for (int q = 0; q < nj; q++)
+				{
+					const int at = (j0 + q) * r + i;
+					rf.F[at] = Y[at] = sh[q];
+					rf.Fl[at] = sl[q];
+				}
+			}
+			__syncthreads();
+			for (int e = tid; e < nb * r; e += svd_threads())
+			{
+				const int b = e / r, i = e % r, j0 = b * XB, nj = min(XB, rf.nown - j0);
+				float acc[XB];
+#pragma unroll
+				for (int q = 0; q < XB; q++) acc[q] = 0.0f;
+#pragma unroll 8
+				for (int k = 0; k < r; k++)
+				{
+					const float xv = __ldcg(rf.X + (i64)k * r + i);
+#pragma unroll
+					for (int q = 0; q < XB; q++)
+						if (q < nj) acc[q] = fmaf(xv, Y[(j0 + q) * r + k], acc[q]);
+				}
+				for (int q = 0; q < nj; q++)
+				{
+					const int at = (j0 + q) * r + i;
+					const float x = rf.Xo[at], h = 0.5f * rf.F[at];
+					const float sum = x + h, bp = sum - x;
+					const float lo = ((x - (sum - bp)) + (h - bp)) + fmaf(0.125f, acc[q], 0.5f * rf.Fl[at]);
+					const float f = sum + lo;
+					rf.F[at] = f;
+					rf.Fl[at] = (sum - f) + lo;
+				}
+			}
+		}
 		// one thread per row i and up to XB own columns at a time: each entry X_ik is loaded once
 		// for all of them (eight loads in flight)
+		else
 		{
 			constexpr int XB = 8;
 			const int nb = (rf.nown + XB - 1) / XB;
@@ -1796,7 +1866,7 @@ __global__ void __launch_bounds__(SVD_THREADS_MAX, 1)
 k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restrict__ a, double* __restrict__ u,
            double* __restrict__ s, double* __restrict__ vh, double* __restrict__ scratch, int* __restrict__ status,
            double* __restrict__ flops, int cl, int smem_bytes, unsigned long long* __restrict__ phase_ts, int f32_min,
-           int f32_cl, int refine, double tail2, int f32_sweeps, float f32_cos, float f32_wide, int full)
+           int f32_cl, int refine, double tail2, int f32_sweeps, float f32_cos, float f32_wide, int full, int steady)
 {
 	extern __shared__ __align__(16) double smem[];
 	cg::cluster_group cluster = cg::this_cluster();
@@ -1896,7 +1966,7 @@ k_svd_tour(const SvdDesc* __restrict__ descs, int first, const double* __restric
 	{
 		const double us = __ldcg(xs.misc + 2);
 		precondition_f32(cluster, t, smem, xs, M, cf, rank, f32_sweeps, f32_cos, f32_wide, (float)(tail2 / (us * us)), cyc);
-		refined = finish_mixed(cluster, t, smem, xs, M, cl, rank, refine != 0, (float)(tail2 / (us * us)), jflops, cyc,
+		refined = finish_mixed(cluster, t, smem, xs, M, cl, rank, refine != 0, steady != 0, (float)(tail2 / (us * us)), jflops, cyc,
 		                       rf_iters);
 	}
 	else
@@ -2653,7 +2723,7 @@ void launch_svd_group(const SvdLaunch& g, int first, int count, const SvdDesc* d
 		});
 	CTG_CUDA(cudaLaunchKernelEx(&cfg, k_svd_tour, descs, first, a, u, s, vh, scratch, status, flops, g.cluster, g.smem,
 	                             phase_ts, f32_min, svd_f32_cluster(), svd_refine(), discard2, svd_f32_sweeps(),
-	                             svd_f32_cos(), steady ? FLT_MAX : svd_f32_wide(), full ? 1 : 0));
+	                             svd_f32_cos(), steady ? FLT_MAX : svd_f32_wide(), full ? 1 : 0, steady ? 1 : 0));
 }
 
 }  // namespace ctg
