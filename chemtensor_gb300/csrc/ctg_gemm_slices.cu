@@ -141,7 +141,7 @@ __device__ __forceinline__ int64_t add_order(int64_t acc, int x, int w)
 // The items of an operand (32 rows of a group, a lane each, by SLICE_ITEM stages of its terms), 8 terms at a time.
 struct SliceReader {
 	const SliceRun* __restrict__ runs;   // the group's
-	const double* __restrict__ x;
+	const double* x;
 	const double* p;
 	int row, nrun;
 	bool valid;
@@ -194,8 +194,7 @@ constexpr int PACK_WARPS = 4;
 // digits need the whole row's code. It reads what the product before has just written, mostly from L2.
 __global__ void __launch_bounds__(PACK_WARPS * 32)
 k_slice_exps(int nitems, const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups,
-             const SliceRun* __restrict__ runs, const double* __restrict__ x, int* __restrict__ codes, int* __restrict__ clear,
-             int nclear)
+             const SliceRun* __restrict__ runs, const double* x, int* codes, int* clear, int nclear)
 {
 	pdl_wait();
 	pdl_trigger();
@@ -238,8 +237,7 @@ __device__ __forceinline__ uint32_t digits_f16x2(uint32_t w, bool upper, uint32_
 // next 8 terms are on their way while these are cut.
 __global__ void __launch_bounds__(PACK_WARPS * 32, 8)
 k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups,
-             const SliceRun* __restrict__ runs, int rows8, const double* __restrict__ x, const int* __restrict__ codes,
-             unsigned char* __restrict__ dst, short* __restrict__ exps)
+             const SliceRun* __restrict__ runs, int rows8, const double* x, const int* codes, unsigned char* dst, short* exps)
 {
 	pdl_wait();
 	pdl_trigger();
@@ -309,7 +307,7 @@ k_slice_pack(int nitems, const SliceItem* __restrict__ items, const SliceGroup* 
 // the nonzero terms of every row (a warp) of an item's 32
 __global__ void __launch_bounds__(1024)
 k_slice_lists(const SliceItem* __restrict__ items, const SliceGroup* __restrict__ groups, const SliceRun* __restrict__ runs,
-              const double* __restrict__ x, SliceTerm* __restrict__ terms, int* __restrict__ counts)
+              const double* x, SliceTerm* terms, int* counts)
 {
 	pdl_wait();
 	pdl_trigger();
@@ -877,8 +875,7 @@ struct MaskTile {
 // list: its length (zero before the launch), then (mask word, its bits)
 __global__ void __launch_bounds__(CHECK_WARPS * 32)
 k_slice_find(int ntiles, int nsplits, const SliceTile* __restrict__ tiles, const GemmOut* __restrict__ outs,
-             const SliceOut* __restrict__ souts, const GemmSplit* __restrict__ splits, int orient, const unsigned* __restrict__ masks,
-             uint2* __restrict__ list)
+             const SliceOut* __restrict__ souts, const GemmSplit* __restrict__ splits, int orient, const unsigned* masks, uint2* list)
 {
 	pdl_wait();
 	pdl_trigger();
@@ -984,9 +981,8 @@ __device__ __forceinline__ void entry_terms(const GemmOut& o, const GemmContrib*
 __global__ void __launch_bounds__(CHECK_WARPS * 32)
 k_slice_check(int ntiles, const SliceTile* __restrict__ tiles, const GemmOut* __restrict__ outs, const SliceOut* __restrict__ souts,
               const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits, int orient, int swap,
-              const SliceGroup* __restrict__ groups, const SliceTerm* __restrict__ terms, const int* __restrict__ counts,
-              const double* __restrict__ A, const double* __restrict__ B, const short* __restrict__ xexps,
-              const short* __restrict__ yexps, double* __restrict__ C, uint2* list)
+              const SliceGroup* __restrict__ groups, const SliceTerm* terms, const int* counts, const double* A, const double* B,
+              const short* xexps, const short* yexps, double* C, uint2* list)
 {
 	pdl_wait();
 	pdl_trigger();

@@ -431,8 +431,7 @@ __device__ __forceinline__ void copy_desc(D* to, const D* __restrict__ from)
 // T = double, or double2 for complex128 entries (same descriptors, element units)
 template <class T>
 __global__ void __launch_bounds__(256)
-k_permute(const Chunk* __restrict__ chunks, const PermDesc* __restrict__ descs, const T* __restrict__ src,
-          T* __restrict__ dst)
+k_permute(const Chunk* __restrict__ chunks, const PermDesc* __restrict__ descs, const T* src, T* dst)
 {
 	__shared__ PermDesc d;
 	const Chunk ch = chunks[blockIdx.x];
@@ -508,8 +507,7 @@ void launch_permute(int nchunks, const Chunk* chunks, const PermDesc* descs, con
 
 template <class T>
 __global__ void __launch_bounds__(256)
-k_rowmap(const Chunk* __restrict__ chunks, const RowDesc* __restrict__ descs, const i64* __restrict__ maps,
-         const T* __restrict__ src, T* __restrict__ dst)
+k_rowmap(const Chunk* __restrict__ chunks, const RowDesc* __restrict__ descs, const i64* __restrict__ maps, const T* src, T* dst)
 {
 	__shared__ RowDesc d;
 	const Chunk ch = chunks[blockIdx.x];

@@ -18,7 +18,9 @@ namespace ctg {
 
 // in every kernel launched by launch_pdl, before the first access to memory that an earlier kernel may have
 // written or may still read. Lists that belong to a plan may be read before it: they were uploaded by a copy
-// in the same stream, for which a kernel launch waits in full, and no kernel writes them.
+// in the same stream, for which a kernel launch waits in full, and no kernel writes them. What kernels do write is
+// not read through const __restrict__ pointers after such early reads: the compiler may take those loads for
+// loads of constants and move them up.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
