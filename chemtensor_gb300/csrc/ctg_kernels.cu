@@ -270,24 +270,18 @@ __device__ __forceinline__ void gemm_tile(const GemmTile& tile, const GemmOut* _
 		{
 			const int i = e / sp.cols, j = e - i * sp.cols;
 			const T* pw = work + sp.part + (i64)i * sp.ld + j;
-			// four sums side by side: a fraction of the rounding of one chain
-			T sum[4] = {T(), T(), T(), T()};
-			if (sp.chain)
+			// in four runs (a fraction of the rounding of one chain) or in one
+			const int run = sp.chain ? sp.nsplit : (sp.nsplit + 3) / 4;
+			T sum = T();
+#pragma unroll 1
+			for (int q0 = 0; q0 < sp.nsplit; q0 += run)
 			{
+				T part_sum = T();
 #pragma unroll 4
-				for (int q = 0; q < sp.nsplit; q++) gemm_add(sum[0], __ldcg(pw + (i64)q * sp.stride));
+				for (int q = q0; q < min(q0 + run, sp.nsplit); q++) gemm_add(part_sum, __ldcg(pw + (i64)q * sp.stride));
+				gemm_add(sum, part_sum);
 			}
-			else
-			{
-				for (int q = 0; q < sp.nsplit; q += 4)
-#pragma unroll
-					for (int u = 0; u < 4; u++)
-						if (q + u < sp.nsplit) gemm_add(sum[u], __ldcg(pw + (i64)(q + u) * sp.stride));
-				gemm_add(sum[0], sum[1]);
-				gemm_add(sum[2], sum[3]);
-				gemm_add(sum[0], sum[2]);
-			}
-			C[gemm_out_index(o, sp.m0 + i, sp.n0 + j)] = sum[0];
+			C[gemm_out_index(o, sp.m0 + i, sp.n0 + j)] = sum;
 		}
 		if (tid == 0) counters[tile.split] = 0;
 		return;

@@ -56,7 +56,7 @@ struct GemmTile {
 struct GemmSplit {
 	int out, m0, n0, rows, cols, nsplit, ld, stride;
 	i64 part;
-	int chain, pad;    // the shares are added one after the other (see Ctx::steady), else in four sums
+	int chain, pad;    // the shares are added one after the other (see Ctx::steady), else in four runs
 };
 
 // tile classes (rows x cols of C per CTA of 256 threads): 256 outputs, one per thread (S 16 x 16,
