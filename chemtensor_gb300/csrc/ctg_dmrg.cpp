@@ -279,7 +279,7 @@ DTensor contraction_step_left(Ctx& c, const DTensor& a, const DTensor& w, const 
 	DTensor s = op_dot(c, l, AX_TRAILING, br, AX_LEADING, 1, precision);
 	const int p0[5] = {0, 1, 4, 2, 3};
 	DTensor t = op_transpose(c, s, p0);
-	s = op_dot(c, t, AX_TRAILING, w, AX_LEADING, 2, precision);
+	s = op_dot(c, t, AX_TRAILING, w, AX_LEADING, 2, precision, 1);
 	const int p1[5] = {1, 3, 4, 2, 0};
 	t = op_transpose(c, s, p1);
 	s = op_dot(c, a, AX_LEADING, t, AX_LEADING, 2, precision);
@@ -294,7 +294,7 @@ DTensor contraction_step_right_ab(Ctx& c, const DTensor& a, const DTensor& b, co
 	DTensor s = op_dot(c, a, AX_TRAILING, r, AX_LEADING, 1, precision);
 	const int p0[5] = {1, 2, 0, 3, 4};
 	DTensor t = op_transpose(c, s, p0);
-	s = op_dot(c, w, AX_TRAILING, t, AX_LEADING, 2, precision);
+	s = op_dot(c, w, AX_TRAILING, t, AX_LEADING, 2, precision, 0);
 	const int p1[5] = {4, 2, 0, 1, 3};
 	t = op_transpose(c, s, p1);
 	// the bra: b with reversed axis directions, complex conjugated (chain_ops.c:138-149)
@@ -473,7 +473,7 @@ struct LocalH {
 		k = op_transpose(c, l, p2);
 		auto plan = [&](bool slices) {
 			d1 = make_dot_plan(c, a, AX_TRAILING, r.m(), AX_LEADING, 1, precision, p0, slices);
-			d2 = make_dot_plan(c, w.m(), AX_TRAILING, *d1.out, AX_LEADING, 2, precision, p1, slices);
+			d2 = make_dot_plan(c, w.m(), AX_TRAILING, *d1.out, AX_LEADING, 2, precision, p1, slices, 0);
 			d3 = make_dot_plan(c, k.m(), AX_TRAILING, *d2.out, AX_LEADING, 2, precision, nullptr, slices);
 		};
 		plan(true);

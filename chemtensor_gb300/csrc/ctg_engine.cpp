@@ -480,12 +480,12 @@ const T* at(const DBufPtr& b, size_t off)
 // dot (block_sparse_tensor.c:1826-2001; dense_tensor.c:1761-1837)
 // ------------------------------------------------------------------------------------
 
-static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn);
+static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn, int sparse = -1);
 static int tuned_tile_width(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision,
                             const int* out_perm, const DotLowering& l64);
 
 static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision,
-                              const int* out_perm, bool slices)
+                              const int* out_perm, bool slices, int sparse)
 {
 	// complex128: the FP64 lists and tiles, over complex entries
 	const bool z = precision == GEMM_Z64;
@@ -497,14 +497,14 @@ static DotPlan build_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int
 		// stays on FP64 is lowered once, one on the tensor cores twice
 		DotLowering l = lower_dot(s, axs, t, axt, nmult, GEMM_FP64, c.num_sms(), out_perm, 64, slices, c.steady);
 		const int bn = tuned_tile_width(c, s, axs, t, axt, nmult, precision, out_perm, l);
-		if (bn == 0) return upload_dot_plan(c, std::move(l), GEMM_FP64, 64);
+		if (bn == 0) return upload_dot_plan(c, std::move(l), GEMM_FP64, 64, sparse);
 		return upload_dot_plan(c, lower_dot(s, axs, t, axt, nmult, precision, c.num_sms(), out_perm, bn), precision, bn);
 	}
 	DotLowering l = lower_dot(s, axs, t, axt, nmult, z ? (int)GEMM_FP64 : precision, c.num_sms(), out_perm, 64, slices && !z, c.steady);
-	return upload_dot_plan(c, std::move(l), precision, 64);
+	return upload_dot_plan(c, std::move(l), precision, 64, sparse);
 }
 
-static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
+static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn, int sparse)
 {
 	DotPlan p;
 	p.out = l.out;
@@ -544,11 +544,13 @@ static DotPlan upload_dot_plan(Ctx& c, DotLowering&& l, int precision, int bn)
 		d.terms = l.spack[q].terms;
 		d.bytes = l.spack[q].bytes;
 	}
-	// lists for the smaller operand (an MPO tensor, whose rows are mostly zeros) where they take less memory than
-	// the other operand has
-	const int small = l.b_entries < l.a_entries ? 1 : 0;
-	p.side[1 - small].terms = 0;
-	if (2 * p.side[small].terms > std::max(l.a_entries, l.b_entries)) p.side[small].terms = 0;
+	// lists for an MPO tensor, whose rows are mostly zeros (they take as much memory as its digits), also where it is
+	// the larger operand: where a wide MPO meets a bond that has become small. A molecular search (n = 24, D = 512, bond
+	// dimension 298 once converged): 342 ms for a converged sweep, 3370 with its terms read one by one, 1841 on
+	// the FP64 pipe. Else for the smaller operand where the lists take less memory than the other one has
+	p.listed = sparse >= 0 ? sparse : l.b_entries < l.a_entries ? 1 : 0;
+	p.side[1 - p.listed].terms = 0;
+	if (sparse < 0 && 2 * p.side[p.listed].terms > std::max(l.a_entries, l.b_entries)) p.side[p.listed].terms = 0;
 	for (const SliceOut& o : l.souts) p.max_k = std::max(p.max_k, o.k);
 	p.tcons = at<TcContrib>(p.desc, o_tcons);
 	p.apacks = at<TcPack>(p.desc, o_apacks);
@@ -671,9 +673,8 @@ void DotPlan::run_slices(Ctx& c, const double* A, const double* B, const void* a
 	launch_gemm_slices(nstiles, stiles, outs, souts, cons, nsplits, splits, counters ? (int*)counters->ptr : nullptr, orient, A, B,
 	                   (const char*)pack[x] + slice_head(side[x]), (const char*)pack[1 - x] + slice_head(side[1 - x]), xe, ye, C,
 	                   max_k, check, c.split_work(work_bytes), c.tc_error(), c.num_sms(), c.stream());
-	const int small = b_entries < a_entries ? 1 : 0;
-	launch_slice_check(nstiles, nsplits, stiles, outs, souts, cons, splits, orient, small == 1, side[small].groups,
-	                   slice_lists(side[small], pack[small]), slice_counts(side[small], pack[small]), A, B, xe, ye, C, max_k, check,
+	launch_slice_check(nstiles, nsplits, stiles, outs, souts, cons, splits, orient, listed == 1, side[listed].groups,
+	                   slice_lists(side[listed], pack[listed]), slice_counts(side[listed], pack[listed]), A, B, xe, ye, C, max_k, check,
 	                   c.num_sms(), c.stream());
 }
 
@@ -993,13 +994,13 @@ static void dump_plan_request(int kind, const std::vector<i64>& params, const Me
 	fflush(f);
 }
 
-constexpr i64 PLAN_STEADY = 1 << 16, PLAN_TILES = 1 << 17;      // beside the precision in a plan's key
+constexpr i64 PLAN_STEADY = 1 << 16, PLAN_TILES = 1 << 17, PLAN_SPARSE = 1 << 18;      // beside the precision in a plan's key
 
 DotPlan make_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision,
-                      const int* out_perm, bool slices)
+                      const int* out_perm, bool slices, int sparse)
 {
 	PlanTimer plan_timer(c);
-	std::vector<i64> params = {axs, axt, nmult, precision + (c.steady ? PLAN_STEADY : 0) + (slices ? 0 : PLAN_TILES)};
+	std::vector<i64> params = {axs, axt, nmult, precision + (c.steady ? PLAN_STEADY : 0) + (slices ? 0 : PLAN_TILES) + (sparse + 1) * PLAN_SPARSE};
 	if (out_perm)
 		for (int i = 0; i < s.ndim + t.ndim - 2 * nmult; i++) params.push_back(out_perm[i]);
 	const uint64_t key = plan_key(0, params, s, &t);
@@ -1010,7 +1011,7 @@ DotPlan make_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, in
 	e.params = params;
 	e.s = StructSig(s);
 	e.t = StructSig(t);
-	e.dot = build_dot_plan(c, s, axs, t, axt, nmult, precision, out_perm, slices);
+	e.dot = build_dot_plan(c, s, axs, t, axt, nmult, precision, out_perm, slices, sparse);
 	const size_t bytes = e.dot.desc ? e.dot.desc->bytes : 0;
 	DotPlan p = e.dot;
 	plan_insert(c, key, std::move(e), bytes);
@@ -1068,7 +1069,7 @@ CopyPlan make_slice_plan(Ctx& c, const Meta& t, int ax, const std::vector<i64>& 
 // one-shot operations
 // ------------------------------------------------------------------------------------
 
-DTensor op_dot(Ctx& c, const DTensor& s, int axs, const DTensor& t, int axt, int nmult, int precision)
+DTensor op_dot(Ctx& c, const DTensor& s, int axs, const DTensor& t, int axt, int nmult, int precision, int sparse)
 {
 	if (s.cplx || t.cplx)
 	{
@@ -1078,7 +1079,7 @@ DTensor op_dot(Ctx& c, const DTensor& s, int axs, const DTensor& t, int axt, int
 		p.run_z(c, s.data(), t.data(), r.data(), s.conj, t.conj);
 		return r;
 	}
-	DotPlan p = make_dot_plan(c, s.m(), axs, t.m(), axt, nmult, precision);
+	DotPlan p = make_dot_plan(c, s.m(), axs, t.m(), axt, nmult, precision, nullptr, true, sparse);
 	DTensor r;
 	r.meta = p.out;
 	r.buf = std::make_shared<DBuf>(&c, (size_t)std::max<i64>(p.out->nnz, 1) * sizeof(double));

@@ -192,6 +192,7 @@ struct DotPlan {
 	DBufPtr counters;                    // their completion counters (one int per split tile)
 	// FP64 on the tensor cores by digit slices (then ntiles is 0); side 0 is operand A, 1 is B
 	int nstiles = 0, orient = 0, max_k = 0;
+	int listed = 0;                      // the operand that the check of the results reads first (0: A, 1: B)
 	const SliceTile* stiles = nullptr;
 	const SliceOut* souts = nullptr;
 	struct Side {
@@ -244,8 +245,9 @@ struct DotPlan {
 };
 // out_perm (every precision): the result is written straight in the layout of its transpose by out_perm
 // (see lower_dot), and the plan's `out` is that transposed structure. slices: an FP64 product may run by digit slices.
+// sparse: the operand whose rows are mostly zeros (0: s, 1: t), such as an MPO tensor; -1: not known.
 DotPlan make_dot_plan(Ctx& c, const Meta& s, int axs, const Meta& t, int axt, int nmult, int precision = GEMM_FP64,
-                      const int* out_perm = nullptr, bool slices = true);
+                      const int* out_perm = nullptr, bool slices = true, int sparse = -1);
 
 // Tile autotuner of the reduced-precision GEMMs: the column width (64, 128 or 256) of a product's
 // tensor-core tiles, or FP64 (0) where the product is too small for the tensor cores to pay for the
@@ -284,7 +286,8 @@ CopyPlan make_slice_plan(Ctx& c, const Meta& t, int ax, const std::vector<i64>& 
 
 // ---- one-shot operations (plan + run) ------------------------------------------------
 
-DTensor op_dot(Ctx& c, const DTensor& s, int axs, const DTensor& t, int axt, int nmult, int precision = GEMM_FP64);
+DTensor op_dot(Ctx& c, const DTensor& s, int axs, const DTensor& t, int axt, int nmult, int precision = GEMM_FP64,
+               int sparse = -1);
 DTensor op_transpose(Ctx& c, const DTensor& t, const int* perm);
 DTensor op_flatten(Ctx& c, const DTensor& t, int ax, int newdir);
 DTensor op_split(Ctx& c, const DTensor& t, int ax, const i64 nd[2], const int ndir[2], const std::vector<q32>* nq);
