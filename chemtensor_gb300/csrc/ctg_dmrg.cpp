@@ -594,7 +594,7 @@ struct LocalH {
 		}
 		else if (s1)
 		{
-			KScope ks(c, K_GEMM, 5, d1.flops, 0);
+			KScope ks(c, K_GEMM, 6, d1.flops, 0);
 			d1.slice_pack(c, 0, x, sp_x->ptr, turn);
 			d1.run_slices(c, x, r.data(), sp_x->ptr, sp_r->ptr, t1, check->ptr);
 			c.gemm_flops += d1.flops;
@@ -608,7 +608,7 @@ struct LocalH {
 		}
 		else if (s2)
 		{
-			KScope ks(c, K_GEMM, 5, d2.flops, 0);
+			KScope ks(c, K_GEMM, 6, d2.flops, 0);
 			d2.slice_pack(c, 1, t1, sp_t1->ptr, turn);
 			d2.run_slices(c, w.data(), t1, sp_w->ptr, sp_t1->ptr, t2, check->ptr);
 			c.gemm_flops += d2.flops;
@@ -622,7 +622,7 @@ struct LocalH {
 		}
 		else if (s3)
 		{
-			KScope ks(c, K_GEMM, 5, d3.flops, 0);
+			KScope ks(c, K_GEMM, 6, d3.flops, 0);
 			d3.slice_pack(c, 1, t2, sp_t2->ptr, turn);
 			d3.run_slices(c, k.data(), t2, sp_k->ptr, sp_t2->ptr, y, check->ptr);
 			c.gemm_flops += d3.flops;

@@ -596,7 +596,7 @@ bool DotPlan::run(Ctx& c, const double* A, const double* B, double* C) const
 	}
 	if (ntiles[0] > 0 || nstiles > 0)
 	{
-		KScope ks(c, K_GEMM, nstiles > 0 ? 7 : 1, flops, 0);
+		KScope ks(c, K_GEMM, nstiles > 0 ? 8 : 1, flops, 0);
 		if (!launch_f64(c, A, B, C)) return false;
 	}
 	c.gemm_flops += flops;

@@ -14,8 +14,9 @@
 //   k_gemm_slices  persistent, one CTA per SM, output tiles of 128 x 64 (SliceTile): warp 0 copies the
 //                  digits of 16 terms per stage (up to 32 + 16 KiB), warp 1 issues the MMAs, warps 4-19 add
 //                  the orders up and write, and mark the results whose digits may not be enough
-//   k_slice_find, k_slice_check   look at the marked results and sum those in FP64 that need it; k_slice_lists
-//                  makes lists of the nonzero terms of a small operand for them
+//   k_slice_find, k_slice_check, k_slice_parts   look at the marked results and sum those in FP64 that need it, one by
+//                  one or, where a part of a tile has many, all of its results at a time; k_slice_lists makes lists of
+//                  the nonzero terms of an MPO tensor or a small operand for them
 // The 64 columns of a tile are two halves of 32 with an accumulator each in tensor memory: columns 32 o ..
 // 32 o + 31 of it hold order o. Digit s of the 128 rows meets the digits 0 .. 7 - s of the 32 columns,
 // which lie one after the other as rows of one B operand, in one MMA of N = 32 (8 - s) that writes
@@ -872,10 +873,22 @@ struct MaskTile {
 	}
 };
 
-// list: its length (zero before the launch), then (mask word, its bits)
+// A part of a tile, 32 MMA rows by 8 columns, of which many results are suspect, such as those of a row that is
+// graded against the other operand's columns, is summed as a whole, its operands read once for all of it
+// (k_slice_parts). The words keep the parts if these are too few to fill the SMs (two for each). A result of the words
+// costs 4 to 6 times the terms that one of a part costs, 1.3 to 2.7 times with lists. Products of which all results are
+// suspect (ms by words, by parts, on the FP64 pipe): 2048 x 2048 x 2048 terms 90, 14.0, 14.3; with lists
+// 512 x 4096 x 2048 20.4, 7.0, 7.5; 4096 x 512 x 2048 9.4, 7.0, 7.5. From half the results on, with lists or without,
+// the molecular search (n = 24, D = 512) is slower by 2 %: there the words of long sums read the same terms at a time.
+constexpr double CHECK_WHOLE = 3, CHECK_WHOLE_LISTS = 1.25;
+constexpr int CHECK_TERMS = 32, PARTS_SM = 5;
+
+// list: the numbers of its words and parts (zero before the launch), then (mask word, its bits); from its end, the
+// parts (of mask word by column group, rows: 32 id + 4 group + rows)
 __global__ void __launch_bounds__(CHECK_WARPS * 32)
 k_slice_find(int ntiles, int nsplits, const SliceTile* __restrict__ tiles, const GemmOut* __restrict__ outs,
-             const SliceOut* __restrict__ souts, const GemmSplit* __restrict__ splits, int orient, const unsigned* masks, uint2* list)
+             const SliceOut* __restrict__ souts, const GemmSplit* __restrict__ splits, int orient, int swap,
+             const SliceGroup* __restrict__ groups, const int* counts, const unsigned* masks, uint2* list, unsigned last)
 {
 	pdl_wait();
 	pdl_trigger();
@@ -888,7 +901,31 @@ k_slice_find(int ntiles, int nsplits, const SliceTile* __restrict__ tiles, const
 		unsigned word = col < t.mc && row0 < t.mr ? masks[at] : 0;
 		if (t.mr - row0 < 32) word &= (1u << max(t.mr - row0, 0)) - 1;
 		if (!__any_sync(0xffffffffu, word != 0)) continue;
-		const int width = check_rows(souts[t.out].k);
+		const SliceOut so = souts[t.out];
+		// the suspects of the lane's 32 rows, and their terms: with lists, as many as a row of them has here
+		auto sum = [](int v) {
+			for (int q = 4; q < 32; q <<= 1) v += __shfl_xor_sync(0xffffffffu, v, q);
+			return v;
+		};
+		const int cols = min(8, t.mc - (unit & 7) * 8), nrow = min(32, t.mr - row0);
+		const double suspects = (counts ? CHECK_WHOLE_LISTS : CHECK_WHOLE) * sum(__popc(word)), whole = 32.0 * cols * so.k;
+		bool part = suspects * so.k > whole;
+		if (counts && __any_sync(0xffffffffu, part))
+		{
+			const bool rows = swap != orient;
+			const int* len = counts + groups[rows ? so.xgroup : so.ygroup].row0 + (rows == (orient != 0) ? t.m0 : t.n0) + (rows ? row0 : (unit & 7) * 8);
+			const int nlen = rows ? nrow : cols;
+			int n = 0;
+			for (int r = lane >> 2; r < nlen; r += 8) n += len[r];
+			const double terms = sum(n);
+			part = part && suspects * terms > whole * nlen;
+		}
+		if (part)
+		{
+			if (lane < 4) list[last - atomicAdd(&list[0].y, 1u)] = make_uint2((unsigned)unit * 4 + lane, 0);
+			word = 0;
+		}
+		const int width = check_rows(so.k);
 		int n = 0;
 		for (int q = 0; q < 32; q += width) n += (word >> q & (0xffffffffu >> (32 - width))) != 0;
 		int end = n;
@@ -910,8 +947,8 @@ k_slice_find(int ntiles, int nsplits, const SliceTile* __restrict__ tiles, const
 }
 
 // use(a, b) for the terms of an entry that are the lane's (sub, sub + lanes, ..), for all lanes of a warp at once,
-// until done() holds in all of them. x is the operand with fewer entries (i its row: an MPO tensor, whose rows are
-// mostly zeros) and read first: unless all terms are asked for, y is read where x is not zero, and terms that
+// until done() holds in all of them. x is the MPO tensor, whose rows are mostly zeros, or else the operand with fewer
+// entries (i its row), and read first: unless all terms are asked for, y is read where x is not zero, and terms that
 // are zero in every lane are left out. Contributions of more terms than an entry has lanes are taken one by one;
 // those of shorter ones, 32 at a time, are one list.
 template <bool ALL, class Use, class Done>
@@ -978,24 +1015,146 @@ __device__ __forceinline__ void entry_terms(const GemmOut& o, const GemmContrib*
 	}
 }
 
+// The parts of k_slice_find, a block each: 32 terms at a time, a quarter of them for each warp, a lane's row by 8 columns.
+// Bound by the FP64 pipe (a warp's FMA takes 64 clocks of a quarter of the SM, beside a row's entry and 8 staged ones).
+__global__ void __launch_bounds__(CHECK_WARPS * 32, PARTS_SM)
+k_slice_parts(int ntiles, const SliceTile* __restrict__ tiles, const GemmOut* __restrict__ outs, const SliceOut* __restrict__ souts,
+              const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits, int orient, const double* A, const double* B,
+              const short* xexps, const short* yexps, const unsigned* masks, double* C, const uint2* list, unsigned last, unsigned least)
+{
+	__shared__ double stage[CHECK_TERMS][8], sums[CHECK_WARPS - 1][8][32];
+	__shared__ unsigned cleared[32];
+	pdl_wait();
+	pdl_trigger();
+	const unsigned nparts = list[0].y;
+	if (nparts < least) return;
+	for (unsigned p = blockIdx.x; p < nparts; p += gridDim.x)
+	{
+		const unsigned part = list[last - p].x;
+		const int id = (int)(part >> 5), c0 = (int)(part >> 2 & 7) * 8, q0 = (int)(part & 3);
+		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = q0 * 32 + lane;
+		const MaskTile t(id, ntiles, tiles, splits, outs, orient);
+		const GemmOut o = outs[t.out];
+		const SliceOut so = souts[t.out];
+		const int cols = min(8, t.mc - c0), xr = (orient ? t.m0 : t.n0) + row, yr = (orient ? t.n0 : t.m0) + c0;
+		const bool in = row < t.mr;
+		const int e = in ? xexps[so.xrow + xr] : 0;
+		unsigned left = 0, look = 0;           // results that are suspect and not cleared; those in range
+		int limit[8], most[8];
+		double s[8];
+	#pragma unroll
+		for (int c = 0; c < 8; c++)
+		{
+			s[c] = 0.0;
+			limit[c] = most[c] = 0;
+			if (!in || c >= cols || !(masks[(unsigned)id * SL_MASKS + (c0 + c) * 4 + q0] >> lane & 1)) continue;
+			const int f = yexps[so.yrow + yr + c];
+			limit[c] = slice_term_limit(e, f);
+			left |= 1u << c;
+			look |= (unsigned)slice_in_range(slice_top(e, f)) << c;
+		}
+		if (warp == 0) cleared[lane] = 0;
+		// a sum that may overflow stays one chain (see k_slice_check): the first warp's
+		const bool chain = __syncthreads_or((left & ~look) != 0);
+		const int u0 = chain ? 0 : warp * (CHECK_TERMS / CHECK_WARPS), u1 = chain ? (warp ? 0 : CHECK_TERMS) : u0 + CHECK_TERMS / CHECK_WARPS;
+		const int st = threadIdx.x & (CHECK_TERMS - 1), sc = (threadIdx.x / CHECK_TERMS) * 2;
+		bool some = true;
+		for (int q = 0; q < o.nc && some; q++)
+		{
+			const GemmContrib g = cons[o.c0 + q];
+			const double* px = orient ? A + g.a_off + (i64)xr * g.sAm : B + g.b_off + (i64)xr * g.sBn;
+			const double* py = orient ? B + g.b_off + (i64)yr * g.sBn : A + g.a_off + (i64)yr * g.sAm;
+			const int kx = orient ? g.sAk : g.sBk, ky = orient ? g.sBk : g.sAk, ny = orient ? g.sBn : g.sAm;
+			for (int k0 = 0; k0 < g.k; k0 += CHECK_TERMS)
+			{
+				const int n = min(CHECK_TERMS, g.k - k0);
+				// the warps have read the stage before; a result that one of them has cleared is done
+				some = __syncthreads_or(left != 0);
+				if (!some) break;
+				left &= ~cleared[lane];
+	#pragma unroll
+				for (int c = 0; c < 2; c++)
+					stage[st][sc + c] = st < n && sc + c < cols ? py[(i64)(k0 + st) * ky + (i64)(sc + c) * ny] : 0.0;
+				__syncthreads();
+				for (int u = u0; u < min(n, u1); u += CHECK_UNROLL)
+				{
+					double x[CHECK_UNROLL];
+	#pragma unroll
+					for (int v = 0; v < CHECK_UNROLL; v++) x[v] = in && u + v < n ? px[(i64)(k0 + u + v) * kx] : 0.0;
+	#pragma unroll
+					for (int v = 0; v < CHECK_UNROLL; v++)
+					{
+						if (u + v >= n) break;
+						const int ex = biased_exponent(x[v]);
+	#pragma unroll
+						for (int c = 0; c < 8; c++)
+						{
+							const double y = stage[u + v][c];
+							s[c] = fma(x[v], y, s[c]);
+							most[c] = max(most[c], ex + biased_exponent(y));
+						}
+					}
+				}
+				unsigned enough = 0;
+	#pragma unroll
+				for (int c = 0; c < 8; c++) enough |= (unsigned)(most[c] >= limit[c]) << c;
+				enough &= left & look;
+				if (enough) atomicOr(&cleared[lane], enough);
+				left &= ~enough;
+			}
+		}
+		if (warp > 0)
+		{
+	#pragma unroll
+			for (int c = 0; c < 8; c++) sums[warp - 1][c][lane] = s[c];
+		}
+		__syncthreads();
+		if (warp == 0)
+		{
+			left &= ~cleared[lane];
+	#pragma unroll
+			for (int c = 0; c < 8; c++)
+			{
+				double r = s[c];
+				if (!chain)
+					for (int w = 0; w < CHECK_WARPS - 1; w++) r += sums[w][c][lane];
+				if (left >> c & 1) C[orient ? gemm_out_index(o, xr, yr + c) : gemm_out_index(o, yr + c, xr)] = r;
+			}
+		}
+		__syncthreads();
+	}
+}
+
 __global__ void __launch_bounds__(CHECK_WARPS * 32)
 k_slice_check(int ntiles, const SliceTile* __restrict__ tiles, const GemmOut* __restrict__ outs, const SliceOut* __restrict__ souts,
               const GemmContrib* __restrict__ cons, const GemmSplit* __restrict__ splits, int orient, int swap,
               const SliceGroup* __restrict__ groups, const SliceTerm* terms, const int* counts, const double* A, const double* B,
-              const short* xexps, const short* yexps, double* C, uint2* list)
+              const short* xexps, const short* yexps, const unsigned* masks, double* C, const uint2* list, unsigned last, unsigned least, unsigned pieces)
 {
 	pdl_wait();
 	pdl_trigger();
 	const int lane = threadIdx.x & 31;
-	const unsigned n = list[0].x;
-	// the smaller operand, and the other one
+	const unsigned nword = list[0].x, nparts = list[0].y;
+	const unsigned n = nword + (nparts < least ? nparts * 8 * pieces : 0);
+	// an entry of the list, or a piece of a part's word
+	auto word_at = [&](unsigned at) -> uint2 {
+		if (at < nword) return list[1 + at];
+		const unsigned v = at - nword, p = list[last - v / (8 * pieces)].x, col = (p >> 2 & 7) * 8 + v / pieces % 8, row0 = (p & 3) * 32;
+		const MaskTile t((int)(p >> 5), ntiles, tiles, splits, outs, orient);
+		if ((int)col >= t.mc) return make_uint2(0, 0);
+		const unsigned wd = (p >> 5) * SL_MASKS + col * 4 + (p & 3);
+		const int rows = min(32, t.mr - (int)row0);
+		return make_uint2(wd, masks[wd] & 0xffffffffu >> (32 - rows) & 0xffffffffu >> (32 - 32 / pieces) << (v % pieces * (32 / pieces)));
+	};
+	// the operand that is read first, and the other one
 	const double *x = swap ? B : A, *y = swap ? A : B;
 	unsigned item = blockIdx.x * CHECK_WARPS + (threadIdx.x >> 5);
-	uint2 next = item < n ? list[1 + item] : make_uint2(0, 0);
+	uint2 next = item < n ? word_at(item) : make_uint2(0, 0);
 	for (; item < n; item += gridDim.x * CHECK_WARPS)
 	{
 		const uint2 w = next;
-		if (item + gridDim.x * CHECK_WARPS < n) next = list[1 + item + gridDim.x * CHECK_WARPS];
+		if (item + gridDim.x * CHECK_WARPS < n) next = word_at(item + gridDim.x * CHECK_WARPS);
+		if (w.y == 0) continue;
 		const int wd = (int)(w.x % SL_MASKS), col = wd >> 2;
 		const MaskTile t((int)(w.x / SL_MASKS), ntiles, tiles, splits, outs, orient);
 		const GemmOut o = outs[t.out];
@@ -1076,9 +1235,11 @@ i64 slice_check_bytes(int ntiles, int nsplits, int max_k)
 	return 8 + (i64)(ntiles + nsplits) * SL_MASKS * (32 / check_rows(max_k) * (i64)sizeof(uint2) + (i64)sizeof(unsigned));
 }
 
+// last entry of the list
+static i64 check_last(int ntiles, int nsplits, int max_k) { return (i64)(ntiles + nsplits) * SL_MASKS * (32 / check_rows(max_k)); }
 static unsigned* check_masks(void* check, int ntiles, int nsplits, int max_k)
 {
-	return (unsigned*)((uint2*)check + 1 + (i64)(ntiles + nsplits) * SL_MASKS * (32 / check_rows(max_k)));
+	return (unsigned*)((uint2*)check + 1 + check_last(ntiles, nsplits, max_k));
 }
 
 void launch_slice_exps(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, const double* x,
@@ -1131,10 +1292,15 @@ void launch_slice_check(int ntiles, int nsplits, const SliceTile* tiles, const G
 	if (ntiles <= 0) return;
 	uint2* list = (uint2*)check;
 	const int all = num_sms * 8;
+	const unsigned* masks = check_masks(check, ntiles, nsplits, max_k);
+	const unsigned last = (unsigned)check_last(ntiles, nsplits, max_k);
 	launch_pdl(launch_config(dim3(std::min((ntiles + nsplits) * 8 / CHECK_WARPS, 2 * all)), dim3(CHECK_WARPS * 32), 0, st), k_slice_find,
-	           ntiles, nsplits, tiles, outs, souts, splits, orient, check_masks(check, ntiles, nsplits, max_k), list);
+	           ntiles, nsplits, tiles, outs, souts, splits, orient, b_smaller ? 1 : 0, groups, terms ? counts : nullptr, masks, list, last);
 	launch_pdl(launch_config(dim3(all), dim3(CHECK_WARPS * 32), 0, st), k_slice_check, ntiles, tiles, outs, souts, cons, splits, orient,
-	           b_smaller ? 1 : 0, groups, terms, counts, A, B, xexps, yexps, C, list);
+	           b_smaller ? 1 : 0, groups, terms, counts, A, B, xexps, yexps, masks, C, list, last,
+	           2u * num_sms, (unsigned)(32 / check_rows(max_k)));
+	launch_pdl(launch_config(dim3(num_sms * PARTS_SM), dim3(CHECK_WARPS * 32), 0, st), k_slice_parts, ntiles, tiles, outs, souts, cons, splits,
+	           orient, A, B, xexps, yexps, masks, C, list, last, 2u * num_sms);
 }
 
 }  // namespace ctg

@@ -139,7 +139,7 @@ void launch_gemm_slices(int ntiles, const SliceTile* tiles, const GemmOut* outs,
 void launch_slice_lists(int nitems, const SliceItem* items, const SliceGroup* groups, const SliceRun* runs, const double* x,
                         SliceTerm* terms, int* counts, cudaStream_t st);
 i64 slice_check_bytes(int ntiles, int nsplits, int max_k);     // max_k: most terms of an output block
-// terms (may be null), counts, groups: of the operand with fewer entries, which is B if b_smaller
+// terms (may be null), counts, groups: of the operand that is read first (see DotPlan::listed), B if b_smaller
 void launch_slice_check(int ntiles, int nsplits, const SliceTile* tiles, const GemmOut* outs, const SliceOut* souts,
                         const GemmContrib* cons, const GemmSplit* splits, int orient, bool b_smaller, const SliceGroup* groups,
                         const SliceTerm* terms, const int* counts, const double* A, const double* B, const short* xexps,

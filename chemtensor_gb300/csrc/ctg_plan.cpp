@@ -134,7 +134,7 @@ int slice_orient(const std::vector<GemmOut>& outs, const std::vector<i64>& ksum,
 	return clocks[1] < clocks[0] ? 1 : 0;
 }
 
-// SM clocks of the five launches that a product by digit slices has besides the GEMM (exponents, digits, the
+// SM clocks of the six launches that a product by digit slices has besides the GEMM (exponents, digits, the
 // results to look at again, of which graded states have many), and of those for an entry of an operand and of
 // the result
 constexpr double SLICE_OVERHEAD = 150000, SLICE_ENTRY = 3.0, SLICE_RESULT = 4.0;
